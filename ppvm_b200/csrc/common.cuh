@@ -51,6 +51,8 @@ struct Ctrl {
   unsigned long long fb_cut;   // fused-run fallback: gates at the head of the run to apply one at a time, 0 = none
   unsigned long long done;     // blocks of the current launch that finished (last_block_done)
   unsigned long long scr_top;  // fused run in scratch mode: group outputs placed in the scratch so far
+  unsigned long long rot_s;      // rotation: anticommuting terms found by k_rot_pair (0 between rotations)
+  unsigned long long rot_pairs;  // rotation: partner pairs among them (0 between rotations)
   unsigned spin_limit;         // polls a look-back waits before it gives up; 0 = kSpinLimit
   unsigned reserved;
 };
@@ -116,6 +118,22 @@ __device__ __forceinline__ bool last_block_done(unsigned long long* counter) {
   if (threadIdx.x == 0) {
     const unsigned long long prev = atomicAdd(counter, 1ull);
     s_last = prev == (unsigned long long)gridDim.x * gridDim.y * gridDim.z - 1;
+    if (s_last) *counter = 0;
+  }
+  __syncthreads();
+  if (s_last) __threadfence();
+  return s_last;
+}
+
+// last_block_done for a launch of which only the first `blocks` blocks take part (the others
+// returned at once): the last of those to call it.
+__device__ __forceinline__ bool last_of_blocks(unsigned long long* counter, unsigned blocks) {
+  __shared__ bool s_last;
+  if (blocks == 1) return true;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    s_last = atomicAdd(counter, 1ull) == (unsigned long long)blocks - 1;
     if (s_last) *counter = 0;
   }
   __syncthreads();

@@ -460,6 +460,7 @@ ppvm_status grow(ppvm_sum* s, unsigned long long new_cap) {
   free_scratch(s);
   CUDA_TRY(pool_malloc((void**)&s->s_idx, sizeof(uint32_t) * new_cap, site));
   CUDA_TRY(pool_malloc((void**)&s->partner, sizeof(uint32_t) * new_cap, site));
+  CUDA_TRY(cudaMemsetAsync(s->partner, 0xFF, sizeof(uint32_t) * new_cap, s->stream));  // kNone between rotations
   CUDA_TRY(pool_malloc((void**)&s->s_rec, sizeof(uint64_t) * (size_t)(2 * W + 1) * new_cap, site));
   s->table_cap = next_pow2(std::max<unsigned long long>(2 * new_cap, 1024));
   CUDA_TRY(pool_malloc((void**)&s->table, sizeof(unsigned long long) * s->table_cap, site));
@@ -611,12 +612,15 @@ uint64_t launch_bytes(const ppvm_sum* s, const ProfLaunch& L, const std::vector<
   const uint64_t B = 16ull * s->W + 8;
   const OpLog& g = s->h_log[L.op];
   switch (L.family) {
-    case F_SCAN: {
+    case F_SCAN: return g.n_in * 16ull + g.n_s * (B + B + 8);  // damping: test words + gather + record/idx/partner
+    case F_PAIR: {  // test words of every term, the anticommuting terms' keys, one table slot each
       const int tw = (L.op < (int)test_words.size()) ? test_words[L.op] : 1;
-      return g.n_in * 8ull * tw + g.n_s * (B + B + 8);  // test words + gather + record/idx/partner
+      return g.n_in * 8ull * tw + g.n_s * (B - 8 + 8);
     }
-    case F_PAIR: return g.n_s * B * 2;                 // own record + partner record
-    case F_APPLY: return g.n_s * (B + 8) + g.n_new * B;  // records, coeff writes, children
+    case F_APPLY: {  // test words, partner links, coefficients read and written, children
+      const int tw = (L.op < (int)test_words.size()) ? test_words[L.op] : 1;
+      return g.n_in * 8ull * tw + g.n_s * (4 + 16) + g.n_new * (B - 8 + B);
+    }
     case F_CLIFF: return 2ull * g.n_in * B;
     case F_TRUNC: return g.n_in * B + g.n_out * B;
     case F_RUN_CLASSIFY: return g.n_in * B + g.n_in * 4;       // every term read once, group slots
@@ -864,27 +868,19 @@ struct K {
       if (g.gx[w]) zmask |= 1u << w;
     }
     const double sn = std::sin(theta), cs = std::cos(theta);
+    // the words the sign (and, on a lossy sum, the lost qubits) need, beside the test's
+    unsigned gm = xmask | zmask;
+    if (g.lw) gm = (1u << W) - 1;
     const unsigned long long nub = std::max<unsigned long long>(s->n_ub, 1);
-    {
-      ProfScope ps(s, F_SCAN, op, 1);
-      launch(k_rot_scan<W, kScanBlock, ITEMS>, grid_for(nub, TILE, 8), kScanBlock, 0, s->stream,
-          P, s->d_ctrl, g, xmask, zmask, s->s_idx, s->s_rec, s->partner, s->tstate,
-          s->next_tile_epoch(), op, s->d_log);
-    }
     {
       ProfScope ps(s, F_PAIR, op, 1);
       launch(k_rot_pair<W>, grid_for(nub, kPairBlock, 8), kPairBlock, 0, s->stream,
-          s->d_ctrl, g, s->s_rec, s->partner, s->table, s->table_cap, s->next_table_epoch(), op);
+          P, s->d_ctrl, g, xmask, zmask, s->partner, s->table, s->table_cap, s->next_table_epoch(), op);
     }
     {
       ProfScope ps(s, F_APPLY, op, 1);
       launch(k_rot_apply<W, kScanBlock, ITEMS>, grid_for(nub, TILE, 8), kScanBlock, 0, s->stream,
-          P, s->d_ctrl, g, sn, cs, s->s_idx, s->s_rec, s->partner, s->tstate, s->next_tile_epoch(),
-          op, s->d_log);
-    }
-    {
-      ProfScope ps(s, F_COMMIT, op, 1);
-      launch(k_commit_rot, 1, 1, 0, s->stream, s->d_ctrl, op, s->d_log);
+          P, s->d_ctrl, g, xmask, zmask, gm, sn, cs, s->partner, s->tstate, s->next_tile_epoch(), op, s->d_log);
     }
     s->n_ub = std::min<unsigned long long>(s->cap, 2 * s->n_ub);
   }
@@ -901,8 +897,8 @@ struct K {
     const unsigned long long nub = std::max<unsigned long long>(s->n_ub, 1);
     {
       ProfScope ps(s, F_SCAN, op, 1);
-      launch(k_rot_scan<W, kScanBlock, ITEMS, true>, grid_for(nub, TILE, 8), kScanBlock, 0, s->stream,
-          P, s->d_ctrl, g, 0u, qmask, s->s_idx, s->s_rec, s->partner, s->tstate,
+      launch(k_damp_scan<W, kScanBlock, ITEMS>, grid_for(nub, TILE, 8), kScanBlock, 0, s->stream,
+          P, s->d_ctrl, g, qmask, s->s_idx, s->s_rec, s->partner, s->tstate,
           s->next_tile_epoch(), op, s->d_log);
     }
     const unsigned tep = s->next_table_epoch();
@@ -1246,6 +1242,7 @@ ppvm_status clear_err(ppvm_sum* s) {
   c.fb_cut = 0;
   c.done = 0;  // blocks that returned early on the error never counted
   c.scr_top = 0;
+  c.rot_s = c.rot_pairs = 0;
   for (int t = 0; t < 4; ++t) c.tickets[t] = 0;
   CUDA_TRY(cudaMemcpyAsync(s->d_ctrl, &c, sizeof(Ctrl), cudaMemcpyHostToDevice, s->stream));
   CUDA_TRY(cudaStreamSynchronize(s->stream));
@@ -1429,6 +1426,8 @@ ppvm_status run_list(ppvm_sum* s, const ppvm_op* ops, size_t n_ops, const std::v
     }
     if (s->prof) prof_collect(s, test_words);
     PPVM_TRY(clear_run_tables(s, s->run_slots_used));  // a run stopped part-way leaves its slots set
+    // and a rotation stopped between its kernels leaves partner links
+    CUDA_TRY(cudaMemsetAsync(s->partner, 0xFF, sizeof(uint32_t) * std::min(s->cap, s->n_ub), s->stream));
     // fused runs at or after the failing op did not run: give their buffers back
     for (int op0 : s->swaps)
       if (op0 >= c.err_op) std::swap(s->planes, s->alt);

@@ -2,13 +2,13 @@
 //
 // Rotation exp(-i theta/2 G) on a sum held in SoA planes, reference semantics of
 // PauliSum::map_insert (crates/ppvm-pauli-sum/src/sum/data.rs:204-226):
-//   k_rot_scan   ordered compaction of the anticommuting terms into a dense record buffer
-//   k_rot_pair   partner search: each record inserts min(K, K^G) into an epoch-tagged table;
-//                the second of a pair to arrive links both (a child K^G can only collide with
-//                its partner term, so every key receives at most two contributions)
+//   k_rot_pair   partner search: each anticommuting term inserts min(K, K^G) into an
+//                epoch-tagged table; the second of a pair to arrive links both (a child K^G can
+//                only collide with its partner term, so every key receives at most two
+//                contributions)
 //   k_rot_apply  parent <- c*cos (+ partner's c*(eps*sin)); partnerless parents append their
-//                child in parent order, so the term order stays the reference's IndexMap order
-//   k_commit     publishes the new live count and resets the tile tickets
+//                child in parent order, so the term order stays the reference's IndexMap order;
+//                its last block publishes the new live count
 // Clifford runs (sum/clifford.rs) and diagonal noise (sum/noise.rs) are one in-place pass
 // (k_clifford); truncation (data.rs:275-311, strategy.rs) is an in-place stable compaction.
 #pragma once
@@ -76,110 +76,59 @@ struct ItemsFor {
 };
 
 // ---------------------------------------------------------------------------------------
-// k_rot_scan: flags anticommuting terms, writes their index and record in index order.
-// With DAMP the flagged terms are those with Z (x = 0, z = 1) on the qubit of g.gz instead:
-// the parents of amplitude damping.
+// Rotations.  Both kernels read the terms in place: a term's anticommutation test needs only the
+// generator's words, so a term that commutes costs those words and nothing is copied aside.
+// (Copying the anticommuting terms into dense records first, as an ordered compaction of its
+// own, and committing in a fourth kernel made a gate four launches and moved about 3 (16W + 8)
+// bytes more per anticommuting term.)
 // ---------------------------------------------------------------------------------------
-template <int W, int BLOCK, int ITEMS, bool DAMP = false>
-__global__ void __launch_bounds__(BLOCK)
-k_rot_scan(Planes P, Ctrl* ctrl, Gen g, unsigned xmask, unsigned zmask, uint32_t* s_idx, uint64_t* s_rec,
-           uint32_t* partner, unsigned long long* ts, unsigned epoch, int op, OpLog* log) {
-  pdl_wait();
-  __shared__ unsigned s_tile;
-  __shared__ unsigned long long s_slot;
-  __shared__ unsigned s_base[ITEMS * (BLOCK / 32) + 1];
-  if (ld_volatile_int(&ctrl->err)) return;
-  const unsigned long long N = ld_volatile(&ctrl->n);
-  constexpr unsigned long long TILE = (unsigned long long)BLOCK * ITEMS;
-  const unsigned long long ntiles = (N + TILE - 1) / TILE;
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    log[op].n_in = N;
-    ctrl->n_pairs = 0;
-    if (N == 0) {
-      ctrl->n_s = 0;
-      log[op].n_s = 0;
-    }
-  }
-  const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  constexpr int NW = BLOCK / 32;
-  for (;;) {
-    const unsigned tile = next_tile(&ctrl->tickets[0], &s_tile);
-    if (tile >= ntiles) break;
-    const unsigned long long base = (unsigned long long)tile * TILE;
-    unsigned ballots[ITEMS];
+
+// The words of term i that a rotation by g needs (word masks: xm of the X plane, zm of the Z
+// plane); the others are zero.
+template <int W>
+__device__ __forceinline__ void load_words(const Planes& P, unsigned long long i, unsigned xm, unsigned zm,
+                                           uint64_t (&x)[W], uint64_t (&z)[W]) {
 #pragma unroll
-    for (int k = 0; k < ITEMS; ++k) {
-      const unsigned long long i = base + (unsigned long long)k * BLOCK + threadIdx.x;
-      bool a = false;
-      if (i < N) {
-        uint64_t acc = 0;
-        if constexpr (DAMP) {
-#pragma unroll
-          for (int w = 0; w < W; ++w)
-            if ((zmask >> w) & 1u)
-              acc |= P.z[(unsigned long long)w * P.cap + i] & ~P.x[(unsigned long long)w * P.cap + i] & g.gz[w];
-          a = acc != 0;
-        } else {
-#pragma unroll
-          for (int w = 0; w < W; ++w) {
-            if ((xmask >> w) & 1u) acc ^= P.x[(unsigned long long)w * P.cap + i] & g.gz[w];
-            if ((zmask >> w) & 1u) acc ^= P.z[(unsigned long long)w * P.cap + i] & g.gx[w];
-          }
-          a = __popcll(acc) & 1;
-        }
-      }
-      ballots[k] = __ballot_sync(kFull, a);
-    }
-    const unsigned agg = tile_ranks<BLOCK, ITEMS>(ballots, s_base);
-    const unsigned long long excl = lookback(ts, tile, agg, epoch, ctrl, op, &s_slot);
-#pragma unroll
-    for (int k = 0; k < ITEMS; ++k) {
-      if ((ballots[k] >> lane) & 1u) {
-        const unsigned long long i = base + (unsigned long long)k * BLOCK + threadIdx.x;
-        const unsigned long long r =
-            excl + s_base[k * NW + warp] + __popc(ballots[k] & ((1u << lane) - 1u));
-        s_idx[r] = (uint32_t)i;
-        partner[r] = kNone;
-        uint64_t* rec = s_rec + r * (2 * W + 1);
-#pragma unroll
-        for (int w = 0; w < W; ++w) rec[w] = P.x[(unsigned long long)w * P.cap + i];
-#pragma unroll
-        for (int w = 0; w < W; ++w) rec[W + w] = P.z[(unsigned long long)w * P.cap + i];
-        rec[2 * W] = (uint64_t)__double_as_longlong(P.c[i]);
-      }
-    }
-    if (tile == ntiles - 1 && threadIdx.x == 0) {
-      ctrl->n_s = excl + agg;
-      log[op].n_s = excl + agg;
-    }
+  for (int w = 0; w < W; ++w) {
+    x[w] = (xm >> w) & 1u ? P.x[(unsigned long long)w * P.cap + i] : 0ull;
+    z[w] = (zm >> w) & 1u ? P.z[(unsigned long long)w * P.cap + i] : 0ull;
   }
 }
 
-// ---------------------------------------------------------------------------------------
-// k_rot_pair: finds, for each anticommuting term, whether its partner K^G is also present.
-// ---------------------------------------------------------------------------------------
+// k_rot_pair: finds, for each anticommuting term, whether its partner K^G is also present.  The
+// term inserts its index at min(K, K^G) in an epoch-tagged table; the second of a pair to
+// arrive links both in partner[] (all kNone between rotations: k_rot_apply clears the links
+// it reads).  xmask/zmask: the words of the X/Z plane that the test reads.
+// Bound by the random 8-byte table accesses: one thread per term at full occupancy keeps as many
+// in flight as the SMs can hold.
 template <int W>
 __global__ void __launch_bounds__(256)
-k_rot_pair(Ctrl* ctrl, Gen g, const uint64_t* s_rec, uint32_t* partner,
+k_rot_pair(Planes P, Ctrl* ctrl, Gen g, unsigned xmask, unsigned zmask, uint32_t* partner,
            unsigned long long* table, unsigned long long table_cap, unsigned tepoch, int op) {
   pdl_wait();
+  __shared__ unsigned s_cnt[2];
   if (ld_volatile_int(&ctrl->err)) return;
-  const unsigned long long ns = ld_volatile(&ctrl->n_s);
-  if (ns == 0) return;
-  unsigned long long tsize = next_pow2_ull(ns * 2 < 1024 ? 1024 : ns * 2);
+  const unsigned long long N = ld_volatile(&ctrl->n);
+  const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
+  if ((unsigned long long)blockIdx.x * blockDim.x >= N) return;
+  if (threadIdx.x < 2) s_cnt[threadIdx.x] = 0;
+  __syncthreads();
+  // at most N entries: full to 2/3 when every term anticommutes and none has a partner
+  unsigned long long tsize = next_pow2_ull(N + N / 2 < 1024 ? 1024 : N + N / 2);
   if (tsize > table_cap) tsize = table_cap;
   const unsigned long long mask = tsize - 1;
-  const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
-  for (unsigned long long s = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; s < ns;
-       s += stride) {
-    uint64_t x[W], z[W], px[W], pz[W], ex[W], ez[W];
-    double c;
-    load_rec<W>(s_rec, s, x, z, c);
-    gen_on<W>(g, x, ex, ez);
+  unsigned mine_s = 0, mine_p = 0;
+  for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += stride) {
+    uint64_t x[W], z[W], px[W], pz[W];
+    load_words<W>(P, i, xmask, zmask, x, z);
+    if (!anticommutes<W>(g, x, z)) continue;
+    ++mine_s;
+    load_key<W>(P, i, x, z);
+    gen_on<W>(g, x, px, pz);
 #pragma unroll
     for (int w = 0; w < W; ++w) {
-      px[w] = x[w] ^ ex[w];
-      pz[w] = z[w] ^ ez[w];
+      px[w] ^= x[w];
+      pz[w] ^= z[w];
     }
     const bool use_p = key_less<W>(px, pz, x, z);
     uint64_t rx[W], rz[W];
@@ -190,7 +139,7 @@ k_rot_pair(Ctrl* ctrl, Gen g, const uint64_t* s_rec, uint32_t* partner,
     }
     const uint64_t h = hash_key<W>(rx, rz);
     const unsigned tag = (unsigned)(h >> 48) & 0xFFFFu;
-    const unsigned long long mine = make_slot(tepoch, tag, (unsigned)s);
+    const unsigned long long mine = make_slot(tepoch, tag, (unsigned)i);
     unsigned long long slot = h & mask;
     unsigned long long probes = 0;
     while (true) {
@@ -203,16 +152,15 @@ k_rot_pair(Ctrl* ctrl, Gen g, const uint64_t* s_rec, uint32_t* partner,
       if (slot_tag(cur) == tag) {
         const unsigned j = slot_idx(cur);
         uint64_t jx[W], jz[W];
-        double jc;
-        load_rec<W>(s_rec, j, jx, jz, jc);
+        load_key<W>(P, j, jx, jz);
         // j is our partner iff its key is exactly K ^ G
         bool eq = true;
 #pragma unroll
         for (int w = 0; w < W; ++w) eq &= (jx[w] == px[w]) & (jz[w] == pz[w]);
         if (eq) {
-          partner[s] = j;
-          partner[j] = (uint32_t)s;
-          atomicAdd(&ctrl->n_pairs, 1ull);
+          partner[i] = j;
+          partner[j] = (uint32_t)i;
+          ++mine_p;
           break;
         }
       }
@@ -223,101 +171,128 @@ k_rot_pair(Ctrl* ctrl, Gen g, const uint64_t* s_rec, uint32_t* partner,
       }
     }
   }
+  mine_s = __reduce_add_sync(kFull, mine_s);
+  mine_p = __reduce_add_sync(kFull, mine_p);
+  if ((threadIdx.x & 31) == 0) {
+    if (mine_s) atomicAdd(&s_cnt[0], mine_s);
+    if (mine_p) atomicAdd(&s_cnt[1], mine_p);
+  }
+  __syncthreads();
+  if (threadIdx.x < 2 && s_cnt[threadIdx.x])
+    atomicAdd(threadIdx.x == 0 ? &ctrl->rot_s : &ctrl->rot_pairs, (unsigned long long)s_cnt[threadIdx.x]);
 }
 
-// ---------------------------------------------------------------------------------------
-// k_rot_apply: new coefficients of anticommuting parents; children appended in order.
-// ---------------------------------------------------------------------------------------
+// k_rot_apply: new coefficients in place, children appended in parent order (one decoupled
+// look-back per tile of terms).  Of a pair, the term of lower index computes both coefficients
+// from the old ones, so nothing is read after it was written.  xmask/zmask: the test's words, gm:
+// the words of the generator (of both planes; the sign needs them).  The last of the blocks that have tiles publishes the live count.
 template <int W, int BLOCK, int ITEMS>
 __global__ void __launch_bounds__(BLOCK)
-k_rot_apply(Planes P, Ctrl* ctrl, Gen g, double sn, double cs, const uint32_t* s_idx,
-            const uint64_t* s_rec, const uint32_t* partner, unsigned long long* ts,
-            unsigned epoch, int op, OpLog* log) {
+k_rot_apply(Planes P, Ctrl* ctrl, Gen g, unsigned xmask, unsigned zmask, unsigned gm, double sn, double cs,
+            uint32_t* partner, unsigned long long* ts, unsigned epoch, int op, OpLog* log) {
   pdl_wait();
   __shared__ unsigned s_tile;
   __shared__ unsigned long long s_slot;
   __shared__ unsigned s_base[ITEMS * (BLOCK / 32) + 1];
   if (ld_volatile_int(&ctrl->err)) return;
   const unsigned long long N = ld_volatile(&ctrl->n);
-  const unsigned long long ns = ld_volatile(&ctrl->n_s);
-  const unsigned long long np = ld_volatile(&ctrl->n_pairs);
-  const unsigned long long nchild = ns - 2 * np;
-  if (N + nchild > P.cap) {
+  const unsigned long long ns = ld_volatile(&ctrl->rot_s);
+  const unsigned long long nchild = ns - 2 * ld_volatile(&ctrl->rot_pairs);
+  if (N + nchild > P.cap) {  // nothing has been written: the host grows the storage and replays this op
     if (blockIdx.x == 0 && threadIdx.x == 0) {
       ctrl->cap_needed = N + nchild;
       set_err(ctrl, kErrCapacity, op);
     }
     return;
   }
-  if (ns == 0) return;
   constexpr unsigned long long TILE = (unsigned long long)BLOCK * ITEMS;
-  const unsigned long long ntiles = (ns + TILE - 1) / TILE;
+  const unsigned long long ntiles = ns == 0 ? 0 : (N + TILE - 1) / TILE;
+  const unsigned blocks = (unsigned)(ntiles < 1 ? 1 : ntiles < gridDim.x ? ntiles : gridDim.x);
+  if (blockIdx.x >= blocks) return;
   const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   constexpr int NW = BLOCK / 32;
-  for (;;) {
+  while (ntiles) {
     const unsigned tile = next_tile(&ctrl->tickets[1], &s_tile);
     if (tile >= ntiles) break;
     const unsigned long long base = (unsigned long long)tile * TILE;
     unsigned ballots[ITEMS];
+    double kc[ITEMS];  // a childbearing parent's old coefficient
 #pragma unroll
     for (int k = 0; k < ITEMS; ++k) {
-      const unsigned long long s = base + (unsigned long long)k * BLOCK + threadIdx.x;
+      const unsigned long long i = base + (unsigned long long)k * BLOCK + threadIdx.x;
       bool child = false;
-      if (s < ns) {
+      if (i < N) {
         uint64_t x[W], z[W];
-        double c;
-        load_rec<W>(s_rec, s, x, z, c);
-        const uint32_t j = partner[s];
-        double nc;
-        if (j != kNone) {
-          uint64_t jx[W], jz[W];
-          double jc;
-          load_rec<W>(s_rec, j, jx, jz, jc);
-          const double eps_j = rot_sign<W>(g, jx, jz);
-          nc = __dadd_rn(__dmul_rn(c, cs), __dmul_rn(jc, eps_j * sn));
-        } else {
-          nc = __dmul_rn(c, cs);
-          child = true;
+        load_words<W>(P, i, xmask, zmask, x, z);
+        if (anticommutes<W>(g, x, z)) {
+          const uint32_t j = partner[i];
+          if (j == kNone) {
+            child = true;
+            kc[k] = P.c[i];
+            P.c[i] = __dmul_rn(kc[k], cs);
+          } else {
+            partner[i] = kNone;
+            if (i < j) {
+              const double ci = P.c[i], cj = P.c[j];
+              uint64_t x2[W], z2[W];  // the sign's words that the test did not read
+              load_words<W>(P, i, gm & ~xmask, gm & ~zmask, x2, z2);
+#pragma unroll
+              for (int w = 0; w < W; ++w) {
+                x[w] |= x2[w];
+                z[w] |= z2[w];
+              }
+              const double eps_i = rot_sign<W>(g, x, z);
+              uint64_t ex[W], ez[W];
+              gen_on<W>(g, x, ex, ez);
+#pragma unroll
+              for (int w = 0; w < W; ++w) {
+                x[w] ^= ex[w];
+                z[w] ^= ez[w];
+              }
+              const double eps_j = rot_sign<W>(g, x, z);
+              P.c[i] = __dadd_rn(__dmul_rn(ci, cs), __dmul_rn(cj, eps_j * sn));
+              P.c[j] = __dadd_rn(__dmul_rn(cj, cs), __dmul_rn(ci, eps_i * sn));
+            }
+          }
         }
-        P.c[s_idx[s]] = nc;
       }
       ballots[k] = __ballot_sync(kFull, child);
     }
-    const unsigned agg = tile_ranks<BLOCK, ITEMS>(ballots, s_base);
-    const unsigned long long excl = lookback(ts, tile, agg, epoch, ctrl, op, &s_slot);
+    if (nchild) {
+      const unsigned agg = tile_ranks<BLOCK, ITEMS>(ballots, s_base);
+      const unsigned long long excl = lookback(ts, tile, agg, epoch, ctrl, op, &s_slot);
 #pragma unroll
-    for (int k = 0; k < ITEMS; ++k) {
-      if ((ballots[k] >> lane) & 1u) {
-        const unsigned long long s = base + (unsigned long long)k * BLOCK + threadIdx.x;
-        const unsigned long long r =
-            N + excl + s_base[k * NW + warp] + __popc(ballots[k] & ((1u << lane) - 1u));
-        uint64_t x[W], z[W];
-        double c;
-        load_rec<W>(s_rec, s, x, z, c);
-        const double eps = rot_sign<W>(g, x, z);
-        uint64_t ex[W], ez[W];
-        gen_on<W>(g, x, ex, ez);
+      for (int k = 0; k < ITEMS; ++k) {
+        if ((ballots[k] >> lane) & 1u) {
+          const unsigned long long i = base + (unsigned long long)k * BLOCK + threadIdx.x;
+          const unsigned long long r =
+              N + excl + s_base[k * NW + warp] + __popc(ballots[k] & ((1u << lane) - 1u));
+          uint64_t x[W], z[W];
+          load_key<W>(P, i, x, z);
+          const double eps = rot_sign<W>(g, x, z);
+          uint64_t ex[W], ez[W];
+          gen_on<W>(g, x, ex, ez);
 #pragma unroll
-        for (int w = 0; w < W; ++w) {
-          x[w] ^= ex[w];
-          z[w] ^= ez[w];
+          for (int w = 0; w < W; ++w) {
+            x[w] ^= ex[w];
+            z[w] ^= ez[w];
+          }
+          store_key<W>(P, r, x, z);
+          P.c[r] = __dmul_rn(kc[k], eps * sn);
         }
-        store_key<W>(P, r, x, z);
-        P.c[r] = __dmul_rn(c, eps * sn);
       }
     }
   }
-}
-
-// Publishes the live count after a rotation and resets the tile tickets (one thread).
-static __global__ void k_commit_rot(Ctrl* ctrl, int op, OpLog* log) {
-  pdl_wait();
-  for (int t = 0; t < 4; ++t) ctrl->tickets[t] = 0;
-  if (ctrl->err) return;
-  const unsigned long long nchild = ctrl->n_s - 2 * ctrl->n_pairs;
-  log[op].n_new = nchild;
-  ctrl->n = ctrl->n + nchild;
-  log[op].n_out = ctrl->n;
+  if (last_of_blocks(&ctrl->done, blocks) && threadIdx.x == 0) {
+    for (int t = 0; t < 4; ++t) ctrl->tickets[t] = 0;
+    ctrl->rot_s = ctrl->rot_pairs = 0;
+    if (ld_volatile_int(&ctrl->err)) return;
+    log[op].n_in = N;
+    log[op].n_s = ns;
+    log[op].n_new = nchild;
+    log[op].n_out = N + nchild;
+    ctrl->n = N + nchild;
+  }
 }
 
 // ---------------------------------------------------------------------------------------

@@ -8,7 +8,7 @@
 // only land on a term with I on q, which is not a parent itself, so every key still receives
 // at most two contributions and the result is bit-identical to the reference's.
 //
-//   k_rot_scan<..., DAMP>  parents (Z on q) in index order: s_idx, s_rec (key + coefficient)
+//   k_damp_scan            parents (Z on q) in index order: s_idx, s_rec (key + coefficient)
 //   k_damp_index           the parents' child keys into an epoch-tagged hash table
 //   k_damp_probe           every term with I on q looks its own key up (a hit is the partner
 //                          of that child); X and Y terms are scaled by sqrt(1-g) here
@@ -23,6 +23,76 @@
 #include "kernels.cuh"
 
 namespace ppvm {
+
+// ---------------------------------------------------------------------------------------
+// k_damp_scan: flags the parents (Z, x = 0 and z = 1, on the qubit of g.gz) and writes their
+// index and record in index order.
+// ---------------------------------------------------------------------------------------
+template <int W, int BLOCK, int ITEMS>
+__global__ void __launch_bounds__(BLOCK)
+k_damp_scan(Planes P, Ctrl* ctrl, Gen g, unsigned zmask, uint32_t* s_idx, uint64_t* s_rec,
+            uint32_t* partner, unsigned long long* ts, unsigned epoch, int op, OpLog* log) {
+  pdl_wait();
+  __shared__ unsigned s_tile;
+  __shared__ unsigned long long s_slot;
+  __shared__ unsigned s_base[ITEMS * (BLOCK / 32) + 1];
+  if (ld_volatile_int(&ctrl->err)) return;
+  const unsigned long long N = ld_volatile(&ctrl->n);
+  constexpr unsigned long long TILE = (unsigned long long)BLOCK * ITEMS;
+  const unsigned long long ntiles = (N + TILE - 1) / TILE;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    log[op].n_in = N;
+    ctrl->n_pairs = 0;
+    if (N == 0) {
+      ctrl->n_s = 0;
+      log[op].n_s = 0;
+    }
+  }
+  const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int NW = BLOCK / 32;
+  for (;;) {
+    const unsigned tile = next_tile(&ctrl->tickets[0], &s_tile);
+    if (tile >= ntiles) break;
+    const unsigned long long base = (unsigned long long)tile * TILE;
+    unsigned ballots[ITEMS];
+#pragma unroll
+    for (int k = 0; k < ITEMS; ++k) {
+      const unsigned long long i = base + (unsigned long long)k * BLOCK + threadIdx.x;
+      bool a = false;
+      if (i < N) {
+        uint64_t acc = 0;
+#pragma unroll
+        for (int w = 0; w < W; ++w)
+          if ((zmask >> w) & 1u)
+            acc |= P.z[(unsigned long long)w * P.cap + i] & ~P.x[(unsigned long long)w * P.cap + i] & g.gz[w];
+        a = acc != 0;
+      }
+      ballots[k] = __ballot_sync(kFull, a);
+    }
+    const unsigned agg = tile_ranks<BLOCK, ITEMS>(ballots, s_base);
+    const unsigned long long excl = lookback(ts, tile, agg, epoch, ctrl, op, &s_slot);
+#pragma unroll
+    for (int k = 0; k < ITEMS; ++k) {
+      if ((ballots[k] >> lane) & 1u) {
+        const unsigned long long i = base + (unsigned long long)k * BLOCK + threadIdx.x;
+        const unsigned long long r =
+            excl + s_base[k * NW + warp] + __popc(ballots[k] & ((1u << lane) - 1u));
+        s_idx[r] = (uint32_t)i;
+        partner[r] = kNone;
+        uint64_t* rec = s_rec + r * (2 * W + 1);
+#pragma unroll
+        for (int w = 0; w < W; ++w) rec[w] = P.x[(unsigned long long)w * P.cap + i];
+#pragma unroll
+        for (int w = 0; w < W; ++w) rec[W + w] = P.z[(unsigned long long)w * P.cap + i];
+        rec[2 * W] = (uint64_t)__double_as_longlong(P.c[i]);
+      }
+    }
+    if (tile == ntiles - 1 && threadIdx.x == 0) {
+      ctrl->n_s = excl + agg;
+      log[op].n_s = excl + agg;
+    }
+  }
+}
 
 template <int W>
 __device__ __forceinline__ void damp_child_key(const uint64_t* s_rec, unsigned long long s, const Gen& g,
@@ -124,7 +194,7 @@ k_damp_probe(Planes P, Ctrl* ctrl, Gen g, unsigned qw, const uint64_t* s_rec, ui
 template <int W, int BLOCK, int ITEMS>
 __global__ void __launch_bounds__(BLOCK)
 k_damp_apply(Planes P, Ctrl* ctrl, Gen g, double om, double gm, const uint32_t* s_idx, const uint64_t* s_rec,
-             const uint32_t* partner, unsigned long long* ts, unsigned epoch, int op) {
+             uint32_t* partner, unsigned long long* ts, unsigned epoch, int op) {
   pdl_wait();
   __shared__ unsigned s_tile;
   __shared__ unsigned long long s_slot;
@@ -154,6 +224,7 @@ k_damp_apply(Planes P, Ctrl* ctrl, Gen g, double om, double gm, const uint32_t* 
         const uint32_t j = partner[s];
         if (j != kNone) {
           P.c[j] = __dadd_rn(P.c[j], __dmul_rn(c, gm));  // the partner is no parent: one writer
+          partner[s] = kNone;  // the array is all kNone between ops (rotations rely on it)
         } else {
           child = true;
         }
