@@ -148,7 +148,7 @@ struct ppvm_sum {
   std::map<size_t, int> run_len;   // run start -> gates of the fused run enqueued there (this attempt)
   uint32_t* s_idx = nullptr;
   uint64_t* s_rec = nullptr;
-  uint32_t* partner = nullptr;
+  unsigned long long* link = nullptr;  // per term: its rotation partner's coefficient (kNoLink between rotations)
   unsigned long long* table = nullptr;
   unsigned long long table_cap = 0;
   unsigned long long run_slots_used = 0;  // group-table slots the fused runs since the last clean state hashed into
@@ -417,12 +417,12 @@ void free_scratch(ppvm_sum* s) {
   s->tstate2 = nullptr;
   pool_free(s->s_idx);
   pool_free(s->s_rec);
-  pool_free(s->partner);
+  pool_free(s->link);
   pool_free(s->table);
   pool_free(s->tstate);
   s->s_idx = nullptr;
   s->s_rec = nullptr;
-  s->partner = nullptr;
+  s->link = nullptr;
   s->table = nullptr;
   s->tstate = nullptr;
 }
@@ -459,8 +459,8 @@ ppvm_status grow(ppvm_sum* s, unsigned long long new_cap) {
   s->cap = new_cap;
   free_scratch(s);
   CUDA_TRY(pool_malloc((void**)&s->s_idx, sizeof(uint32_t) * new_cap, site));
-  CUDA_TRY(pool_malloc((void**)&s->partner, sizeof(uint32_t) * new_cap, site));
-  CUDA_TRY(cudaMemsetAsync(s->partner, 0xFF, sizeof(uint32_t) * new_cap, s->stream));  // kNone between rotations
+  CUDA_TRY(pool_malloc((void**)&s->link, sizeof(unsigned long long) * new_cap, site));
+  CUDA_TRY(cudaMemsetAsync(s->link, 0xFF, sizeof(unsigned long long) * new_cap, s->stream));  // all kNoLink
   CUDA_TRY(pool_malloc((void**)&s->s_rec, sizeof(uint64_t) * (size_t)(2 * W + 1) * new_cap, site));
   s->table_cap = next_pow2(std::max<unsigned long long>(2 * new_cap, 1024));
   CUDA_TRY(pool_malloc((void**)&s->table, sizeof(unsigned long long) * s->table_cap, site));
@@ -619,7 +619,7 @@ uint64_t launch_bytes(const ppvm_sum* s, const ProfLaunch& L, const std::vector<
     }
     case F_APPLY: {  // test words, partner links, coefficients read and written, children
       const int tw = (L.op < (int)test_words.size()) ? test_words[L.op] : 1;
-      return g.n_in * 8ull * tw + g.n_s * (4 + 16) + g.n_new * (B - 8 + B);
+      return g.n_in * 8ull * tw + g.n_s * (8 + 16) + g.n_new * (B - 8 + B);
     }
     case F_CLIFF: return 2ull * g.n_in * B;
     case F_TRUNC: return g.n_in * B + g.n_out * B;
@@ -875,12 +875,12 @@ struct K {
     {
       ProfScope ps(s, F_PAIR, op, 1);
       launch(k_rot_pair<W>, grid_for(nub, kPairBlock, 8), kPairBlock, 0, s->stream,
-          P, s->d_ctrl, g, xmask, zmask, s->partner, s->table, s->table_cap, s->next_table_epoch(), op);
+          P, s->d_ctrl, g, xmask, zmask, s->link, s->table, s->table_cap, s->next_table_epoch(), op);
     }
     {
       ProfScope ps(s, F_APPLY, op, 1);
       launch(k_rot_apply<W, kScanBlock, ITEMS>, grid_for(nub, TILE, 8), kScanBlock, 0, s->stream,
-          P, s->d_ctrl, g, xmask, zmask, gm, sn, cs, s->partner, s->tstate, s->next_tile_epoch(), op, s->d_log);
+          P, s->d_ctrl, g, xmask, zmask, gm, sn, cs, s->link, s->tstate, s->next_tile_epoch(), op, s->d_log);
     }
     s->n_ub = std::min<unsigned long long>(s->cap, 2 * s->n_ub);
   }
@@ -898,8 +898,8 @@ struct K {
     {
       ProfScope ps(s, F_SCAN, op, 1);
       launch(k_damp_scan<W, kScanBlock, ITEMS>, grid_for(nub, TILE, 8), kScanBlock, 0, s->stream,
-          P, s->d_ctrl, g, qmask, s->s_idx, s->s_rec, s->partner, s->tstate,
-          s->next_tile_epoch(), op, s->d_log);
+          P, s->d_ctrl, g, qmask, s->s_idx, s->s_rec, s->R.gslot, s->tstate,
+          s->next_tile_epoch(), op, s->d_log);  // gslot: free outside fused runs, the parents' partners here
     }
     const unsigned tep = s->next_table_epoch();
     {
@@ -907,12 +907,12 @@ struct K {
       launch(k_damp_index<W>, grid_for(nub, kPairBlock, 8), kPairBlock, 0, s->stream,
           s->d_ctrl, g, s->s_rec, s->table, s->table_cap, tep, op);
       launch(k_damp_probe<W>, grid_for(nub, kPairBlock, 8), kPairBlock, 0, s->stream,
-          P, s->d_ctrl, g, q >> 6, s->s_rec, s->partner, s->table, s->table_cap, tep, sxy, op);
+          P, s->d_ctrl, g, q >> 6, s->s_rec, s->R.gslot, s->table, s->table_cap, tep, sxy, op);
     }
     {
       ProfScope ps(s, F_APPLY, op, 1);
       launch(k_damp_apply<W, kScanBlock, ITEMS>, grid_for(nub, TILE, 8), kScanBlock, 0, s->stream,
-          P, s->d_ctrl, g, om, gamma, s->s_idx, s->s_rec, s->partner, s->tstate, s->next_tile_epoch(), op);
+          P, s->d_ctrl, g, om, gamma, s->s_idx, s->s_rec, s->R.gslot, s->tstate, s->next_tile_epoch(), op);
     }
     {
       ProfScope ps(s, F_COMMIT, op, 1);
@@ -1426,8 +1426,8 @@ ppvm_status run_list(ppvm_sum* s, const ppvm_op* ops, size_t n_ops, const std::v
     }
     if (s->prof) prof_collect(s, test_words);
     PPVM_TRY(clear_run_tables(s, s->run_slots_used));  // a run stopped part-way leaves its slots set
-    // and a rotation stopped between its kernels leaves partner links
-    CUDA_TRY(cudaMemsetAsync(s->partner, 0xFF, sizeof(uint32_t) * std::min(s->cap, s->n_ub), s->stream));
+    // and a rotation stopped between its kernels leaves links
+    CUDA_TRY(cudaMemsetAsync(s->link, 0xFF, sizeof(unsigned long long) * std::min(s->cap, s->n_ub), s->stream));
     // fused runs at or after the failing op did not run: give their buffers back
     for (int op0 : s->swaps)
       if (op0 >= c.err_op) std::swap(s->planes, s->alt);

@@ -95,15 +95,24 @@ __device__ __forceinline__ void load_words(const Planes& P, unsigned long long i
   }
 }
 
+// link[i]: the bits of the coefficient of term i's partner, or kNoLink.  kNoLink is a NaN that no
+// arithmetic makes; a coefficient that is that very NaN is linked as another NaN.
+constexpr unsigned long long kNoLink = ~0ull;
+__device__ __forceinline__ unsigned long long link_bits(double c) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(c);
+  return b == kNoLink ? kNoLink - 1 : b;
+}
+
 // k_rot_pair: finds, for each anticommuting term, whether its partner K^G is also present.  The
 // term inserts its index at min(K, K^G) in an epoch-tagged table; the second of a pair to
-// arrive links both in partner[] (all kNone between rotations: k_rot_apply clears the links
-// it reads).  xmask/zmask: the words of the X/Z plane that the test reads.
+// arrive hands each the other's coefficient in link[] (all kNoLink between rotations: k_rot_apply
+// clears the links it reads), so that the apply pass reads and writes nothing at random.
+// xmask/zmask: the words of the X/Z plane that the test reads.
 // Bound by the random 8-byte table accesses: one thread per term at full occupancy keeps as many
 // in flight as the SMs can hold.
 template <int W>
 __global__ void __launch_bounds__(256)
-k_rot_pair(Planes P, Ctrl* ctrl, Gen g, unsigned xmask, unsigned zmask, uint32_t* partner,
+k_rot_pair(Planes P, Ctrl* ctrl, Gen g, unsigned xmask, unsigned zmask, unsigned long long* link,
            unsigned long long* table, unsigned long long table_cap, unsigned tepoch, int op) {
   pdl_wait();
   __shared__ unsigned s_cnt[2];
@@ -158,8 +167,8 @@ k_rot_pair(Planes P, Ctrl* ctrl, Gen g, unsigned xmask, unsigned zmask, uint32_t
 #pragma unroll
         for (int w = 0; w < W; ++w) eq &= (jx[w] == px[w]) & (jz[w] == pz[w]);
         if (eq) {
-          partner[i] = j;
-          partner[j] = (uint32_t)i;
+          link[i] = link_bits(P.c[j]);
+          link[j] = link_bits(P.c[i]);
           ++mine_p;
           break;
         }
@@ -183,13 +192,13 @@ k_rot_pair(Planes P, Ctrl* ctrl, Gen g, unsigned xmask, unsigned zmask, uint32_t
 }
 
 // k_rot_apply: new coefficients in place, children appended in parent order (one decoupled
-// look-back per tile of terms).  Of a pair, the term of lower index computes both coefficients
-// from the old ones, so nothing is read after it was written.  xmask/zmask: the test's words, gm:
-// the words of the generator (of both planes; the sign needs them).  The last of the blocks that have tiles publishes the live count.
+// look-back per tile of terms).  xmask/zmask: the test's words, gm: the words of the generator (of
+// both planes; the sign needs them).  The last of the blocks that have tiles publishes the
+// live count.  A streaming pass: every access but the appended children is at the term itself.
 template <int W, int BLOCK, int ITEMS>
 __global__ void __launch_bounds__(BLOCK)
 k_rot_apply(Planes P, Ctrl* ctrl, Gen g, unsigned xmask, unsigned zmask, unsigned gm, double sn, double cs,
-            uint32_t* partner, unsigned long long* ts, unsigned epoch, int op, OpLog* log) {
+            unsigned long long* link, unsigned long long* ts, unsigned epoch, int op, OpLog* log) {
   pdl_wait();
   __shared__ unsigned s_tile;
   __shared__ unsigned long long s_slot;
@@ -215,46 +224,50 @@ k_rot_apply(Planes P, Ctrl* ctrl, Gen g, unsigned xmask, unsigned zmask, unsigne
     const unsigned tile = next_tile(&ctrl->tickets[1], &s_tile);
     if (tile >= ntiles) break;
     const unsigned long long base = (unsigned long long)tile * TILE;
-    unsigned ballots[ITEMS];
-    double kc[ITEMS];  // a childbearing parent's old coefficient
+    // loads of all the thread's terms first, stores after them
+    unsigned ballots[ITEMS], bits[ITEMS];  // 1: anticommutes, 2: eps of its child is +1, 4: eps of its partner's
+    double kc[ITEMS];
+    unsigned long long kl[ITEMS];
 #pragma unroll
     for (int k = 0; k < ITEMS; ++k) {
       const unsigned long long i = base + (unsigned long long)k * BLOCK + threadIdx.x;
-      bool child = false;
+      bits[k] = 0;
       if (i < N) {
         uint64_t x[W], z[W];
         load_words<W>(P, i, xmask, zmask, x, z);
-        if (anticommutes<W>(g, x, z)) {
-          const uint32_t j = partner[i];
-          if (j == kNone) {
-            child = true;
-            kc[k] = P.c[i];
-            P.c[i] = __dmul_rn(kc[k], cs);
-          } else {
-            partner[i] = kNone;
-            if (i < j) {
-              const double ci = P.c[i], cj = P.c[j];
-              uint64_t x2[W], z2[W];  // the sign's words that the test did not read
-              load_words<W>(P, i, gm & ~xmask, gm & ~zmask, x2, z2);
+        bits[k] = anticommutes<W>(g, x, z);
+      }
+    }
 #pragma unroll
-              for (int w = 0; w < W; ++w) {
-                x[w] |= x2[w];
-                z[w] |= z2[w];
-              }
-              const double eps_i = rot_sign<W>(g, x, z);
-              uint64_t ex[W], ez[W];
-              gen_on<W>(g, x, ex, ez);
+    for (int k = 0; k < ITEMS; ++k) {
+      const unsigned long long i = base + (unsigned long long)k * BLOCK + threadIdx.x;
+      if (bits[k]) {
+        uint64_t x[W], z[W], ex[W], ez[W];
+        load_words<W>(P, i, gm, gm, x, z);
+        kl[k] = link[i];
+        kc[k] = P.c[i];
+        if (rot_sign<W>(g, x, z) > 0.0) bits[k] |= 2u;
+        gen_on<W>(g, x, ex, ez);
 #pragma unroll
-              for (int w = 0; w < W; ++w) {
-                x[w] ^= ex[w];
-                z[w] ^= ez[w];
-              }
-              const double eps_j = rot_sign<W>(g, x, z);
-              P.c[i] = __dadd_rn(__dmul_rn(ci, cs), __dmul_rn(cj, eps_j * sn));
-              P.c[j] = __dadd_rn(__dmul_rn(cj, cs), __dmul_rn(ci, eps_i * sn));
-            }
-          }
+        for (int w = 0; w < W; ++w) {
+          x[w] ^= ex[w];
+          z[w] ^= ez[w];
         }
+        if (rot_sign<W>(g, x, z) > 0.0) bits[k] |= 4u;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < ITEMS; ++k) {
+      const unsigned long long i = base + (unsigned long long)k * BLOCK + threadIdx.x;
+      const bool child = bits[k] && kl[k] == kNoLink;
+      if (bits[k]) {
+        double nc = __dmul_rn(kc[k], cs);
+        if (!child) {
+          const double eps_j = bits[k] & 4u ? 1.0 : -1.0;
+          nc = __dadd_rn(nc, __dmul_rn(__longlong_as_double((long long)kl[k]), eps_j * sn));
+          link[i] = kNoLink;
+        }
+        P.c[i] = nc;
       }
       ballots[k] = __ballot_sync(kFull, child);
     }
@@ -267,10 +280,8 @@ k_rot_apply(Planes P, Ctrl* ctrl, Gen g, unsigned xmask, unsigned zmask, unsigne
           const unsigned long long i = base + (unsigned long long)k * BLOCK + threadIdx.x;
           const unsigned long long r =
               N + excl + s_base[k * NW + warp] + __popc(ballots[k] & ((1u << lane) - 1u));
-          uint64_t x[W], z[W];
+          uint64_t x[W], z[W], ex[W], ez[W];
           load_key<W>(P, i, x, z);
-          const double eps = rot_sign<W>(g, x, z);
-          uint64_t ex[W], ez[W];
           gen_on<W>(g, x, ex, ez);
 #pragma unroll
           for (int w = 0; w < W; ++w) {
@@ -278,7 +289,7 @@ k_rot_apply(Planes P, Ctrl* ctrl, Gen g, unsigned xmask, unsigned zmask, unsigne
             z[w] ^= ez[w];
           }
           store_key<W>(P, r, x, z);
-          P.c[r] = __dmul_rn(kc[k], eps * sn);
+          P.c[r] = __dmul_rn(kc[k], (bits[k] & 2u ? 1.0 : -1.0) * sn);
         }
       }
     }

@@ -194,7 +194,7 @@ k_damp_probe(Planes P, Ctrl* ctrl, Gen g, unsigned qw, const uint64_t* s_rec, ui
 template <int W, int BLOCK, int ITEMS>
 __global__ void __launch_bounds__(BLOCK)
 k_damp_apply(Planes P, Ctrl* ctrl, Gen g, double om, double gm, const uint32_t* s_idx, const uint64_t* s_rec,
-             uint32_t* partner, unsigned long long* ts, unsigned epoch, int op) {
+             const uint32_t* partner, unsigned long long* ts, unsigned epoch, int op) {
   pdl_wait();
   __shared__ unsigned s_tile;
   __shared__ unsigned long long s_slot;
@@ -224,7 +224,6 @@ k_damp_apply(Planes P, Ctrl* ctrl, Gen g, double om, double gm, const uint32_t* 
         const uint32_t j = partner[s];
         if (j != kNone) {
           P.c[j] = __dadd_rn(P.c[j], __dmul_rn(c, gm));  // the partner is no parent: one writer
-          partner[s] = kNone;  // the array is all kNone between ops (rotations rely on it)
         } else {
           child = true;
         }
