@@ -15,9 +15,11 @@
 // built from host circuits therefore costs little more than its kernels.
 //
 // Per op, with reference semantics (crates/ppvm-pauli-sum/src/sum/data.rs:204-311):
-//   rotation   scan (anticommuting terms, in order) -> pair (partner K^G through an
-//              epoch-tagged table) -> apply (parent c*cos + partner's c*(eps*sin); the
-//              partnerless append their child c*(eps*sin) at the end, in parent order)
+//   rotation   scan (anticommuting terms, in order; not at all when the sum's support rules
+//              them out) -> pair (partner K^G through an epoch-tagged table, the second of
+//              a pair hands each the other's coefficient) -> apply (parent c*cos + partner's
+//              c*(eps*sin); the partnerless append their child c*(eps*sin) at the end, in
+//              parent order)
 //   Clifford / noise   in place, consecutive ops fused per term
 //   TRUNCATE   stable in-place compaction (|c| < thr or weight > cap dropped)
 // Term order therefore stays the reference's IndexMap order, and every coefficient is the
@@ -112,10 +114,8 @@ struct BInst {
   int pad;
 };
 
-constexpr unsigned kBNone = 0xFFFFFFFFu;
-
 __host__ __device__ inline unsigned long long region_words(int W, unsigned long long cap, unsigned long long tsize) {
-  return (unsigned long long)(2 * W + 3) * cap + tsize;
+  return (unsigned long long)(2 * W + 2) * cap + (cap + 1) / 2 + tsize;
 }
 
 template <int W>
@@ -123,9 +123,8 @@ struct Region {
   uint64_t* x;
   uint64_t* z;
   double* c;
-  double* rc;      // coefficients of the anticommuting terms, before the op
-  uint32_t* sidx;  // index of anticommuting term r
-  uint32_t* part;  // its partner record, or kBNone
+  unsigned long long* link;  // per term: its partner's coefficient, complemented (0 = none; all 0 between ops)
+  uint32_t* sidx;            // anticommuting terms: each warp's list at the start of its chunk of terms
   unsigned long long* table;
   unsigned long long cap, tsize;
 };
@@ -139,10 +138,9 @@ __device__ __forceinline__ Region<W> region_at(uint64_t* b, unsigned long long c
   r.x = b;
   r.z = b + (size_t)W * cap;
   r.c = reinterpret_cast<double*>(b + (size_t)2 * W * cap);
-  r.rc = reinterpret_cast<double*>(b + (size_t)(2 * W + 1) * cap);
+  r.link = reinterpret_cast<unsigned long long*>(b + (size_t)(2 * W + 1) * cap);
   r.sidx = reinterpret_cast<uint32_t*>(b + (size_t)(2 * W + 2) * cap);
-  r.part = r.sidx + cap;
-  r.table = reinterpret_cast<unsigned long long*>(b + (size_t)(2 * W + 3) * cap);
+  r.table = reinterpret_cast<unsigned long long*>(b + (size_t)(2 * W + 2) * cap + (cap + 1) / 2);
   return r;
 }
 template <int W>
@@ -180,6 +178,12 @@ __device__ __forceinline__ void wflip(uint64_t (&a)[W], unsigned w, uint64_t m) 
 #pragma unroll
   for (int k = 0; k < W; ++k)
     if (k == (int)w) a[k] ^= m;
+}
+template <int W>
+__device__ __forceinline__ void wset_bits(uint64_t (&a)[W], unsigned w, uint64_t m) {
+#pragma unroll
+  for (int k = 0; k < W; ++k)
+    if (k == (int)w) a[k] |= m;
 }
 template <int W>
 __device__ __forceinline__ void wset(uint64_t (&a)[W], unsigned w, unsigned b, bool v) {
@@ -270,31 +274,34 @@ __device__ __forceinline__ void local_op(const DevOp& d, uint64_t (&x)[W], uint6
   }
 }
 
-// Sums of two counts over the block in one pass (three barriers instead of six).
-template <int BLOCK>
-__device__ __forceinline__ void block_sum2_u64(unsigned long long& a, unsigned long long& b,
-                                               unsigned long long* s_red) {
+// ORs the block's masks into s_or (2W words) and returns them to every thread.
+template <int W>
+__device__ __forceinline__ void block_or(uint64_t (&ox)[W], uint64_t (&oz)[W], unsigned long long* s_or) {
+  __syncthreads();
+  if (threadIdx.x < 2 * W) s_or[threadIdx.x] = 0ull;
+  __syncthreads();
 #pragma unroll
-  for (int o = 16; o; o >>= 1) {
-    a += __shfl_down_sync(kFull, a, o);
-    b += __shfl_down_sync(kFull, b, o);
-  }
-  const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  __syncthreads();
-  if (lane == 0) {
-    s_red[warp] = a;
-    s_red[BLOCK / 32 + warp] = b;
+  for (int w = 0; w < W; ++w) {
+    const unsigned xl = __reduce_or_sync(kFull, (unsigned)ox[w]), xh = __reduce_or_sync(kFull, (unsigned)(ox[w] >> 32));
+    const unsigned zl = __reduce_or_sync(kFull, (unsigned)oz[w]), zh = __reduce_or_sync(kFull, (unsigned)(oz[w] >> 32));
+    if ((threadIdx.x & 31) == 0) {
+      atomicOr(&s_or[w], (unsigned long long)xh << 32 | xl);
+      atomicOr(&s_or[W + w], (unsigned long long)zh << 32 | zl);
+    }
   }
   __syncthreads();
-  unsigned long long ta = 0, tb = 0;
 #pragma unroll
-  for (int w = 0; w < BLOCK / 32; ++w) {
-    ta += s_red[w];
-    tb += s_red[BLOCK / 32 + w];
+  for (int w = 0; w < W; ++w) {
+    ox[w] = s_or[w];
+    oz[w] = s_or[W + w];
   }
-  __syncthreads();
-  a = ta;
-  b = tb;
+}
+
+// The coefficient in a link word (its complement), and back: 0 means no link, so the one NaN
+// whose complement is 0 is linked as another NaN.
+__device__ __forceinline__ unsigned long long link_word(double c) {
+  const unsigned long long v = ~(unsigned long long)__double_as_longlong(c);
+  return v ? v : 1ull;
 }
 
 // One layer (or, with layer < 0, everything left) of every instance; CTA b = instance b.
@@ -305,7 +312,9 @@ k_batch(BInst* insts, const BOp* __restrict__ ops, const uint32_t* __restrict__ 
   constexpr int NW = BLOCK / 32;
   constexpr unsigned long long TILE = (unsigned long long)BLOCK * ITEMS;
   __shared__ unsigned s_base[ITEMS * NW + 1];
-  __shared__ unsigned long long s_red[2 * NW];
+  __shared__ unsigned long long s_or[2 * W];
+  __shared__ unsigned s_cnt[NW], s_child[NW];  // per warp: its list's length, its children
+  __shared__ int s_perr;
   extern __shared__ __align__(16) uint64_t s_region[];  // resident_bytes of dynamic shared memory
   BInst& I = insts[blockIdx.x];
   if (I.err) return;
@@ -332,8 +341,10 @@ k_batch(BInst* insts, const BOp* __restrict__ ops, const uint32_t* __restrict__ 
       R.c[i] = G.c[i];
     }
     for (unsigned long long t = threadIdx.x; t < R.tsize; t += BLOCK) R.table[t] = 0ull;
+    for (unsigned long long t = threadIdx.x; t < R.cap; t += BLOCK) R.link[t] = 0ull;
     __syncthreads();
   }
+  if (threadIdx.x == 0) s_perr = 0;
   const double* __restrict__ P = params + I.param_off;
   const double thr = I.thr;
   const unsigned long long maxw = I.maxw;
@@ -343,6 +354,20 @@ k_batch(BInst* insts, const BOp* __restrict__ ops, const uint32_t* __restrict__ 
   int err = 0;
   const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned lt = (1u << lane) - 1u;
+  // bits that some term may have in its X and Z planes: a rotation that none of them lets
+  // anticommute changes nothing and is skipped (a Trotter list acts on every qubit, while the
+  // observable's light cone covers a part of them)
+  uint64_t sx[W], sz[W];
+#pragma unroll
+  for (int w = 0; w < W; ++w) sx[w] = sz[w] = 0ull;
+  for (unsigned long long i = threadIdx.x; i < N; i += BLOCK) {
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+      sx[w] |= R.x[(size_t)w * R.cap + i];
+      sz[w] |= R.z[(size_t)w * R.cap + i];
+    }
+  }
+  block_or<W>(sx, sz, s_or);
   while (pc < end) {
     const BOp op = ops[pc];
     const uint32_t kind = bop_kind(op.h);
@@ -350,6 +375,8 @@ k_batch(BInst* insts, const BOp* __restrict__ ops, const uint32_t* __restrict__ 
       // stable in-place compaction: a tile's reads finish (inside tile_ranks) before its
       // writes, and every write goes to a position at or below the word it came from
       unsigned long long kept = 0;
+#pragma unroll
+      for (int w = 0; w < W; ++w) sx[w] = sz[w] = 0ull;
       for (unsigned long long base = 0; base < N; base += TILE) {
         uint64_t kx[ITEMS][W], kz[ITEMS][W];
         double kc[ITEMS];
@@ -373,10 +400,16 @@ k_batch(BInst* insts, const BOp* __restrict__ ops, const uint32_t* __restrict__ 
             const unsigned long long r = kept + s_base[k * NW + warp] + __popc(bal[k] & lt);
             rstore<W>(R, r, kx[k], kz[k]);
             R.c[r] = kc[k];
+#pragma unroll
+            for (int w = 0; w < W; ++w) {
+              sx[w] |= kx[k][w];
+              sz[w] |= kz[k][w];
+            }
           }
         kept += agg;
         __syncthreads();
       }
+      block_or<W>(sx, sz, s_or);
       N = kept;
       ++pc;
       continue;
@@ -384,6 +417,8 @@ k_batch(BInst* insts, const BOp* __restrict__ ops, const uint32_t* __restrict__ 
     if (kind == B_LOCAL) {
       unsigned j = pc;
       while (j < end && bop_kind(ops[j].h) == B_LOCAL) ++j;
+#pragma unroll
+      for (int w = 0; w < W; ++w) sx[w] = sz[w] = 0ull;
       for (unsigned long long i = threadIdx.x; i < N; i += BLOCK) {
         uint64_t x[W], z[W];
         rload<W>(R, i, x, z);
@@ -392,54 +427,90 @@ k_batch(BInst* insts, const BOp* __restrict__ ops, const uint32_t* __restrict__ 
         for (unsigned o = pc; o < j; ++o) local_op<W>(bop_decode(ops[o], P), x, z, c, neg);
         rstore<W>(R, i, x, z);
         R.c[i] = neg ? -c : c;
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+          sx[w] |= x[w];
+          sz[w] |= z[w];
+        }
       }
+      block_or<W>(sx, sz, s_or);
       tgu += N * (unsigned long long)(j - pc);
       pc = j;
-      __syncthreads();
       continue;
     }
     // ---- rotation exp(-i theta/2 G), G on op.d's one or two qubits ----
     const DevOp d = bop_decode(op, P);
     const double sn = P[op.param], cs = P[op.param + 1];
+    {
+      bool x0 = (wsel<W>(sx, d.w0) >> d.b0) & 1ull, z0 = (wsel<W>(sz, d.w0) >> d.b0) & 1ull;
+      bool any = ((d.az & 1) && x0) || ((d.ax & 1) && z0);
+      if (d.two) {
+        bool x1 = (wsel<W>(sx, d.w1) >> d.b1) & 1ull, z1 = (wsel<W>(sz, d.w1) >> d.b1) & 1ull;
+        any = any || ((d.az & 2) && x1) || ((d.ax & 2) && z1);
+      }
+      if (!any) {  // no term anticommutes
+        tgu += N;
+        ++pc;
+        continue;
+      }
+    }
     if (++epoch >= 0xFFFFu) {  // pair-table epochs wrapped: clear the table once
       for (unsigned long long t = threadIdx.x; t < R.tsize; t += BLOCK) R.table[t] = 0ull;
       __syncthreads();
       epoch = 1;
     }
-    // scan: anticommuting terms, in order
-    unsigned long long S = 0;
-    for (unsigned long long base = 0; base < N; base += TILE) {
-      unsigned bal[ITEMS];
+    // scan: each warp lists the anticommuting terms of its chunk, in order.  No barrier inside: a
+    // scan by block-wide tiles waited three times per 1024 terms
+    const unsigned n32 = (unsigned)N;
+    const unsigned chunk = ((n32 + NW - 1) / NW + 31u) & ~31u;
+    const unsigned lo = min(n32, warp * chunk), hi = min(n32, lo + chunk);
+    unsigned cnt = 0;
+    for (unsigned b0 = lo; b0 < hi; b0 += 32 * ITEMS) {
+      bool a[ITEMS];
 #pragma unroll
       for (int k = 0; k < ITEMS; ++k) {
-        const unsigned long long i = base + (unsigned long long)k * BLOCK + threadIdx.x;
-        bool a = false;
-        if (i < N) {
+        const unsigned i = b0 + k * 32 + lane;
+        a[k] = false;
+        if (i < hi) {
           bool x0, z0, x1, z1;
           term_bits<W>(R, d, i, x0, z0, x1, z1);
-          a = rot_bits(d, x0, z0, x1, z1).anti;
+          a[k] = rot_bits(d, x0, z0, x1, z1).anti;
         }
-        bal[k] = __ballot_sync(kFull, a);
       }
-      const unsigned agg = tile_ranks<BLOCK, ITEMS>(bal, s_base);
 #pragma unroll
-      for (int k = 0; k < ITEMS; ++k)
-        if ((bal[k] >> lane) & 1u) {
-          const unsigned long long i = base + (unsigned long long)k * BLOCK + threadIdx.x;
-          const unsigned long long r = S + s_base[k * NW + warp] + __popc(bal[k] & lt);
-          R.sidx[r] = (uint32_t)i;
-          R.part[r] = kBNone;
-          R.rc[r] = R.c[i];
-        }
-      S += agg;
-      __syncthreads();
+      for (int k = 0; k < ITEMS; ++k) {
+        const unsigned m = __ballot_sync(kFull, a[k]);
+        if (a[k]) R.sidx[lo + cnt + __popc(m & lt)] = b0 + k * 32 + lane;
+        cnt += __popc(m);
+      }
     }
-    // pair: the record of K and the record of K^G (if both exist) meet at min(K, K^G)
-    unsigned long long mine = 0;
+    if (lane == 0) s_cnt[warp] = cnt;
+    if (!__syncthreads_or(cnt != 0)) {
+      tgu += N;
+      ++pc;
+      continue;
+    }
+    unsigned pre[NW];  // lists before warp w's (every thread holds the same)
+    unsigned S = 0;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) {
+      pre[w] = S;
+      S += s_cnt[w];
+    }
+    // term of rank r among the anticommuting ones
+    auto nth = [&](unsigned r) -> unsigned {
+      unsigned at = r;  // lists of the same chunk layout: warp w's starts at w * chunk
+#pragma unroll
+      for (int w = 1; w < NW; ++w)
+        if (r >= pre[w]) at = w * chunk + (r - pre[w]);
+      return R.sidx[at];
+    };
+    // pair: K and K^G (if both exist) meet at min(K, K^G)
     const unsigned long long mask = R.tsize - 1;
-    for (unsigned long long r = threadIdx.x; r < S; r += BLOCK) {
+    for (unsigned r = threadIdx.x; r < S; r += BLOCK) {
+      const unsigned i = nth(r);
       uint64_t x[W], z[W], px[W], pz[W];
-      rload<W>(R, R.sidx[r], x, z);
+      rload<W>(R, i, x, z);
 #pragma unroll
       for (int w = 0; w < W; ++w) {
         px[w] = x[w];
@@ -455,7 +526,7 @@ k_batch(BInst* insts, const BOp* __restrict__ ops, const uint32_t* __restrict__ 
       }
       const uint64_t h = hash_key<W>(kx, kz);
       const unsigned tag = (unsigned)(h >> 48) & 0xFFFFu;
-      const unsigned long long me = make_slot(epoch, tag, (unsigned)r);
+      const unsigned long long me = make_slot(epoch, tag, i);
       unsigned long long slot = h & mask, probes = 0;
       while (true) {
         const unsigned long long cur = ld_volatile(&R.table[slot]);
@@ -466,87 +537,99 @@ k_batch(BInst* insts, const BOp* __restrict__ ops, const uint32_t* __restrict__ 
         if (slot_tag(cur) == tag) {
           const unsigned j = slot_idx(cur);
           uint64_t jx[W], jz[W];
-          rload<W>(R, R.sidx[j], jx, jz);
+          rload<W>(R, j, jx, jz);
           bool eq = true;
 #pragma unroll
           for (int w = 0; w < W; ++w) eq &= (jx[w] == px[w]) & (jz[w] == pz[w]);
           if (eq) {
-            R.part[r] = j;
-            R.part[j] = (uint32_t)r;
-            ++mine;
+            R.link[i] = link_word(R.c[j]);
+            R.link[j] = link_word(R.c[i]);
             break;
           }
         }
         slot = (slot + 1) & mask;
         if (++probes > mask) {
-          err = kErrProbe;  // cannot happen with tsize >= 2 * cap; reported, not trapped
+          s_perr = 1;  // cannot happen with tsize >= 2 * cap; reported, not trapped
           break;
         }
       }
     }
-    unsigned long long pairs = mine, perr = (unsigned long long)err;
-    block_sum2_u64<BLOCK>(pairs, perr, s_red);
-    if (perr) {
+    __syncthreads();
+    if (s_perr) {
       err = kErrProbe;
       break;
     }
-    const unsigned long long children = S - 2 * pairs;
-    if (N + children > R.cap) {
-      if (threadIdx.x == 0) I.need = N + children;
+    // each warp counts the children of its share of the ranks; their places follow from the
+    // counts, and nothing is written before the total is known to fit
+    const unsigned share = ((S + NW - 1) / NW + 31u) & ~31u;
+    const unsigned rlo = min(S, warp * share), rhi = min(S, rlo + share);
+    unsigned kids = 0;
+    for (unsigned r = rlo + lane; r < rhi; r += 32) kids += R.link[nth(r)] == 0ull;
+    kids = __reduce_add_sync(kFull, kids);
+    if (lane == 0) s_child[warp] = kids;
+    __syncthreads();
+    unsigned C = 0, at = 0;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) {
+      if (w < (int)warp) at += s_child[w];
+      C += s_child[w];
+    }
+    if (N + C > R.cap) {
+      if (threadIdx.x == 0) I.need = N + C;
       err = kErrCapacity;
       break;
     }
     // apply: parents in place, partnerless children appended in parent order
-    unsigned long long C = 0;
-    for (unsigned long long base = 0; base < S; base += TILE) {
-      unsigned bal[ITEMS];
-#pragma unroll
-      for (int k = 0; k < ITEMS; ++k) {
-        const unsigned long long r = base + (unsigned long long)k * BLOCK + threadIdx.x;
-        bool child = false;
-        if (r < S) {
-          const uint32_t i = R.sidx[r], j = R.part[r];
-          const double c = R.rc[r];
-          double nc;
-          if (j != kBNone) {
-            // the partner's key is K^G: its eps from this term's bits with G's bits flipped
-            bool x0, z0, x1, z1;
-            term_bits<W>(R, d, i, x0, z0, x1, z1);
-            x0 ^= (bool)(d.ax & 1);
-            z0 ^= (bool)(d.az & 1);
-            if (d.two) {
-              x1 ^= (bool)(d.ax & 2);
-              z1 ^= (bool)(d.az & 2);
-            }
-            const double eps_j = rot_bits(d, x0, z0, x1, z1).eps_plus ? 1.0 : -1.0;
-            nc = __dadd_rn(__dmul_rn(c, cs), __dmul_rn(R.rc[j], eps_j * sn));
-          } else {
-            nc = __dmul_rn(c, cs);
-            child = true;
-          }
-          R.c[i] = nc;
-        }
-        bal[k] = __ballot_sync(kFull, child);
-      }
-      const unsigned agg = tile_ranks<BLOCK, ITEMS>(bal, s_base);
-#pragma unroll
-      for (int k = 0; k < ITEMS; ++k)
-        if ((bal[k] >> lane) & 1u) {
-          const unsigned long long r = base + (unsigned long long)k * BLOCK + threadIdx.x;
-          const unsigned long long pos = N + C + s_base[k * NW + warp] + __popc(bal[k] & lt);
-          uint64_t x[W], z[W];
-          rload<W>(R, R.sidx[r], x, z);
+    for (unsigned r0 = rlo; r0 < rhi; r0 += 32) {
+      const unsigned r = r0 + lane;
+      unsigned i = 0;
+      bool child = false;
+      double c = 0.0;
+      if (r < rhi) {
+        i = nth(r);
+        c = R.c[i];
+        const unsigned long long lw = R.link[i];
+        double nc = __dmul_rn(c, cs);
+        if (lw) {
+          // the partner's key is K^G: its eps from this term's bits with G's bits flipped
           bool x0, z0, x1, z1;
-          op_bits<W>(d, x, z, x0, z0, x1, z1);
-          if (!d.two) x1 = z1 = false;
-          const double eps = rot_bits(d, x0, z0, x1, z1).eps_plus ? 1.0 : -1.0;
-          flip_gen<W>(d, x, z);
-          rstore<W>(R, pos, x, z);
-          R.c[pos] = __dmul_rn(R.rc[r], eps * sn);
+          term_bits<W>(R, d, i, x0, z0, x1, z1);
+          x0 ^= (bool)(d.ax & 1);
+          z0 ^= (bool)(d.az & 1);
+          if (d.two) {
+            x1 ^= (bool)(d.ax & 2);
+            z1 ^= (bool)(d.az & 2);
+          }
+          const double eps_j = rot_bits(d, x0, z0, x1, z1).eps_plus ? 1.0 : -1.0;
+          nc = __dadd_rn(nc, __dmul_rn(__longlong_as_double((long long)~lw), eps_j * sn));
+          R.link[i] = 0ull;
+        } else {
+          child = true;
         }
-      C += agg;
-      __syncthreads();
+        R.c[i] = nc;
+      }
+      const unsigned m = __ballot_sync(kFull, child);
+      if (child) {
+        const unsigned long long pos = N + at + __popc(m & lt);
+        uint64_t x[W], z[W];
+        rload<W>(R, i, x, z);
+        bool x0, z0, x1, z1;
+        op_bits<W>(d, x, z, x0, z0, x1, z1);
+        if (!d.two) x1 = z1 = false;
+        const double eps = rot_bits(d, x0, z0, x1, z1).eps_plus ? 1.0 : -1.0;
+        flip_gen<W>(d, x, z);
+        rstore<W>(R, pos, x, z);
+        R.c[pos] = __dmul_rn(c, eps * sn);
+      }
+      at += __popc(m);
     }
+    if (d.ax & 1) wset_bits<W>(sx, d.w0, 1ull << d.b0);
+    if (d.az & 1) wset_bits<W>(sz, d.w0, 1ull << d.b0);
+    if (d.two) {
+      if (d.ax & 2) wset_bits<W>(sx, d.w1, 1ull << d.b1);
+      if (d.az & 2) wset_bits<W>(sz, d.w1, 1ull << d.b1);
+    }
+    __syncthreads();
     tgu += N;
     N += C;
     ++pc;
