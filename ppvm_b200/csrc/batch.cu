@@ -24,8 +24,9 @@
 //   TRUNCATE   stable in-place compaction (|c| < thr or weight > cap dropped)
 // Term order therefore stays the reference's IndexMap order, and every coefficient is the
 // same IEEE result, so each instance equals a PauliSum run on its own.  A rotation that
-// would overflow its instance's capacity stops before writing anything; the host grows that
-// instance's region and resumes from the failing op.
+// would overflow its instance's capacity moves the instance to a larger region of the pool's
+// spare words, inside the kernel; with none left it stops before writing anything, and the
+// host grows that instance's region and resumes from the failing op.
 
 #include <cuda_runtime.h>
 
@@ -113,6 +114,18 @@ struct BInst {
   int err;
   int pad;
 };
+
+// The pool's unused end: an instance that runs out of room takes its next region from here
+// without leaving the kernel (word offset of the next free word; the pool ends at `end`).
+struct BSpare {
+  unsigned long long top, end;
+};
+
+// The capacity a region grows to when it needs `need` terms: 4 times a small one, twice a large one.
+__host__ __device__ inline unsigned long long grown_cap(unsigned long long cap, unsigned long long need) {
+  const unsigned long long a = (cap < 4096 ? 4 : 2) * cap, b = need + need / 2 + 64;
+  return a > b ? a : b;
+}
 
 __host__ __device__ inline unsigned long long region_words(int W, unsigned long long cap, unsigned long long tsize) {
   return (unsigned long long)(2 * W + 2) * cap + (cap + 1) / 2 + tsize;
@@ -306,15 +319,18 @@ __device__ __forceinline__ unsigned long long link_word(double c) {
 
 // One layer (or, with layer < 0, everything left) of every instance; CTA b = instance b.
 template <int W, int BLOCK, int ITEMS>
-__global__ void __launch_bounds__(BLOCK)
+__global__ void __launch_bounds__(BLOCK, 512 / BLOCK)
 k_batch(BInst* insts, const BOp* __restrict__ ops, const uint32_t* __restrict__ layer_ends,
-        const double* __restrict__ params, int layer, uint64_t* pool, unsigned long long resident_bytes) {
+        const double* __restrict__ params, int layer, uint64_t* pool, unsigned long long resident_bytes,
+        BSpare* spare, int tfac) {
   constexpr int NW = BLOCK / 32;
   constexpr unsigned long long TILE = (unsigned long long)BLOCK * ITEMS;
+  constexpr int UB = 1;  // anticommuting terms a thread works on at a time
   __shared__ unsigned s_base[ITEMS * NW + 1];
   __shared__ unsigned long long s_or[2 * W];
   __shared__ unsigned s_cnt[NW], s_child[NW];  // per warp: its list's length, its children
   __shared__ int s_perr;
+  __shared__ unsigned long long s_off;
   extern __shared__ __align__(16) uint64_t s_region[];  // resident_bytes of dynamic shared memory
   BInst& I = insts[blockIdx.x];
   if (I.err) return;
@@ -327,8 +343,8 @@ k_batch(BInst* insts, const BOp* __restrict__ ops, const uint32_t* __restrict__ 
   // live terms are copied in, its pair table starts empty (a zero slot holds no epoch), and
   // the terms go back to the pool at the end.  The op loop is the same code either way (R's
   // arrays are generic pointers).  A region that does not fit runs from the pool.
-  const bool resident = 8ull * region_words(W, I.cap, I.tsize) <= resident_bytes;
-  const Region<W> R = resident ? region_at<W>(s_region, I.cap, I.tsize) : region_of<W>(pool, I);
+  bool resident = 8ull * region_words(W, I.cap, I.tsize) <= resident_bytes;
+  Region<W> R = resident ? region_at<W>(s_region, I.cap, I.tsize) : region_of<W>(pool, I);
   if (resident) {
     const Region<W> G = region_of<W>(pool, I);
     const unsigned long long n0 = I.n;
@@ -505,52 +521,81 @@ k_batch(BInst* insts, const BOp* __restrict__ ops, const uint32_t* __restrict__ 
         if (r >= pre[w]) at = w * chunk + (r - pre[w]);
       return R.sidx[at];
     };
-    // pair: K and K^G (if both exist) meet at min(K, K^G)
+    // pair: K and K^G (if both exist) meet at the same one of the two
     const unsigned long long mask = R.tsize - 1;
-    for (unsigned r = threadIdx.x; r < S; r += BLOCK) {
-      const unsigned i = nth(r);
-      uint64_t x[W], z[W], px[W], pz[W];
-      rload<W>(R, i, x, z);
+#pragma unroll 1
+    for (unsigned r0 = threadIdx.x; r0 < S; r0 += BLOCK * UB) {
+      // the loads of UB terms in flight together, down to the first table slot of each
+      unsigned idx[UB];
+      uint64_t x[UB][W], z[UB][W];
+      unsigned long long hh[UB], first[UB];
 #pragma unroll
-      for (int w = 0; w < W; ++w) {
-        px[w] = x[w];
-        pz[w] = z[w];
+      for (int u = 0; u < UB; ++u) {
+        const unsigned r = r0 + u * BLOCK;
+        if (r < S) idx[u] = nth(r);
       }
-      flip_gen<W>(d, px, pz);
-      const bool use_p = key_less<W>(px, pz, x, z);
-      uint64_t kx[W], kz[W];
 #pragma unroll
-      for (int w = 0; w < W; ++w) {
-        kx[w] = use_p ? px[w] : x[w];
-        kz[w] = use_p ? pz[w] : z[w];
-      }
-      const uint64_t h = hash_key<W>(kx, kz);
-      const unsigned tag = (unsigned)(h >> 48) & 0xFFFFu;
-      const unsigned long long me = make_slot(epoch, tag, i);
-      unsigned long long slot = h & mask, probes = 0;
-      while (true) {
-        const unsigned long long cur = ld_volatile(&R.table[slot]);
-        if (slot_epoch(cur) != (epoch & 0xFFFFu)) {
-          if (atomicCAS(&R.table[slot], cur, me) == cur) break;
-          continue;
+      for (int u = 0; u < UB; ++u)
+        if (r0 + u * BLOCK < S) rload<W>(R, idx[u], x[u], z[u]);
+#pragma unroll
+      for (int u = 0; u < UB; ++u)
+        if (r0 + u * BLOCK < S) {
+          uint64_t px[W], pz[W], kx[W], kz[W];
+#pragma unroll
+          for (int w = 0; w < W; ++w) {
+            px[w] = x[u][w];
+            pz[w] = z[u][w];
+          }
+          flip_gen<W>(d, px, pz);
+          // of the two keys, the one without the generator's bit on q0
+          const bool use_p = ((d.ax & 1 ? wsel<W>(x[u], d.w0) : wsel<W>(z[u], d.w0)) >> d.b0) & 1ull;
+#pragma unroll
+          for (int w = 0; w < W; ++w) {
+            kx[w] = use_p ? px[w] : x[u][w];
+            kz[w] = use_p ? pz[w] : z[u][w];
+          }
+          hh[u] = table_hash<W>(kx, kz);
+          first[u] = ld_volatile(&R.table[hh[u] & mask]);
         }
-        if (slot_tag(cur) == tag) {
-          const unsigned j = slot_idx(cur);
-          uint64_t jx[W], jz[W];
-          rload<W>(R, j, jx, jz);
-          bool eq = true;
 #pragma unroll
-          for (int w = 0; w < W; ++w) eq &= (jx[w] == px[w]) & (jz[w] == pz[w]);
-          if (eq) {
-            R.link[i] = link_word(R.c[j]);
-            R.link[j] = link_word(R.c[i]);
+      for (int u = 0; u < UB; ++u) {
+        if (r0 + u * BLOCK >= S) continue;
+        const unsigned i = idx[u];
+        const unsigned tag = (unsigned)(hh[u] >> 48) & 0xFFFFu;
+        const unsigned long long me = make_slot(epoch, tag, i);
+        unsigned long long slot = hh[u] & mask, probes = 0, cur = first[u];
+        while (true) {
+          if (slot_epoch(cur) != (epoch & 0xFFFFu)) {
+            const unsigned long long prev = atomicCAS(&R.table[slot], cur, me);
+            if (prev == cur) break;
+            cur = prev;  // taken meanwhile: examine what is there now
+            continue;
+          }
+          if (slot_tag(cur) == tag) {
+            const unsigned j = slot_idx(cur);
+            uint64_t px[W], pz[W], jx[W], jz[W];
+#pragma unroll
+            for (int w = 0; w < W; ++w) {
+              px[w] = x[u][w];
+              pz[w] = z[u][w];
+            }
+            flip_gen<W>(d, px, pz);
+            rload<W>(R, j, jx, jz);
+            bool eq = true;
+#pragma unroll
+            for (int w = 0; w < W; ++w) eq &= (jx[w] == px[w]) & (jz[w] == pz[w]);
+            if (eq) {
+              R.link[i] = link_word(R.c[j]);
+              R.link[j] = link_word(R.c[i]);
+              break;
+            }
+          }
+          slot = (slot + 1) & mask;
+          if (++probes > mask) {
+            s_perr = 1;  // cannot happen with tsize >= 2 * cap; reported, not trapped
             break;
           }
-        }
-        slot = (slot + 1) & mask;
-        if (++probes > mask) {
-          s_perr = 1;  // cannot happen with tsize >= 2 * cap; reported, not trapped
-          break;
+          cur = ld_volatile(&R.table[slot]);
         }
       }
     }
@@ -564,7 +609,15 @@ k_batch(BInst* insts, const BOp* __restrict__ ops, const uint32_t* __restrict__ 
     const unsigned share = ((S + NW - 1) / NW + 31u) & ~31u;
     const unsigned rlo = min(S, warp * share), rhi = min(S, rlo + share);
     unsigned kids = 0;
-    for (unsigned r = rlo + lane; r < rhi; r += 32) kids += R.link[nth(r)] == 0ull;
+    for (unsigned r0 = rlo + lane; r0 < rhi; r0 += 32 * UB) {
+      unsigned idx[UB];
+#pragma unroll
+      for (int u = 0; u < UB; ++u)
+        if (r0 + u * 32 < rhi) idx[u] = nth(r0 + u * 32);
+#pragma unroll
+      for (int u = 0; u < UB; ++u)
+        if (r0 + u * 32 < rhi) kids += R.link[idx[u]] == 0ull;
+    }
     kids = __reduce_add_sync(kFull, kids);
     if (lane == 0) s_child[warp] = kids;
     __syncthreads();
@@ -575,53 +628,101 @@ k_batch(BInst* insts, const BOp* __restrict__ ops, const uint32_t* __restrict__ 
       C += s_child[w];
     }
     if (N + C > R.cap) {
-      if (threadIdx.x == 0) I.need = N + C;
-      err = kErrCapacity;
-      break;
+      // a larger region from the pool's spare end: terms, links and lists move over, the table
+      // starts empty (its entries of this op are no longer needed)
+      const unsigned long long ncap = grown_cap(R.cap, N + C);
+      const unsigned long long nts = next_pow2_ull(tfac * ncap < 64 ? 64 : tfac * ncap);
+      if (threadIdx.x == 0) {
+        const unsigned long long words = (region_words(W, ncap, nts) + 31) & ~31ull;
+        s_off = spare->end;  // none left
+        if (ld_volatile(&spare->top) + words <= spare->end) {
+          const unsigned long long o = atomicAdd(&spare->top, words);
+          if (o + words <= spare->end) s_off = o;
+        }
+      }
+      __syncthreads();
+      if (s_off >= spare->end) {  // the host lays the pool out anew
+        if (threadIdx.x == 0) I.need = N + C;
+        err = kErrCapacity;
+        break;
+      }
+      const Region<W> G = region_at<W>(pool + s_off, ncap, nts);
+      for (unsigned long long i = threadIdx.x; i < ncap; i += BLOCK) {
+        if (i < N) {
+#pragma unroll
+          for (int w = 0; w < W; ++w) {
+            G.x[(size_t)w * ncap + i] = R.x[(size_t)w * R.cap + i];
+            G.z[(size_t)w * ncap + i] = R.z[(size_t)w * R.cap + i];
+          }
+          G.c[i] = R.c[i];
+          G.sidx[i] = R.sidx[i];
+        }
+        G.link[i] = i < N ? R.link[i] : 0ull;
+      }
+      for (unsigned long long t = threadIdx.x; t < nts; t += BLOCK) G.table[t] = 0ull;
+      if (threadIdx.x == 0) {
+        I.off = s_off;
+        I.cap = ncap;
+        I.tsize = nts;
+      }
+      R = G;
+      resident = false;
+      __syncthreads();
     }
     // apply: parents in place, partnerless children appended in parent order
-    for (unsigned r0 = rlo; r0 < rhi; r0 += 32) {
-      const unsigned r = r0 + lane;
-      unsigned i = 0;
-      bool child = false;
-      double c = 0.0;
-      if (r < rhi) {
-        i = nth(r);
-        c = R.c[i];
-        const unsigned long long lw = R.link[i];
-        double nc = __dmul_rn(c, cs);
-        if (lw) {
-          // the partner's key is K^G: its eps from this term's bits with G's bits flipped
+    for (unsigned r0 = rlo; r0 < rhi; r0 += 32 * UB) {  // loads of UB terms together, then stores
+      unsigned idx[UB];
+      double c[UB];
+      unsigned long long lw[UB];
+      bool own[UB], other[UB];  // eps of the term's child, of its partner's, is +1
+#pragma unroll
+      for (int u = 0; u < UB; ++u) {
+        const unsigned r = r0 + u * 32 + lane;
+        if (r < rhi) idx[u] = nth(r);
+      }
+#pragma unroll
+      for (int u = 0; u < UB; ++u) {
+        own[u] = other[u] = false;
+        if (r0 + u * 32 + lane < rhi) {
+          c[u] = R.c[idx[u]];
+          lw[u] = R.link[idx[u]];
           bool x0, z0, x1, z1;
-          term_bits<W>(R, d, i, x0, z0, x1, z1);
+          term_bits<W>(R, d, idx[u], x0, z0, x1, z1);
+          own[u] = rot_bits(d, x0, z0, x1, z1).eps_plus;
+          // the partner's key is K^G: its eps from this term's bits with G's bits flipped
           x0 ^= (bool)(d.ax & 1);
           z0 ^= (bool)(d.az & 1);
           if (d.two) {
             x1 ^= (bool)(d.ax & 2);
             z1 ^= (bool)(d.az & 2);
           }
-          const double eps_j = rot_bits(d, x0, z0, x1, z1).eps_plus ? 1.0 : -1.0;
-          nc = __dadd_rn(nc, __dmul_rn(__longlong_as_double((long long)~lw), eps_j * sn));
-          R.link[i] = 0ull;
-        } else {
-          child = true;
+          other[u] = rot_bits(d, x0, z0, x1, z1).eps_plus;
         }
-        R.c[i] = nc;
       }
-      const unsigned m = __ballot_sync(kFull, child);
-      if (child) {
-        const unsigned long long pos = N + at + __popc(m & lt);
-        uint64_t x[W], z[W];
-        rload<W>(R, i, x, z);
-        bool x0, z0, x1, z1;
-        op_bits<W>(d, x, z, x0, z0, x1, z1);
-        if (!d.two) x1 = z1 = false;
-        const double eps = rot_bits(d, x0, z0, x1, z1).eps_plus ? 1.0 : -1.0;
-        flip_gen<W>(d, x, z);
-        rstore<W>(R, pos, x, z);
-        R.c[pos] = __dmul_rn(c, eps * sn);
+#pragma unroll
+      for (int u = 0; u < UB; ++u) {
+        bool child = false;
+        if (r0 + u * 32 + lane < rhi) {
+          double nc = __dmul_rn(c[u], cs);
+          if (lw[u]) {
+            nc = __dadd_rn(nc, __dmul_rn(__longlong_as_double((long long)~lw[u]), (other[u] ? 1.0 : -1.0) * sn));
+            R.link[idx[u]] = 0ull;
+          } else {
+            child = true;
+          }
+          R.c[idx[u]] = nc;
+        }
+        const unsigned m = __ballot_sync(kFull, child);
+        if (child) {
+          const unsigned long long pos = N + at + __popc(m & lt);
+          uint64_t x[W], z[W];
+          rload<W>(R, idx[u], x, z);
+          flip_gen<W>(d, x, z);
+          rstore<W>(R, pos, x, z);
+          R.c[pos] = __dmul_rn(c[u], (own[u] ? 1.0 : -1.0) * sn);
+        }
+        at += __popc(m);
       }
-      at += __popc(m);
     }
     if (d.ax & 1) wset_bits<W>(sx, d.w0, 1ull << d.b0);
     if (d.az & 1) wset_bits<W>(sz, d.w0, 1ull << d.b0);
@@ -777,7 +878,7 @@ struct ppvm_batch {
   double* d_params = nullptr;
   uint64_t* d_init = nullptr;
   uint64_t* pool = nullptr;
-  size_t pool_words = 0;
+  BSpare* d_spare = nullptr;
   unsigned long long resident_bytes = 0;  // dynamic shared memory per CTA for resident instances
   double* d_out = nullptr;
   bool inputs_dirty = true;
@@ -814,7 +915,8 @@ cudaError_t launch_layer(ppvm_batch* b, int layer) {
     if (e != cudaSuccess) return e;
   }
   k_batch<W, BLOCK, ITEMS><<<(unsigned)b->ninst, BLOCK, dyn, b->stream>>>(b->d_inst, b->d_ops, b->d_lends,
-                                                                           b->d_params, layer, b->pool, dyn);
+                                                                           b->d_params, layer, b->pool, dyn,
+                                                                           b->d_spare, b->tfac);
   return cudaGetLastError();
 }
 
@@ -972,6 +1074,17 @@ ppvm_status choose_resident(ppvm_batch* b) {
   return PPVM_OK;
 }
 
+constexpr size_t kSpareMax = (size_t)1 << 30;
+
+// PPVM_BATCH_GROW=host: no spare words, every growth through the host (for the tests).
+bool grow_on_device() {
+  static const bool v = [] {
+    const char* e = std::getenv("PPVM_BATCH_GROW");
+    return !(e && std::strcmp(e, "host") == 0);
+  }();
+  return v;
+}
+
 // Lays the pool out for the current capacities.  With keep, live terms move over.
 ppvm_status layout(ppvm_batch* b, bool keep) {
   std::vector<BInst> old(b->h_inst, b->h_inst + b->ninst);
@@ -986,12 +1099,25 @@ ppvm_status layout(ppvm_batch* b, bool keep) {
     I.epoch = 0;
   }
   const size_t bytes = sizeof(uint64_t) * std::max<unsigned long long>(words, 1);
+  // Spare words after the regions, for instances to grow into inside a launch: 31 times the
+  // regions, between 16 MB and 1 GB.  A device that cannot spare them runs without (growth
+  // through the host).
+  size_t spare = bytes >= kSpareMax / 31 ? kSpareMax : std::max<size_t>(31 * bytes, (size_t)16 << 20);
+  if (!grow_on_device()) spare = 0;
   BTRY(choose_resident(b));
   BCUDA(cudaStreamSynchronize(b->stream));
   void* np = nullptr;
-  BCUDA(ppvm::cache_malloc(&np, bytes));
-  // zeroed: pair-table slots of an earlier user must not carry a live epoch
+  if (spare && ppvm::cache_malloc(&np, bytes + spare) != cudaSuccess) {
+    cudaGetLastError();
+    np = nullptr;
+    spare = 0;
+  }
+  if (!np) BCUDA(ppvm::cache_malloc(&np, bytes));
+  // zeroed: pair-table slots of an earlier user must not carry a live epoch (an instance that
+  // takes spare words clears them itself)
   cudaError_t e = cudaMemsetAsync(np, 0, bytes, b->stream);
+  const BSpare sp = {(bytes / 8 + 31) & ~31ull, (bytes + spare) / 8};
+  if (e == cudaSuccess) e = cudaMemcpyAsync(b->d_spare, &sp, sizeof(sp), cudaMemcpyHostToDevice, b->stream);
   void* d_old = nullptr;
   if (e == cudaSuccess && keep && b->pool) {
     e = ppvm::cache_malloc(&d_old, sizeof(BInst) * b->ninst);
@@ -1015,7 +1141,6 @@ ppvm_status layout(ppvm_batch* b, bool keep) {
   }
   ppvm::cache_free(b->pool);
   b->pool = static_cast<uint64_t*>(np);
-  b->pool_words = words;
   b->layout_dirty = false;
   drop_graphs(b);
   return PPVM_OK;
@@ -1071,12 +1196,13 @@ ppvm_status ensure_graphs(ppvm_batch* b) {
 ppvm_status grow_failed(ppvm_batch* b, uint32_t* first) {
   *first = 0xFFFFFFFFu;
   bool grow = false;
+  for (size_t i = 0; i < b->ninst; ++i) b->cap[i] = b->h_inst[i].cap;  // some grew inside the launches
   for (size_t i = 0; i < b->ninst; ++i) {
     BInst& I = b->h_inst[i];
     if (!I.err) continue;
     if (I.err != kErrCapacity)
       return bfail(PPVM_ECUDA, "batch instance " + std::to_string(i) + ": device error " + std::to_string(I.err));
-    b->cap[i] = std::max<unsigned long long>(2 * b->cap[i], I.need + I.need / 2 + 64);
+    b->cap[i] = grown_cap(b->cap[i], I.need);
     if (b->cap[i] >= 0xFFFFFFF0ull) return bfail(PPVM_ECAPACITY, "batch instance capacity limit (2^32) exceeded");
     I.err = 0;
     grow = true;
@@ -1110,6 +1236,17 @@ ppvm_status run_all(ppvm_batch* b, bool use_graphs, bool persistent) {
     BTRY(grow_failed(b, &first));
     if (first == 0xFFFFFFFFu) {
       b->ran = true;
+      bool grown = false;  // inside the launches, into the pool's spare words
+      for (size_t i = 0; i < b->ninst; ++i) {
+        grown |= b->cap[i] != b->h_inst[i].cap;
+        b->cap[i] = b->h_inst[i].cap;
+      }
+      if (grown) {  // lay the next run out anew if every instance could be resident at these sizes
+        const unsigned long long now = b->resident_bytes;
+        BTRY(choose_resident(b));
+        b->layout_dirty |= b->resident_bytes > now;
+        b->resident_bytes = now;
+      }
       return PPVM_OK;
     }
   }
@@ -1251,6 +1388,7 @@ ppvm_status ppvm_batch_destroy(ppvm_batch* b) {
   ppvm::cache_free(b->d_input);
   ppvm::cache_free(b->pool);
   ppvm::cache_free(b->d_out);
+  ppvm::cache_free(b->d_spare);
   if (b->stream && b->own_stream) cudaStreamDestroy(b->stream);
   delete b;
   return PPVM_OK;
@@ -1290,6 +1428,7 @@ ppvm_status ppvm_batch_create(ppvm_batch** out, size_t n_inst, const uint32_t* n
   if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess ||
       ppvm::cache_malloc((void**)&b->d_inst, sizeof(BInst) * n_inst) != cudaSuccess ||
       cudaMallocHost(&b->h_inst, sizeof(BInst) * n_inst) != cudaSuccess ||
+      ppvm::cache_malloc((void**)&b->d_spare, sizeof(BSpare)) != cudaSuccess ||
       ppvm::cache_malloc((void**)&b->d_out, sizeof(double) * n_inst) != cudaSuccess) {
     ppvm_batch_destroy(b);
     return bfail(PPVM_ECAPACITY, "device allocation failed");

@@ -348,6 +348,21 @@ __device__ __forceinline__ uint64_t hash_key(const uint64_t (&x)[W], const uint6
   return h;
 }
 
+// Hash of a key for the kernels' own tables: one multiply per word, independent of each other,
+// and one mix (hash_key's chain of 2W mixes costs about 2W times as many dependent
+// instructions).  hash_key stays where the host computes the same value or the hash decides
+// where a term goes.
+template <int W>
+__device__ __forceinline__ uint64_t table_hash(const uint64_t (&x)[W], const uint64_t (&z)[W]) {
+  uint64_t h = 0x9E3779B97F4A7C15ull;
+#pragma unroll
+  for (int w = 0; w < W; ++w) {
+    h += (x[w] ^ (x[w] >> 32)) * (0xD1B54A32D192ED03ull + 0x6A09E667F3BCC908ull * (uint64_t)(2 * w));
+    h ^= (z[w] ^ (z[w] >> 31)) * (0x8CB92BA72F3D8DD7ull + 0x6A09E667F3BCC908ull * (uint64_t)(2 * w + 1));
+  }
+  return mix64(h);
+}
+
 template <int W>
 __device__ __forceinline__ bool anticommutes(const Gen& g, const uint64_t (&x)[W],
                                              const uint64_t (&z)[W]) {

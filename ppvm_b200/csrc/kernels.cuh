@@ -2,7 +2,7 @@
 //
 // Rotation exp(-i theta/2 G) on a sum held in SoA planes, reference semantics of
 // PauliSum::map_insert (crates/ppvm-pauli-sum/src/sum/data.rs:204-226):
-//   k_rot_pair   partner search: each anticommuting term inserts min(K, K^G) into an
+//   k_rot_pair   partner search: each anticommuting term inserts one of K, K^G into an
 //                epoch-tagged table; the second of a pair to arrive links both (a child K^G can
 //                only collide with its partner term, so every key receives at most two
 //                contributions)
@@ -104,8 +104,9 @@ __device__ __forceinline__ unsigned long long link_bits(double c) {
 }
 
 // k_rot_pair: finds, for each anticommuting term, whether its partner K^G is also present.  The
-// term inserts its index at min(K, K^G) in an epoch-tagged table; the second of a pair to
-// arrive hands each the other's coefficient in link[] (all kNoLink between rotations: k_rot_apply
+// term inserts its index at the one of K and K^G without the generator's first bit (on a lossy
+// sum, whose terms each see their own part of the generator: the smaller) in an epoch-tagged
+// table; the second of a pair to arrive hands each the other's coefficient in link[] (all kNoLink between rotations: k_rot_apply
 // clears the links it reads), so that the apply pass reads and writes nothing at random.
 // xmask/zmask: the words of the X/Z plane that the test reads.
 // Bound by the random 8-byte table accesses: one thread per term at full occupancy keeps as many
@@ -126,6 +127,18 @@ k_rot_pair(Planes P, Ctrl* ctrl, Gen g, unsigned xmask, unsigned zmask, unsigned
   unsigned long long tsize = next_pow2_ull(N + N / 2 < 1024 ? 1024 : N + N / 2);
   if (tsize > table_cap) tsize = table_cap;
   const unsigned long long mask = tsize - 1;
+  // the generator's first bit: word cw of the X plane (cx) or of the Z plane, mask cm
+  int cw = 0;
+  bool cx = false;
+  uint64_t cm = 0;
+#pragma unroll
+  for (int w = W - 1; w >= 0; --w)
+    if (g.gx[w] | g.gz[w]) {
+      cw = w;
+      cx = g.gx[w] != 0;
+      cm = cx ? g.gx[w] : g.gz[w];
+    }
+  cm &= ~cm + 1;
   unsigned mine_s = 0, mine_p = 0;
   for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += stride) {
     uint64_t x[W], z[W], px[W], pz[W];
@@ -139,14 +152,23 @@ k_rot_pair(Planes P, Ctrl* ctrl, Gen g, unsigned xmask, unsigned zmask, unsigned
       px[w] ^= x[w];
       pz[w] ^= z[w];
     }
-    const bool use_p = key_less<W>(px, pz, x, z);
+    bool use_p;
+    if (g.lw) {
+      use_p = key_less<W>(px, pz, x, z);
+    } else {  // of the two keys, the one without the generator's first bit
+      uint64_t b = 0;
+#pragma unroll
+      for (int w = 0; w < W; ++w)
+        if (w == cw) b = cx ? x[w] : z[w];
+      use_p = b & cm;
+    }
     uint64_t rx[W], rz[W];
 #pragma unroll
     for (int w = 0; w < W; ++w) {
       rx[w] = use_p ? px[w] : x[w];
       rz[w] = use_p ? pz[w] : z[w];
     }
-    const uint64_t h = hash_key<W>(rx, rz);
+    const uint64_t h = table_hash<W>(rx, rz);
     const unsigned tag = (unsigned)(h >> 48) & 0xFFFFu;
     const unsigned long long mine = make_slot(tepoch, tag, (unsigned)i);
     unsigned long long slot = h & mask;
@@ -774,7 +796,7 @@ __device__ __forceinline__ void index_insert(const Planes& P, unsigned long long
                                              unsigned tepoch, Ctrl* ctrl) {
   uint64_t x[W], z[W];
   load_key<W>(P, i, x, z);
-  const uint64_t h = hash_key<W>(x, z);
+  const uint64_t h = table_hash<W>(x, z);
   const unsigned long long mine = make_slot(tepoch, (unsigned)(h >> 48), (unsigned)i);
   unsigned long long slot = h & mask;
   for (unsigned long long probe = 0; probe <= mask; ++probe) {
@@ -793,7 +815,7 @@ template <int W>
 __device__ __forceinline__ long long index_find(const Planes& P, const uint64_t (&x)[W],
                                                 const uint64_t (&z)[W], const unsigned long long* table,
                                                 unsigned long long mask, unsigned tepoch) {
-  const uint64_t h = hash_key<W>(x, z);
+  const uint64_t h = table_hash<W>(x, z);
   const unsigned tag = (unsigned)(h >> 48) & 0xFFFFu;
   unsigned long long slot = h & mask;
   for (unsigned long long probe = 0; probe <= mask; ++probe) {

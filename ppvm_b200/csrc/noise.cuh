@@ -118,7 +118,7 @@ k_damp_index(Ctrl* ctrl, Gen g, const uint64_t* s_rec, unsigned long long* table
     uint64_t x[W], z[W];
     double c;
     damp_child_key<W>(s_rec, s, g, x, z, c);
-    const uint64_t h = hash_key<W>(x, z);
+    const uint64_t h = table_hash<W>(x, z);
     const unsigned long long mine = make_slot(tepoch, (unsigned)(h >> 48) & 0xFFFFu, (unsigned)s);
     unsigned long long slot = h & mask;
     unsigned long long probes = 0;
@@ -166,7 +166,7 @@ k_damp_probe(Planes P, Ctrl* ctrl, Gen g, unsigned qw, const uint64_t* s_rec, ui
     if (ns == 0 || (P.z[(unsigned long long)qw * P.cap + i] & bit)) continue;  // Z: a parent
     uint64_t x[W], z[W];
     load_key<W>(P, i, x, z);
-    const uint64_t h = hash_key<W>(x, z);
+    const uint64_t h = table_hash<W>(x, z);
     const unsigned tag = (unsigned)(h >> 48) & 0xFFFFu;
     unsigned long long slot = h & mask;
     for (unsigned long long probes = 0; probes <= tsize; ++probes) {

@@ -155,7 +155,7 @@ k_run_classify(Planes P, Planes O, Ctrl* ctrl, const RunDesc* rd, RunScratch R, 
           fb = max(fb, hi[kRunMaxK] + 1u);  // reported once per warp below
           R.gslot[i] = kNone;
         } else {
-          const uint64_t h = hash_key<W>(v, f);
+          const uint64_t h = table_hash<W>(v, f);
           const unsigned tag = (unsigned)(h >> 48) & 0xFFFFu;
           const unsigned long long mine = make_slot(tepoch, tag, (unsigned)i);
           unsigned long long slot = h & tmask;
