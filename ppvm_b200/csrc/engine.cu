@@ -162,7 +162,6 @@ struct ppvm_sum {
   OpLog* h_log = nullptr;
   size_t log_cap = 0;
   size_t last_nops = 0;
-  PatItem* d_pat = nullptr;
   double* d_partials = nullptr;
   unsigned long long* d_counter = nullptr;
   SelState* d_sel = nullptr;   // radix select state of budget truncation
@@ -1146,14 +1145,18 @@ struct K {
     k_owz<W><<<nblocks, kRedBlock, 0, s->stream>>>(s->planes_view(), s->d_ctrl, s->d_partials);
     k_sum_partials<<<1, kRedBlock, 0, s->stream>>>(s->d_partials, nblocks, s->d_ctrl);
   }
-  static void trace(ppvm_sum* s, int nblocks, int nitems) {
-    k_trace<W><<<nblocks, kRedBlock, 0, s->stream>>>(s->planes_view(), s->d_ctrl, s->d_pat, nitems,
+  static void trace(ppvm_sum* s, int nblocks, const PatItem* pat, int nitems) {
+    k_trace<W><<<nblocks, kRedBlock, 0, s->stream>>>(s->planes_view(), s->d_ctrl, pat, nitems,
                                                      s->n, s->d_partials, s->lossy ? (unsigned)s->wr : 0u);
     k_sum_partials<<<1, kRedBlock, 0, s->stream>>>(s->d_partials, nblocks, s->d_ctrl);
   }
   static void weights(ppvm_sum* s, uint32_t* out) {
     k_weights<W><<<grid_for(std::max<unsigned long long>(s->n_host, 1), kRedBlock, 8), kRedBlock, 0,
                    s->stream>>>(s->planes_view(), s->d_ctrl, out);
+  }
+  static void max_weight(ppvm_sum* s) {
+    k_max_weight<W><<<grid_for(std::max<unsigned long long>(s->n_host, 1), kRedBlock, 8), kRedBlock, 0, s->stream>>>(
+        s->planes_view(), s->d_ctrl, s->d_counter);
   }
   static void build_index(ppvm_sum* s, unsigned long long mask, unsigned ep) {
     k_build_index<W><<<grid_for(std::max<unsigned long long>(s->n_host, 1), kRedBlock, 8), kRedBlock, 0,
@@ -1496,8 +1499,14 @@ ppvm_status run_gate(ppvm_sum* s, uint32_t code, const uint32_t* t, size_t k, bo
   return run_list(s, ops.data(), ops.size(), {});
 }
 
+// Blocks of a reduction over the sum's terms: enough to fill the GPU (8 blocks of 256 an SM: the
+// reductions wait on memory), at least 4 terms a thread.
+int reduce_blocks(const ppvm_sum* s) {
+  return (int)grid_for(std::max<unsigned long long>(s->n_host, 1), kRedBlock * 4, 8);
+}
+
 ppvm_status do_reduce_owz(ppvm_sum* s, double* out) {
-  const int nb = (int)grid_for(std::max<unsigned long long>(s->n_host, 1), kRedBlock * 4, 2);
+  const int nb = reduce_blocks(s);
   DISPATCH_W(s->W, owz(s, nb));
   CUDA_TRY(cudaGetLastError());
   PPVM_TRY(sync_state(s, 0));
@@ -1699,7 +1708,6 @@ void destroy_now(ppvm_sum* s) {
   cudaFreeHost(s->h_ctrl);
   cudaFree(s->d_log);
   cudaFreeHost(s->h_log);
-  cudaFree(s->d_pat);
   cudaFree(s->d_partials);
   cudaFree(s->d_counter);
   cudaFree(s->d_sel);
@@ -1752,10 +1760,8 @@ ppvm_status ppvm_sum_destroy(ppvm_sum* s) {
       s->event_pool.push_back(L.b);
     }
     s->prof_pending.clear();
-    cudaFree(s->d_pat);
-    cudaFree(s->d_pres_keys);
+      cudaFree(s->d_pres_keys);
     cudaFree(s->d_pres_table);
-    s->d_pat = nullptr;
     s->d_pres_keys = nullptr;
     s->d_pres_table = nullptr;
     std::lock_guard<std::mutex> lk(g_pool_mu);
@@ -2021,13 +2027,19 @@ ppvm_status ppvm_weights(const ppvm_sum* cs, uint32_t* w, size_t cap, size_t* n_
   return PPVM_OK;
 }
 
-ppvm_status ppvm_current_max_weight(const ppvm_sum* s, uint64_t* out) {
-  if (!s || !out) return fail(PPVM_EINVAL, "null argument");
-  std::vector<uint32_t> w(s->n_host);
-  size_t n = 0;
-  PPVM_TRY(ppvm_weights(s, w.data(), w.size(), &n));
-  uint64_t m = 0;
-  for (size_t i = 0; i < n; ++i) m = std::max<uint64_t>(m, w[i]);
+ppvm_status ppvm_current_max_weight(const ppvm_sum* cs, uint64_t* out) {
+  if (!cs || !out) return fail(PPVM_EINVAL, "null argument");
+  REQUIRE_USABLE(cs);
+  ppvm_sum* s = const_cast<ppvm_sum*>(cs);
+  PPVM_TRY(ensure_device(s->device));
+  *out = 0;
+  if (s->n_host == 0) return PPVM_OK;
+  unsigned long long m = 0;
+  CUDA_TRY(cudaMemsetAsync(s->d_counter, 0, sizeof(unsigned long long), s->stream));
+  DISPATCH_W(s->W, max_weight(s));
+  CUDA_TRY(cudaGetLastError());
+  CUDA_TRY(cudaMemcpyAsync(&m, s->d_counter, sizeof(m), cudaMemcpyDeviceToHost, s->stream));
+  CUDA_TRY(cudaStreamSynchronize(s->stream));
   *out = m;
   return PPVM_OK;
 }
@@ -2284,13 +2296,11 @@ ppvm_status ppvm_trace(ppvm_sum* s, const char* pattern, double* out) {
   PPVM_TRY(ensure_device(s->device));
   if (items.size() == 1 && items[0].kind == 1 && items[0].accept == (1u | 4u))  // "Z?*"
     return do_reduce_owz(s, out);
-  cudaFree(s->d_pat);
-  s->d_pat = nullptr;
-  CUDA_TRY(cudaMalloc(&s->d_pat, sizeof(PatItem) * std::max<size_t>(items.size(), 1)));
-  if (!items.empty())
-    CUDA_TRY(cudaMemcpyAsync(s->d_pat, items.data(), sizeof(PatItem) * items.size(), cudaMemcpyHostToDevice, s->stream));
-  const int nb = (int)grid_for(std::max<unsigned long long>(s->n_host, 1), kRedBlock * 4, 2);
-  DISPATCH_W(s->W, trace(s, nb, (int)items.size()));
+  const void* d_pat = nullptr;
+  stage_reset(s);  // the stream is idle between calls
+  if (!items.empty()) PPVM_TRY(stage_put(s, items.data(), sizeof(PatItem) * items.size(), &d_pat));
+  const int nb = reduce_blocks(s);
+  DISPATCH_W(s->W, trace(s, nb, static_cast<const PatItem*>(d_pat), (int)items.size()));
   CUDA_TRY(cudaGetLastError());
   PPVM_TRY(sync_state(s, 0));
   *out = s->h_ctrl->sum;
@@ -2309,7 +2319,7 @@ ppvm_status ppvm_overlap(ppvm_sum* a, ppvm_sum* b, double* out) {
   unsigned ep;
   PPVM_TRY(build_index(a, a->n_host, &mask, &ep));
   CUDA_TRY(cudaMemsetAsync(a->d_counter, 0, sizeof(unsigned long long), a->stream));
-  const int nb = (int)grid_for(std::max<unsigned long long>(b->n_host, 1), kRedBlock * 4, 2);
+  const int nb = reduce_blocks(b);
   DISPATCH_W(a->W, overlap(a, b, mask, ep, nb, a->d_counter));
   CUDA_TRY(cudaGetLastError());
   PPVM_TRY(sync_state(a, 0));
@@ -2335,7 +2345,7 @@ ppvm_status ppvm_equal(const ppvm_sum* ca, const ppvm_sum* cb, int* out) {
   unsigned ep;
   PPVM_TRY(build_index(a, a->n_host, &mask, &ep));
   CUDA_TRY(cudaMemsetAsync(a->d_counter, 0, sizeof(unsigned long long), a->stream));
-  const int nb = (int)grid_for(std::max<unsigned long long>(b->n_host, 1), kRedBlock * 4, 2);
+  const int nb = reduce_blocks(b);
   DISPATCH_W(a->W, overlap(a, b, mask, ep, nb, a->d_counter));
   unsigned long long miss = 1;
   CUDA_TRY(cudaMemcpyAsync(&miss, a->d_counter, sizeof(miss), cudaMemcpyDeviceToHost, a->stream));

@@ -685,78 +685,56 @@ struct PatItem {
   uint64_t arg;
 };
 
+// First qubit at or after pos whose bit in m is clear; n if there is none below n.
 template <int W>
-__device__ __forceinline__ unsigned pauli_code(const uint64_t (&x)[W], const uint64_t (&z)[W],
-                                               unsigned q) {
-  uint64_t xw = 0, zw = 0;
+__device__ __forceinline__ unsigned first_clear(const uint64_t (&m)[W], unsigned pos, unsigned n) {
+  unsigned r = n;
 #pragma unroll
-  for (int w = 0; w < W; ++w)
-    if ((int)(q >> 6) == w) {
-      xw = x[w];
-      zw = z[w];
-    }
-  return (unsigned)((xw >> (q & 63)) & 1u) | ((unsigned)((zw >> (q & 63)) & 1u) << 1);
-}
-
-// Pattern code of qubit q: pauli_code, or 4 for a lost qubit of a lossy sum (lw: first loss
-// word of the X plane, 0 for a plain sum).  No pattern item accepts 4 (accept masks have four
-// bits): L matches no Pauli pattern (crates/ppvm-pauli-word/src/pattern/contains.rs:25-41).
-template <int W>
-__device__ __forceinline__ unsigned pat_code(const uint64_t (&x)[W], const uint64_t (&z)[W], unsigned lw,
-                                             unsigned q) {
-  if (lw) {
-    uint64_t l = 0;
-#pragma unroll
-    for (int w = 0; w < W; ++w)
-      if ((int)(lw + (q >> 6)) == w) l = x[w];
-    if ((l >> (q & 63)) & 1u) return 4u;
+  for (int w = W - 1; w >= 0; --w) {
+    uint64_t c = ~m[w];
+    if ((int)(pos >> 6) == w) c &= ~0ull << (pos & 63);
+    if (w >= (int)(pos >> 6) && c) r = w * 64 + (unsigned)__ffsll((long long)c) - 1;
   }
-  return pauli_code<W>(x, z, q);
+  return r < n ? r : n;
 }
 
+// Whether the word matches the pattern (items in order, then only I).  The qubits an item accepts
+// are one mask per word, and a step over a stretch of them is one search for a clear bit: the
+// cost is per item, not per qubit.  x, z: the qubits' words (wr of them on a lossy sum, whose
+// lost qubits, lost[], match no item; crates/ppvm-pauli-word/src/pattern/contains.rs:25-41).
 template <int W>
 __device__ bool pattern_match(const PatItem* items, int nitems, unsigned n, const uint64_t (&x)[W],
-                              const uint64_t (&z)[W], unsigned lw) {
+                              const uint64_t (&z)[W], const uint64_t (&lost)[W]) {
   unsigned pos = 0;
+  uint64_t id[W];  // qubits that hold I
+#pragma unroll
+  for (int w = 0; w < W; ++w) id[w] = ~(x[w] | z[w] | lost[w]);
   for (int it = 0; it < nitems; ++it) {
     const PatItem p = items[it];
-    if (p.kind == 0) {
-      bool next = false;
-      while (pos < n) {
-        const unsigned q = pos++;
-        const unsigned c = pat_code<W>(x, z, lw, q);
-        if (q == p.arg) {
-          next = (p.accept >> c) & 1u;
-          break;
-        }
-        if (c == 0) continue;
-        break;
-      }
-      if (!next) return false;
-    } else if (p.kind == 1) {
-      while (pos < n && ((p.accept >> pat_code<W>(x, z, lw, pos)) & 1u)) ++pos;
+    uint64_t acc[W];
+#pragma unroll
+    for (int w = 0; w < W; ++w)
+      acc[w] = ((p.accept & 1u ? id[w] : 0ull) | (p.accept & 2u ? x[w] & ~z[w] : 0ull) |
+                (p.accept & 4u ? ~x[w] & z[w] : 0ull) | (p.accept & 8u ? x[w] & z[w] : 0ull)) & ~lost[w];
+    if (p.kind == 0) {  // I up to qubit arg, which is accepted
+      if (p.arg < pos || p.arg >= n || first_clear<W>(id, pos, n) < p.arg) return false;
+      const unsigned q = (unsigned)p.arg;
+      if (first_clear<W>(acc, q, n) == q) return false;
+      pos = q + 1;
     } else {
-      unsigned long long matched = 0;
-      bool done = false;
-      while (pos < n) {
-        if ((p.accept >> pat_code<W>(x, z, lw, pos)) & 1u) {
-          ++pos;
-          if (++matched == p.arg) {
-            done = true;
-            break;
-          }
-        } else {
-          if (matched < p.arg) return false;
-          done = true;
-          break;
-        }
+      const unsigned to = first_clear<W>(acc, pos, n);
+      if (p.kind == 1) {
+        pos = to;
+      } else if (p.arg == 0) {  // takes the accepted stretch; fails if that reaches the end
+        if (to == n && to != pos) return false;
+        pos = to;
+      } else {
+        if (to - pos < p.arg) return false;
+        pos += (unsigned)p.arg;
       }
-      if (!done && matched != p.arg) return false;
     }
   }
-  for (; pos < n; ++pos)
-    if (pat_code<W>(x, z, lw, pos) != 0) return false;
-  return true;
+  return first_clear<W>(id, pos, n) == n;
 }
 
 template <int W>
@@ -770,7 +748,15 @@ k_trace(Planes P, const Ctrl* ctrl, const PatItem* items, int nitems, unsigned n
        i += (unsigned long long)gridDim.x * blockDim.x) {
     uint64_t x[W], z[W];
     load_key<W>(P, i, x, z);
-    if (pattern_match<W>(items, nitems, nq, x, z, lw)) acc = __dadd_rn(acc, P.c[i]);
+    uint64_t lost[W];
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+      lost[w] = 0ull;
+#pragma unroll
+      for (int v = 0; v < W; ++v)
+        if (lw && v == w + (int)lw) lost[w] = x[v];
+    }
+    if (pattern_match<W>(items, nitems, nq, x, z, lost)) acc = __dadd_rn(acc, P.c[i]);
   }
   const double b = block_sum(acc, s_red);
   if (threadIdx.x == 0) partials[blockIdx.x] = b;
@@ -785,6 +771,21 @@ __global__ void __launch_bounds__(256) k_weights(Planes P, const Ctrl* ctrl, uin
     load_key<W>(P, i, x, z);
     out[i] = weight<W>(x, z);
   }
+}
+
+// The largest weight into *out (0 before the launch).
+template <int W>
+__global__ void __launch_bounds__(256) k_max_weight(Planes P, const Ctrl* ctrl, unsigned long long* out) {
+  const unsigned long long N = ld_volatile(&ctrl->n);
+  unsigned m = 0;
+  for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < N;
+       i += (unsigned long long)gridDim.x * blockDim.x) {
+    uint64_t x[W], z[W];
+    load_key<W>(P, i, x, z);
+    m = max(m, weight<W>(x, z));
+  }
+  m = __reduce_max_sync(kFull, m);
+  if ((threadIdx.x & 31) == 0 && m) atomicMax(out, (unsigned long long)m);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -883,7 +884,7 @@ k_overlap(Planes A, Planes B, const Ctrl* bctrl, const unsigned long long* table
   __shared__ double s_red[8];
   const unsigned long long NB = ld_volatile(&bctrl->n);
   double acc = 0.0;
-  unsigned long long miss = 0;
+  unsigned miss = 0;
   for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < NB;
        i += (unsigned long long)gridDim.x * blockDim.x) {
     uint64_t x[W], z[W];
@@ -900,7 +901,9 @@ k_overlap(Planes A, Planes B, const Ctrl* bctrl, const unsigned long long* table
   }
   const double b = block_sum(acc, s_red);
   if (threadIdx.x == 0) partials[blockIdx.x] = b;
-  if (miss) atomicAdd(mismatch, miss);
+  // one count per warp: an atomic per thread on the one word cost more than the lookups
+  miss = __reduce_add_sync(kFull, miss);
+  if ((threadIdx.x & 31) == 0 && miss) atomicAdd(mismatch, (unsigned long long)miss);
 }
 
 }  // namespace ppvm
