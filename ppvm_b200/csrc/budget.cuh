@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(128) k_score(Planes P, const Ctrl* ctrl, const
     }
     __syncwarp();
     MlpTile T;
-    mlp_forward(X, Ws, T);
+    mlp_forward<false>(X, Ws, T);
     if (t == 0) {
       if (tile * 16 + g < N) keys[tile * 16 + g] = score_key(T.y[0]);
       if (tile * 16 + g + 8 < N) keys[tile * 16 + g + 8] = score_key(T.y[1]);

@@ -11,6 +11,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
 #include <string>
 #include <vector>
@@ -37,7 +38,10 @@ struct ppvm_mlp {
   int step = 0;
   float* d_feats = nullptr;  // training / prediction inputs (grown on demand)
   float* d_tgt = nullptr;
-  uint32_t* d_order = nullptr;
+  uint32_t* d_order = nullptr;  // sample orders and learning rates of two epochs, and their pinned twin
+  uint32_t* h_order = nullptr;
+  size_t order_cap = 0;
+  cudaEvent_t half_free[2] = {nullptr, nullptr};  // each half's last upload
   float* d_out = nullptr;
   size_t data_cap = 0;
 };
@@ -92,26 +96,16 @@ __global__ void k_mlp_pack(const float* p, MlpWeights* w) {
   if (threadIdx.x == 0) w->b3 = p[kOffB3];
 }
 
-// Adam on the flat parameter vector, one thread per parameter: the minibatch gradient (the
-// training blocks' slabs summed in block order), the update, and the parameter's own packed
-// copies written (W1's zero padding is set once by k_mlp_pack), so no thread waits for another.
-__global__ void __launch_bounds__(256) k_mlp_adam(float* p, float* m, float* v, const float* slabs, int nslabs,
-                                                  float* loss, MlpWeights* w, float lr_t, float b1, float b2,
-                                                  float eps) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i > kMlpParams) return;
-  float gi = 0.0f;  // the minibatch gradient: slabs summed in block order
-  for (int b = 0; b < nslabs; ++b) gi += slabs[(size_t)b * kSlab + i];
-  if (i == kMlpParams) {  // the loss slot
-    *loss += gi;
-    return;
-  }
-  const float mi = b1 * m[i] + (1.0f - b1) * gi;
-  const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-  m[i] = mi;
-  v[i] = vi;
-  const float pi = p[i] - lr_t * mi / (sqrtf(vi) + eps);
-  p[i] = pi;
+// One Adam update: the moments in place, the new parameter returned.
+__device__ __forceinline__ float adam_step(float p, float& m, float& v, float g, float lr_t, float b1, float b2,
+                                           float eps) {
+  m = b1 * m + (1.0f - b1) * g;
+  v = b2 * v + (1.0f - b2) * g * g;
+  return p - lr_t * m / (sqrtf(v) + eps);
+}
+
+// Parameter i's packed copies (W1's zero padding is set once by k_mlp_pack).
+__device__ __forceinline__ void pack_param(MlpWeights* w, int i, float pi) {
   if (i < kOffB1) {
     const int n = (i - kOffW1) / kMlpIn, k = (i - kOffW1) % kMlpIn;
     w->w1[n * kMlpK1 + k] = __float2bfloat16_rn(pi);
@@ -131,29 +125,90 @@ __global__ void __launch_bounds__(256) k_mlp_adam(float* p, float* m, float* v, 
   }
 }
 
-// Stages the features of rows [r0, r0+16) of the sample list into a BF16 [16][16] tile.
-__device__ __forceinline__ void stage_features(__nv_bfloat16* sX, const float* feats, const uint32_t* order,
-                                               unsigned long long r0, unsigned long long rend) {
-  const int lane = threadIdx.x & 31;
-  for (int e = lane; e < 16 * kMlpK1; e += 32) {
-    const int r = e / kMlpK1, k = e % kMlpK1;
-    float v = 0.0f;
-    const unsigned long long row = r0 + r;
-    if (k < kMlpIn && row < rend) {
-      const unsigned long long s = order ? order[row] : row;
-      v = feats[s * kMlpIn + k];
-    }
-    sX[e] = __float2bfloat16_rn(v);
+// Adam on the flat parameter vector, one thread per parameter: the minibatch gradient (the
+// training blocks' slabs summed in block order), the update, and the parameter's own packed
+// copies written, so no thread waits for another.
+__global__ void __launch_bounds__(256) k_mlp_adam(float* p, float* m, float* v, const float* slabs, int nslabs,
+                                                  float* loss, MlpWeights* w, float lr_t, float b1, float b2,
+                                                  float eps) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i > kMlpParams) return;
+  float gi = 0.0f;  // the minibatch gradient: slabs summed in block order
+  for (int b = 0; b < nslabs; ++b) gi += slabs[(size_t)b * kSlab + i];
+  if (i == kMlpParams) {  // the loss slot
+    *loss += gi;
+    return;
   }
+  float mi = m[i], vi = v[i];
+  const float pi = adam_step(p[i], mi, vi, gi, lr_t, b1, b2, eps);
+  m[i] = mi;
+  v[i] = vi;
+  p[i] = pi;
+  pack_param(w, i, pi);
+}
+
+// A lane's share of a 16-row sample tile: half of row r0 + lane/2's features, and the targets of
+// rows r0 + g and r0 + g + 8 (0 past the end).  Loaded apart from its use, so that the loads of
+// the next minibatch's tile are in flight across the update of this one.
+struct SampleTile {
+  float4 f;
+  float tg[2];
+};
+__device__ __forceinline__ void load_samples(SampleTile& S, const float* feats, const float* targets,
+                                             const uint32_t* order, unsigned long long r0, unsigned long long rend) {
+  const int lane = threadIdx.x & 31;
+  const unsigned long long row = r0 + (lane >> 1);
+  S.f = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  if (row < rend) {
+    const unsigned long long s = order ? order[row] : row;
+    S.f = *reinterpret_cast<const float4*>(feats + s * kMlpIn + 4 * (lane & 1));
+  }
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const unsigned long long r = r0 + (lane >> 2) + 8 * h;
+    S.tg[h] = targets && r < rend ? targets[order ? order[r] : r] : 0.0f;
+  }
+}
+
+// The tile's features as a BF16 [16][16] tile (upper 8 columns 0).
+__device__ __forceinline__ void stage_features(__nv_bfloat16* sX, const SampleTile& S) {
+  const int lane = threadIdx.x & 31;
+  uint2* row = reinterpret_cast<uint2*>(sX + (lane >> 1) * kMlpK1);
+  row[lane & 1] = make_uint2(pack_bf16(S.f.x, S.f.y), pack_bf16(S.f.z, S.f.w));
+  row[2 + (lane & 1)] = make_uint2(0u, 0u);
   __syncwarp();
 }
 
-__device__ __forceinline__ uint32_t pack2(const __nv_bfloat16 lo, const __nv_bfloat16 hi) {
-  return (uint32_t)__bfloat16_as_ushort(lo) | ((uint32_t)__bfloat16_as_ushort(hi) << 16);
+// Row stride of the warps' [16][64] staging tiles: 144 bytes, so that the 8 rows of an ldmatrix land
+// in different banks.
+constexpr int kStageLd = kMlpH + 8;
+constexpr int kTileHalves = 16 * kMlpK1 + 2 * 16 * kStageLd;  // sX, sD, sH of a warp
+
+// Four transposed 8 x 8 blocks; lane i gives the address of row i % 8 of block i / 8.
+__device__ __forceinline__ void ldmatrix4_t(uint32_t (&r)[4], const __nv_bfloat16* p) {
+  const unsigned a = (unsigned)__cvta_generic_to_shared(p);
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(a)
+               : "memory");
+}
+
+// sG[i] += v, or sG[i] = v for a warp's first tile (FIRST: nothing has been added yet).
+template <bool FIRST>
+__device__ __forceinline__ void acc_to(float* sG, int i, float v) {
+  sG[i] = FIRST ? v : sG[i] + v;
+}
+// The same for entries i (even), i + 1.
+template <bool FIRST>
+__device__ __forceinline__ void acc_to2(float* sG, int i, float lo, float hi) {
+  float2* d = reinterpret_cast<float2*>(sG + i);
+  const float2 o = FIRST ? make_float2(0.0f, 0.0f) : *d;
+  *d = FIRST ? make_float2(lo, hi) : make_float2(o.x + lo, o.y + hi);
 }
 
 // Sums a per-thread column partial over the 8 row groups of the warp (lanes with equal t)
 // and adds it to the CTA gradient: cols 8j + 2t, 8j + 2t + 1 of vector `off`.
+template <bool FIRST>
 __device__ __forceinline__ void add_cols(float* sG, int off, int j, float lo, float hi) {
   lo += __shfl_xor_sync(0xffffffffu, lo, 4);
   lo += __shfl_xor_sync(0xffffffffu, lo, 8);
@@ -163,173 +218,168 @@ __device__ __forceinline__ void add_cols(float* sG, int off, int j, float lo, fl
   hi += __shfl_xor_sync(0xffffffffu, hi, 16);
   const int lane = threadIdx.x & 31;
   if (lane < 4) {  // the warp's own gradient copy: each entry always written by the same lane
-    sG[off + 8 * j + 2 * lane] += lo;
-    sG[off + 8 * j + 2 * lane + 1] += hi;
+    acc_to<FIRST>(sG, off + 8 * j + 2 * lane, lo);
+    acc_to<FIRST>(sG, off + 8 * j + 2 * lane + 1, hi);
   }
 }
 
-// Forward + backward over samples order[start .. start+count) of (feats, targets): squared
-// error loss scaled by inv_n.  Deterministic: every warp accumulates into its own gradient copy
-// (each entry always updated by the same lane), the block sums its warps' copies in a fixed
-// order into its slab (slabs[blockIdx.x]: gradients, then the loss), and the consumer sums the
-// slabs in block order.
-__global__ void __launch_bounds__(kTrainWarps * 32)
-k_mlp_train(const MlpWeights* Wg, const float* feats, const float* targets, const uint32_t* order,
-            unsigned long long start, unsigned long long count, float inv_n, float* slabs) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  MlpWeights& W = *reinterpret_cast<MlpWeights*>(smem);
-  float* sG0 = reinterpret_cast<float*>(smem + sizeof(MlpWeights));  // kTrainWarps copies of kSlab
-  __nv_bfloat16* sX0 = reinterpret_cast<__nv_bfloat16*>(sG0 + kTrainWarps * kSlab);
-  __shared__ float s_loss[kTrainWarps];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+// Forward + backward of one warp over a 16-sample tile at row r0 (rows below `end`): gradients of the
+// squared error scaled by inv_n into the warp's copy sG, the squared errors into lsum.
+template <bool FIRST>
+__device__ __forceinline__ void train_tile(const MlpWeights& W, const SampleTile& S, unsigned long long r0,
+                                           unsigned long long end, float inv_n, __nv_bfloat16* sX, float* sG,
+                                           float& lsum) {
+  const int lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
-  __nv_bfloat16* sX = sX0 + warp * (16 * kMlpK1 + 2 * 16 * kMlpH);
-  float* sG = sG0 + warp * kSlab;
-  __nv_bfloat16* sD = sX + 16 * kMlpK1;  // [16][64]: dZ2, later dZ1
-  __nv_bfloat16* sH = sD + 16 * kMlpH;   // [16][64]: H1
-  {
-    const uint32_t* src = reinterpret_cast<const uint32_t*>(Wg);
-    uint32_t* dst = reinterpret_cast<uint32_t*>(&W);
-    for (int i = threadIdx.x; i < (int)(sizeof(MlpWeights) / 4); i += blockDim.x) dst[i] = src[i];
-    for (int i = threadIdx.x; i < kTrainWarps * kSlab; i += blockDim.x) sG0[i] = 0.0f;
+  __nv_bfloat16* sD = sX + 16 * kMlpK1;   // [16][64]: dZ2, later dZ1
+  __nv_bfloat16* sH = sD + 16 * kStageLd;  // [16][64]: H1
+  stage_features(sX, S);
+  MlpTile T;
+  mlp_forward<true>(sX, W, T);
+  // output error of rows g and g+8
+  float dy[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    float d = 0.0f;
+    if (r0 + g + 8 * h < end) {
+      const float e = T.y[h] - S.tg[h];
+      if (t == 0) lsum += e * e;
+      d = 2.0f * e * inv_n;
+    }
+    dy[h] = d;
   }
-  __syncthreads();
-  float lsum = 0.0f;
-  const unsigned long long end = start + count;
-  const unsigned long long ntiles = (count + 15) / 16;
-  for (unsigned long long tile = (unsigned long long)blockIdx.x * kTrainWarps + warp; tile < ntiles;
-       tile += (unsigned long long)gridDim.x * kTrainWarps) {
-    const unsigned long long r0 = start + tile * 16;
-    stage_features(sX, feats, order, r0, end);
-    MlpTile T;
-    mlp_forward(sX, W, T);
-    // output error of rows g and g+8
-    float dy[2];
+  // layer 3: dW3 = sum dy h2, db3 = sum dy; layer-2 pre-activation gradient dZ2
+  float dz2[8][4];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const unsigned long long row = r0 + g + 8 * h;
-      float d = 0.0f;
-      if (row < end) {
-        const float tg = targets[order ? order[row] : row];
-        const float e = T.y[h] - tg;
-        if (t == 0) lsum += e * e;
-        d = 2.0f * e * inv_n;
-      }
-      dy[h] = d;
-    }
-    // layer 3: dW3 = sum dy h2, db3 = sum dy; layer-2 pre-activation gradient dZ2
-    float dz2[8][4];
+  for (int j = 0; j < 8; ++j) {
+    add_cols<FIRST>(sG, kOffW3, j, dy[0] * T.h2[j][0] + dy[1] * T.h2[j][2], dy[0] * T.h2[j][1] + dy[1] * T.h2[j][3]);
+    const float wl = W.w3[8 * j + 2 * t], wh = W.w3[8 * j + 2 * t + 1];
+    dz2[j][0] = dy[0] * wl * T.g2[j][0];
+    dz2[j][1] = dy[0] * wh * T.g2[j][1];
+    dz2[j][2] = dy[1] * wl * T.g2[j][2];
+    dz2[j][3] = dy[1] * wh * T.g2[j][3];
+    add_cols<FIRST>(sG, kOffB2, j, dz2[j][0] + dz2[j][2], dz2[j][1] + dz2[j][3]);
+  }
+  {
+    float s = (t == 0) ? dy[0] + dy[1] : 0.0f;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      add_cols(sG, kOffW3, j, dy[0] * T.h2[j][0] + dy[1] * T.h2[j][2], dy[0] * T.h2[j][1] + dy[1] * T.h2[j][3]);
-      const float wl = W.w3[8 * j + 2 * t], wh = W.w3[8 * j + 2 * t + 1];
-      dz2[j][0] = dy[0] * wl * gelu_grad(T.z2[j][0]);
-      dz2[j][1] = dy[0] * wh * gelu_grad(T.z2[j][1]);
-      dz2[j][2] = dy[1] * wl * gelu_grad(T.z2[j][2]);
-      dz2[j][3] = dy[1] * wh * gelu_grad(T.z2[j][3]);
-      add_cols(sG, kOffB2, j, dz2[j][0] + dz2[j][2], dz2[j][1] + dz2[j][3]);
-    }
-    {
-      float s = (t == 0) ? dy[0] + dy[1] : 0.0f;
+    for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) acc_to<FIRST>(sG, kOffB3, s);
+  }
+  // stage dZ2 and H1 (BF16, row-major [16][64]) for the weight gradient of layer 2
 #pragma unroll
-      for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      if (lane == 0) sG[kOffB3] += s;
-    }
-    // stage dZ2 and H1 (BF16, row-major [16][64]) for the weight gradient of layer 2
+  for (int j = 0; j < 8; ++j) {
+    const int c = 8 * j + 2 * t;
+    *reinterpret_cast<uint32_t*>(sD + g * kStageLd + c) = pack_bf16(dz2[j][0], dz2[j][1]);
+    *reinterpret_cast<uint32_t*>(sD + (g + 8) * kStageLd + c) = pack_bf16(dz2[j][2], dz2[j][3]);
+    *reinterpret_cast<uint32_t*>(sH + g * kStageLd + c) = T.h1[j / 2][2 * (j % 2)];
+    *reinterpret_cast<uint32_t*>(sH + (g + 8) * kStageLd + c) = T.h1[j / 2][2 * (j % 2) + 1];
+  }
+  __syncwarp();
+  // rows of the 8 x 8 blocks that this lane addresses: A blocks (k half, column half) in the order
+  // (0,0) (0,1) (1,0) (1,1); B blocks (k half, n-tile) in the order (0,0) (1,0) (0,1) (1,1)
+  const int lr = lane & 7, lb = lane >> 3;
+  const __nv_bfloat16* aD = sD + (lr + 8 * (lb >> 1)) * kStageLd + 8 * (lb & 1);
+  const __nv_bfloat16* bH = sH + (lr + 8 * (lb & 1)) * kStageLd + 8 * (lb >> 1);
+  // dW2[n][k] += sum_r dZ2[r][n] H1[r][k]: A = dZ2^T (64 x 16), B = H1 (16 x 64)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int c = 8 * j + 2 * t;
-      sD[g * kMlpH + c] = __float2bfloat16_rn(dz2[j][0]);
-      sD[g * kMlpH + c + 1] = __float2bfloat16_rn(dz2[j][1]);
-      sD[(g + 8) * kMlpH + c] = __float2bfloat16_rn(dz2[j][2]);
-      sD[(g + 8) * kMlpH + c + 1] = __float2bfloat16_rn(dz2[j][3]);
-      sH[g * kMlpH + c] = __float2bfloat16_rn(gelu_f(T.z1[j][0]));
-      sH[g * kMlpH + c + 1] = __float2bfloat16_rn(gelu_f(T.z1[j][1]));
-      sH[(g + 8) * kMlpH + c] = __float2bfloat16_rn(gelu_f(T.z1[j][2]));
-      sH[(g + 8) * kMlpH + c + 1] = __float2bfloat16_rn(gelu_f(T.z1[j][3]));
-    }
-    __syncwarp();
-    // dW2[n][k] += sum_r dZ2[r][n] H1[r][k]: A = dZ2^T (64 x 16), B = H1 (16 x 64)
-#pragma unroll 1
+  for (int jj = 0; jj < 4; ++jj) {
+    uint32_t b[4];
+    ldmatrix4_t(b, bH + 16 * jj);
+#pragma unroll
     for (int mt = 0; mt < 4; ++mt) {
       uint32_t a[4];
+      ldmatrix4_t(a, aD + 16 * mt);
       const int n0 = 16 * mt + g;
-      a[0] = pack2(sD[(2 * t) * kMlpH + n0], sD[(2 * t + 1) * kMlpH + n0]);
-      a[1] = pack2(sD[(2 * t) * kMlpH + n0 + 8], sD[(2 * t + 1) * kMlpH + n0 + 8]);
-      a[2] = pack2(sD[(2 * t + 8) * kMlpH + n0], sD[(2 * t + 9) * kMlpH + n0]);
-      a[3] = pack2(sD[(2 * t + 8) * kMlpH + n0 + 8], sD[(2 * t + 9) * kMlpH + n0 + 8]);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int k0 = 8 * j + g;
-        const uint32_t b0 = pack2(sH[(2 * t) * kMlpH + k0], sH[(2 * t + 1) * kMlpH + k0]);
-        const uint32_t b1 = pack2(sH[(2 * t + 8) * kMlpH + k0], sH[(2 * t + 9) * kMlpH + k0]);
+      for (int e = 0; e < 2; ++e) {
         float acc[4] = {0.f, 0.f, 0.f, 0.f};
-        mma_bf16(acc, a, b0, b1);
-        const int col = 8 * j + 2 * t;
-        sG[kOffW2 + n0 * kMlpH + col] += acc[0];
-        sG[kOffW2 + n0 * kMlpH + col + 1] += acc[1];
-        sG[kOffW2 + (n0 + 8) * kMlpH + col] += acc[2];
-        sG[kOffW2 + (n0 + 8) * kMlpH + col + 1] += acc[3];
+        mma_bf16(acc, a, b[2 * e], b[2 * e + 1]);
+        const int col = 16 * jj + 8 * e + 2 * t;
+        acc_to2<FIRST>(sG, kOffW2 + n0 * kMlpH + col, acc[0], acc[1]);
+        acc_to2<FIRST>(sG, kOffW2 + (n0 + 8) * kMlpH + col, acc[2], acc[3]);
       }
     }
-    // dH1 = dZ2 W2 (A from the dZ2 fragments, B = W2T), dZ1 = dH1 * gelu'(Z1)
-    float dz1[8][4];
+  }
+  // dH1 = dZ2 W2 (A from the dZ2 fragments, B = W2T), dZ1 = dH1 * gelu'(Z1)
+  float dz1[8][4];
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
+  for (int j = 0; j < 8; ++j)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) dz1[j][e] = 0.0f;
+    for (int e = 0; e < 4; ++e) dz1[j][e] = 0.0f;
 #pragma unroll
-    for (int kk = 0; kk < 4; ++kk) {
-      uint32_t a[4];
-      a[0] = pack_bf16(dz2[2 * kk][0], dz2[2 * kk][1]);
-      a[1] = pack_bf16(dz2[2 * kk][2], dz2[2 * kk][3]);
-      a[2] = pack_bf16(dz2[2 * kk + 1][0], dz2[2 * kk + 1][1]);
-      a[3] = pack_bf16(dz2[2 * kk + 1][2], dz2[2 * kk + 1][3]);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const __nv_bfloat16* wr = W.w2t + (8 * j + g) * kMlpH + 16 * kk;
-        mma_bf16(dz1[j], a, *reinterpret_cast<const uint32_t*>(wr + 2 * t),
-                 *reinterpret_cast<const uint32_t*>(wr + 2 * t + 8));
-      }
-    }
-    __syncwarp();  // every lane has read sD before it is overwritten with dZ1
+  for (int kk = 0; kk < 4; ++kk) {
+    uint32_t a[4];
+    a[0] = pack_bf16(dz2[2 * kk][0], dz2[2 * kk][1]);
+    a[1] = pack_bf16(dz2[2 * kk][2], dz2[2 * kk][3]);
+    a[2] = pack_bf16(dz2[2 * kk + 1][0], dz2[2 * kk + 1][1]);
+    a[3] = pack_bf16(dz2[2 * kk + 1][2], dz2[2 * kk + 1][3]);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
+      const __nv_bfloat16* wr = W.w2t + (8 * j + g) * kMlpH + 16 * kk;
+      mma_bf16(dz1[j], a, *reinterpret_cast<const uint32_t*>(wr + 2 * t),
+               *reinterpret_cast<const uint32_t*>(wr + 2 * t + 8));
+    }
+  }
+  __syncwarp();  // every lane has read sD before it is overwritten with dZ1
 #pragma unroll
-      for (int e = 0; e < 4; ++e) dz1[j][e] *= gelu_grad(T.z1[j][e]);
-      add_cols(sG, kOffB1, j, dz1[j][0] + dz1[j][2], dz1[j][1] + dz1[j][3]);
-      const int c = 8 * j + 2 * t;
-      sD[g * kMlpH + c] = __float2bfloat16_rn(dz1[j][0]);
-      sD[g * kMlpH + c + 1] = __float2bfloat16_rn(dz1[j][1]);
-      sD[(g + 8) * kMlpH + c] = __float2bfloat16_rn(dz1[j][2]);
-      sD[(g + 8) * kMlpH + c + 1] = __float2bfloat16_rn(dz1[j][3]);
-    }
-    __syncwarp();
-    // dW1[n][k] += sum_r dZ1[r][n] X[r][k]: A = dZ1^T (64 x 16), B = X (16 x 8 real columns)
-#pragma unroll 1
-    for (int mt = 0; mt < 4; ++mt) {
-      uint32_t a[4];
-      const int n0 = 16 * mt + g;
-      a[0] = pack2(sD[(2 * t) * kMlpH + n0], sD[(2 * t + 1) * kMlpH + n0]);
-      a[1] = pack2(sD[(2 * t) * kMlpH + n0 + 8], sD[(2 * t + 1) * kMlpH + n0 + 8]);
-      a[2] = pack2(sD[(2 * t + 8) * kMlpH + n0], sD[(2 * t + 9) * kMlpH + n0]);
-      a[3] = pack2(sD[(2 * t + 8) * kMlpH + n0 + 8], sD[(2 * t + 9) * kMlpH + n0 + 8]);
-      const uint32_t b0 = pack2(sX[(2 * t) * kMlpK1 + g], sX[(2 * t + 1) * kMlpK1 + g]);
-      const uint32_t b1 = pack2(sX[(2 * t + 8) * kMlpK1 + g], sX[(2 * t + 9) * kMlpK1 + g]);
-      float acc[4] = {0.f, 0.f, 0.f, 0.f};
-      mma_bf16(acc, a, b0, b1);
-      sG[kOffW1 + n0 * kMlpIn + 2 * t] += acc[0];
-      sG[kOffW1 + n0 * kMlpIn + 2 * t + 1] += acc[1];
-      sG[kOffW1 + (n0 + 8) * kMlpIn + 2 * t] += acc[2];
-      sG[kOffW1 + (n0 + 8) * kMlpIn + 2 * t + 1] += acc[3];
-    }
-    __syncwarp();  // sX, sD and sH are rewritten by the next tile
+  for (int j = 0; j < 8; ++j) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) dz1[j][e] *= T.g1[j][e];
+    add_cols<FIRST>(sG, kOffB1, j, dz1[j][0] + dz1[j][2], dz1[j][1] + dz1[j][3]);
+    const int c = 8 * j + 2 * t;
+    *reinterpret_cast<uint32_t*>(sD + g * kStageLd + c) = pack_bf16(dz1[j][0], dz1[j][1]);
+    *reinterpret_cast<uint32_t*>(sD + (g + 8) * kStageLd + c) = pack_bf16(dz1[j][2], dz1[j][3]);
+  }
+  __syncwarp();
+  // dW1[n][k] += sum_r dZ1[r][n] X[r][k]: A = dZ1^T (64 x 16), B = X (16 x 8 real columns)
+  uint32_t bx[4];
+  ldmatrix4_t(bx, sX + (lr + 8 * (lb & 1)) * kMlpK1 + 8 * (lb >> 1));  // blocks 2 and 3: the zero columns
+#pragma unroll
+  for (int mt = 0; mt < 4; ++mt) {
+    uint32_t a[4];
+    ldmatrix4_t(a, aD + 16 * mt);
+    const int n0 = 16 * mt + g;
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    mma_bf16(acc, a, bx[0], bx[1]);
+    acc_to2<FIRST>(sG, kOffW1 + n0 * kMlpIn + 2 * t, acc[0], acc[1]);
+    acc_to2<FIRST>(sG, kOffW1 + (n0 + 8) * kMlpIn + 2 * t, acc[2], acc[3]);
+  }
+  __syncwarp();  // sX, sD and sH are rewritten by the next tile
+}
+
+// One virtual block (kTrainWarps warps) of a minibatch of `count` samples spread over `blocks` of
+// them: block `block`'s warps take tiles block * kTrainWarps + warp, then every
+// blocks * kTrainWarps-th.  Deterministic: every warp accumulates into its own gradient copy
+// (each entry always updated by the same lane), block_slab sums the copies in a fixed order
+// into the block's slab (gradients, then the loss), and the consumer sums the slabs in block
+// order.  `first` holds the samples of the warp's first tile.  Called by warps 0 .. kTrainWarps - 1.
+__device__ __forceinline__ void train_tiles(const MlpWeights& W, const float* feats, const float* targets,
+                                            const uint32_t* order, unsigned long long start, unsigned long long count,
+                                            float inv_n, unsigned block, unsigned blocks, const SampleTile& first,
+                                            __nv_bfloat16* sX, float* sG, float* s_loss) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float lsum = 0.0f;
+  const unsigned long long end = start + count, ntiles = (count + 15) / 16;
+  unsigned long long tile = (unsigned long long)block * kTrainWarps + warp;
+  if (tile < ntiles) {
+    train_tile<true>(W, first, start + tile * 16, end, inv_n, sX, sG, lsum);
+  } else {
+    for (int i = lane; i < kMlpParams; i += 32) sG[i] = 0.0f;
+  }
+  for (tile += (unsigned long long)blocks * kTrainWarps; tile < ntiles; tile += (unsigned long long)blocks * kTrainWarps) {
+    SampleTile S;
+    load_samples(S, feats, targets, order, start + tile * 16, end);
+    train_tile<false>(W, S, start + tile * 16, end, inv_n, sX, sG, lsum);
   }
 #pragma unroll
   for (int o = 16; o; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
   if (lane == 0) s_loss[warp] = lsum;
-  __syncthreads();
-  float* slab = slabs + (size_t)blockIdx.x * kSlab;
+}
+
+// The warps' gradient copies and losses summed in warp order into the block's slab (all threads,
+// after a block barrier).
+__device__ __forceinline__ void block_slab(const float* sG0, const float* s_loss, float* slab) {
   for (int i = threadIdx.x; i < kMlpParams; i += blockDim.x) {
     float v = sG0[i];
 #pragma unroll
@@ -340,6 +390,135 @@ k_mlp_train(const MlpWeights* Wg, const float* feats, const float* targets, cons
     float l = s_loss[0];
     for (int w = 1; w < kTrainWarps; ++w) l += s_loss[w];
     slab[kMlpParams] = l;
+  }
+}
+
+// Forward + backward over samples order[start .. start+count) of (feats, targets), one minibatch.
+__global__ void __launch_bounds__(kTrainWarps * 32)
+k_mlp_train(const MlpWeights* Wg, const float* feats, const float* targets, const uint32_t* order,
+            unsigned long long start, unsigned long long count, float inv_n, float* slabs) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  MlpWeights& W = *reinterpret_cast<MlpWeights*>(smem);
+  float* sG0 = reinterpret_cast<float*>(smem + sizeof(MlpWeights));  // kTrainWarps copies of kSlab
+  __nv_bfloat16* sX0 = reinterpret_cast<__nv_bfloat16*>(sG0 + kTrainWarps * kSlab);
+  __shared__ float s_loss[kTrainWarps];
+  const int warp = threadIdx.x >> 5;
+  {
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(Wg);
+    uint32_t* dst = reinterpret_cast<uint32_t*>(&W);
+    for (int i = threadIdx.x; i < (int)(sizeof(MlpWeights) / 4); i += blockDim.x) dst[i] = src[i];
+  }
+  __syncthreads();
+  SampleTile S;
+  load_samples(S, feats, targets, order, start + ((unsigned long long)blockIdx.x * kTrainWarps + warp) * 16,
+               start + count);
+  train_tiles(W, feats, targets, order, start, count, inv_n, blockIdx.x, gridDim.x, S, sX0 + warp * kTileHalves,
+              sG0 + warp * kSlab, s_loss);
+  __syncthreads();
+  block_slab(sG0, s_loss, slabs + (size_t)blockIdx.x * kSlab);
+}
+
+// A whole epoch of minibatch steps in one launch: one cluster of at most kMaxCluster CTAs, CTA b
+// standing for block b of each step's k_mlp_train launch.  Every CTA keeps the parameters,
+// the Adam moments and the packed weights in its shared memory and applies the same update to all
+// of them from all slabs (summed in block order), so a step needs one cluster barrier and no
+// weight ever crosses the CTAs.  The slabs alternate between two buffers: a CTA writes a
+// buffer again only after a barrier that every reader of its last contents has reached.  The
+// results are those of the launches, bit for bit.  Warps kTrainWarps and up only help to sum
+// and update.  A step was two dependent launches (29 us at 512 samples); what bounds it now is
+// the chain of one tile's products and the cluster's reads of the slabs (L2).
+constexpr int kMaxCluster = 16;
+constexpr int kEpochThreads = 256;
+
+__global__ void __launch_bounds__(kEpochThreads)
+k_mlp_epoch(float* p_g, float* m_g, float* v_g, MlpWeights* Wg, const float* feats, const float* targets,
+            const uint32_t* order, unsigned long long n, unsigned long long batch, const float* lr_t, float b1,
+            float b2, float eps, float* slabs, float* loss) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  MlpWeights& W = *reinterpret_cast<MlpWeights*>(smem);
+  float* sG0 = reinterpret_cast<float*>(smem + sizeof(MlpWeights));
+  __nv_bfloat16* sX0 = reinterpret_cast<__nv_bfloat16*>(sG0 + kTrainWarps * kSlab);
+  float* sp = reinterpret_cast<float*>(sX0 + kTrainWarps * kTileHalves);  // parameters, moments
+  float* sm = sp + kSlab;
+  float* sv = sm + kSlab;
+  __shared__ float s_loss[kTrainWarps];
+  const int warp = threadIdx.x >> 5;
+  const unsigned cta = blockIdx.x;  // one cluster: the rank in it
+  for (int i = threadIdx.x; i < (int)(sizeof(MlpWeights) / 4); i += blockDim.x)
+    reinterpret_cast<uint32_t*>(&W)[i] = reinterpret_cast<const uint32_t*>(Wg)[i];
+  for (int i = threadIdx.x; i < kMlpParams; i += blockDim.x) {
+    sp[i] = p_g[i];
+    sm[i] = m_g[i];
+    sv[i] = v_g[i];
+  }
+  float lsum = threadIdx.x == 0 ? *loss : 0.0f;
+  SampleTile S;  // the warp's first tile of the coming step
+  const unsigned long long mine = ((unsigned long long)cta * kTrainWarps + warp) * 16;
+  if (warp < kTrainWarps) load_samples(S, feats, targets, order, mine, n < batch ? n : batch);
+  __syncthreads();
+  unsigned step = 0;
+  for (unsigned long long st = 0; st < n; st += batch, ++step) {
+    const unsigned long long cnt = n - st < batch ? n - st : batch;
+    const unsigned tiles = (unsigned)((cnt + 15) / 16);
+    const unsigned blocks = (tiles + kTrainWarps - 1) / kTrainWarps;  // as launch_train: at most the cluster
+    float* buf = slabs + (size_t)(step & 1) * kMaxCluster * kSlab;
+    if (cta < blocks) {
+      if (warp < kTrainWarps)
+        train_tiles(W, feats, targets, order, st, cnt, 1.0f / (float)cnt, cta, blocks, S, sX0 + warp * kTileHalves,
+                    sG0 + warp * kSlab, s_loss);
+      __syncthreads();
+      block_slab(sG0, s_loss, buf + (size_t)cta * kSlab);
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    if (warp < kTrainWarps && st + batch < n)
+      load_samples(S, feats, targets, order, st + batch + mine, n - st - batch < batch ? n : st + 2 * batch);
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    const float lr = lr_t[step];
+    // four parameters at a time, four slabs' loads in flight; each parameter's slabs still added in
+    // block order (entries past kMlpParams, the loss's and the padding's, are updated by nobody)
+    for (int q = threadIdx.x; q < kSlab / 4; q += blockDim.x) {
+      float gq[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+      const float4* src = reinterpret_cast<const float4*>(buf) + q;
+      for (unsigned b = 0; b < blocks; b += 4) {
+        float4 v[4];
+#pragma unroll
+        for (unsigned u = 0; u < 4; ++u)
+          if (b + u < blocks) v[u] = __ldcg(src + (size_t)(b + u) * (kSlab / 4));
+#pragma unroll
+        for (unsigned u = 0; u < 4; ++u)
+          if (b + u < blocks) {
+            gq[0] += v[u].x;
+            gq[1] += v[u].y;
+            gq[2] += v[u].z;
+            gq[3] += v[u].w;
+          }
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int i = 4 * q + e;
+        if (i == kMlpParams) s_loss[0] = gq[e];
+        if (i >= kMlpParams) continue;
+        float mi = sm[i], vi = sv[i];
+        const float pi = adam_step(sp[i], mi, vi, gq[e], lr, b1, b2, eps);
+        sm[i] = mi;
+        sv[i] = vi;
+        sp[i] = pi;
+        pack_param(&W, i, pi);
+      }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) lsum += s_loss[0];
+    __syncthreads();  // before the next step's losses
+  }
+  if (cta == 0) {
+    for (int i = threadIdx.x; i < (int)(sizeof(MlpWeights) / 4); i += blockDim.x)
+      reinterpret_cast<uint32_t*>(Wg)[i] = reinterpret_cast<const uint32_t*>(&W)[i];
+    for (int i = threadIdx.x; i < kMlpParams; i += blockDim.x) {
+      p_g[i] = sp[i];
+      m_g[i] = sm[i];
+      v_g[i] = sv[i];
+    }
+    if (threadIdx.x == 0) *loss = lsum;
   }
 }
 
@@ -358,7 +537,7 @@ __global__ void __launch_bounds__(256) k_mlp_reduce(const float* slabs, int nsla
 __global__ void __launch_bounds__(128) k_mlp_predict(const MlpWeights* Wg, const float* feats, unsigned long long n,
                                                      float* out) {
   __shared__ MlpWeights W;
-  __shared__ __nv_bfloat16 sX[4][16 * kMlpK1];
+  __shared__ __align__(16) __nv_bfloat16 sX[4][16 * kMlpK1];
   {
     const uint32_t* src = reinterpret_cast<const uint32_t*>(Wg);
     uint32_t* dst = reinterpret_cast<uint32_t*>(&W);
@@ -369,9 +548,11 @@ __global__ void __launch_bounds__(128) k_mlp_predict(const MlpWeights* Wg, const
   const unsigned long long ntiles = (n + 15) / 16;
   for (unsigned long long tile = (unsigned long long)blockIdx.x * 4 + warp; tile < ntiles;
        tile += (unsigned long long)gridDim.x * 4) {
-    stage_features(sX[warp], feats, nullptr, tile * 16, n);
+    SampleTile S;
+    load_samples(S, feats, nullptr, nullptr, tile * 16, n);
+    stage_features(sX[warp], S);
     MlpTile T;
-    mlp_forward(sX[warp], W, T);
+    mlp_forward<false>(sX[warp], W, T);
     if (t == 0) {
       if (tile * 16 + g < n) out[tile * 16 + g] = T.y[0];
       if (tile * 16 + g + 8 < n) out[tile * 16 + g + 8] = T.y[1];
@@ -381,31 +562,78 @@ __global__ void __launch_bounds__(128) k_mlp_predict(const MlpWeights* Wg, const
 }
 
 size_t train_smem() {
-  return sizeof(MlpWeights) + sizeof(float) * kTrainWarps * kSlab +
-         sizeof(__nv_bfloat16) * kTrainWarps * (16 * kMlpK1 + 2 * 16 * kMlpH);
+  return sizeof(MlpWeights) + sizeof(float) * kTrainWarps * kSlab + sizeof(__nv_bfloat16) * kTrainWarps * kTileHalves;
+}
+size_t epoch_smem() { return train_smem() + sizeof(float) * 3 * kSlab; }
+
+// One epoch of minibatches of at most kMaxCluster blocks as a single cluster; *done says whether it
+// was launched (false: the device cannot place such a cluster).
+ppvm_status launch_epoch(ppvm_mlp* m, unsigned blocks, unsigned long long n, unsigned long long batch,
+                         const uint32_t* d_order, const float* d_lr, float b1, float b2, float eps, bool* done) {
+  *done = false;
+  static const bool never = [] {  // PPVM_MLP_EPOCH=never: two launches per step (for the tests)
+    const char* e = std::getenv("PPVM_MLP_EPOCH");
+    return e && std::strcmp(e, "never") == 0;
+  }();
+  if (never) return PPVM_OK;
+  MCUDA(cudaFuncSetAttribute(k_mlp_epoch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)epoch_smem()));
+  MCUDA(cudaFuncSetAttribute(k_mlp_epoch, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(kEpochThreads);
+  cfg.dynamicSmemBytes = epoch_smem();
+  cfg.stream = m->stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = blocks;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  int fit = 0;
+  if (cudaOccupancyMaxActiveClusters(&fit, k_mlp_epoch, &cfg) != cudaSuccess || fit < 1) {
+    cudaGetLastError();
+    return PPVM_OK;
+  }
+  MCUDA(cudaLaunchKernelEx(&cfg, k_mlp_epoch, m->params, m->m, m->v, m->w, (const float*)m->d_feats,
+                           (const float*)m->d_tgt, d_order, n, batch, d_lr, b1, b2, eps, m->slabs, m->loss));
+  *done = true;
+  return PPVM_OK;
 }
 
 ppvm_status ensure_data(ppvm_mlp* m, size_t n) {
   if (n <= m->data_cap) return PPVM_OK;
   cudaFree(m->d_feats);
   cudaFree(m->d_tgt);
-  cudaFree(m->d_order);
   cudaFree(m->d_out);
   m->d_feats = nullptr;
   m->d_tgt = nullptr;
-  m->d_order = nullptr;
   m->d_out = nullptr;
   m->data_cap = 0;
   MCUDA(cudaMalloc(&m->d_feats, sizeof(float) * kMlpIn * n));
   MCUDA(cudaMalloc(&m->d_tgt, sizeof(float) * n));
-  MCUDA(cudaMalloc(&m->d_order, sizeof(uint32_t) * n));
   MCUDA(cudaMalloc(&m->d_out, sizeof(float) * n));
   m->data_cap = n;
   return PPVM_OK;
 }
 
+// Room for `words` 4-byte words of orders and learning rates (the stream is idle).
+ppvm_status ensure_order(ppvm_mlp* m, size_t words) {
+  for (cudaEvent_t& e : m->half_free)
+    if (!e) MCUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  if (words <= m->order_cap) return PPVM_OK;
+  cudaFree(m->d_order);
+  cudaFreeHost(m->h_order);
+  m->d_order = nullptr;
+  m->h_order = nullptr;
+  m->order_cap = 0;
+  MCUDA(cudaMalloc(&m->d_order, sizeof(uint32_t) * words));
+  MCUDA(cudaMallocHost(&m->h_order, sizeof(uint32_t) * words));
+  m->order_cap = words;
+  return PPVM_OK;
+}
+
 // Forward + backward of one minibatch into the slabs; *nslabs = the number of slabs written.
-ppvm_status launch_train(ppvm_mlp* m, bool use_order, unsigned long long start, unsigned long long count, float inv_n,
+ppvm_status launch_train(ppvm_mlp* m, const uint32_t* d_order, unsigned long long start, unsigned long long count, float inv_n,
                          int* nslabs) {
   static unsigned long long attr = 0;
   if (!((attr >> m->device) & 1ull)) {
@@ -416,8 +644,7 @@ ppvm_status launch_train(ppvm_mlp* m, bool use_order, unsigned long long start, 
   const unsigned grid = (unsigned)std::max<unsigned long long>(
       1, std::min<unsigned long long>((tiles + kTrainWarps - 1) / kTrainWarps, kMaxTrainBlocks));
   k_mlp_train<<<grid, kTrainWarps * 32, train_smem(), m->stream>>>(m->w, m->d_feats, m->d_tgt,
-                                                                   use_order ? m->d_order : nullptr, start, count,
-                                                                   inv_n, m->slabs);
+                                                                   d_order, start, count, inv_n, m->slabs);
   MCUDA(cudaGetLastError());
   *nslabs = (int)grid;
   return PPVM_OK;
@@ -449,6 +676,9 @@ ppvm_status ppvm_mlp_destroy(ppvm_mlp* m) {
   cudaFree(m->d_feats);
   cudaFree(m->d_tgt);
   cudaFree(m->d_order);
+  cudaFreeHost(m->h_order);
+  for (cudaEvent_t e : m->half_free)
+    if (e) cudaEventDestroy(e);
   cudaFree(m->d_out);
   if (m->stream) cudaStreamDestroy(m->stream);
   delete m;
@@ -520,7 +750,7 @@ ppvm_status ppvm_mlp_grad(ppvm_mlp* m, const float* feats, const float* targets,
   MCUDA(cudaMemcpyAsync(m->d_tgt, targets, sizeof(float) * n, cudaMemcpyHostToDevice, m->stream));
   MCUDA(cudaMemsetAsync(m->loss, 0, sizeof(float), m->stream));
   int nslabs = 0;
-  MTRY(launch_train(m, false, 0, n, 1.0f / (float)n, &nslabs));
+  MTRY(launch_train(m, nullptr, 0, n, 1.0f / (float)n, &nslabs));
   k_mlp_reduce<<<(kMlpParams + 1 + 255) / 256, 256, 0, m->stream>>>(m->slabs, nslabs, m->grads, m->loss);
   MCUDA(cudaGetLastError());
   MCUDA(cudaMemcpyAsync(grads, m->grads, sizeof(float) * kMlpParams, cudaMemcpyDeviceToHost, m->stream));
@@ -540,28 +770,46 @@ ppvm_status ppvm_mlp_train(ppvm_mlp* m, const float* feats, const float* targets
   MTRY(ensure_data(m, n));
   MCUDA(cudaMemcpyAsync(m->d_feats, feats, sizeof(float) * kMlpIn * n, cudaMemcpyHostToDevice, m->stream));
   MCUDA(cudaMemcpyAsync(m->d_tgt, targets, sizeof(float) * n, cudaMemcpyHostToDevice, m->stream));
-  std::vector<uint32_t> order(n);
+  // Each epoch's sample order and learning rates are written into one half of a pinned buffer while
+  // the GPU trains on the other half's.
+  const size_t nsteps = (n + (size_t)batch - 1) / (size_t)batch, half = n + nsteps;  // 4-byte words
+  MTRY(ensure_order(m, 2 * half));
   uint64_t s = seed;
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+  const unsigned long long first_tiles = (std::min<size_t>((size_t)batch, n) + 15) / 16;
+  const unsigned long long blocks = (first_tiles + kTrainWarps - 1) / kTrainWarps;
   float ls = 0.f;
   for (int ep = 0; ep < epochs; ++ep) {
+    uint32_t* order = m->h_order + (ep & 1) * half;
+    float* lr_t = reinterpret_cast<float*>(order + n);
+    const uint32_t* d_order = m->d_order + (ep & 1) * half;
+    const float* d_lr = reinterpret_cast<const float*>(d_order + n);
+    if (ep >= 2) MCUDA(cudaEventSynchronize(m->half_free[ep & 1]));  // its copy of two epochs ago is done
     for (size_t i = 0; i < n; ++i) order[i] = (uint32_t)i;
     for (size_t i = n - 1; i > 0; --i) std::swap(order[i], order[splitmix(s) % (i + 1)]);  // Fisher-Yates
-    MCUDA(cudaMemcpyAsync(m->d_order, order.data(), sizeof(uint32_t) * n, cudaMemcpyHostToDevice, m->stream));
+    for (size_t k = 0; k < nsteps; ++k) {
+      const float step = (float)(m->step + (int)k + 1);
+      lr_t[k] = lr * std::sqrt(1.0f - std::pow(b2, step)) / (1.0f - std::pow(b1, step));
+    }
+    MCUDA(cudaMemcpyAsync(m->d_order + (ep & 1) * half, order, sizeof(uint32_t) * half, cudaMemcpyHostToDevice,
+                          m->stream));
+    MCUDA(cudaEventRecord(m->half_free[ep & 1], m->stream));
     MCUDA(cudaMemsetAsync(m->loss, 0, sizeof(float), m->stream));
-    for (size_t st = 0; st < n; st += (size_t)batch) {
+    bool done = false;
+    if (blocks <= (unsigned long long)kMaxCluster)
+      MTRY(launch_epoch(m, (unsigned)blocks, n, (unsigned long long)batch, d_order, d_lr, b1, b2, eps, &done));
+    for (size_t st = 0, k = 0; !done && st < n; st += (size_t)batch, ++k) {
       const size_t cnt = std::min<size_t>((size_t)batch, n - st);
       int nslabs = 0;
-      MTRY(launch_train(m, true, st, cnt, 1.0f / (float)cnt, &nslabs));
-      ++m->step;
-      const float lr_t = lr * std::sqrt(1.0f - std::pow(b2, (float)m->step)) / (1.0f - std::pow(b1, (float)m->step));
+      MTRY(launch_train(m, d_order, st, cnt, 1.0f / (float)cnt, &nslabs));
       k_mlp_adam<<<(kMlpParams + 1 + 255) / 256, 256, 0, m->stream>>>(m->params, m->m, m->v, m->slabs, nslabs,
-                                                                       m->loss, m->w, lr_t, b1, b2, eps);
+                                                                       m->loss, m->w, lr_t[k], b1, b2, eps);
       MCUDA(cudaGetLastError());
     }
-    MCUDA(cudaMemcpyAsync(&ls, m->loss, sizeof(float), cudaMemcpyDeviceToHost, m->stream));
-    MCUDA(cudaStreamSynchronize(m->stream));  // the host order buffer is rewritten next epoch
+    m->step += (int)nsteps;
   }
+  MCUDA(cudaMemcpyAsync(&ls, m->loss, sizeof(float), cudaMemcpyDeviceToHost, m->stream));
+  MCUDA(cudaStreamSynchronize(m->stream));
   if (last_epoch_loss) *last_epoch_loss = ls / (float)n;
   return PPVM_OK;
 }

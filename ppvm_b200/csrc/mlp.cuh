@@ -25,8 +25,9 @@ constexpr int kMlpParams = kMlpH * kMlpIn + kMlpH + kMlpH * kMlpH + kMlpH + kMlp
 constexpr int kOffW1 = 0, kOffB1 = kOffW1 + kMlpH * kMlpIn, kOffW2 = kOffB1 + kMlpH,
               kOffB2 = kOffW2 + kMlpH * kMlpH, kOffW3 = kOffB2 + kMlpH, kOffB3 = kOffW3 + kMlpH;
 
-// Device weights (what k_adam writes after every step).
-struct MlpWeights {
+// Device weights (what k_adam writes after every step).  A multiple of 16 bytes: the training
+// kernels place vector-accessed arrays behind it.
+struct alignas(16) MlpWeights {
   __nv_bfloat16 w1[kMlpH * kMlpK1];
   __nv_bfloat16 w2[kMlpH * kMlpH];
   __nv_bfloat16 w2t[kMlpH * kMlpH];
@@ -47,19 +48,22 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], 
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// GELU (erf form) and its derivative.
-__device__ __forceinline__ float gelu_f(float x) { return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f)); }
-__device__ __forceinline__ float gelu_grad(float x) {
-  return 0.5f * (1.0f + erff(x * 0.70710678118654752f)) + x * 0.3989422804014327f * expf(-0.5f * x * x);
+// GELU (erf form) and its derivative, which share 1 + erf(x / sqrt 2).
+__device__ __forceinline__ float gelu_q(float x) { return 1.0f + erff(x * 0.70710678118654752f); }
+__device__ __forceinline__ float gelu_of(float x, float q) { return 0.5f * x * q; }
+__device__ __forceinline__ float gelu_grad_of(float x, float q) {
+  return 0.5f * q + x * 0.3989422804014327f * expf(-0.5f * x * x);
 }
 
 // Per-warp activations of a 16-row tile, in accumulator-fragment layout: tile j covers
 // output columns 8j..8j+7; element e of thread (g = lane/4, t = lane%4) is row g + 8*(e/2),
 // column 8j + 2t + (e%2).
 struct MlpTile {
-  float z1[8][4], z2[8][4];  // pre-activations (kept for the backward pass)
-  float h2[8][4];            // layer-2 activations
-  float y[2];                // outputs of rows g and g+8 (valid in every lane of the quad)
+  float h2[8][4];       // layer-2 activations
+  float y[2];           // outputs of rows g and g+8 (valid in every lane of the quad)
+  // with GRAD, for the backward pass:
+  float g1[8][4], g2[8][4];  // derivatives of the activations
+  uint32_t h1[4][4];         // layer-1 activations as the packed A fragments of layer 2
 };
 
 // A fragment (16 x 16, row-major) from a BF16 tile in shared memory with row stride ld.
@@ -72,41 +76,51 @@ __device__ __forceinline__ void load_a(uint32_t (&a)[4], const __nv_bfloat16* s,
 }
 
 // Forward pass of one warp over a 16-row feature tile X (BF16, [16][16] in shared memory).
-// W: the weights in shared memory.
+// W: the weights in shared memory.  The erf of each pre-activation, which dominates the pass, is
+// evaluated once, for the activation and (GRAD) its derivative.
+template <bool GRAD>
 __device__ __forceinline__ void mlp_forward(const __nv_bfloat16* X, const MlpWeights& W, MlpTile& T) {
   const int g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
   uint32_t a[4];
+  float z1[8][4], z2[8][4];
   load_a(a, X, kMlpK1, 0);
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     const float bl = W.b1[8 * j + 2 * t], bh = W.b1[8 * j + 2 * t + 1];
-    T.z1[j][0] = bl;
-    T.z1[j][1] = bh;
-    T.z1[j][2] = bl;
-    T.z1[j][3] = bh;
+    z1[j][0] = bl;
+    z1[j][1] = bh;
+    z1[j][2] = bl;
+    z1[j][3] = bh;
     const __nv_bfloat16* wr = W.w1 + (8 * j + g) * kMlpK1;
-    mma_bf16(T.z1[j], a, *reinterpret_cast<const uint32_t*>(wr + 2 * t),
+    mma_bf16(z1[j], a, *reinterpret_cast<const uint32_t*>(wr + 2 * t),
              *reinterpret_cast<const uint32_t*>(wr + 2 * t + 8));
   }
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     const float bl = W.b2[8 * j + 2 * t], bh = W.b2[8 * j + 2 * t + 1];
-    T.z2[j][0] = bl;
-    T.z2[j][1] = bh;
-    T.z2[j][2] = bl;
-    T.z2[j][3] = bh;
+    z2[j][0] = bl;
+    z2[j][1] = bh;
+    z2[j][2] = bl;
+    z2[j][3] = bh;
   }
 #pragma unroll
   for (int kk = 0; kk < 4; ++kk) {
     uint32_t h[4];
-    h[0] = pack_bf16(gelu_f(T.z1[2 * kk][0]), gelu_f(T.z1[2 * kk][1]));
-    h[1] = pack_bf16(gelu_f(T.z1[2 * kk][2]), gelu_f(T.z1[2 * kk][3]));
-    h[2] = pack_bf16(gelu_f(T.z1[2 * kk + 1][0]), gelu_f(T.z1[2 * kk + 1][1]));
-    h[3] = pack_bf16(gelu_f(T.z1[2 * kk + 1][2]), gelu_f(T.z1[2 * kk + 1][3]));
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {  // n-tile 2kk + u/2, elements 2 (u%2) and 2 (u%2) + 1
+      const float xl = z1[2 * kk + u / 2][2 * (u % 2)], xh = z1[2 * kk + u / 2][2 * (u % 2) + 1];
+      const float ql = gelu_q(xl), qh = gelu_q(xh);
+      h[u] = pack_bf16(gelu_of(xl, ql), gelu_of(xh, qh));
+      if (GRAD) {
+        T.g1[2 * kk + u / 2][2 * (u % 2)] = gelu_grad_of(xl, ql);
+        T.g1[2 * kk + u / 2][2 * (u % 2) + 1] = gelu_grad_of(xh, qh);
+        T.h1[kk][u] = h[u];
+      }
+    }
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const __nv_bfloat16* wr = W.w2 + (8 * j + g) * kMlpH + 16 * kk;
-      mma_bf16(T.z2[j], h, *reinterpret_cast<const uint32_t*>(wr + 2 * t),
+      mma_bf16(z2[j], h, *reinterpret_cast<const uint32_t*>(wr + 2 * t),
                *reinterpret_cast<const uint32_t*>(wr + 2 * t + 8));
     }
   }
@@ -115,7 +129,11 @@ __device__ __forceinline__ void mlp_forward(const __nv_bfloat16* X, const MlpWei
   for (int j = 0; j < 8; ++j) {
     const float wl = W.w3[8 * j + 2 * t], wh = W.w3[8 * j + 2 * t + 1];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) T.h2[j][e] = gelu_f(T.z2[j][e]);
+    for (int e = 0; e < 4; ++e) {
+      const float q = gelu_q(z2[j][e]);
+      T.h2[j][e] = gelu_of(z2[j][e], q);
+      if (GRAD) T.g2[j][e] = gelu_grad_of(z2[j][e], q);
+    }
     p0 += T.h2[j][0] * wl + T.h2[j][1] * wh;
     p1 += T.h2[j][2] * wl + T.h2[j][3] * wh;
   }
