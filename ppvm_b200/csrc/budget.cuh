@@ -22,14 +22,15 @@ struct SelState {
 };
 
 template <int W>
-__global__ void __launch_bounds__(256) k_features(Planes P, const Ctrl* ctrl, int L, int layers_left, float* out) {
+__global__ void __launch_bounds__(256) k_features(Planes P, const Ctrl* ctrl, Lattice lat, int layers_left,
+                                                  float* out) {
   const unsigned long long N = ld_volatile(&ctrl->n);
   for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < N;
        i += (unsigned long long)gridDim.x * blockDim.x) {
     uint64_t x[W], z[W];
     load_key<W>(P, i, x, z);
     float f[kMlpIn];
-    term_features<W>(x, z, P.c[i], L, layers_left, f);
+    term_features<W>(x, z, P.c[i], lat, layers_left, f);
 #pragma unroll
     for (int k = 0; k < kMlpIn; ++k) out[i * kMlpIn + k] = f[k];
   }
@@ -37,10 +38,10 @@ __global__ void __launch_bounds__(256) k_features(Planes P, const Ctrl* ctrl, in
 
 // Priority key of every live term: plain (Wg == nullptr) or the network's score.
 template <int W>
-__global__ void __launch_bounds__(128) k_score(Planes P, const Ctrl* ctrl, const MlpWeights* Wg, int L,
+__global__ void __launch_bounds__(128) k_score(Planes P, const Ctrl* ctrl, const MlpWeights* Wg, Lattice lat,
                                                int layers_left, uint32_t* keys) {
   __shared__ MlpWeights Ws;
-  __shared__ __nv_bfloat16 sX[4][16 * kMlpK1];
+  __shared__ __align__(16) __nv_bfloat16 sX[4][2][16 * kMlpK1];
   const unsigned long long N = ld_volatile(&ctrl->n);
   if (!Wg) {
     for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < N;
@@ -55,30 +56,36 @@ __global__ void __launch_bounds__(128) k_score(Planes P, const Ctrl* ctrl, const
   }
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const unsigned long long ntiles = (N + 15) / 16;
-  __nv_bfloat16* X = sX[warp];
-  for (unsigned long long tile = (unsigned long long)blockIdx.x * 4 + warp; tile < ntiles;
-       tile += (unsigned long long)gridDim.x * 4) {
-    if (lane < 16) {
-      const unsigned long long i = tile * 16 + lane;
+  // 32 terms at a time: every lane computes one term's features, then the warp runs the network on
+  // the two 16-row tiles
+  const unsigned long long npairs = (N + 31) / 32;
+  for (unsigned long long pair = (unsigned long long)blockIdx.x * 4 + warp; pair < npairs;
+       pair += (unsigned long long)gridDim.x * 4) {
+    {
+      const unsigned long long i = pair * 32 + lane;
       float f[kMlpIn];
       if (i < N) {
         uint64_t x[W], z[W];
         load_key<W>(P, i, x, z);
-        term_features<W>(x, z, P.c[i], L, layers_left, f);
+        term_features<W>(x, z, P.c[i], lat, layers_left, f);
       } else {
 #pragma unroll
         for (int k = 0; k < kMlpIn; ++k) f[k] = 0.0f;
       }
-#pragma unroll
-      for (int k = 0; k < kMlpK1; ++k) X[lane * kMlpK1 + k] = __float2bfloat16_rn(k < kMlpIn ? f[k] : 0.0f);
+      uint4* row = reinterpret_cast<uint4*>(sX[warp][lane >> 4] + (lane & 15) * kMlpK1);
+      row[0] = make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
+      row[1] = make_uint4(0u, 0u, 0u, 0u);
     }
     __syncwarp();
-    MlpTile T;
-    mlp_forward<false>(X, Ws, T);
-    if (t == 0) {
-      if (tile * 16 + g < N) keys[tile * 16 + g] = score_key(T.y[0]);
-      if (tile * 16 + g + 8 < N) keys[tile * 16 + g + 8] = score_key(T.y[1]);
+#pragma unroll 1
+    for (int h = 0; h < 2; ++h) {
+      MlpTile T;
+      mlp_forward<false>(sX[warp][h], Ws, T);
+      const unsigned long long i = pair * 32 + 16 * h + g;
+      if (t == 0) {
+        if (i < N) keys[i] = score_key(T.y[0]);
+        if (i + 8 < N) keys[i + 8] = score_key(T.y[1]);
+      }
     }
     __syncwarp();
   }

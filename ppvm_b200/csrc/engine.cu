@@ -853,6 +853,16 @@ void compose_tableau(int W, const DevOp* d, int L, HostTableau& t) {
   }
 }
 
+// The lattice of the term features (at most 22 x 22 on 512 qubits; L = 0: none).
+Lattice lattice_of(int L) {
+  Lattice lat;
+  std::memset(&lat, 0, sizeof(lat));
+  lat.L = L;
+  for (int q = 0; L > 0 && q < 64 * kMaxW; ++q)
+    if (q % L + 1 < L) lat.inner[q >> 6] |= 1ull << (q & 63);
+  return lat;
+}
+
 // ---- kernel enqueue (templated on W) ------------------------------------------------------------
 template <int W>
 struct K {
@@ -1114,7 +1124,7 @@ struct K {
     const Planes P = s->planes_view();
     uint32_t* keys = s->s_idx;  // cap entries, free outside the rotation pipeline
     const unsigned long long nub = std::max<unsigned long long>(s->n_host, 1);
-    k_score<W><<<grid_for(nub, 128, 8), 128, 0, s->stream>>>(P, s->d_ctrl, mw, L, layers_left, keys);
+    k_score<W><<<grid_for(nub, 128, 8), 128, 0, s->stream>>>(P, s->d_ctrl, mw, lattice_of(L), layers_left, keys);
     k_sel_init<<<1, 1, 0, s->stream>>>(s->d_ctrl, B, s->d_sel);
     if (bits == 11) {
       for (int shift : {21, 10, 0}) {
@@ -1135,7 +1145,7 @@ struct K {
   }
   static void features(ppvm_sum* s, int L, int layers_left, float* out) {
     k_features<W><<<grid_for(std::max<unsigned long long>(s->n_host, 1), 256, 8), 256, 0, s->stream>>>(
-        s->planes_view(), s->d_ctrl, L, layers_left, out);
+        s->planes_view(), s->d_ctrl, lattice_of(L), layers_left, out);
   }
 
   static void owz(ppvm_sum* s, int nblocks) {

@@ -78,15 +78,15 @@ ppvm_status mfail(ppvm_status s, const std::string& msg) {
 
 // FP32 master parameters -> packed BF16/FP32 device weights.
 __global__ void k_mlp_pack(const float* p, MlpWeights* w) {
-  for (int i = threadIdx.x; i < kMlpH * kMlpK1; i += blockDim.x) {
-    const int n = i / kMlpK1, k = i % kMlpK1;
+  for (int i = threadIdx.x; i < kMlpH * kLdW1; i += blockDim.x) {
+    const int n = i / kLdW1, k = i % kLdW1;
     w->w1[i] = __float2bfloat16_rn(k < kMlpIn ? p[kOffW1 + n * kMlpIn + k] : 0.0f);
   }
   for (int i = threadIdx.x; i < kMlpH * kMlpH; i += blockDim.x) {
     const int n = i / kMlpH, k = i % kMlpH;
     const __nv_bfloat16 b = __float2bfloat16_rn(p[kOffW2 + i]);
-    w->w2[i] = b;
-    w->w2t[k * kMlpH + n] = b;
+    w->w2[n * kLdW2 + k] = b;
+    w->w2t[k * kLdW2 + n] = b;
   }
   for (int i = threadIdx.x; i < kMlpH; i += blockDim.x) {
     w->b1[i] = p[kOffB1 + i];
@@ -108,14 +108,14 @@ __device__ __forceinline__ float adam_step(float p, float& m, float& v, float g,
 __device__ __forceinline__ void pack_param(MlpWeights* w, int i, float pi) {
   if (i < kOffB1) {
     const int n = (i - kOffW1) / kMlpIn, k = (i - kOffW1) % kMlpIn;
-    w->w1[n * kMlpK1 + k] = __float2bfloat16_rn(pi);
+    w->w1[n * kLdW1 + k] = __float2bfloat16_rn(pi);
   } else if (i < kOffW2) {
     w->b1[i - kOffB1] = pi;
   } else if (i < kOffB2) {
     const int n = (i - kOffW2) / kMlpH, k = (i - kOffW2) % kMlpH;
     const __nv_bfloat16 b = __float2bfloat16_rn(pi);
-    w->w2[n * kMlpH + k] = b;
-    w->w2t[k * kMlpH + n] = b;
+    w->w2[n * kLdW2 + k] = b;
+    w->w2t[k * kLdW2 + n] = b;
   } else if (i < kOffW3) {
     w->b2[i - kOffB2] = pi;
   } else if (i < kOffB3) {
@@ -316,7 +316,7 @@ __device__ __forceinline__ void train_tile(const MlpWeights& W, const SampleTile
     a[3] = pack_bf16(dz2[2 * kk + 1][2], dz2[2 * kk + 1][3]);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const __nv_bfloat16* wr = W.w2t + (8 * j + g) * kMlpH + 16 * kk;
+      const __nv_bfloat16* wr = W.w2t + (8 * j + g) * kLdW2 + 16 * kk;
       mma_bf16(dz1[j], a, *reinterpret_cast<const uint32_t*>(wr + 2 * t),
                *reinterpret_cast<const uint32_t*>(wr + 2 * t + 8));
     }
@@ -493,18 +493,20 @@ k_mlp_epoch(float* p_g, float* m_g, float* v_g, MlpWeights* Wg, const float* fea
             gq[3] += v[u].w;
           }
       }
+      float4 p4 = reinterpret_cast<float4*>(sp)[q], m4 = reinterpret_cast<float4*>(sm)[q],
+             v4 = reinterpret_cast<float4*>(sv)[q];
+      float pe[4] = {p4.x, p4.y, p4.z, p4.w}, me[4] = {m4.x, m4.y, m4.z, m4.w}, ve[4] = {v4.x, v4.y, v4.z, v4.w};
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const int i = 4 * q + e;
         if (i == kMlpParams) s_loss[0] = gq[e];
         if (i >= kMlpParams) continue;
-        float mi = sm[i], vi = sv[i];
-        const float pi = adam_step(sp[i], mi, vi, gq[e], lr, b1, b2, eps);
-        sm[i] = mi;
-        sv[i] = vi;
-        sp[i] = pi;
-        pack_param(&W, i, pi);
+        pe[e] = adam_step(pe[e], me[e], ve[e], gq[e], lr, b1, b2, eps);
+        pack_param(&W, i, pe[e]);
       }
+      reinterpret_cast<float4*>(sp)[q] = make_float4(pe[0], pe[1], pe[2], pe[3]);
+      reinterpret_cast<float4*>(sm)[q] = make_float4(me[0], me[1], me[2], me[3]);
+      reinterpret_cast<float4*>(sv)[q] = make_float4(ve[0], ve[1], ve[2], ve[3]);
     }
     __syncthreads();
     if (threadIdx.x == 0) lsum += s_loss[0];

@@ -9,7 +9,7 @@
 //
 // Parameters (FP32 master copy, flat): W1[64][8], b1[64], W2[64][64], b2[64], w3[64], b3.
 // The device copy used by the kernels: W1 as BF16 [64][16] (k padded), W2 as BF16 [64][64]
-// ([out][in]) and its transpose W2T [in][out] (for the backward pass), b1, b2, w3, b3 FP32.
+// ([out][in]), rows padded (below), and its transpose W2T [in][out] (for the backward pass), b1, b2, w3, b3 FP32.
 #pragma once
 
 #include <cuda_bf16.h>
@@ -20,6 +20,10 @@ namespace ppvm {
 constexpr int kMlpIn = 8;
 constexpr int kMlpK1 = 16;
 constexpr int kMlpH = 64;
+// Row strides of the packed BF16 matrices: 48 and 144 bytes, so that the 8 rows that a warp's B
+// fragment reads at once lie in different shared-memory banks (64-wide rows put them in one).
+constexpr int kLdW1 = kMlpK1 + 8;
+constexpr int kLdW2 = kMlpH + 8;
 constexpr int kMlpParams = kMlpH * kMlpIn + kMlpH + kMlpH * kMlpH + kMlpH + kMlpH + 1;  // 4801
 // offsets in the flat FP32 parameter vector
 constexpr int kOffW1 = 0, kOffB1 = kOffW1 + kMlpH * kMlpIn, kOffW2 = kOffB1 + kMlpH,
@@ -28,9 +32,9 @@ constexpr int kOffW1 = 0, kOffB1 = kOffW1 + kMlpH * kMlpIn, kOffW2 = kOffB1 + kM
 // Device weights (what k_adam writes after every step).  A multiple of 16 bytes: the training
 // kernels place vector-accessed arrays behind it.
 struct alignas(16) MlpWeights {
-  __nv_bfloat16 w1[kMlpH * kMlpK1];
-  __nv_bfloat16 w2[kMlpH * kMlpH];
-  __nv_bfloat16 w2t[kMlpH * kMlpH];
+  __nv_bfloat16 w1[kMlpH * kLdW1];
+  __nv_bfloat16 w2[kMlpH * kLdW2];
+  __nv_bfloat16 w2t[kMlpH * kLdW2];
   float b1[kMlpH], b2[kMlpH], w3[kMlpH];
   float b3;
 };
@@ -91,7 +95,7 @@ __device__ __forceinline__ void mlp_forward(const __nv_bfloat16* X, const MlpWei
     z1[j][1] = bh;
     z1[j][2] = bl;
     z1[j][3] = bh;
-    const __nv_bfloat16* wr = W.w1 + (8 * j + g) * kMlpK1;
+    const __nv_bfloat16* wr = W.w1 + (8 * j + g) * kLdW1;
     mma_bf16(z1[j], a, *reinterpret_cast<const uint32_t*>(wr + 2 * t),
              *reinterpret_cast<const uint32_t*>(wr + 2 * t + 8));
   }
@@ -119,7 +123,7 @@ __device__ __forceinline__ void mlp_forward(const __nv_bfloat16* X, const MlpWei
     }
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const __nv_bfloat16* wr = W.w2 + (8 * j + g) * kMlpH + 16 * kk;
+      const __nv_bfloat16* wr = W.w2 + (8 * j + g) * kLdW2 + 16 * kk;
       mma_bf16(z2[j], h, *reinterpret_cast<const uint32_t*>(wr + 2 * t),
                *reinterpret_cast<const uint32_t*>(wr + 2 * t + 8));
     }
@@ -145,13 +149,21 @@ __device__ __forceinline__ void mlp_forward(const __nv_bfloat16* X, const MlpWei
   T.y[1] = p1 + W.b3;
 }
 
+// The lattice of the term features: L x L, qubit r*L + c; inner: the qubits with a right neighbour in
+// their row (bit q set when q % L + 1 < L).
+struct Lattice {
+  int L;
+  uint64_t inner[8];
+};
+
 // Term features of learned truncation on an L x L lattice (qubit r*L + c), 8 values:
 //   weight/16, (log10|c| + 6)/6, layers_left/8, #X/8, #Y/8, #Z/8,
 //   nearest-neighbour bonds inside the support/8, weight*layers_left/64 (the support's
 //   overlap with the remaining RX layers, which act on every qubit).
+// Bonds are counted by words: the support against itself shifted by one qubit and by one row.
 template <int W>
-__device__ __forceinline__ void term_features(const uint64_t (&x)[W], const uint64_t (&z)[W], double c, int L,
-                                              int layers_left, float (&f)[kMlpIn]) {
+__device__ __forceinline__ void term_features(const uint64_t (&x)[W], const uint64_t (&z)[W], double c,
+                                              const Lattice& lat, int layers_left, float (&f)[kMlpIn]) {
   int nx = 0, ny = 0, nz = 0, bonds = 0;
 #pragma unroll
   for (int w = 0; w < W; ++w) {
@@ -159,17 +171,13 @@ __device__ __forceinline__ void term_features(const uint64_t (&x)[W], const uint
     ny += __popcll(x[w] & z[w]);
     nz += __popcll(~x[w] & z[w]);
   }
-  const int wt = nx + ny + nz;
+  const int wt = nx + ny + nz, L = lat.L;
+  if (L > 0) {
 #pragma unroll
-  for (int w = 0; w < W; ++w) {
-    uint64_t m = x[w] | z[w];
-    while (m) {
-      const int q = w * 64 + __ffsll((long long)m) - 1;
-      m &= m - 1;
-      const int col = L > 0 ? q % L : 0;
-      const int r = q + 1, d = q + L;
-      if (L > 0 && col + 1 < L && r < 64 * W && (((x[r >> 6] | z[r >> 6]) >> (r & 63)) & 1ull)) ++bonds;
-      if (L > 0 && d < 64 * W && (((x[d >> 6] | z[d >> 6]) >> (d & 63)) & 1ull)) ++bonds;
+    for (int w = 0; w < W; ++w) {
+      const uint64_t s = x[w] | z[w], up = w + 1 < W ? x[w + 1 < W ? w + 1 : w] | z[w + 1 < W ? w + 1 : w] : 0ull;
+      bonds += __popcll(s & (s >> 1 | up << 63) & lat.inner[w]);
+      bonds += __popcll(s & (s >> L | up << (64 - L)));  // 1 <= L <= 22
     }
   }
   const double a = fabs(c);
