@@ -41,7 +41,7 @@
 #include <vector>
 
 #include "../../include/ppvm_cuda.h"
-#include "tableau.cuh"
+#include "cta.cuh"
 
 namespace ppvm {
 void set_last_error(const std::string& msg);
@@ -127,194 +127,9 @@ __host__ __device__ inline unsigned long long grown_cap(unsigned long long cap, 
   return a > b ? a : b;
 }
 
-__host__ __device__ inline unsigned long long region_words(int W, unsigned long long cap, unsigned long long tsize) {
-  return (unsigned long long)(2 * W + 2) * cap + (cap + 1) / 2 + tsize;
-}
-
-template <int W>
-struct Region {
-  uint64_t* x;
-  uint64_t* z;
-  double* c;
-  unsigned long long* link;  // per term: its partner's coefficient, complemented (0 = none; all 0 between ops)
-  uint32_t* sidx;            // anticommuting terms: each warp's list at the start of its chunk of terms
-  unsigned long long* table;
-  unsigned long long cap, tsize;
-};
-
-// The region layout from its first word b (in the pool, or in shared memory).
-template <int W>
-__device__ __forceinline__ Region<W> region_at(uint64_t* b, unsigned long long cap, unsigned long long tsize) {
-  Region<W> r;
-  r.cap = cap;
-  r.tsize = tsize;
-  r.x = b;
-  r.z = b + (size_t)W * cap;
-  r.c = reinterpret_cast<double*>(b + (size_t)2 * W * cap);
-  r.link = reinterpret_cast<unsigned long long*>(b + (size_t)(2 * W + 1) * cap);
-  r.sidx = reinterpret_cast<uint32_t*>(b + (size_t)(2 * W + 2) * cap);
-  r.table = reinterpret_cast<unsigned long long*>(b + (size_t)(2 * W + 2) * cap + (cap + 1) / 2);
-  return r;
-}
 template <int W>
 __device__ __forceinline__ Region<W> region_of(uint64_t* pool, const BInst& I) {
   return region_at<W>(pool + I.off, I.cap, I.tsize);
-}
-
-template <int W>
-__device__ __forceinline__ void rload(const Region<W>& R, unsigned long long i, uint64_t (&x)[W], uint64_t (&z)[W]) {
-#pragma unroll
-  for (int w = 0; w < W; ++w) {
-    x[w] = R.x[(size_t)w * R.cap + i];
-    z[w] = R.z[(size_t)w * R.cap + i];
-  }
-}
-template <int W>
-__device__ __forceinline__ void rstore(const Region<W>& R, unsigned long long i, const uint64_t (&x)[W],
-                                       const uint64_t (&z)[W]) {
-#pragma unroll
-  for (int w = 0; w < W; ++w) {
-    R.x[(size_t)w * R.cap + i] = x[w];
-    R.z[(size_t)w * R.cap + i] = z[w];
-  }
-}
-// word w of a W-word array without dynamic register indexing
-template <int W>
-__device__ __forceinline__ uint64_t wsel(const uint64_t (&a)[W], unsigned w) {
-  uint64_t v = 0;
-#pragma unroll
-  for (int k = 0; k < W; ++k) v = (k == (int)w) ? a[k] : v;
-  return v;
-}
-template <int W>
-__device__ __forceinline__ void wflip(uint64_t (&a)[W], unsigned w, uint64_t m) {
-#pragma unroll
-  for (int k = 0; k < W; ++k)
-    if (k == (int)w) a[k] ^= m;
-}
-template <int W>
-__device__ __forceinline__ void wset_bits(uint64_t (&a)[W], unsigned w, uint64_t m) {
-#pragma unroll
-  for (int k = 0; k < W; ++k)
-    if (k == (int)w) a[k] |= m;
-}
-template <int W>
-__device__ __forceinline__ void wset(uint64_t (&a)[W], unsigned w, unsigned b, bool v) {
-#pragma unroll
-  for (int k = 0; k < W; ++k)
-    if (k == (int)w) a[k] = (a[k] & ~(1ull << b)) | ((uint64_t)v << b);
-}
-
-// Rotation on at most two qubits with axes (ax, az) (bit 0: q0, bit 1: q1).  For a word with
-// bits (x0, z0) at q0 and (x1, z1) at q1: whether it anticommutes, and eps of its child
-// (+1 exactly when the anticommuting qubit's single-qubit phase in G*P is -1, as rot_sign).
-struct RotBits {
-  bool anti;
-  bool eps_plus;
-};
-__device__ __forceinline__ RotBits rot_bits(const DevOp& d, bool x0, bool z0, bool x1, bool z1) {
-  const bool ax0 = d.ax & 1, az0 = d.az & 1, ax1 = d.two && (d.ax & 2), az1 = d.two && (d.az & 2);
-  RotBits r;
-  r.anti = ((x0 & az0) ^ (z0 & ax0)) ^ ((x1 & az1) ^ (z1 & ax1));
-  const bool m0 = (ax0 & !az0 & !x0 & z0) | (ax0 & az0 & x0 & !z0) | (!ax0 & az0 & x0 & z0);
-  const bool m1 = (ax1 & !az1 & !x1 & z1) | (ax1 & az1 & x1 & !z1) | (!ax1 & az1 & x1 & z1);
-  r.eps_plus = m0 | m1;
-  return r;
-}
-
-template <int W>
-__device__ __forceinline__ void op_bits(const DevOp& d, const uint64_t (&x)[W], const uint64_t (&z)[W], bool& x0,
-                                        bool& z0, bool& x1, bool& z1) {
-  x0 = (wsel<W>(x, d.w0) >> d.b0) & 1ull;
-  z0 = (wsel<W>(z, d.w0) >> d.b0) & 1ull;
-  x1 = (wsel<W>(x, d.w1) >> d.b1) & 1ull;
-  z1 = (wsel<W>(z, d.w1) >> d.b1) & 1ull;
-}
-
-template <int W>
-__device__ __forceinline__ void flip_gen(const DevOp& d, uint64_t (&x)[W], uint64_t (&z)[W]) {
-  if (d.ax & 1) wflip<W>(x, d.w0, 1ull << d.b0);
-  if (d.az & 1) wflip<W>(z, d.w0, 1ull << d.b0);
-  if (d.two) {
-    if (d.ax & 2) wflip<W>(x, d.w1, 1ull << d.b1);
-    if (d.az & 2) wflip<W>(z, d.w1, 1ull << d.b1);
-  }
-}
-
-// Bits of term i at the op's qubits, read from the planes (two words at most).
-template <int W>
-__device__ __forceinline__ void term_bits(const Region<W>& R, const DevOp& d, unsigned long long i, bool& x0,
-                                          bool& z0, bool& x1, bool& z1) {
-  x0 = (R.x[(size_t)d.w0 * R.cap + i] >> d.b0) & 1ull;
-  z0 = (R.z[(size_t)d.w0 * R.cap + i] >> d.b0) & 1ull;
-  x1 = z1 = false;
-  if (d.two) {
-    x1 = (R.x[(size_t)d.w1 * R.cap + i] >> d.b1) & 1ull;
-    z1 = (R.z[(size_t)d.w1 * R.cap + i] >> d.b1) & 1ull;
-  }
-}
-
-// One local op (Clifford, Clifford-angle rotation or diagonal noise) on a word, the rules of
-// the per-op pass (crates/ppvm-pauli-sum/src/sum/clifford.rs:37-221, sum/noise.rs:17-129).
-template <int W>
-__device__ __forceinline__ void local_op(const DevOp& d, uint64_t (&x)[W], uint64_t (&z)[W], double& c, bool& neg) {
-  bool x0, z0, x1, z1;
-  op_bits<W>(d, x, z, x0, z0, x1, z1);
-  switch (d.code) {
-    case C_PAULI_ERROR: {
-      const int k = (int)x0 | ((int)z0 << 1);
-      if (k == 1) c = __dmul_rn(c, d.f0);
-      else if (k == 2) c = __dmul_rn(c, d.f1);
-      else if (k == 3) c = __dmul_rn(c, d.f2);
-      return;
-    }
-    case C_DEP1:
-      if (x0 | z0) c = __dmul_rn(c, d.f0);
-      return;
-    case C_DEP2:
-      if (x0 | z0 | x1 | z1) c = __dmul_rn(c, d.f0);
-      return;
-    default: break;
-  }
-  const bool two = d.code == C_CNOT || d.code == C_CZ || d.code == C_CY || (d.code == C_ROTC && d.two);
-  if (!two) x1 = z1 = false;
-  cliff_rule<bool>(d, x0, z0, x1, z1, neg);
-  wset<W>(x, d.w0, d.b0, x0);
-  wset<W>(z, d.w0, d.b0, z0);
-  if (two) {
-    wset<W>(x, d.w1, d.b1, x1);
-    wset<W>(z, d.w1, d.b1, z1);
-  }
-}
-
-// ORs the block's masks into s_or (2W words) and returns them to every thread.
-template <int W>
-__device__ __forceinline__ void block_or(uint64_t (&ox)[W], uint64_t (&oz)[W], unsigned long long* s_or) {
-  __syncthreads();
-  if (threadIdx.x < 2 * W) s_or[threadIdx.x] = 0ull;
-  __syncthreads();
-#pragma unroll
-  for (int w = 0; w < W; ++w) {
-    const unsigned xl = __reduce_or_sync(kFull, (unsigned)ox[w]), xh = __reduce_or_sync(kFull, (unsigned)(ox[w] >> 32));
-    const unsigned zl = __reduce_or_sync(kFull, (unsigned)oz[w]), zh = __reduce_or_sync(kFull, (unsigned)(oz[w] >> 32));
-    if ((threadIdx.x & 31) == 0) {
-      atomicOr(&s_or[w], (unsigned long long)xh << 32 | xl);
-      atomicOr(&s_or[W + w], (unsigned long long)zh << 32 | zl);
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int w = 0; w < W; ++w) {
-    ox[w] = s_or[w];
-    oz[w] = s_or[W + w];
-  }
-}
-
-// The coefficient in a link word (its complement), and back: 0 means no link, so the one NaN
-// whose complement is 0 is linked as another NaN.
-__device__ __forceinline__ unsigned long long link_word(double c) {
-  const unsigned long long v = ~(unsigned long long)__double_as_longlong(c);
-  return v ? v : 1ull;
 }
 
 // One layer (or, with layer < 0, everything left) of every instance; CTA b = instance b.
@@ -324,12 +139,8 @@ k_batch(BInst* insts, const BOp* __restrict__ ops, const uint32_t* __restrict__ 
         const double* __restrict__ params, int layer, uint64_t* pool, unsigned long long resident_bytes,
         BSpare* spare, int tfac) {
   constexpr int NW = BLOCK / 32;
-  constexpr unsigned long long TILE = (unsigned long long)BLOCK * ITEMS;
-  constexpr int UB = 1;  // anticommuting terms a thread works on at a time
   __shared__ unsigned s_base[ITEMS * NW + 1];
-  __shared__ unsigned long long s_or[2 * W];
-  __shared__ unsigned s_cnt[NW], s_child[NW];  // per warp: its list's length, its children
-  __shared__ int s_perr;
+  __shared__ CtaShared<W, NW> sh;
   __shared__ unsigned long long s_off;
   extern __shared__ __align__(16) uint64_t s_region[];  // resident_bytes of dynamic shared memory
   BInst& I = insts[blockIdx.x];
@@ -360,16 +171,13 @@ k_batch(BInst* insts, const BOp* __restrict__ ops, const uint32_t* __restrict__ 
     for (unsigned long long t = threadIdx.x; t < R.cap; t += BLOCK) R.link[t] = 0ull;
     __syncthreads();
   }
-  if (threadIdx.x == 0) s_perr = 0;
+  if (threadIdx.x == 0) sh.perr = 0;
   const double* __restrict__ P = params + I.param_off;
   const double thr = I.thr;
   const unsigned long long maxw = I.maxw;
-  const bool wcap = maxw != ~0ull;
   unsigned long long N = I.n, tgu = 0;
   unsigned epoch = I.epoch;
   int err = 0;
-  const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const unsigned lt = (1u << lane) - 1u;
   // bits that some term may have in its X and Z planes: a rotation that none of them lets
   // anticommute changes nothing and is skipped (a Trotter list acts on every qubit, while the
   // observable's light cone covers a part of them)
@@ -383,50 +191,12 @@ k_batch(BInst* insts, const BOp* __restrict__ ops, const uint32_t* __restrict__ 
       sz[w] |= R.z[(size_t)w * R.cap + i];
     }
   }
-  block_or<W>(sx, sz, s_or);
+  block_or<W>(sx, sz, sh.orw);
   while (pc < end) {
     const BOp op = ops[pc];
     const uint32_t kind = bop_kind(op.h);
     if (kind == B_TRUNC) {
-      // stable in-place compaction: a tile's reads finish (inside tile_ranks) before its
-      // writes, and every write goes to a position at or below the word it came from
-      unsigned long long kept = 0;
-#pragma unroll
-      for (int w = 0; w < W; ++w) sx[w] = sz[w] = 0ull;
-      for (unsigned long long base = 0; base < N; base += TILE) {
-        uint64_t kx[ITEMS][W], kz[ITEMS][W];
-        double kc[ITEMS];
-        unsigned bal[ITEMS];
-#pragma unroll
-        for (int k = 0; k < ITEMS; ++k) {
-          const unsigned long long i = base + (unsigned long long)k * BLOCK + threadIdx.x;
-          bool keep = false;
-          if (i < N) {
-            rload<W>(R, i, kx[k], kz[k]);
-            kc[k] = R.c[i];
-            keep = !(fabs(kc[k]) < thr);
-            if (wcap) keep = keep && (weight<W>(kx[k], kz[k]) <= maxw);
-          }
-          bal[k] = __ballot_sync(kFull, keep);
-        }
-        const unsigned agg = tile_ranks<BLOCK, ITEMS>(bal, s_base);
-#pragma unroll
-        for (int k = 0; k < ITEMS; ++k)
-          if ((bal[k] >> lane) & 1u) {
-            const unsigned long long r = kept + s_base[k * NW + warp] + __popc(bal[k] & lt);
-            rstore<W>(R, r, kx[k], kz[k]);
-            R.c[r] = kc[k];
-#pragma unroll
-            for (int w = 0; w < W; ++w) {
-              sx[w] |= kx[k][w];
-              sz[w] |= kz[k][w];
-            }
-          }
-        kept += agg;
-        __syncthreads();
-      }
-      block_or<W>(sx, sz, s_or);
-      N = kept;
+      N = cta_truncate<W, BLOCK, ITEMS>(R, N, thr, maxw, s_base, sh.orw, sx, sz);
       ++pc;
       continue;
     }
@@ -449,188 +219,40 @@ k_batch(BInst* insts, const BOp* __restrict__ ops, const uint32_t* __restrict__ 
           sz[w] |= z[w];
         }
       }
-      block_or<W>(sx, sz, s_or);
+      block_or<W>(sx, sz, sh.orw);
       tgu += N * (unsigned long long)(j - pc);
       pc = j;
       continue;
     }
-    // ---- rotation exp(-i theta/2 G), G on op.d's one or two qubits ----
+    // ---- rotation exp(-i theta/2 G), G on the op's one or two qubits ----
     const DevOp d = bop_decode(op, P);
     const double sn = P[op.param], cs = P[op.param + 1];
-    {
-      bool x0 = (wsel<W>(sx, d.w0) >> d.b0) & 1ull, z0 = (wsel<W>(sz, d.w0) >> d.b0) & 1ull;
-      bool any = ((d.az & 1) && x0) || ((d.ax & 1) && z0);
-      if (d.two) {
-        bool x1 = (wsel<W>(sx, d.w1) >> d.b1) & 1ull, z1 = (wsel<W>(sz, d.w1) >> d.b1) & 1ull;
-        any = any || ((d.az & 2) && x1) || ((d.ax & 2) && z1);
-      }
-      if (!any) {  // no term anticommutes
-        tgu += N;
-        ++pc;
-        continue;
-      }
+    // a Trotter list acts on every qubit, while the observable's light cone covers a part of
+    // them: a rotation that no term's bits let anticommute is over at once
+    if (!rot_may_touch<W>(d, sx, sz)) {
+      tgu += N;
+      ++pc;
+      continue;
     }
     if (++epoch >= 0xFFFFu) {  // pair-table epochs wrapped: clear the table once
       for (unsigned long long t = threadIdx.x; t < R.tsize; t += BLOCK) R.table[t] = 0ull;
       __syncthreads();
       epoch = 1;
     }
-    // scan: each warp lists the anticommuting terms of its chunk, in order.  No barrier inside: a
-    // scan by block-wide tiles waited three times per 1024 terms
-    const unsigned n32 = (unsigned)N;
-    const unsigned chunk = ((n32 + NW - 1) / NW + 31u) & ~31u;
-    const unsigned lo = min(n32, warp * chunk), hi = min(n32, lo + chunk);
-    unsigned cnt = 0;
-    for (unsigned b0 = lo; b0 < hi; b0 += 32 * ITEMS) {
-      bool a[ITEMS];
-#pragma unroll
-      for (int k = 0; k < ITEMS; ++k) {
-        const unsigned i = b0 + k * 32 + lane;
-        a[k] = false;
-        if (i < hi) {
-          bool x0, z0, x1, z1;
-          term_bits<W>(R, d, i, x0, z0, x1, z1);
-          a[k] = rot_bits(d, x0, z0, x1, z1).anti;
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < ITEMS; ++k) {
-        const unsigned m = __ballot_sync(kFull, a[k]);
-        if (a[k]) R.sidx[lo + cnt + __popc(m & lt)] = b0 + k * 32 + lane;
-        cnt += __popc(m);
-      }
-    }
-    if (lane == 0) s_cnt[warp] = cnt;
-    if (!__syncthreads_or(cnt != 0)) {
+    CtaPlan<NW> p;
+    if (!cta_pair<W, BLOCK, ITEMS, false>(R, d, (unsigned)N, epoch, sh, p)) {
       tgu += N;
       ++pc;
       continue;
     }
-    unsigned pre[NW];  // lists before warp w's (every thread holds the same)
-    unsigned S = 0;
-#pragma unroll
-    for (int w = 0; w < NW; ++w) {
-      pre[w] = S;
-      S += s_cnt[w];
-    }
-    // term of rank r among the anticommuting ones
-    auto nth = [&](unsigned r) -> unsigned {
-      unsigned at = r;  // lists of the same chunk layout: warp w's starts at w * chunk
-#pragma unroll
-      for (int w = 1; w < NW; ++w)
-        if (r >= pre[w]) at = w * chunk + (r - pre[w]);
-      return R.sidx[at];
-    };
-    // pair: K and K^G (if both exist) meet at the same one of the two
-    const unsigned long long mask = R.tsize - 1;
-#pragma unroll 1
-    for (unsigned r0 = threadIdx.x; r0 < S; r0 += BLOCK * UB) {
-      // the loads of UB terms in flight together, down to the first table slot of each
-      unsigned idx[UB];
-      uint64_t x[UB][W], z[UB][W];
-      unsigned long long hh[UB], first[UB];
-#pragma unroll
-      for (int u = 0; u < UB; ++u) {
-        const unsigned r = r0 + u * BLOCK;
-        if (r < S) idx[u] = nth(r);
-      }
-#pragma unroll
-      for (int u = 0; u < UB; ++u)
-        if (r0 + u * BLOCK < S) rload<W>(R, idx[u], x[u], z[u]);
-#pragma unroll
-      for (int u = 0; u < UB; ++u)
-        if (r0 + u * BLOCK < S) {
-          uint64_t px[W], pz[W], kx[W], kz[W];
-#pragma unroll
-          for (int w = 0; w < W; ++w) {
-            px[w] = x[u][w];
-            pz[w] = z[u][w];
-          }
-          flip_gen<W>(d, px, pz);
-          // of the two keys, the one without the generator's bit on q0
-          const bool use_p = ((d.ax & 1 ? wsel<W>(x[u], d.w0) : wsel<W>(z[u], d.w0)) >> d.b0) & 1ull;
-#pragma unroll
-          for (int w = 0; w < W; ++w) {
-            kx[w] = use_p ? px[w] : x[u][w];
-            kz[w] = use_p ? pz[w] : z[u][w];
-          }
-          hh[u] = table_hash<W>(kx, kz);
-          first[u] = ld_volatile(&R.table[hh[u] & mask]);
-        }
-#pragma unroll
-      for (int u = 0; u < UB; ++u) {
-        if (r0 + u * BLOCK >= S) continue;
-        const unsigned i = idx[u];
-        const unsigned tag = (unsigned)(hh[u] >> 48) & 0xFFFFu;
-        const unsigned long long me = make_slot(epoch, tag, i);
-        unsigned long long slot = hh[u] & mask, probes = 0, cur = first[u];
-        while (true) {
-          if (slot_epoch(cur) != (epoch & 0xFFFFu)) {
-            const unsigned long long prev = atomicCAS(&R.table[slot], cur, me);
-            if (prev == cur) break;
-            cur = prev;  // taken meanwhile: examine what is there now
-            continue;
-          }
-          if (slot_tag(cur) == tag) {
-            const unsigned j = slot_idx(cur);
-            uint64_t px[W], pz[W], jx[W], jz[W];
-#pragma unroll
-            for (int w = 0; w < W; ++w) {
-              px[w] = x[u][w];
-              pz[w] = z[u][w];
-            }
-            flip_gen<W>(d, px, pz);
-            rload<W>(R, j, jx, jz);
-            bool eq = true;
-#pragma unroll
-            for (int w = 0; w < W; ++w) eq &= (jx[w] == px[w]) & (jz[w] == pz[w]);
-            if (eq) {
-              R.link[i] = link_word(R.c[j]);
-              R.link[j] = link_word(R.c[i]);
-              break;
-            }
-          }
-          slot = (slot + 1) & mask;
-          if (++probes > mask) {
-            s_perr = 1;  // cannot happen with tsize >= 2 * cap; reported, not trapped
-            break;
-          }
-          cur = ld_volatile(&R.table[slot]);
-        }
-      }
-    }
-    __syncthreads();
-    if (s_perr) {
+    if (sh.perr) {
       err = kErrProbe;
       break;
     }
-    // each warp counts the children of its share of the ranks; their places follow from the
-    // counts, and nothing is written before the total is known to fit
-    const unsigned share = ((S + NW - 1) / NW + 31u) & ~31u;
-    const unsigned rlo = min(S, warp * share), rhi = min(S, rlo + share);
-    unsigned kids = 0;
-    for (unsigned r0 = rlo + lane; r0 < rhi; r0 += 32 * UB) {
-      unsigned idx[UB];
-#pragma unroll
-      for (int u = 0; u < UB; ++u)
-        if (r0 + u * 32 < rhi) idx[u] = nth(r0 + u * 32);
-#pragma unroll
-      for (int u = 0; u < UB; ++u)
-        if (r0 + u * 32 < rhi) kids += R.link[idx[u]] == 0ull;
-    }
-    kids = __reduce_add_sync(kFull, kids);
-    if (lane == 0) s_child[warp] = kids;
-    __syncthreads();
-    unsigned C = 0, at = 0;
-#pragma unroll
-    for (int w = 0; w < NW; ++w) {
-      if (w < (int)warp) at += s_child[w];
-      C += s_child[w];
-    }
-    if (N + C > R.cap) {
+    if (N + p.C > R.cap) {
       // a larger region from the pool's spare end: terms, links and lists move over, the table
       // starts empty (its entries of this op are no longer needed)
-      const unsigned long long ncap = grown_cap(R.cap, N + C);
+      const unsigned long long ncap = grown_cap(R.cap, N + p.C);
       const unsigned long long nts = next_pow2_ull(tfac * ncap < 64 ? 64 : tfac * ncap);
       if (threadIdx.x == 0) {
         const unsigned long long words = (region_words(W, ncap, nts) + 31) & ~31ull;
@@ -642,7 +264,7 @@ k_batch(BInst* insts, const BOp* __restrict__ ops, const uint32_t* __restrict__ 
       }
       __syncthreads();
       if (s_off >= spare->end) {  // the host lays the pool out anew
-        if (threadIdx.x == 0) I.need = N + C;
+        if (threadIdx.x == 0) I.need = N + p.C;
         err = kErrCapacity;
         break;
       }
@@ -669,70 +291,11 @@ k_batch(BInst* insts, const BOp* __restrict__ ops, const uint32_t* __restrict__ 
       resident = false;
       __syncthreads();
     }
-    // apply: parents in place, partnerless children appended in parent order
-    for (unsigned r0 = rlo; r0 < rhi; r0 += 32 * UB) {  // loads of UB terms together, then stores
-      unsigned idx[UB];
-      double c[UB];
-      unsigned long long lw[UB];
-      bool own[UB], other[UB];  // eps of the term's child, of its partner's, is +1
-#pragma unroll
-      for (int u = 0; u < UB; ++u) {
-        const unsigned r = r0 + u * 32 + lane;
-        if (r < rhi) idx[u] = nth(r);
-      }
-#pragma unroll
-      for (int u = 0; u < UB; ++u) {
-        own[u] = other[u] = false;
-        if (r0 + u * 32 + lane < rhi) {
-          c[u] = R.c[idx[u]];
-          lw[u] = R.link[idx[u]];
-          bool x0, z0, x1, z1;
-          term_bits<W>(R, d, idx[u], x0, z0, x1, z1);
-          own[u] = rot_bits(d, x0, z0, x1, z1).eps_plus;
-          // the partner's key is K^G: its eps from this term's bits with G's bits flipped
-          x0 ^= (bool)(d.ax & 1);
-          z0 ^= (bool)(d.az & 1);
-          if (d.two) {
-            x1 ^= (bool)(d.ax & 2);
-            z1 ^= (bool)(d.az & 2);
-          }
-          other[u] = rot_bits(d, x0, z0, x1, z1).eps_plus;
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < UB; ++u) {
-        bool child = false;
-        if (r0 + u * 32 + lane < rhi) {
-          double nc = __dmul_rn(c[u], cs);
-          if (lw[u]) {
-            nc = __dadd_rn(nc, __dmul_rn(__longlong_as_double((long long)~lw[u]), (other[u] ? 1.0 : -1.0) * sn));
-            R.link[idx[u]] = 0ull;
-          } else {
-            child = true;
-          }
-          R.c[idx[u]] = nc;
-        }
-        const unsigned m = __ballot_sync(kFull, child);
-        if (child) {
-          const unsigned long long pos = N + at + __popc(m & lt);
-          uint64_t x[W], z[W];
-          rload<W>(R, idx[u], x, z);
-          flip_gen<W>(d, x, z);
-          rstore<W>(R, pos, x, z);
-          R.c[pos] = __dmul_rn(c[u], (own[u] ? 1.0 : -1.0) * sn);
-        }
-        at += __popc(m);
-      }
-    }
-    if (d.ax & 1) wset_bits<W>(sx, d.w0, 1ull << d.b0);
-    if (d.az & 1) wset_bits<W>(sz, d.w0, 1ull << d.b0);
-    if (d.two) {
-      if (d.ax & 2) wset_bits<W>(sx, d.w1, 1ull << d.b1);
-      if (d.az & 2) wset_bits<W>(sz, d.w1, 1ull << d.b1);
-    }
+    cta_apply<W, BLOCK, false>(R, d, sn, cs, N, p);
+    join_gen<W>(d, sx, sz);
     __syncthreads();
     tgu += N;
-    N += C;
+    N += p.C;
     ++pc;
   }
   __syncthreads();

@@ -28,6 +28,7 @@
 #include "loss.cuh"
 #include "noise.cuh"
 #include "shard.cuh"
+#include "small.cuh"
 
 using namespace ppvm;
 
@@ -96,12 +97,12 @@ struct ProfLaunch {
 
 enum Family {
   F_SCAN = 0, F_PAIR, F_APPLY, F_COMMIT, F_CLIFF, F_TRUNC, F_READ,
-  F_RUN_CLASSIFY, F_RUN_ORDER, F_RUN_SCATTER, F_RUN_GROUPS, F_RUN_PLACE, F_TABLEAU, F_LOSS, F_COUNT
+  F_RUN_CLASSIFY, F_RUN_ORDER, F_RUN_SCATTER, F_RUN_GROUPS, F_RUN_PLACE, F_TABLEAU, F_LOSS, F_SMALL, F_COUNT
 };
 const char* kFamilyNames[F_COUNT] = {"rot_scan", "rot_pair", "rot_apply", "rot_commit",
                                      "clifford", "truncate", "readout",
                                      "run_classify", "run_order", "run_scatter", "run_groups", "run_place",
-                                     "tableau", "loss"};
+                                     "tableau", "loss", "small"};
 
 // One pinned host chunk and its device twin: per-call uploads (op descriptors, run
 // descriptors, tableaux) are packed here and copied with truly asynchronous copies.
@@ -1119,6 +1120,20 @@ struct K {
     return PPVM_OK;
   }
 
+  // ops[0..nops) (small ops, list indices from op0) on a sum of at most kSmallStart terms.
+  static ppvm_status small(ppvm_sum* s, const SmallOp* d_ops, int nops, int op0) {
+    static unsigned long long attr_set = 0;  // one bit per device
+    if (!((attr_set >> s->device) & 1ull)) {
+      CUDA_TRY(cudaFuncSetAttribute(k_small<W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)SmallFor<W>::smem));
+      attr_set |= 1ull << s->device;
+    }
+    ProfScope ps(s, F_SMALL, op0, nops);
+    launch(k_small<W>, 1, kSmallBlock, SmallFor<W>::smem, s->stream, s->planes_view(), s->d_ctrl, d_ops,
+           (unsigned)nops, op0, s->thr, s->maxw, s->d_log);
+    return PPVM_OK;
+  }
+
   // Term-budget truncation: priority keys, radix select of the budget-th largest, compaction.
   static void budget(ppvm_sum* s, unsigned long long B, const MlpWeights* mw, int L, int layers_left, int bits) {
     const Planes P = s->planes_view();
@@ -1233,6 +1248,10 @@ ppvm_status enqueue_tableau(ppvm_sum* s, const HostTableau& t, int op0, int nops
   DISPATCH_W_RET(s->W, tableau(s, t, op0, nops, trunc_op));
 }
 
+ppvm_status enqueue_small(ppvm_sum* s, const SmallOp* d_ops, int nops, int op0) {
+  DISPATCH_W_RET(s->W, small(s, d_ops, nops, op0));
+}
+
 int test_words_of(int W, const Gen& g) {
   int n = 0;
   for (int w = 0; w < W; ++w) n += (g.gz[w] != 0) + (g.gx[w] != 0);
@@ -1270,6 +1289,27 @@ bool tab_ok(const ppvm_sum* s, const DevOp& d) {
   if (!is_cliff_code(d.code)) return false;
   if (!s->lossy) return true;
   return !(d.code == C_CNOT || d.code == C_CZ || d.code == C_CY || (d.code == C_ROTC && d.two));
+}
+
+// Gates of the fused run that starts at ops[i] (RX or RZ rotations on distinct qubits, none at a
+// Clifford angle; at most max_gates), or 0 if none of at least two gates does.  Not on a lossy
+// sum: its correlated loss channel sums up to three children per key in the reference's term
+// order, which a fused run (same terms, another order) would change in the last bit.
+int run_length(const ppvm_sum* s, const ppvm_op* ops, size_t n_ops, size_t i, int max_gates) {
+  const ppvm_op& op = ops[i];
+  if (!(op.code == PPVM_OP_RX || op.code == PPVM_OP_RZ) || (s->flags & PPVM_FLAG_EXACT_ORDER) || s->lossy ||
+      s->npres || max_gates < 2)
+    return 0;
+  uint64_t Q[kMaxW] = {};
+  size_t j = i;
+  while (j < n_ops && (int)(j - i) < max_gates) {
+    const ppvm_op& o = ops[j];
+    if (o.flags != 0 || o.code != op.code || is_clifford_angle(s, o.theta)) break;
+    if ((Q[o.q0 >> 6] >> (o.q0 & 63)) & 1ull) break;  // qubit repeats: end the run
+    Q[o.q0 >> 6] |= 1ull << (o.q0 & 63);
+    ++j;
+  }
+  return j - i >= 2 ? (int)(j - i) : 0;
 }
 
 // Enqueues ops[start..n) (gate-list indices start..n).  Generators of explicit Pauli rotations
@@ -1363,34 +1403,27 @@ ppvm_status enqueue(ppvm_sum* s, const ppvm_op* ops, size_t n_ops, size_t start,
       run.push_back(d);
       continue;
     }
-    // fused run of single-qubit RX (or RZ) rotations on distinct qubits.  Not on a lossy sum:
-    // its correlated loss channel sums up to three children per key in the reference's term
-    // order, which a fused run (same terms, another order) would change in the last bit.
+    // fused run of single-qubit RX (or RZ) rotations on distinct qubits
     const auto cap_it = s->run_cap.find(i);
     int max_gates = cap_it == s->run_cap.end() ? kRunMaxGates : cap_it->second;
     if (max_gates < 0) {  // the run starting here goes gate by gate: -max_gates gates
       per_gate_end = i + (size_t)(-max_gates);
       max_gates = 0;
     }
-    const bool fusable = (op.code == PPVM_OP_RX || op.code == PPVM_OP_RZ) &&
-                         !(s->flags & PPVM_FLAG_EXACT_ORDER) && !s->lossy && s->npres == 0 && max_gates >= 2 &&
-                         i >= per_gate_end;
-    if (fusable) {
-      RunDesc rd;
-      std::memset(&rd, 0, sizeof(rd));
-      rd.cls = op.code == PPVM_OP_RX ? 0 : 1;
-      size_t j = i;
-      while (j < n_ops && (int)(j - i) < max_gates) {
-        const ppvm_op& o = ops[j];
-        if (o.flags != 0 || o.code != op.code || is_clifford_angle(s, o.theta)) break;
-        if ((rd.Q[o.q0 >> 6] >> (o.q0 & 63)) & 1ull) break;  // qubit repeats: end the run
-        rd.Q[o.q0 >> 6] |= 1ull << (o.q0 & 63);
-        rd.q[rd.L] = o.q0;
-        trig.get(o.theta, rd.sn[rd.L], rd.cs[rd.L]);
-        ++rd.L;
-        ++j;
-      }
-      if (rd.L >= 2) {
+    {
+      const int len = i >= per_gate_end ? run_length(s, ops, n_ops, i, max_gates) : 0;
+      if (len) {
+        RunDesc rd;
+        std::memset(&rd, 0, sizeof(rd));
+        rd.cls = op.code == PPVM_OP_RX ? 0 : 1;
+        rd.L = (uint32_t)len;
+        const size_t j = i + (size_t)len;
+        for (int k = 0; k < len; ++k) {
+          const ppvm_op& o = ops[i + k];
+          rd.Q[o.q0 >> 6] |= 1ull << (o.q0 & 63);
+          rd.q[k] = o.q0;
+          trig.get(o.theta, rd.sn[k], rd.cs[k]);
+        }
         PPVM_TRY(flush(-1, nullptr));
         const int trunc_op =
             (j < n_ops && ops[j].code == PPVM_OP_TRUNCATE && ops[j].flags == 0 && s->maxlw == UINT64_MAX) ? (int)j
@@ -1412,6 +1445,94 @@ ppvm_status enqueue(ppvm_sum* s, const ppvm_op* ops, size_t n_ops, size_t start,
   return PPVM_OK;
 }
 
+// PPVM_SMALL=never: small sums take the pipelines from the first op on (for the tests).
+bool small_enabled() {
+  static const bool v = [] {
+    const char* e = std::getenv("PPVM_SMALL");
+    return !(e && std::strcmp(e, "never") == 0);
+  }();
+  return v;
+}
+
+// Applies the head of ops[start..n_ops) with k_small while the sum is small; *start moves past what
+// was applied.  Launches of up to kSmallOps ops, each followed by a synchronisation (the host
+// goes on from where the kernel stopped).  It is not worth it for sums above kSmallStart terms,
+// which soon outgrow one CTA, and it leaves long stretches of local ops to the composed pass.
+ppvm_status run_small(ppvm_sum* s, const ppvm_op* ops, size_t n_ops, size_t* start) {
+  if (!small_enabled() || s->lossy || s->npres) return PPVM_OK;
+  SinCosMemo trig;
+  std::vector<SmallOp> rec;
+  while (*start < n_ops && s->n_host > 0 && s->n_host <= kSmallStart) {
+    rec.clear();
+    size_t i = *start, run_end = 0;
+    while (i < n_ops && rec.size() < (size_t)kSmallOps) {
+      const ppvm_op& op = ops[i];
+      if (op.flags != 0 || op.code == kOpPauliError2) break;
+      SmallOp r;
+      std::memset(&r, 0, sizeof(r));
+      if (op.code == PPVM_OP_TRUNCATE) {
+        r.kind = S_TRUNC;
+      } else if (op.code == PPVM_OP_AMPLITUDE_DAMPING) {
+        r.kind = S_DAMP;
+        r.d.w0 = r.d.w1 = (uint16_t)(op.q0 >> 6);
+        r.d.b0 = r.d.b1 = (uint16_t)(op.q0 & 63);
+        r.a = op.theta;
+        r.b = 1.0 - op.theta;
+        r.c = std::sqrt(r.b);
+      } else if (is_local(s, op)) {
+        size_t j = i;
+        while (j < n_ops && j - i <= (size_t)kSmallLocal && ops[j].flags == 0 && is_local(s, ops[j])) ++j;
+        if (j - i > (size_t)kSmallLocal) break;
+        for (; i < j; ++i) {
+          r.kind = S_LOCAL;
+          r.d = to_devop(ops[i]);
+          rec.push_back(r);
+        }
+        continue;
+      } else {
+        r.kind = S_ROT;
+        Gen g;  // axes from the generator
+        gen_from_op(s, op, g);
+        const bool two = op.code == PPVM_OP_RXX || op.code == PPVM_OP_RYY || op.code == PPVM_OP_RZZ;
+        const uint32_t q1 = two ? op.q1 : op.q0;
+        r.d.w0 = (uint16_t)(op.q0 >> 6), r.d.b0 = (uint16_t)(op.q0 & 63);
+        r.d.w1 = (uint16_t)(q1 >> 6), r.d.b1 = (uint16_t)(q1 & 63);
+        r.d.two = two ? 1 : 0;
+        const bool gx = (g.gx[op.q0 >> 6] >> (op.q0 & 63)) & 1ull, gz = (g.gz[op.q0 >> 6] >> (op.q0 & 63)) & 1ull;
+        r.d.ax = (uint16_t)(gx ? (two ? 3 : 1) : 0);
+        r.d.az = (uint16_t)(gz ? (two ? 3 : 1) : 0);
+        trig.get(op.theta, r.a, r.b);
+        if (i >= run_end) {
+          const int len = run_length(s, ops, n_ops, i, kRunMaxGates);
+          if (len) {
+            if (rec.size() + (size_t)len > (size_t)kSmallOps) break;  // a run is applied whole
+            r.run = (uint32_t)len;
+            run_end = i + (size_t)len;
+          }
+        }
+      }
+      rec.push_back(r);
+      ++i;
+    }
+    if (rec.empty()) return PPVM_OK;
+    stage_reset(s);
+    const void* d_ops = nullptr;
+    PPVM_TRY(stage_put(s, rec.data(), sizeof(SmallOp) * rec.size(), &d_ops));
+    PPVM_TRY(enqueue_small(s, static_cast<const SmallOp*>(d_ops), (int)rec.size(), (int)*start));
+    CUDA_TRY(cudaGetLastError());
+    const bool all = *start + rec.size() == n_ops;
+    PPVM_TRY(sync_state(s, all ? n_ops : 0));
+    if (s->h_ctrl->err) {
+      s->poisoned = true;
+      return fail(PPVM_ECUDA, "device error " + std::to_string(s->h_ctrl->err) + " in a small op list");
+    }
+    s->n_host = s->n_ub = s->h_ctrl->n;
+    *start += s->h_ctrl->small_pc;
+    if (s->h_ctrl->small_pc < rec.size()) return PPVM_OK;  // outgrown, or a run too wide
+  }
+  return PPVM_OK;
+}
+
 // Runs a validated op list with capacity growth and replay.
 ppvm_status run_list(ppvm_sum* s, const ppvm_op* ops, size_t n_ops, const std::vector<Gen>& gens) {
   if (s->poisoned) return fail(PPVM_ECUDA, "sum is in an error state from an earlier failure");
@@ -1420,6 +1541,12 @@ ppvm_status run_list(ppvm_sum* s, const ppvm_op* ops, size_t n_ops, const std::v
   std::vector<int> test_words(n_ops, 0);
   size_t start = 0;
   s->run_cap.clear();
+  PPVM_TRY(run_small(s, ops, n_ops, &start));
+  if (s->prof) prof_collect(s, test_words);
+  if (start == n_ops) {
+    s->last_nops = n_ops;
+    return PPVM_OK;
+  }
   // every failed attempt grows the capacity or cuts a run, so the loop ends; the bound only
   // turns a logic error into a status
   const size_t max_attempts = 64 + 8 * n_ops;

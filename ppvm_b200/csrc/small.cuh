@@ -1,0 +1,373 @@
+// small.cuh — op lists on small sums: one CTA, one launch, the sum in shared memory.
+//
+// A sum of a few hundred terms leaves the GPU idle, and every kernel of the per-op pipelines is then
+// a few microseconds of launch and memory latency: a 20-qubit Trotter chain of 410 ops took
+// 2.2 ms for at most 900 terms, a single-gate call 40 us.  k_small interprets the list in one CTA
+// (cta.cuh), at block-barrier cost per op, as long as the terms fit into shared memory.  An op
+// that would outgrow it, or one it does not know, ends the launch before anything of that op
+// is written; the host goes on from there with the pipelines, which are the faster from about
+// that size on (they spread over all SMs).
+//
+// Every op gives the pipelines' terms, coefficients and order: rotations, damping, Cliffords,
+// diagonal noise and TRUNCATE keep the reference's IndexMap order; a fused run (rotations on
+// distinct qubits, RX or RZ, in a sum without exact order) is applied gate by gate and its
+// terms are then sorted as the fused run writes them: untouched terms in order, then the
+// groups by their first member, members by coordinate (runs.cuh).
+#pragma once
+
+#include "cta.cuh"
+#include "runs.cuh"
+
+namespace ppvm {
+
+constexpr int kSmallBlock = 512;
+constexpr int kSmallItems = 4;
+constexpr int kSmallOps = 2048;                  // ops per launch
+constexpr unsigned long long kSmallStart = 512;  // sums of more terms take the pipelines at once
+constexpr int kSmallLocal = 128;                 // longer stretches of local ops: the composed pass
+
+// Terms the region holds: as many as fit into shared memory with the pair table and the sort keys.
+template <int W>
+struct SmallFor {
+  static constexpr unsigned cap = W <= 3 ? 2048 : 1024;
+  static constexpr size_t smem = 8 * ((size_t)(2 * W + 2) * cap + cap / 2 + 2 * cap) + 8 * (size_t)cap;
+};
+
+enum SKind : uint32_t { S_ROT = 0, S_LOCAL, S_TRUNC, S_DAMP };
+
+struct alignas(8) SmallOp {
+  DevOp d;       // qubits, axes; local ops: code and factors
+  uint32_t kind;
+  uint32_t run;  // gates of the fused run that starts here (0: none starts)
+  double a, b, c;  // rotation: sin, cos; damping: gamma, 1 - gamma, sqrt(1 - gamma)
+};
+
+// The run's qubits, and whether every group fits the fused run (at most kRunMaxK coordinates).
+template <int W>
+__device__ __forceinline__ bool small_run_begin(const Region<W>& R, unsigned N, const SmallOp* ops, unsigned len,
+                                                bool rx, unsigned long long* s_q, uint64_t (&Q)[W]) {
+  __syncthreads();
+  if (threadIdx.x < W) s_q[threadIdx.x] = 0ull;
+  __syncthreads();
+  for (unsigned j = threadIdx.x; j < len; j += kSmallBlock) atomicOr(&s_q[ops[j].d.w0], 1ull << ops[j].d.b0);
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < W; ++w) Q[w] = s_q[w];
+  bool wide = false;
+  for (unsigned i = threadIdx.x; i < N; i += kSmallBlock) {
+    unsigned k = 0;
+#pragma unroll
+    for (int w = 0; w < W; ++w) k += __popcll((rx ? R.z : R.x)[(size_t)w * R.cap + i] & Q[w]);
+    wide |= k > (unsigned)kRunMaxK;
+  }
+  return !__syncthreads_or(wide);
+}
+
+// The sum's terms after the gates of a run that began with N0 terms, sorted as the fused run writes
+// them.  The original terms still hold indices below N0 (gates only append), so a group's
+// first member is the smallest of them with the group's key.
+template <int W>
+__device__ __forceinline__ void small_run_sort(const Region<W>& R, unsigned N0, unsigned N, bool rx,
+                                               const uint64_t (&Q)[W], unsigned epoch, unsigned long long* key) {
+  const unsigned long long mask = R.tsize - 1;
+  const uint64_t* V = rx ? R.z : R.x;
+  const uint64_t* F = rx ? R.x : R.z;
+  auto group = [&](unsigned i, uint64_t (&v)[W], uint64_t (&f)[W]) {
+    unsigned k = 0;
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+      v[w] = V[(size_t)w * R.cap + i];
+      f[w] = F[(size_t)w * R.cap + i] & ~(v[w] & Q[w]);
+      k += __popcll(v[w] & Q[w]);
+    }
+    return k;
+  };
+  // the slot of a group holds the smallest index seen of it
+  for (unsigned i = threadIdx.x; i < N0; i += kSmallBlock) {
+    uint64_t v[W], f[W];
+    if (group(i, v, f) == 0) continue;
+    const uint64_t h = table_hash<W>(v, f);
+    const unsigned tag = (unsigned)(h >> 48) & 0xFFFFu;
+    const unsigned long long me = make_slot(epoch, tag, i);
+    unsigned long long slot = h & mask, cur = ld_volatile(&R.table[slot]);
+    for (unsigned long long probes = 0; probes <= mask;) {
+      if (slot_epoch(cur) != (epoch & 0xFFFFu)) {
+        const unsigned long long prev = atomicCAS(&R.table[slot], cur, me);
+        if (prev == cur) break;
+        cur = prev;
+        continue;
+      }
+      if (slot_tag(cur) == tag) {
+        uint64_t jv[W], jf[W];
+        group(slot_idx(cur), jv, jf);
+        bool eq = true;
+#pragma unroll
+        for (int w = 0; w < W; ++w) eq &= (jv[w] == v[w]) & (jf[w] == f[w]);
+        if (eq) {
+          atomicMin(&R.table[slot], me);  // same epoch and tag: the smaller index
+          break;
+        }
+      }
+      slot = (slot + 1) & mask;
+      ++probes;
+      cur = ld_volatile(&R.table[slot]);
+    }
+  }
+  __syncthreads();
+  unsigned n2 = 1;
+  while (n2 < N) n2 <<= 1;
+  // sort keys: untouched by index; touched after them by (first member, coordinate); the term's
+  // index below
+  for (unsigned i = threadIdx.x; i < n2; i += kSmallBlock) {
+    unsigned long long k = ~0ull;
+    if (i < N) {
+      uint64_t v[W], f[W];
+      unsigned hi = i;
+      if (group(i, v, f)) {
+        const uint64_t h = table_hash<W>(v, f);
+        const unsigned tag = (unsigned)(h >> 48) & 0xFFFFu;
+        unsigned long long slot = h & mask;
+        unsigned first = 0;
+        for (unsigned long long probes = 0; probes <= mask; ++probes) {  // found: the group has an original member
+          const unsigned long long cur = R.table[slot];
+          if (slot_epoch(cur) == (epoch & 0xFFFFu) && slot_tag(cur) == tag) {
+            uint64_t jv[W], jf[W];
+            group(slot_idx(cur), jv, jf);
+            bool eq = true;
+#pragma unroll
+            for (int w = 0; w < W; ++w) eq &= (jv[w] == v[w]) & (jf[w] == f[w]);
+            if (eq) {
+              first = slot_idx(cur);
+              break;
+            }
+          }
+          slot = (slot + 1) & mask;
+        }
+        unsigned c = 0, t = 0;
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+          const uint64_t fw = F[(size_t)w * R.cap + i];
+          uint64_t m = v[w] & Q[w];
+          while (m) {
+            const int b = __ffsll((long long)m) - 1;
+            c |= (unsigned)((fw >> b) & 1ull) << t;
+            ++t;
+            m &= m - 1;
+          }
+        }
+        hi = 1u << 30 | first << kRunMaxK | c;
+      }
+      k = (unsigned long long)hi << 32 | i;
+    }
+    key[i] = k;
+  }
+  __syncthreads();
+  for (unsigned size = 2; size <= n2; size <<= 1)
+    for (unsigned d = size >> 1; d; d >>= 1) {
+      for (unsigned e = threadIdx.x; e < n2 / 2; e += kSmallBlock) {
+        const unsigned a = ((e & ~(d - 1)) << 1) | (e & (d - 1)), b = a | d;
+        const unsigned long long ka = key[a], kb = key[b];
+        if ((ka > kb) == ((a & size) == 0)) {
+          key[a] = kb;
+          key[b] = ka;
+        }
+      }
+      __syncthreads();
+    }
+  // every term to its place (all reads before all writes)
+  constexpr int PER = (int)(SmallFor<W>::cap / kSmallBlock);
+  uint64_t x[PER][W], z[PER][W];
+  double c[PER];
+#pragma unroll
+  for (int u = 0; u < PER; ++u) {
+    const unsigned i = u * kSmallBlock + threadIdx.x;
+    if (i < N) {
+      const unsigned from = (unsigned)key[i];
+      rload<W>(R, from, x[u], z[u]);
+      c[u] = R.c[from];
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < PER; ++u) {
+    const unsigned i = u * kSmallBlock + threadIdx.x;
+    if (i < N) {
+      rstore<W>(R, i, x[u], z[u]);
+      R.c[i] = c[u];
+    }
+  }
+  __syncthreads();
+}
+
+template <int W>
+__global__ void __launch_bounds__(kSmallBlock)
+k_small(Planes P, Ctrl* ctrl, const SmallOp* __restrict__ ops, unsigned nops, int op0, double thr,
+        unsigned long long maxw, OpLog* log) {
+  pdl_wait();
+  constexpr int BLOCK = kSmallBlock, ITEMS = kSmallItems, NW = BLOCK / 32;
+  __shared__ unsigned s_base[ITEMS * NW + 1];
+  __shared__ CtaShared<W, NW> sh;
+  __shared__ unsigned long long s_q[W];
+  // the ops from index s0 on: an op read from global memory would cost its latency each time
+  constexpr unsigned OPS = 64;
+  __shared__ SmallOp s_ops[OPS];
+  unsigned s0 = 0;
+  auto fetch = [&](unsigned at) {
+    __syncthreads();
+    s0 = at;
+    const unsigned n = min(OPS, nops - at) * (unsigned)(sizeof(SmallOp) / 8);
+    for (unsigned t = threadIdx.x; t < n; t += BLOCK)
+      reinterpret_cast<unsigned long long*>(s_ops)[t] = reinterpret_cast<const unsigned long long*>(ops + at)[t];
+    __syncthreads();
+  };
+  extern __shared__ __align__(16) uint64_t s_small[];
+  constexpr unsigned CAP = SmallFor<W>::cap;
+  if (ld_volatile_int(&ctrl->err)) return;
+  const Region<W> R = region_at<W>(s_small, CAP, 2 * CAP);
+  unsigned long long* keys = reinterpret_cast<unsigned long long*>(R.table + 2 * CAP);
+  unsigned N = (unsigned)ld_volatile(&ctrl->n);
+  uint64_t sx[W], sz[W];
+#pragma unroll
+  for (int w = 0; w < W; ++w) sx[w] = sz[w] = 0ull;
+  if (N > CAP) return;  // the host asks for at most kSmallStart
+  for (unsigned i = threadIdx.x; i < N; i += BLOCK) {
+    uint64_t x[W], z[W];
+    load_key<W>(P, i, x, z);
+    rstore<W>(R, i, x, z);
+    R.c[i] = P.c[i];
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+      sx[w] |= x[w];
+      sz[w] |= z[w];
+    }
+  }
+  for (unsigned t = threadIdx.x; t < 2 * CAP; t += BLOCK) R.table[t] = 0ull;
+  for (unsigned t = threadIdx.x; t < CAP; t += BLOCK) R.link[t] = 0ull;
+  if (threadIdx.x == 0) sh.perr = 0;
+  block_or<W>(sx, sz, sh.orw);
+  unsigned epoch = 0, pc = 0;
+  unsigned run_end = 0, run_at = 0, run_n = 0;  // the fused run being applied: [run_at, run_end), its first size
+  bool run_rx = false, stop = false;
+  uint64_t Q[W];
+  // an op's live count; n_s and n_new of these ops are not recorded per kernel
+  auto logop = [&](unsigned o, unsigned n_in, unsigned n_out) {
+    if (threadIdx.x == 0) {
+      OpLog& l = log[op0 + o];
+      l.n_in = n_in;
+      l.n_s = 0;
+      l.n_new = n_out > n_in ? n_out - n_in : 0;
+      l.n_out = n_out;
+    }
+  };
+  fetch(0);
+  while (pc < nops && !stop) {
+    if (pc - s0 >= OPS) fetch(pc);
+    const SmallOp& op = s_ops[pc - s0];
+    const uint32_t kind = op.kind;
+    if (epoch >= 0xFFF0u) {  // pair-table epochs about to wrap
+      __syncthreads();
+      for (unsigned t = threadIdx.x; t < 2 * CAP; t += BLOCK) R.table[t] = 0ull;
+      __syncthreads();
+      epoch = 0;
+    }
+    if (kind == S_TRUNC) {
+      const unsigned kept = (unsigned)cta_truncate<W, BLOCK, ITEMS>(R, N, thr, maxw, s_base, sh.orw, sx, sz);
+      logop(pc, N, kept);
+      N = kept;
+      ++pc;
+      continue;
+    }
+    if (kind == S_LOCAL) {
+      unsigned j = pc;
+      while (j < nops && j - s0 < OPS && s_ops[j - s0].kind == S_LOCAL) ++j;
+#pragma unroll
+      for (int w = 0; w < W; ++w) sx[w] = sz[w] = 0ull;
+      for (unsigned i = threadIdx.x; i < N; i += BLOCK) {
+        uint64_t x[W], z[W];
+        rload<W>(R, i, x, z);
+        double c = R.c[i];
+        bool neg = false;
+        for (unsigned o = pc; o < j; ++o) local_op<W>(s_ops[o - s0].d, x, z, c, neg);
+        rstore<W>(R, i, x, z);
+        R.c[i] = neg ? -c : c;
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+          sx[w] |= x[w];
+          sz[w] |= z[w];
+        }
+      }
+      block_or<W>(sx, sz, sh.orw);
+      for (unsigned o = pc; o < j; ++o) logop(o, N, N);
+      pc = j;
+      continue;
+    }
+    const DevOp d = op.d;
+    if (kind == S_DAMP) {
+      CtaPlan<NW> p;
+      const unsigned n_in = N;
+      if (cta_pair<W, BLOCK, ITEMS, true>(R, d, N, ++epoch, sh, p)) {
+        if (N + p.C > CAP || sh.perr) break;
+        cta_apply<W, BLOCK, true>(R, d, op.a, op.b, N, p);
+        N += p.C;
+      }
+      for (unsigned i = threadIdx.x; i < n_in; i += BLOCK)
+        if ((R.x[(size_t)d.w0 * R.cap + i] >> d.b0) & 1ull) R.c[i] = __dmul_rn(R.c[i], op.c);
+      __syncthreads();
+      logop(pc, n_in, N);
+      ++pc;
+      continue;
+    }
+    if (op.run) {  // a fused run starts: its terms as they are, in case it outgrows the region
+      run_rx = (d.ax & 1) != 0;
+      if (!small_run_begin<W>(R, N, ops + pc, op.run, run_rx, s_q, Q)) break;  // too wide: the pipeline cuts it
+      run_at = pc;
+      run_end = pc + op.run;
+      run_n = N;
+      for (unsigned i = threadIdx.x; i < N; i += BLOCK) {
+        uint64_t x[W], z[W];
+        rload<W>(R, i, x, z);
+        store_key<W>(P, i, x, z);
+        P.c[i] = R.c[i];
+      }
+    }
+    const unsigned n_in = N;
+    if (rot_may_touch<W>(d, sx, sz)) {
+      CtaPlan<NW> p;
+      if (cta_pair<W, BLOCK, ITEMS, false>(R, d, N, ++epoch, sh, p)) {
+        if (N + p.C > CAP || sh.perr) {
+          stop = true;
+        } else {
+          cta_apply<W, BLOCK, false>(R, d, op.a, op.b, N, p);
+          join_gen<W>(d, sx, sz);
+          N += p.C;
+          __syncthreads();
+        }
+      }
+    }
+    if (stop) break;
+    logop(pc, n_in, N);
+    ++pc;
+    if (pc == run_end) {
+      small_run_sort<W>(R, run_n, N, run_rx, Q, ++epoch, keys);
+      run_end = 0;
+    }
+  }
+  __syncthreads();
+  if (run_end > pc) {  // stopped inside a run: the terms before it are in P
+    N = run_n;
+    pc = run_at;
+  } else {
+    for (unsigned i = threadIdx.x; i < N; i += BLOCK) {
+      uint64_t x[W], z[W];
+      rload<W>(R, i, x, z);
+      store_key<W>(P, i, x, z);
+      P.c[i] = R.c[i];
+    }
+  }
+  if (threadIdx.x == 0) {
+    ctrl->n = N;
+    ctrl->small_pc = pc;
+  }
+}
+
+}  // namespace ppvm
