@@ -240,7 +240,7 @@ k_batch(BInst* insts, const BOp* __restrict__ ops, const uint32_t* __restrict__ 
       epoch = 1;
     }
     CtaPlan<NW> p;
-    if (!cta_pair<W, BLOCK, ITEMS, false>(R, d, (unsigned)N, epoch, sh, p)) {
+    if (!cta_pair<W, BLOCK, ITEMS>(R, d, (unsigned)N, epoch, sh, p)) {
       tgu += N;
       ++pc;
       continue;
@@ -291,7 +291,7 @@ k_batch(BInst* insts, const BOp* __restrict__ ops, const uint32_t* __restrict__ 
       resident = false;
       __syncthreads();
     }
-    cta_apply<W, BLOCK, false>(R, d, sn, cs, N, p);
+    cta_apply<W, BLOCK>(R, d, sn, cs, N, p);
     join_gen<W>(d, sx, sz);
     __syncthreads();
     tgu += N;

@@ -222,16 +222,13 @@ __device__ __forceinline__ unsigned cta_nth(const Region<W>& R, const CtaPlan<NW
   return R.sidx[at];
 }
 
-// First half of a rotation exp(-i theta/2 G), G on d's one or two qubits (DAMP: of amplitude damping
-// of d's q0): lists the touched terms, links the pairs and counts the children.  Nothing but
-// links, lists and table entries is written, so a caller without room for the children can
-// stop here.  Returns false when nothing is touched.
-//
-// Touched terms are those that anticommute with G (DAMP: those with I or Z on q0; the Z ones are the
-// parents, the I ones where their children may land).  Each warp lists its own chunk of the
-// terms, in order and without a barrier; the pair K, K^G meets in the table at one of the two
-// keys, and the second to arrive hands each the other's coefficient.
-template <int W, int BLOCK, int ITEMS, bool DAMP>
+// First half of a rotation exp(-i theta/2 G), G on d's one or two qubits: lists the terms that
+// anticommute with G, links the pairs and counts the children.  Nothing but links, lists and table
+// entries is written, so a caller without room for the children can stop here.  Returns false
+// when nothing is touched.  Each warp lists its own chunk of the terms, in order and without a
+// barrier; the pair K, K^G meets in the table at one of the two keys, and the second to arrive
+// hands each the other's coefficient.
+template <int W, int BLOCK, int ITEMS>
 __device__ __forceinline__ bool cta_pair(const Region<W>& R, const DevOp& d, unsigned N, unsigned epoch,
                                          CtaShared<W, BLOCK / 32>& sh, CtaPlan<BLOCK / 32>& p) {
   constexpr int NW = BLOCK / 32;
@@ -248,7 +245,7 @@ __device__ __forceinline__ bool cta_pair(const Region<W>& R, const DevOp& d, uns
       if (i < hi) {
         bool x0, z0, x1, z1;
         term_bits<W>(R, d, i, x0, z0, x1, z1);
-        a[k] = DAMP ? !x0 : rot_bits(d, x0, z0, x1, z1).anti;
+        a[k] = rot_bits(d, x0, z0, x1, z1).anti;
       }
     }
 #pragma unroll
@@ -276,10 +273,9 @@ __device__ __forceinline__ bool cta_pair(const Region<W>& R, const DevOp& d, uns
       px[w] = x[w];
       pz[w] = z[w];
     }
-    if constexpr (DAMP) wflip<W>(pz, d.w0, 1ull << d.b0);
-    else flip_gen<W>(d, px, pz);
+    flip_gen<W>(d, px, pz);
     // of the two keys, the one without the flipped bit on q0
-    const bool use_p = ((!DAMP && (d.ax & 1) ? wsel<W>(x, d.w0) : wsel<W>(z, d.w0)) >> d.b0) & 1ull;
+    const bool use_p = ((d.ax & 1 ? wsel<W>(x, d.w0) : wsel<W>(z, d.w0)) >> d.b0) & 1ull;
 #pragma unroll
     for (int w = 0; w < W; ++w) {
       kx[w] = use_p ? px[w] : x[w];
@@ -324,9 +320,7 @@ __device__ __forceinline__ bool cta_pair(const Region<W>& R, const DevOp& d, uns
   p.rhi = min(p.S, p.rlo + share);
   unsigned kids = 0;
   for (unsigned r = p.rlo + lane; r < p.rhi; r += 32) {
-    const unsigned i = cta_nth<W, NW>(R, p, r);
-    if constexpr (DAMP) kids += R.link[i] == 0ull && ((R.z[(size_t)d.w0 * R.cap + i] >> d.b0) & 1ull);
-    else kids += R.link[i] == 0ull;
+    kids += R.link[cta_nth<W, NW>(R, p, r)] == 0ull;
   }
   kids = __reduce_add_sync(kFull, kids);
   if (lane == 0) sh.child[warp] = kids;
@@ -340,11 +334,9 @@ __device__ __forceinline__ bool cta_pair(const Region<W>& R, const DevOp& d, uns
   return true;
 }
 
-// Second half: new coefficients in place, children appended in parent order (there is room).
-// Rotation: parent c*cs (+ partner's c*(eps*sn)), child c*(eps*sn); DAMP: parent c*cs, child c*sn,
-// added to the term that holds its key if there is one (X and Y terms, which it also scales, are not
-// touched here).
-template <int W, int BLOCK, bool DAMP>
+// Second half: new coefficients in place (parent c*cs, + partner's c*(eps*sn)), children c*(eps*sn)
+// appended in parent order (there is room).
+template <int W, int BLOCK>
 __device__ __forceinline__ void cta_apply(const Region<W>& R, const DevOp& d, double sn, double cs,
                                           unsigned long long N, const CtaPlan<BLOCK / 32>& p) {
   constexpr int NW = BLOCK / 32;
@@ -353,36 +345,29 @@ __device__ __forceinline__ void cta_apply(const Region<W>& R, const DevOp& d, do
   for (unsigned r0 = p.rlo; r0 < p.rhi; r0 += 32) {
     const unsigned r = r0 + lane;
     unsigned i = 0;
-    double c = 0.0, made = 0.0;
+    double made = 0.0;
     bool child = false;
     if (r < p.rhi) {
       i = cta_nth<W, NW>(R, p, r);
-      c = R.c[i];
+      const double c = R.c[i];
       const unsigned long long lw = R.link[i];
-      const double lc = __longlong_as_double((long long)~lw);
       bool x0, z0, x1, z1;
       term_bits<W>(R, d, i, x0, z0, x1, z1);
-      double nc;
-      if constexpr (DAMP) {
-        child = z0 && lw == 0ull;
-        made = __dmul_rn(c, sn);
-        nc = z0 ? __dmul_rn(c, cs) : lw ? __dadd_rn(c, __dmul_rn(lc, sn)) : c;
-      } else {
-        child = lw == 0ull;
-        made = __dmul_rn(c, (rot_bits(d, x0, z0, x1, z1).eps_plus ? 1.0 : -1.0) * sn);
-        nc = __dmul_rn(c, cs);
-        if (lw) {
-          // the partner's key is K^G: its eps from this term's bits with G's bits flipped
-          x0 ^= (bool)(d.ax & 1);
-          z0 ^= (bool)(d.az & 1);
-          if (d.two) {
-            x1 ^= (bool)(d.ax & 2);
-            z1 ^= (bool)(d.az & 2);
-          }
-          nc = __dadd_rn(nc, __dmul_rn(lc, (rot_bits(d, x0, z0, x1, z1).eps_plus ? 1.0 : -1.0) * sn));
+      child = lw == 0ull;
+      made = __dmul_rn(c, (rot_bits(d, x0, z0, x1, z1).eps_plus ? 1.0 : -1.0) * sn);
+      double nc = __dmul_rn(c, cs);
+      if (lw) {
+        // the partner's key is K^G: its eps from this term's bits with G's bits flipped
+        x0 ^= (bool)(d.ax & 1);
+        z0 ^= (bool)(d.az & 1);
+        if (d.two) {
+          x1 ^= (bool)(d.ax & 2);
+          z1 ^= (bool)(d.az & 2);
         }
+        nc = __dadd_rn(nc, __dmul_rn(__longlong_as_double((long long)~lw),
+                                     (rot_bits(d, x0, z0, x1, z1).eps_plus ? 1.0 : -1.0) * sn));
+        R.link[i] = 0ull;
       }
-      if (lw) R.link[i] = 0ull;
       R.c[i] = nc;
     }
     const unsigned m = __ballot_sync(kFull, child);
@@ -390,8 +375,7 @@ __device__ __forceinline__ void cta_apply(const Region<W>& R, const DevOp& d, do
       const unsigned long long pos = N + at + __popc(m & lt);
       uint64_t x[W], z[W];
       rload<W>(R, i, x, z);
-      if constexpr (DAMP) wflip<W>(z, d.w0, 1ull << d.b0);
-      else flip_gen<W>(d, x, z);
+      flip_gen<W>(d, x, z);
       rstore<W>(R, pos, x, z);
       R.c[pos] = made;
     }

@@ -1121,7 +1121,7 @@ struct K {
   }
 
   // ops[0..nops) (small ops, list indices from op0) on a sum of at most kSmallStart terms.
-  static ppvm_status small(ppvm_sum* s, const SmallOp* d_ops, int nops, int op0) {
+  static ppvm_status small(ppvm_sum* s, const SmallOp* d_ops, const SmallInline& few, int nops, int op0) {
     static unsigned long long attr_set = 0;  // one bit per device
     if (!((attr_set >> s->device) & 1ull)) {
       CUDA_TRY(cudaFuncSetAttribute(k_small<W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1129,8 +1129,8 @@ struct K {
       attr_set |= 1ull << s->device;
     }
     ProfScope ps(s, F_SMALL, op0, nops);
-    launch(k_small<W>, 1, kSmallBlock, SmallFor<W>::smem, s->stream, s->planes_view(), s->d_ctrl, d_ops,
-           (unsigned)nops, op0, s->thr, s->maxw, s->d_log);
+    launch(k_small<W>, 1, kSmallBlock, SmallFor<W>::smem, s->stream, s->planes_view(), s->d_ctrl, d_ops, few,
+           (unsigned)nops, op0, s->thr, s->maxw, s->h_log, s->h_ctrl);
     return PPVM_OK;
   }
 
@@ -1248,8 +1248,8 @@ ppvm_status enqueue_tableau(ppvm_sum* s, const HostTableau& t, int op0, int nops
   DISPATCH_W_RET(s->W, tableau(s, t, op0, nops, trunc_op));
 }
 
-ppvm_status enqueue_small(ppvm_sum* s, const SmallOp* d_ops, int nops, int op0) {
-  DISPATCH_W_RET(s->W, small(s, d_ops, nops, op0));
+ppvm_status enqueue_small(ppvm_sum* s, const SmallOp* d_ops, const SmallInline& few, int nops, int op0) {
+  DISPATCH_W_RET(s->W, small(s, d_ops, few, nops, op0));
 }
 
 int test_words_of(int W, const Gen& g) {
@@ -1258,11 +1258,13 @@ int test_words_of(int W, const Gen& g) {
   return n;
 }
 
-// Reads the control block and the op log back; synchronises.
-ppvm_status sync_state(ppvm_sum* s, size_t nops) {
+// Reads the control block and the op log's entries [from, nops) back; synchronises.
+ppvm_status sync_state(ppvm_sum* s, size_t nops, size_t from = 0) {
   CUDA_TRY(cudaMemcpyAsync(s->h_ctrl, s->d_ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, s->stream));
-  if (nops) CUDA_TRY(cudaMemcpyAsync(s->h_log, s->d_log, sizeof(OpLog) * nops, cudaMemcpyDeviceToHost, s->stream));
-  s->xfer_d2h += sizeof(Ctrl) + sizeof(OpLog) * nops;
+  if (nops > from)
+    CUDA_TRY(cudaMemcpyAsync(s->h_log + from, s->d_log + from, sizeof(OpLog) * (nops - from), cudaMemcpyDeviceToHost,
+                             s->stream));
+  s->xfer_d2h += sizeof(Ctrl) + sizeof(OpLog) * (nops - from);
   CUDA_TRY(cudaStreamSynchronize(s->stream));
   return PPVM_OK;
 }
@@ -1514,14 +1516,22 @@ ppvm_status run_small(ppvm_sum* s, const ppvm_op* ops, size_t n_ops, size_t* sta
       rec.push_back(r);
       ++i;
     }
-    if (rec.empty()) return PPVM_OK;
-    stage_reset(s);
+    // a short head of a long list is not worth the launch and the synchronisation
+    if (rec.empty() || (rec.size() < 64 && *start + rec.size() < n_ops)) return PPVM_OK;
     const void* d_ops = nullptr;
-    PPVM_TRY(stage_put(s, rec.data(), sizeof(SmallOp) * rec.size(), &d_ops));
-    PPVM_TRY(enqueue_small(s, static_cast<const SmallOp*>(d_ops), (int)rec.size(), (int)*start));
+    SmallInline few;
+    if (rec.size() <= (size_t)kSmallInline) {
+      std::copy(rec.begin(), rec.end(), few.op);
+      s->xfer_h2d += sizeof(SmallOp) * rec.size();
+    } else {
+      stage_reset(s);
+      PPVM_TRY(stage_put(s, rec.data(), sizeof(SmallOp) * rec.size(), &d_ops));
+    }
+    s->h_ctrl->err = kErrProbe;  // the kernel clears it when it is through
+    PPVM_TRY(enqueue_small(s, static_cast<const SmallOp*>(d_ops), few, (int)rec.size(), (int)*start));
     CUDA_TRY(cudaGetLastError());
-    const bool all = *start + rec.size() == n_ops;
-    PPVM_TRY(sync_state(s, all ? n_ops : 0));
+    CUDA_TRY(cudaStreamSynchronize(s->stream));
+    s->xfer_d2h += 24 + sizeof(OpLog) * s->h_ctrl->small_pc;
     if (s->h_ctrl->err) {
       s->poisoned = true;
       return fail(PPVM_ECUDA, "device error " + std::to_string(s->h_ctrl->err) + " in a small op list");
@@ -1547,6 +1557,7 @@ ppvm_status run_list(ppvm_sum* s, const ppvm_op* ops, size_t n_ops, const std::v
     s->last_nops = n_ops;
     return PPVM_OK;
   }
+  const size_t first = start;  // k_small has written the log of the ops before
   // every failed attempt grows the capacity or cuts a run, so the loop ends; the bound only
   // turns a logic error into a status
   const size_t max_attempts = 64 + 8 * n_ops;
@@ -1555,7 +1566,7 @@ ppvm_status run_list(ppvm_sum* s, const ppvm_op* ops, size_t n_ops, const std::v
     s->run_len.clear();
     stage_reset(s);  // the stream is idle here: every earlier upload has completed
     PPVM_TRY(enqueue(s, ops, n_ops, start, gens, test_words));
-    PPVM_TRY(sync_state(s, n_ops));
+    PPVM_TRY(sync_state(s, n_ops, first));
     const Ctrl& c = *s->h_ctrl;
     s->n_host = c.n;
     if (c.err == kOk) {

@@ -24,7 +24,7 @@ constexpr int kSmallBlock = 512;
 constexpr int kSmallItems = 4;
 constexpr int kSmallOps = 2048;                  // ops per launch
 constexpr unsigned long long kSmallStart = 512;  // sums of more terms take the pipelines at once
-constexpr int kSmallLocal = 128;                 // longer stretches of local ops: the composed pass
+constexpr int kSmallLocal = 64;                  // longer stretches of local ops: the composed pass
 
 // Terms the region holds: as many as fit into shared memory with the pair table and the sort keys.
 template <int W>
@@ -41,6 +41,133 @@ struct alignas(8) SmallOp {
   uint32_t run;  // gates of the fused run that starts here (0: none starts)
   double a, b, c;  // rotation: sin, cos; damping: gamma, 1 - gamma, sqrt(1 - gamma)
 };
+
+// Up to this many ops travel as a kernel argument instead of an upload (a single-gate call).
+constexpr int kSmallInline = 4;
+struct SmallInline {
+  SmallOp op[kSmallInline];
+};
+
+// A rotation (DAMP: amplitude damping) with the reference's semantics on N <= BLOCK * ITEMS terms:
+// thread t owns terms t, t + BLOCK, ... throughout, so nothing is listed, and three barriers
+// separate linking the pairs, ranking the children and using the results.  Returns the new size, or
+// more than the region holds, with no term changed.
+template <int W, bool DAMP>
+__device__ __forceinline__ unsigned small_rotate(const Region<W>& R, const SmallOp& op, unsigned N, unsigned epoch,
+                                                 unsigned* s_base, int& perr) {
+  constexpr int BLOCK = kSmallBlock, ITEMS = kSmallItems, NW = BLOCK / 32;
+  const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lt = (1u << lane) - 1u;
+  const DevOp d = op.d;
+  const unsigned long long mask = R.tsize - 1;
+  unsigned bits = 0;  // per item, 4 bits: touched, eps of the child is +1, eps of the partner's is +1; DAMP: touched, Z
+#pragma unroll
+  for (int k = 0; k < ITEMS; ++k) {
+    const unsigned i = k * BLOCK + threadIdx.x;
+    if (i >= N) continue;
+    bool x0, z0, x1, z1;
+    term_bits<W>(R, d, i, x0, z0, x1, z1);
+    if constexpr (DAMP) {
+      if (x0) continue;
+      bits |= (1u | (unsigned)z0 << 1) << (4 * k);
+    } else {
+      const RotBits rb = rot_bits(d, x0, z0, x1, z1);
+      if (!rb.anti) continue;
+      const RotBits pb = rot_bits(d, x0 ^ (bool)(d.ax & 1), z0 ^ (bool)(d.az & 1), x1 ^ (d.two && (d.ax & 2)),
+                                  z1 ^ (d.two && (d.az & 2)));
+      bits |= (1u | (unsigned)rb.eps_plus << 1 | (unsigned)pb.eps_plus << 2) << (4 * k);
+    }
+    uint64_t x[W], z[W], px[W], pz[W], kx[W], kz[W];
+    rload<W>(R, i, x, z);
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+      px[w] = x[w];
+      pz[w] = z[w];
+    }
+    if constexpr (DAMP) wflip<W>(pz, d.w0, 1ull << d.b0);
+    else flip_gen<W>(d, px, pz);
+    const bool use_p = (!DAMP && (d.ax & 1)) ? x0 : z0;  // meet at the key without the flipped bit on q0
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+      kx[w] = use_p ? px[w] : x[w];
+      kz[w] = use_p ? pz[w] : z[w];
+    }
+    const uint64_t h = table_hash<W>(kx, kz);
+    const unsigned tag = (unsigned)(h >> 48) & 0xFFFFu;
+    const unsigned long long me = make_slot(epoch, tag, i);
+    unsigned long long slot = h & mask, probes = 0, cur = ld_volatile(&R.table[slot]);
+    while (true) {
+      if (slot_epoch(cur) != (epoch & 0xFFFFu)) {
+        const unsigned long long prev = atomicCAS(&R.table[slot], cur, me);
+        if (prev == cur) break;
+        cur = prev;
+        continue;
+      }
+      if (slot_tag(cur) == tag) {
+        const unsigned j = slot_idx(cur);
+        uint64_t jx[W], jz[W];
+        rload<W>(R, j, jx, jz);
+        bool eq = true;
+#pragma unroll
+        for (int w = 0; w < W; ++w) eq &= (jx[w] == px[w]) & (jz[w] == pz[w]);
+        if (eq) {
+          R.link[i] = link_word(R.c[j]);
+          R.link[j] = link_word(R.c[i]);
+          break;
+        }
+      }
+      slot = (slot + 1) & mask;
+      if (++probes > mask) {
+        perr = 1;  // cannot happen: twice as many slots as terms
+        break;
+      }
+      cur = ld_volatile(&R.table[slot]);
+    }
+  }
+  if (!__syncthreads_or(bits != 0)) {
+    if constexpr (!DAMP) return N;
+  }
+  unsigned bal[ITEMS];
+  unsigned long long lw[ITEMS];
+#pragma unroll
+  for (int k = 0; k < ITEMS; ++k) {
+    const unsigned b = bits >> (4 * k);
+    lw[k] = b & 1u ? R.link[k * BLOCK + threadIdx.x] : 0ull;
+    bal[k] = __ballot_sync(kFull, (b & 1u) && lw[k] == 0ull && (!DAMP || (b & 2u)));
+  }
+  const unsigned made = tile_ranks<BLOCK, ITEMS>(bal, s_base);
+  if (N + made > (unsigned)R.cap || perr) return (unsigned)R.cap + 1;
+#pragma unroll
+  for (int k = 0; k < ITEMS; ++k) {
+    const unsigned i = k * BLOCK + threadIdx.x, b = bits >> (4 * k);
+    if (b & 1u) {
+      const double c = R.c[i], lc = __longlong_as_double((long long)~lw[k]);
+      double nc, cc;
+      if constexpr (DAMP) {
+        cc = __dmul_rn(c, op.a);
+        nc = b & 2u ? __dmul_rn(c, op.b) : lw[k] ? __dadd_rn(c, __dmul_rn(lc, op.a)) : c;
+      } else {
+        cc = __dmul_rn(c, (b & 2u ? 1.0 : -1.0) * op.a);
+        nc = __dmul_rn(c, op.b);
+        if (lw[k]) nc = __dadd_rn(nc, __dmul_rn(lc, (b & 4u ? 1.0 : -1.0) * op.a));
+      }
+      if (lw[k]) R.link[i] = 0ull;
+      R.c[i] = nc;
+      if ((bal[k] >> lane) & 1u) {
+        const unsigned pos = N + s_base[k * NW + warp] + __popc(bal[k] & lt);
+        uint64_t x[W], z[W];
+        rload<W>(R, i, x, z);
+        if constexpr (DAMP) wflip<W>(z, d.w0, 1ull << d.b0);
+        else flip_gen<W>(d, x, z);
+        rstore<W>(R, pos, x, z);
+        R.c[pos] = cc;
+      }
+    } else if (DAMP && i < N) {  // X or Y
+      R.c[i] = __dmul_rn(R.c[i], op.c);
+    }
+  }
+  __syncthreads();
+  return N + made;
+}
 
 // The run's qubits, and whether every group fits the fused run (at most kRunMaxK coordinates).
 template <int W>
@@ -199,21 +326,29 @@ __device__ __forceinline__ void small_run_sort(const Region<W>& R, unsigned N0, 
   __syncthreads();
 }
 
+// ops: the list in device memory, or null for the ops in `few`.  log and host: the op log and the
+// control block in the host's own (pinned) memory, written directly, so that a call needs no copy
+// back.
 template <int W>
 __global__ void __launch_bounds__(kSmallBlock)
-k_small(Planes P, Ctrl* ctrl, const SmallOp* __restrict__ ops, unsigned nops, int op0, double thr,
-        unsigned long long maxw, OpLog* log) {
+k_small(Planes P, Ctrl* ctrl, const SmallOp* __restrict__ ops, const SmallInline few, unsigned nops, int op0,
+        double thr, unsigned long long maxw, OpLog* log, Ctrl* host) {
   pdl_wait();
   constexpr int BLOCK = kSmallBlock, ITEMS = kSmallItems, NW = BLOCK / 32;
   __shared__ unsigned s_base[ITEMS * NW + 1];
-  __shared__ CtaShared<W, NW> sh;
+  __shared__ unsigned long long s_or[2 * W];
+  __shared__ int s_perr;
   __shared__ unsigned long long s_q[W];
   // the ops from index s0 on: an op read from global memory would cost its latency each time
   constexpr unsigned OPS = 64;
   __shared__ SmallOp s_ops[OPS];
+  static_assert(kSmallInline <= OPS, "the ops in few fit the buffer");
+  if (!ops && threadIdx.x == 0)
+    for (unsigned o = 0; o < nops; ++o) s_ops[o] = few.op[o];
   unsigned s0 = 0;
   auto fetch = [&](unsigned at) {
     __syncthreads();
+    if (!ops) return;
     s0 = at;
     const unsigned n = min(OPS, nops - at) * (unsigned)(sizeof(SmallOp) / 8);
     for (unsigned t = threadIdx.x; t < n; t += BLOCK)
@@ -222,14 +357,12 @@ k_small(Planes P, Ctrl* ctrl, const SmallOp* __restrict__ ops, unsigned nops, in
   };
   extern __shared__ __align__(16) uint64_t s_small[];
   constexpr unsigned CAP = SmallFor<W>::cap;
-  if (ld_volatile_int(&ctrl->err)) return;
   const Region<W> R = region_at<W>(s_small, CAP, 2 * CAP);
   unsigned long long* keys = reinterpret_cast<unsigned long long*>(R.table + 2 * CAP);
-  unsigned N = (unsigned)ld_volatile(&ctrl->n);
+  unsigned N = (unsigned)ld_volatile(&ctrl->n);  // at most kSmallStart: the host knows the count
   uint64_t sx[W], sz[W];
 #pragma unroll
   for (int w = 0; w < W; ++w) sx[w] = sz[w] = 0ull;
-  if (N > CAP) return;  // the host asks for at most kSmallStart
   for (unsigned i = threadIdx.x; i < N; i += BLOCK) {
     uint64_t x[W], z[W];
     load_key<W>(P, i, x, z);
@@ -243,11 +376,11 @@ k_small(Planes P, Ctrl* ctrl, const SmallOp* __restrict__ ops, unsigned nops, in
   }
   for (unsigned t = threadIdx.x; t < 2 * CAP; t += BLOCK) R.table[t] = 0ull;
   for (unsigned t = threadIdx.x; t < CAP; t += BLOCK) R.link[t] = 0ull;
-  if (threadIdx.x == 0) sh.perr = 0;
-  block_or<W>(sx, sz, sh.orw);
+  if (threadIdx.x == 0) s_perr = 0;
+  block_or<W>(sx, sz, s_or);
   unsigned epoch = 0, pc = 0;
   unsigned run_end = 0, run_at = 0, run_n = 0;  // the fused run being applied: [run_at, run_end), its first size
-  bool run_rx = false, stop = false;
+  bool run_rx = false;
   uint64_t Q[W];
   // an op's live count; n_s and n_new of these ops are not recorded per kernel
   auto logop = [&](unsigned o, unsigned n_in, unsigned n_out) {
@@ -260,7 +393,7 @@ k_small(Planes P, Ctrl* ctrl, const SmallOp* __restrict__ ops, unsigned nops, in
     }
   };
   fetch(0);
-  while (pc < nops && !stop) {
+  while (pc < nops) {
     if (pc - s0 >= OPS) fetch(pc);
     const SmallOp& op = s_ops[pc - s0];
     const uint32_t kind = op.kind;
@@ -271,7 +404,7 @@ k_small(Planes P, Ctrl* ctrl, const SmallOp* __restrict__ ops, unsigned nops, in
       epoch = 0;
     }
     if (kind == S_TRUNC) {
-      const unsigned kept = (unsigned)cta_truncate<W, BLOCK, ITEMS>(R, N, thr, maxw, s_base, sh.orw, sx, sz);
+      const unsigned kept = (unsigned)cta_truncate<W, BLOCK, ITEMS>(R, N, thr, maxw, s_base, s_or, sx, sz);
       logop(pc, N, kept);
       N = kept;
       ++pc;
@@ -296,30 +429,23 @@ k_small(Planes P, Ctrl* ctrl, const SmallOp* __restrict__ ops, unsigned nops, in
           sz[w] |= z[w];
         }
       }
-      block_or<W>(sx, sz, sh.orw);
+      block_or<W>(sx, sz, s_or);
       for (unsigned o = pc; o < j; ++o) logop(o, N, N);
       pc = j;
       continue;
     }
-    const DevOp d = op.d;
     if (kind == S_DAMP) {
-      CtaPlan<NW> p;
-      const unsigned n_in = N;
-      if (cta_pair<W, BLOCK, ITEMS, true>(R, d, N, ++epoch, sh, p)) {
-        if (N + p.C > CAP || sh.perr) break;
-        cta_apply<W, BLOCK, true>(R, d, op.a, op.b, N, p);
-        N += p.C;
-      }
-      for (unsigned i = threadIdx.x; i < n_in; i += BLOCK)
-        if ((R.x[(size_t)d.w0 * R.cap + i] >> d.b0) & 1ull) R.c[i] = __dmul_rn(R.c[i], op.c);
-      __syncthreads();
-      logop(pc, n_in, N);
+      const unsigned n_out = small_rotate<W, true>(R, op, N, ++epoch, s_base, s_perr);
+      if (n_out > CAP) break;
+      logop(pc, N, n_out);
+      N = n_out;
       ++pc;
       continue;
     }
+    const DevOp d = op.d;
     if (op.run) {  // a fused run starts: its terms as they are, in case it outgrows the region
       run_rx = (d.ax & 1) != 0;
-      if (!small_run_begin<W>(R, N, ops + pc, op.run, run_rx, s_q, Q)) break;  // too wide: the pipeline cuts it
+      if (!small_run_begin<W>(R, N, ops ? ops + pc : s_ops, op.run, run_rx, s_q, Q)) break;  // too wide: the pipeline cuts it
       run_at = pc;
       run_end = pc + op.run;
       run_n = N;
@@ -332,19 +458,11 @@ k_small(Planes P, Ctrl* ctrl, const SmallOp* __restrict__ ops, unsigned nops, in
     }
     const unsigned n_in = N;
     if (rot_may_touch<W>(d, sx, sz)) {
-      CtaPlan<NW> p;
-      if (cta_pair<W, BLOCK, ITEMS, false>(R, d, N, ++epoch, sh, p)) {
-        if (N + p.C > CAP || sh.perr) {
-          stop = true;
-        } else {
-          cta_apply<W, BLOCK, false>(R, d, op.a, op.b, N, p);
-          join_gen<W>(d, sx, sz);
-          N += p.C;
-          __syncthreads();
-        }
-      }
+      const unsigned n_out = small_rotate<W, false>(R, op, N, ++epoch, s_base, s_perr);
+      if (n_out > CAP) break;
+      N = n_out;
+      join_gen<W>(d, sx, sz);
     }
-    if (stop) break;
     logop(pc, n_in, N);
     ++pc;
     if (pc == run_end) {
@@ -366,7 +484,9 @@ k_small(Planes P, Ctrl* ctrl, const SmallOp* __restrict__ ops, unsigned nops, in
   }
   if (threadIdx.x == 0) {
     ctrl->n = N;
-    ctrl->small_pc = pc;
+    host->n = N;
+    host->small_pc = pc;
+    host->err = 0;
   }
 }
 

@@ -66,9 +66,9 @@ def cases():
             out.append((n, [(w, 1.0)], rx + [G.truncate()] + rx[:2] + [G.truncate()], 1e-9, None))
             out.append((n, [(w, 1.0), ("X" * n, 0.5)], [op for r in rx for op in (r, G.truncate())], 1e-9, None))
     # a run of 13 coordinates (too wide for a group), and one that doubles past the region midway
-    out.append((30, [("Z" * 13 + "I" * 17, 1.0)], [G.r1(G.RX, q, 0.2) for q in range(30)] + [G.truncate()], 1e-4, None))
-    out.append((30, random_terms(rng, 30, 500), [G.r1(G.RX, q, 0.2) for q in range(30)] + [G.truncate()], 1e-4, None))
-    for k in (127, 128, 129, 300):  # local stretches around the composed pass's limit
+    out.append((20, [("Z" * 13 + "I" * 7, 1.0)], [G.r1(G.RX, q, 0.2) for q in range(20)] + [G.truncate()], 1e-4, None))
+    out.append((14, random_terms(rng, 14, 400), [G.r1(G.RX, q, 0.2) for q in range(14)] + [G.truncate()], 1e-3, None))
+    for k in (63, 64, 65, 300):  # local stretches around the composed pass's limit
         ops = [G.g1((G.H, G.S, G.SQRT_X)[i % 3], i % 12) for i in range(k)]
         out.append((12, random_terms(rng, 12, 50), ops + [G.r1(G.RX, 3, 0.4), G.truncate()] + ops[:5], 1e-6, None))
     # more ops than one launch takes, the sum small all along
