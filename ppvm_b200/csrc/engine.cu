@@ -312,15 +312,13 @@ unsigned long long run_scratch_min_groups() {
   return v;
 }
 
-// The group mode of k_run_groups: 0 chosen per run (many single-member groups: one group per
-// lane; otherwise one group per warp), 1 tiles of groups per block, 2 one group per warp, 3 one
-// group per lane.  PPVM_RUN_GROUP_MODE=tiled|warp|lanes forces one; the tests run the
-// fused-run cases in each.
-unsigned run_tile_mode() {
+// The group mode of the fused runs: 0 chosen per run (many single-member groups: one group per lane;
+// otherwise tiles of groups), 1 tiles, 3 one group per lane.  PPVM_RUN_GROUP_MODE=tiled|lanes forces
+// one ("warp", once a mode of its own, is tiles); the tests run the fused-run cases in each.
+unsigned run_group_mode() {
   static const unsigned v = [] {
     const char* e = std::getenv("PPVM_RUN_GROUP_MODE");
-    if (e && std::strcmp(e, "tiled") == 0) return 1u;
-    if (e && std::strcmp(e, "warp") == 0) return 2u;
+    if (e && (std::strcmp(e, "tiled") == 0 || std::strcmp(e, "warp") == 0)) return 1u;
     if (e && std::strcmp(e, "lanes") == 0) return 3u;
     return 0u;
   }();
@@ -1054,24 +1052,39 @@ struct K {
     }
     const Planes S = allow ? s->view_of(s->scr) : O;
     const unsigned long long scratch_min = allow ? smin : ~0ull;
-    {
+    const unsigned mode = run_group_mode();
+    if (mode != 3) {
       ProfScope ps(s, F_RUN_GROUPS, op0, L);
-      // no more blocks than fit on the GPU at once: warps take groups by ticket, so blocks
-      // beyond that would only queue on the ticket counter
+      // no more blocks than fit on the GPU at once: blocks take tiles by ticket, so more would
+      // only queue on the ticket counter
       static int resident = 0;  // blocks per SM (the same on every B200)
       if (!resident) {
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_run_groups<W>, kRunWarps * 32, 0) !=
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_run_tiles<W>, kTileWarps * 32, 0) !=
                 cudaSuccess || resident < 1)
           resident = 1;
       }
-      launch(k_run_groups<W>, grid_for(nub, kRunWarps, std::min(resident, 8)), kRunWarps * 32, 0, s->stream,
+      launch(k_run_tiles<W>, grid_for(nub, kTileWarps, std::min(resident, 8)), kTileWarps * 32, 0, s->stream,
           O, S, s->d_ctrl, d_rd, s->R, trunc, s->thr, s->maxw, s->tstate, s->next_tile_epoch(), op0,
-          trunc_op, s->d_log, scratch_min, run_tile_mode());  // its last block publishes the counts and the op log
+          trunc_op, s->d_log, scratch_min, mode);  // its last block publishes the counts and the op log
     }
-    if (allow) {
+    // ngroups <= live terms <= nub: below the threshold the device takes tiles, and the lane kernel
+    // is not needed
+    if (mode == 3 || (mode == 0 && nub >= kRunTileMinGroups)) {
+      ProfScope ps(s, F_RUN_GROUPS, op0, L);
+      static int resident = 0;
+      if (!resident) {
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_run_lanes<W>, kRunWarps * 32, 0) !=
+                cudaSuccess || resident < 1)
+          resident = 1;
+      }
+      launch(k_run_lanes<W>, grid_for(nub, 32 * kRunWarps, std::min(resident, 8)), kRunWarps * 32, 0, s->stream,
+          O, s->d_ctrl, d_rd, s->R, trunc, s->thr, s->maxw, s->tstate, s->next_tile_epoch(), op0,
+          trunc_op, s->d_log, mode);
+    }
+    if (allow && mode != 3) {
       ProfScope ps(s, F_RUN_PLACE, op0, L);
       launch(k_run_place<W, 256, 2>, grid_for(nub, 512, 4), 256, 0, s->stream,
-          S, O, s->d_ctrl, s->R, scratch_min, s->tstate, s->next_tile_epoch(), op0, run_tile_mode());
+          S, O, s->d_ctrl, s->R, scratch_min, s->tstate, s->next_tile_epoch(), op0, mode);
     }
     std::swap(s->planes, s->alt);
     s->swaps.push_back(op0);

@@ -28,9 +28,8 @@ namespace ppvm {
 
 constexpr int kRunMaxK = 10;       // groups up to 2^10 coordinates in shared memory
 constexpr int kRunMaxGates = 256;  // gates per fused run
-constexpr int kRunWarps = 4;       // warps of a k_run_groups block
-constexpr int kRunTileGroups = 16; // groups per look-back tile of k_run_groups (at most 32)
-constexpr unsigned long long kRunTileMinGroups = 8192;  // fewer groups: one look-back per group
+constexpr int kRunWarps = 4;       // warps of a k_run_lanes block
+constexpr unsigned long long kRunTileMinGroups = 8192;  // fewer groups: never one per lane
 constexpr unsigned long long kRunLogScratchBit = 1ull << 63;  // in the op log of a run's first gate
 constexpr int kErrFallback = 4;    // device error: a group exceeds kRunMaxK; rerun per gate
 
@@ -374,7 +373,7 @@ __global__ void __launch_bounds__(256) k_run_scatter(Planes P, Ctrl* ctrl, const
 }
 
 // Publishes the count after the run and fills the op log of its gates (and its TRUNCATE):
-// one warp of the last block of k_run_groups.  Gate j's live count is n0 plus the children
+// one warp of the last block of k_run_tiles or k_run_lanes.  Gate j's live count is n0 plus the children
 // the gates before it created (an exclusive scan of the created counts, 8 gates per lane).
 __device__ __forceinline__ void run_commit(Ctrl* ctrl, RunScratch R, int op0, int L, int trunc_op, OpLog* log,
                                            bool scratch, unsigned long long cap) {
@@ -439,176 +438,230 @@ __device__ __forceinline__ void run_commit(Ctrl* ctrl, RunScratch R, int op0, in
   }
 }
 
-// A group of a fused run as one warp holds it: key, coordinate qubits (ascending), whether
-// its weight passes the cap.  Its coefficients and existence bits live in the warp's
-// shared-memory slots, its coordinate bits in gate order in the warp's order array.
-template <int W>
-struct RunGroup {
-  uint64_t v[W], f0[W];
-  uint16_t pos[kRunMaxK];
+// ---- a group on a warp ------------------------------------------------------------------------
+constexpr int kTileWarps = 8;             // warps of a k_run_tiles block
+constexpr int kTileSlots = 512;           // slots of shared memory per warp (a group of 2^10 goes through them twice)
+constexpr unsigned long long kNoSlot = ~0ull;  // a slot without a term (see link_bits for that NaN)
+
+// The gates of a group's coordinates in run order.
+struct TileGates {
+  double cs[kRunMaxK], sn[kRunMaxK];
+  uint16_t gate[kRunMaxK];  // r-th gate: its index in the run
+  uint8_t bit[kRunMaxK];    // r-th gate: its coordinate bit
   unsigned k;
-  bool wok;
 };
 
-// Loads group g into the warp's slots: key, coordinates, their gate order, members.
-template <int W>
-__device__ __forceinline__ void group_load(RunGroup<W>& G, unsigned long long g, const RunDesc* rd,
-                                           const RunScratch& R, const uint16_t* s_gidx, uint8_t* ord, double* coef,
-                                           unsigned* ex, bool wcap, unsigned long long maxw) {
+// A group of at most 32 * NR slots on one warp, slot c = 32 r + lane in lane's register r: members loaded
+// through the warp's shared slots, then the gates in run order.  A gate on one of the five low
+// coordinate bits pairs lanes (shuffles), on a higher one registers; either way a slot's new value
+// is the reference's map_insert on the pair (crates/ppvm-pauli-sum/src/sum/rot1.rs:73,124: eps of a member
+// with bit b is +1 for b = 0 under RX, for b = 1 under RZ), with existence tracked apart from the value.
+// part < 0: the survivors of the run's TRUNCATE are counted, and written back to the shared slots
+// (the others empty) when they fit; part 0, 1: those of that half of 1024 slots are written.  Children
+// made per gate are added to created (null: not).  In shared memory, a pair per lane and step, the
+// same butterflies took 4 times the instructions and a round of shared-memory latency per pair.
+template <int NR>
+__device__ __noinline__ unsigned tile_survivors(const TileGates& g, unsigned long long* slots,
+                                                const uint32_t* __restrict__ mcoord, const double* __restrict__ mcoef,
+                                                unsigned cnt, double eps_a, bool trunc, bool wok, double thr,
+                                                unsigned* created, int part) {
   const unsigned lane = threadIdx.x & 31;
-  const uint32_t start = R.g_start[g], cnt = R.g_cnt[g];  // loaded beside the group key
-  uint64_t M[W];
-  G.k = 0;
-  {
-    const uint64_t* gk = R.gkey + g * 2 * W;
+  constexpr int NH = NR < 16 ? NR : 16;  // registers loaded at a time (512 slots)
+  double c[NR];
+  unsigned ex = 0;
 #pragma unroll
-    for (int w = 0; w < W; ++w) {
-      G.v[w] = gk[w];
-      G.f0[w] = gk[W + w];
-      M[w] = G.v[w] & rd->Q[w];
-    }
+  for (int h = 0; h < NR / NH; ++h) {
+    __syncwarp();
 #pragma unroll
-    for (int w = 0; w < W; ++w) {
-      uint64_t m = M[w];
-      while (m) {
-        const int b = __ffsll((long long)m) - 1;
-        G.pos[G.k++] = (uint16_t)(w * 64 + b);
-        m &= m - 1;
-      }
-    }
-  }
-  {  // coordinate bits sorted by the position of their gate in the run (distinct): lane t
-     // takes bit t, its rank is the number of bits whose gate comes earlier
-    unsigned key = 0xFFFFu;
-    for (unsigned t = 0; t < G.k; ++t)
-      if (t == lane) key = s_gidx[G.pos[t]];
-    unsigned rank = 0;
-    for (unsigned t = 0; t < G.k; ++t) rank += __shfl_sync(kFull, key, t) < key;
-    if (lane < G.k) ord[rank] = (uint8_t)lane;
-  }
-  G.wok = true;
-  if (wcap) {
-    unsigned wt = 0;
-#pragma unroll
-    for (int w = 0; w < W; ++w) wt += __popcll(G.v[w] | G.f0[w]);
-    G.wok = wt <= maxw;  // M is inside v, so every member has this weight
-  }
-  const unsigned size = 1u << G.k;
-  for (unsigned e = lane; e < (size + 31) / 32; e += 32) ex[e] = 0u;
-  __syncwarp();
-  for (uint32_t m = lane; m < cnt; m += 32) {
-    const unsigned c = R.mcoord[start + m];
-    coef[c] = R.mcoef[start + m];
-    atomicOr(&ex[c >> 5], 1u << (c & 31));
-  }
-  __syncwarp();
-}
-
-// The gates of the run in order over the group's slots; children created per gate go to
-// s_created when it is given.  eps of a member with bit t = b:
-//   RX: eps = b ? -1 : +1   (crates/ppvm-pauli-sum/src/sum/rot1.rs:73)
-//   RZ: eps = b ? +1 : -1   (rot1.rs:124)
-template <int W>
-__device__ __forceinline__ void group_butterfly(const RunGroup<W>& G, uint32_t cls, const uint8_t* ord,
-                                                const uint16_t* s_gidx, const double* s_cs, const double* s_sn,
-                                                double* coef, unsigned* ex, unsigned long long* s_created) {
-  const unsigned lane = threadIdx.x & 31;
-  const unsigned size = 1u << G.k;
-  const double eps_a = cls == 0 ? 1.0 : -1.0, eps_b = -eps_a;
-  for (unsigned r = 0; r < G.k; ++r) {
-    const unsigned t = ord[r];
-    const unsigned j = s_gidx[G.pos[t]];
-    const unsigned bit = 1u << t;
-    const double cs = s_cs[j], sn = s_sn[j];
-    unsigned made = 0;
-    for (unsigned p = lane; p < size / 2; p += 32) {
-      const unsigned a = ((p >> t) << (t + 1)) | (p & (bit - 1));
-      const unsigned b = a | bit;
-      const bool ea = (ex[a >> 5] >> (a & 31)) & 1u, eb = (ex[b >> 5] >> (b & 31)) & 1u;
-      if (ea && eb) {
-        const double ca = coef[a], cb = coef[b];
-        coef[a] = __dadd_rn(__dmul_rn(ca, cs), __dmul_rn(cb, eps_b * sn));
-        coef[b] = __dadd_rn(__dmul_rn(cb, cs), __dmul_rn(ca, eps_a * sn));
-      } else if (ea) {
-        const double ca = coef[a];
-        coef[a] = __dmul_rn(ca, cs);
-        coef[b] = __dmul_rn(ca, eps_a * sn);
-        atomicOr(&ex[b >> 5], 1u << (b & 31));
-        ++made;
-      } else if (eb) {
-        const double cb = coef[b];
-        coef[b] = __dmul_rn(cb, cs);
-        coef[a] = __dmul_rn(cb, eps_b * sn);
-        atomicOr(&ex[a >> 5], 1u << (a & 31));
-        ++made;
-      }
+    for (int r = 0; r < NH; ++r) slots[32 * r + lane] = kNoSlot;
+    __syncwarp();
+    for (unsigned m = lane; m < cnt; m += 32) {
+      const unsigned s = mcoord[m];
+      if (NR == NH || (int)(s >> 9) == h) slots[s & (32 * NH - 1)] = link_bits(mcoef[m]);
     }
     __syncwarp();
-    if (s_created) {
 #pragma unroll
-      for (int o = 16; o; o >>= 1) made += __shfl_down_sync(kFull, made, o);
-      if (lane == 0 && made) atomicAdd(&s_created[j], (unsigned long long)made);
+    for (int r = 0; r < NH; ++r) {
+      const unsigned long long u = slots[32 * r + lane];
+      c[h * NH + r] = __longlong_as_double((long long)u);
+      ex |= (unsigned)(u != kNoSlot) << (h * NH + r);
     }
   }
-}
-
-// Survivors of the group (existing slots that pass the run's TRUNCATE), on every lane.
-template <int W>
-__device__ __forceinline__ unsigned group_count(const RunGroup<W>& G, const double* coef, const unsigned* ex,
-                                                int trunc, double thr) {
-  const unsigned lane = threadIdx.x & 31;
-  const unsigned size = 1u << G.k;
-  unsigned mine = 0;
-  for (unsigned c = lane; c < size; c += 32) {
-    const bool e = (ex[c >> 5] >> (c & 31)) & 1u;
-    bool keep = e;
-    if (trunc && e) keep = G.wok && !(fabs(coef[c]) < thr);
-    mine += keep;
-  }
+  for (unsigned i = 0; i < g.k; ++i) {
+    const unsigned t = g.bit[i];
+    const double cs = g.cs[i], sn = g.sn[i];
+    unsigned made;
+    if (t < 5) {
+      const bool hi = (lane >> t) & 1u;
+      const double in = (hi ? eps_a : -eps_a) * sn;  // what the partner's value is worth here
+      const unsigned other = __shfl_xor_sync(kFull, ex, 1u << t);
+      made = hi ? 0u : (unsigned)__popc(ex ^ other);
 #pragma unroll
-  for (int o = 16; o; o >>= 1) mine += __shfl_down_sync(kFull, mine, o);
-  return __shfl_sync(kFull, mine, 0);
-}
-
-// Writes the group's survivors, in coordinate order, to D from index out on.
-template <int W>
-__device__ __forceinline__ void group_write(const RunGroup<W>& G, Planes D, unsigned long long out, uint32_t cls,
-                                            const double* coef, const unsigned* ex, int trunc, double thr) {
-  const unsigned lane = threadIdx.x & 31;
-  const unsigned size = 1u << G.k;
-  for (unsigned c0 = 0; c0 < size; c0 += 32) {
-    const unsigned c = c0 + lane;
-    bool keep = false;
-    if (c < size) {
-      keep = (ex[c >> 5] >> (c & 31)) & 1u;
-      if (trunc && keep) keep = G.wok && !(fabs(coef[c]) < thr);
-    }
-    const unsigned bal = __ballot_sync(kFull, keep);
-    if (keep) {
-      const unsigned long long r = out + __popc(bal & ((1u << lane) - 1u));
-      if (r < D.cap) {
-        uint64_t f[W], x[W], z[W];
+      for (int r = 0; r < NR; ++r) {
+        const double o = __shfl_xor_sync(kFull, c[r], 1u << t);
+        const double own = __dmul_rn(c[r], cs), got = __dmul_rn(o, in), sum = __dadd_rn(own, got);
+        c[r] = (ex >> r) & 1u ? ((other >> r) & 1u ? sum : own) : got;
+      }
+      ex |= other;
+    } else {
+      made = 0;
+      const double ia = -eps_a * sn, ib = eps_a * sn;
 #pragma unroll
-        for (int w = 0; w < W; ++w) f[w] = G.f0[w];
-        for (unsigned t = 0; t < G.k; ++t)
-          if ((c >> t) & 1u) {
-            const unsigned q = G.pos[t];
+      for (int u = 0; (1 << u) < NR; ++u) {
+        if ((int)t - 5 != u) continue;
+        unsigned low = 0;  // registers with bit u clear
 #pragma unroll
-            for (int w = 0; w < W; ++w)
-              if (w == (int)(q >> 6)) f[w] |= 1ull << (q & 63);
+        for (int r = 0; r < NR; ++r)
+          if (!((r >> u) & 1)) {
+            low |= 1u << r;
+            const int q = r | 1 << u;
+            const bool ea = (ex >> r) & 1u, eb = (ex >> q) & 1u;
+            const double ca = c[r], cb = c[q];
+            const double oa = __dmul_rn(ca, cs), ga = __dmul_rn(cb, ia), ob = __dmul_rn(cb, cs), gb = __dmul_rn(ca, ib);
+            c[r] = ea ? (eb ? __dadd_rn(oa, ga) : oa) : ga;
+            c[q] = eb ? (ea ? __dadd_rn(ob, gb) : ob) : gb;
           }
-#pragma unroll
-        for (int w = 0; w < W; ++w) {
-          x[w] = cls == 0 ? f[w] : G.v[w];
-          z[w] = cls == 0 ? G.v[w] : f[w];
-        }
-        store_key<W>(D, r, x, z);
-        D.c[r] = coef[c];
+        const unsigned a = ex & low, b = (ex >> (1 << u)) & low;
+        made = (unsigned)__popc(a ^ b);
+        ex = (a | b) | (a | b) << (1 << u);
       }
     }
-    out += __popc(bal);
+    if (created) {
+      made = __reduce_add_sync(kFull, made);
+      if (lane == 0 && made) atomicAdd(&created[g.gate[i]], made);
+    }
   }
+  unsigned keep = trunc && !wok ? 0u : ex;
+  if (trunc) {
+#pragma unroll
+    for (int r = 0; r < NR; ++r)
+      if (fabs(c[r]) < thr) keep &= ~(1u << r);
+  }
+  const unsigned n = __reduce_add_sync(kFull, __popc(keep));
+  __syncwarp();
+  if (NR == NH || part >= 0) {
+#pragma unroll
+    for (int h = 0; h < NR / NH; ++h)
+      if (NR == NH || h == part) {
+#pragma unroll
+        for (int r = 0; r < NH; ++r)
+          slots[32 * r + lane] = (keep >> (h * NH + r)) & 1u ? link_bits(c[h * NH + r]) : kNoSlot;
+      }
+  }
+  __syncwarp();
+  return n;
 }
+
+// A group as its warp holds it: key, coordinates (lane t's q: the t-th coordinate qubit).
+template <int W>
+struct WarpGroup {
+  uint64_t v[W], f0[W];
+  unsigned k, q;
+  bool wok;  // every member's weight (that of v | f0: the coordinates lie inside v) passes the cap
+
+  __device__ __forceinline__ void coordinates(const uint64_t (&Q)[W], unsigned long long maxw) {
+    const unsigned lane = threadIdx.x & 31;
+    unsigned wt = 0;
+    k = q = 0;
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+      uint64_t m = v[w] & Q[w];
+      const unsigned c = __popcll(m);
+      if (lane >= k && lane < k + c) {
+        for (unsigned u = k; u < lane; ++u) m &= m - 1;
+        q = w * 64 + (unsigned)__ffsll((long long)m) - 1;
+      }
+      k += c;
+      wt += __popcll(v[w] | f0[w]);
+    }
+    wok = maxw == ~0ull || wt <= maxw;
+  }
+
+  // The coordinates' gates, in run order.
+  __device__ __forceinline__ void gates(TileGates& G, const RunDesc* rd, const uint16_t* s_gidx) const {
+    const unsigned lane = threadIdx.x & 31;
+    const unsigned key = lane < k ? s_gidx[q] : 0xFFFFu;
+    unsigned rank = 0;
+    for (unsigned t = 0; t < k; ++t) rank += __shfl_sync(kFull, key, t) < key;
+    __syncwarp();
+    if (lane < k) {
+      G.bit[rank] = (uint8_t)lane;
+      G.gate[rank] = (uint16_t)key;
+      G.cs[rank] = rd->cs[key];
+      G.sn[rank] = rd->sn[key];
+    }
+    if (lane == 0) G.k = k;
+    __syncwarp();
+  }
+
+  // Slots of the warp's shared memory that the group's survivors take (at most kTileSlots at a time).
+  __device__ __forceinline__ unsigned slots() const {
+    return k <= 5 ? 32u : k > 9 ? (unsigned)kTileSlots : 1u << k;
+  }
+
+  __device__ __forceinline__ unsigned survivors(const TileGates& G, unsigned long long* sl, const RunScratch& R,
+                                                unsigned start, unsigned cnt, double eps_a, bool trunc, double thr,
+                                                unsigned* created, int part) const {
+    const uint32_t* mc = R.mcoord + start;
+    const double* mv = R.mcoef + start;
+    if (k <= 5) return tile_survivors<1>(G, sl, mc, mv, cnt, eps_a, trunc, wok, thr, created, part);
+    switch (k) {
+      case 6: return tile_survivors<2>(G, sl, mc, mv, cnt, eps_a, trunc, wok, thr, created, part);
+      case 7: return tile_survivors<4>(G, sl, mc, mv, cnt, eps_a, trunc, wok, thr, created, part);
+      case 8: return tile_survivors<8>(G, sl, mc, mv, cnt, eps_a, trunc, wok, thr, created, part);
+      case 9: return tile_survivors<16>(G, sl, mc, mv, cnt, eps_a, trunc, wok, thr, created, part);
+      default: return tile_survivors<32>(G, sl, mc, mv, cnt, eps_a, trunc, wok, thr, created, part);
+    }
+  }
+
+  // Writes the survivors to O from index `out` on, in coordinate order: from sl where tile_survivors
+  // left them, or (again) after running the group once more through sl; 1024 slots always so.
+  __device__ __forceinline__ void emit(const Planes& O, unsigned long long out, uint32_t cls, TileGates& G,
+                                       unsigned long long* sl, bool again, const RunDesc* rd, const uint16_t* s_gidx,
+                                       const RunScratch& R, unsigned start, unsigned cnt, double eps_a, bool trunc,
+                                       double thr) const {
+    const unsigned lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
+    if (again) {
+      gates(G, rd, s_gidx);
+      if (k <= 9) survivors(G, sl, R, start, cnt, eps_a, trunc, thr, nullptr, -1);
+    }
+    uint64_t fl[W];  // f with this lane's low coordinate bits; a chunk of 32 slots adds its high ones
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+      fl[w] = f0[w];
+#pragma unroll
+      for (unsigned t = 0; t < 5; ++t) {
+        const unsigned qt = __shfl_sync(kFull, q, t);
+        if (t < k && (int)(qt >> 6) == w && ((lane >> t) & 1u)) fl[w] |= 1ull << (qt & 63);
+      }
+    }
+    const unsigned nparts = k > 9 ? 2u : 1u, nchunk = k > 9 ? 16u : k > 5 ? 1u << (k - 5) : 1u;
+    for (unsigned part = 0; part < nparts; ++part) {
+      if (nparts > 1) survivors(G, sl, R, start, cnt, eps_a, trunc, thr, nullptr, (int)part);  // half at a time
+      for (unsigned ch = 0; ch < nchunk; ++ch) {
+        const unsigned long long u = sl[32 * ch + lane];
+        const unsigned bal = __ballot_sync(kFull, u != kNoSlot);
+        uint64_t f[W];
+#pragma unroll
+        for (int w = 0; w < W; ++w) f[w] = fl[w];
+        for (unsigned hb = part * 16 + ch; hb; hb &= hb - 1) {
+          const unsigned qt = __shfl_sync(kFull, q, 4u + (unsigned)__ffs((int)hb));
+#pragma unroll
+          for (int w = 0; w < W; ++w)
+            if ((int)(qt >> 6) == w) f[w] |= 1ull << (qt & 63);
+        }
+        const unsigned long long r = out + __popc(bal & lt);
+        if (u != kNoSlot && r < O.cap) {
+          if (cls == 0) store_key<W>(O, r, f, v);
+          else store_key<W>(O, r, v, f);
+          O.c[r] = __longlong_as_double((long long)u);
+        }
+        out += __popc(bal);
+      }
+      __syncwarp();
+    }
+  }
+};
 
 // ---- lane mode: one group per lane ------------------------------------------------------
 constexpr int kRunLaneK = 3;  // groups of up to 3 coordinates (8 slots) run on one lane
@@ -672,13 +725,12 @@ __device__ __forceinline__ bool lane_key(LaneGroup<W>& G, unsigned long long g, 
 }
 
 // The members and the butterfly of a small group on its lane, the same arithmetic in the same
-// gate order as group_butterfly; children made per gate go to s_created.
+// gate order as tile_survivors; children made per gate go to s_created.
 template <int W>
-__device__ __forceinline__ void lane_run(LaneGroup<W>& G, unsigned long long g, uint32_t cls, const RunScratch& R,
-                                         const uint16_t* s_gidx, const double* s_cs, const double* s_sn,
-                                         unsigned long long* s_created) {
+__device__ __forceinline__ void lane_run(LaneGroup<W>& G, unsigned start, unsigned cnt, uint32_t cls,
+                                         const RunScratch& R, const uint16_t* s_gidx, const double* s_cs,
+                                         const double* s_sn, unsigned* s_created) {
   constexpr int SZ = 1 << kRunLaneK;
-  const uint32_t start = R.g_start[g], cnt = R.g_cnt[g];
   G.ex = 0;
 #pragma unroll
   for (int c = 0; c < SZ; ++c) G.coef[c] = 0.0;
@@ -729,7 +781,7 @@ __device__ __forceinline__ void lane_run(LaneGroup<W>& G, unsigned long long g, 
         if (e == b) G.coef[e] = nb;
       }
     }
-    if (made) atomicAdd(&s_created[j], (unsigned long long)made);
+    if (made) atomicAdd(&s_created[j], made);
   }
 }
 
@@ -775,52 +827,44 @@ __device__ __forceinline__ void lane_write(const LaneGroup<W>& G, Planes D, unsi
   }
 }
 
-// Whether a run's groups go one per lane: forced (tile_mode 3), or chosen for many groups of
-// mostly one member.  Lane mode places its 32-group tiles by look-back, never in scratch
-// mode, so k_run_place makes the same decision to stand aside.
-__device__ __forceinline__ bool run_lanes(unsigned long long ngroups, unsigned long long members, unsigned tile_mode) {
-  return tile_mode == 3 || (tile_mode == 0 && ngroups >= kRunTileMinGroups && 2 * members < 3 * ngroups);
+// Whether a run's groups go one per lane: forced (mode 3), or chosen for many groups of mostly one
+// member.
+__device__ __forceinline__ bool run_lanes(unsigned long long ngroups, unsigned long long members, unsigned mode) {
+  return mode == 3 || (mode == 0 && ngroups >= kRunTileMinGroups && 2 * members < 3 * ngroups);
 }
 
-// The groups of a run, in one of four modes chosen per launch (the same in every block):
-// - one group per lane (at least kRunTileMinGroups groups of fewer than 1.5 members on
-//   average; placed by look-back at any group count): see the lane-mode branch;
-// - one group per warp, taken by ticket (groups of several members): the warp runs the
-//   butterfly, counts the survivors, finds the group's output offset by a warp look-back over
-//   the lower-numbered groups, and writes;
-// - tiles of kRunTileGroups groups per block (tile_mode 1 only; lane mode replaced it in the
-//   automatic choice): warp w takes the tile's groups w,
-//   w + kRunWarps, ...; the warps run every butterfly and count, a block scan orders the
-//   counts, one decoupled look-back places the tile after all lower tiles, and the warps then
-//   write, each warp's last group straight from its slots and the others after running their
-//   butterflies again (the same arithmetic in the same order, so the same coefficients).  One
-//   look-back per tile instead of per group; the second butterfly costs less than the
-//   look-backs it saves only when the butterflies are short;
-// - scratch mode (many groups, when not in lane mode): one group per warp, its survivors
-//   written at once to the scratch planes S wherever a counter puts them; k_run_place then
-//   moves every group's block to its place in O.
-// Every mode writes the same terms in the same order: groups by number, members by
-// coordinate.
+// Whether this launch's groups go one per lane (k_run_lanes) or in tiles (k_run_tiles); both
+// kernels of a run read the same counts and decide alike, and the other returns at once.
+struct RunCounts {
+  unsigned long long groups, members, untouched;
+};
+__device__ __forceinline__ RunCounts run_counts(const Ctrl* ctrl) {
+  return {ld_volatile(&ctrl->n_pairs), ld_volatile(&ctrl->n_side), ld_volatile(&ctrl->n_s)};
+}
+
+// One group per lane, for runs of many small groups (run_lanes).  A warp takes 32 consecutive groups
+// by one ticket.  A group of at most kRunLaneK coordinates runs on its lane alone; the larger ones are
+// run by the whole warp, one after the other, and keep their survivors in the warp's slots as long
+// as these hold them (the rest is run again to be written).  One warp scan and one look-back place
+// the 32 groups.
 template <int W>
-__global__ void __launch_bounds__(kRunWarps * 32)
-k_run_groups(Planes O, Planes S, Ctrl* ctrl, const RunDesc* rd, RunScratch R, int trunc, double thr,
-             unsigned long long maxw, unsigned long long* ts, unsigned epoch, int op, int trunc_op, OpLog* log,
-             unsigned long long scratch_min, unsigned tile_mode) {
+__global__ void __launch_bounds__(kRunWarps * 32, 5)
+k_run_lanes(Planes O, Ctrl* ctrl, const RunDesc* rd, RunScratch R, int trunc, double thr, unsigned long long maxw,
+            unsigned long long* ts, unsigned epoch, int op, int trunc_op, OpLog* log, unsigned mode) {
   pdl_wait();
-  constexpr int SZ = 1 << kRunMaxK;
-  constexpr int GT = kRunTileGroups;
-  __shared__ double s_coef[kRunWarps][SZ];
-  __shared__ unsigned s_ex[kRunWarps][SZ / 32];
-  __shared__ unsigned long long s_created[kRunMaxGates];
+  __shared__ unsigned long long s_slot[kRunWarps][kTileSlots];
+  __shared__ TileGates s_g[kRunWarps];
+  __shared__ unsigned s_created[kRunMaxGates];
   __shared__ double s_cs[kRunMaxGates], s_sn[kRunMaxGates];
-  __shared__ uint16_t s_gidx[64 * W];               // qubit -> its gate's index in the run
-  __shared__ uint8_t s_ord[kRunWarps][kRunMaxK];    // a group's coordinate bits in gate order
-  __shared__ unsigned s_cnt[GT], s_off[GT + 1];
-  __shared__ unsigned s_tile;
-  __shared__ unsigned long long s_slot;
-  __shared__ int s_err;
-  if (threadIdx.x == 0) s_err = ld_volatile_int(&ctrl->err);
-  const uint32_t L = rd->L;
+  __shared__ uint16_t s_gidx[64 * W];  // qubit -> its gate's index in the run
+  const RunCounts rc = run_counts(ctrl);
+  if (ld_volatile_int(&ctrl->err) || !run_lanes(rc.groups, rc.members, mode)) return;
+  const unsigned long long ngroups = rc.groups, ubase = rc.untouched;  // untouched survivors go first
+  const unsigned long long ntiles = (ngroups + 31) / 32;
+  const unsigned long long want = (ntiles + kRunWarps - 1) / kRunWarps;
+  const unsigned blocks = (unsigned)(want < 1 ? 1 : want < gridDim.x ? want : gridDim.x);
+  if (blockIdx.x >= blocks) return;
+  const uint32_t L = rd->L, cls = rd->cls;
   for (unsigned j = threadIdx.x; j < L; j += blockDim.x) {
     s_created[j] = 0;
     s_cs[j] = rd->cs[j];
@@ -828,165 +872,267 @@ k_run_groups(Planes O, Planes S, Ctrl* ctrl, const RunDesc* rd, RunScratch R, in
     s_gidx[rd->q[j]] = (uint16_t)j;  // the qubits of a run are distinct
   }
   __syncthreads();
-  if (s_err) return;
-  const unsigned long long ngroups = ld_volatile(&ctrl->n_pairs);
-  const unsigned long long ubase = ld_volatile(&ctrl->n_s);  // untouched survivors go first
-  const unsigned long long members = ld_volatile(&ctrl->n_side);
-  const bool lanes = run_lanes(ngroups, members, tile_mode);  // the same in every block
-  const bool scratch = !lanes && ngroups >= scratch_min;
-  const uint32_t cls = rd->cls;
+  uint64_t Q[W];
+#pragma unroll
+  for (int w = 0; w < W; ++w) Q[w] = rd->Q[w];
   const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool wcap = maxw != ~0ull;
-  double* coef = s_coef[warp];
-  unsigned* ex = s_ex[warp];
-  uint8_t* ord = s_ord[warp];
-  const bool tiled = !lanes && !scratch && tile_mode == 1;
-  if (lanes) {
-    // lane mode: a warp takes 32 consecutive groups by one ticket.  A group of at most
-    // kRunLaneK coordinates runs on its lane alone; a larger one is run by the whole warp.
-    // One warp scan and one look-back place the 32 groups, and
-    // the warp runs its large groups again to write them.
-    const unsigned long long ntiles = (ngroups + 31) / 32;
-    for (;;) {
-      unsigned long long t = 0;
-      if (lane == 0) t = atomicAdd(&ctrl->tickets[2], 1ull);
-      t = __shfl_sync(kFull, t, 0);
-      if (t >= ntiles) break;
-      const unsigned long long g = t * 32 + lane;
-      const bool valid = g < ngroups;
-      LaneGroup<W> LG;
-      bool small = false;
-      unsigned mine = 0;
-      if (valid) {
-        small = lane_key<W>(LG, g, rd, R, s_gidx, wcap, maxw);
-        if (small) {
-          lane_run<W>(LG, g, cls, R, s_gidx, s_cs, s_sn, s_created);
+  const double eps_a = cls == 0 ? 1.0 : -1.0;
+  TileGates& G = s_g[warp];
+  unsigned long long* slots = s_slot[warp];
+  for (;;) {
+    unsigned long long t = 0;
+    if (lane == 0) t = atomicAdd(&ctrl->tickets[2], 1ull);
+    t = __shfl_sync(kFull, t, 0);
+    if (t >= ntiles) break;
+    const unsigned long long g = t * 32 + lane;
+    const bool valid = g < ngroups;
+    LaneGroup<W> LG;
+    bool small = false;
+    unsigned mine = 0, gs = 0, gc = 0;
+    if (valid) {
+      gs = R.g_start[g];
+      gc = R.g_cnt[g];
+      small = lane_key<W>(LG, g, rd, R, s_gidx, wcap, maxw);
+      if (small) {
+        lane_run<W>(LG, gs, gc, cls, R, s_gidx, s_cs, s_sn, s_created);
 #pragma unroll
-          for (int c = 0; c < (1 << kRunLaneK); ++c)
-            if (c < (1 << LG.k)) mine += lane_keep<W>(LG, c, trunc, thr);
-        }
-      }
-      const unsigned big = __ballot_sync(kFull, valid && !small);
-      for (unsigned bb = big; bb; bb &= bb - 1) {
-        const unsigned l = (unsigned)(__ffs(bb) - 1);
-        RunGroup<W> G;
-        group_load<W>(G, t * 32 + l, rd, R, s_gidx, ord, coef, ex, wcap, maxw);
-        group_butterfly<W>(G, cls, ord, s_gidx, s_cs, s_sn, coef, ex, s_created);
-        const unsigned m = group_count<W>(G, coef, ex, trunc, thr);
-        if (lane == l) mine = m;
-        __syncwarp();
-      }
-      unsigned incl = mine;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const unsigned v = __shfl_up_sync(kFull, incl, o);
-        if (lane >= (unsigned)o) incl += v;
-      }
-      const unsigned total = __shfl_sync(kFull, incl, 31);
-      const unsigned pre = incl - mine;
-      const unsigned long long base = ubase + warp_lookback(ts, t, total, epoch, ctrl, op);
-      const Planes D = O;
-      if (valid && small) lane_write<W>(LG, D, base + pre, cls, trunc, thr);
-      for (unsigned bb = big; bb; bb &= bb - 1) {
-        const unsigned l = (unsigned)(__ffs(bb) - 1);
-        const unsigned long long at = base + __shfl_sync(kFull, pre, l);
-        __syncwarp();
-        RunGroup<W> G;
-        group_load<W>(G, t * 32 + l, rd, R, s_gidx, ord, coef, ex, wcap, maxw);
-        group_butterfly<W>(G, cls, ord, s_gidx, s_cs, s_sn, coef, ex, nullptr);
-        group_write<W>(G, D, at, cls, coef, ex, trunc, thr);
-      }
-      if (t == ntiles - 1 && lane == 0) {
-        ctrl->cap_needed = base + total;
-        if (base + total > O.cap) set_err(ctrl, kErrCapacity, op);
-      }
-      __syncwarp();
-    }
-  } else
-  if (!tiled) {
-    for (;;) {
-      unsigned long long g = 0;
-      if (lane == 0) g = atomicAdd(&ctrl->tickets[2], 1ull);
-      g = __shfl_sync(kFull, g, 0);
-      if (g >= ngroups) break;
-      RunGroup<W> G;
-      group_load<W>(G, g, rd, R, s_gidx, ord, coef, ex, wcap, maxw);
-      group_butterfly<W>(G, cls, ord, s_gidx, s_cs, s_sn, coef, ex, s_created);
-      const unsigned mine = group_count<W>(G, coef, ex, trunc, thr);
-      if (scratch) {
-        unsigned long long b = 0;
-        if (lane == 0) {
-          b = atomicAdd(&ctrl->scr_top, (unsigned long long)mine);
-          R.g_rep[g] = (uint32_t)(b < 0xFFFFFFFFull ? b : 0xFFFFFFFFull);  // scratch offset (< capacity < 2^32)
-          R.g_fill[g] = mine;                                                // survivors
-        }
-        group_write<W>(G, S, __shfl_sync(kFull, b, 0), cls, coef, ex, trunc, thr);
-      } else {
-        const unsigned long long excl = warp_lookback(ts, g, mine, epoch, ctrl, op);
-        group_write<W>(G, O, ubase + excl, cls, coef, ex, trunc, thr);
-        if (g == ngroups - 1 && lane == 0) {
-          ctrl->cap_needed = ubase + excl + mine;
-          if (ubase + excl + mine > O.cap) set_err(ctrl, kErrCapacity, op);
-        }
-      }
-      __syncwarp();  // the slots and the order array are rewritten by the warp's next group
-    }
-  } else {
-    const unsigned long long ntiles = (ngroups + GT - 1) / GT;
-    for (;;) {
-      const unsigned tile = next_tile(&ctrl->tickets[2], &s_tile);
-      if (tile >= ntiles) break;
-      const unsigned long long g0 = (unsigned long long)tile * GT;
-      const unsigned ng = (unsigned)min((unsigned long long)GT, ngroups - g0);
-      RunGroup<W> G;
-      unsigned last = GT;  // this warp's last group of the tile (its slots stay loaded)
-      for (unsigned j = warp; j < ng; j += kRunWarps) {
-        group_load<W>(G, g0 + j, rd, R, s_gidx, ord, coef, ex, wcap, maxw);
-        group_butterfly<W>(G, cls, ord, s_gidx, s_cs, s_sn, coef, ex, s_created);
-        const unsigned mine = group_count<W>(G, coef, ex, trunc, thr);
-        if (lane == 0) s_cnt[j] = mine;
-        last = j;
-        __syncwarp();  // the slots and the order array are rewritten by the warp's next group
-      }
-      __syncthreads();
-      if (warp == 0) {  // exclusive scan of the tile's counts (GT <= 32)
-        const unsigned c = lane < ng ? s_cnt[lane] : 0u;
-        unsigned v = c;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const unsigned t = __shfl_up_sync(kFull, v, o);
-          if (lane >= (unsigned)o) v += t;
-        }
-        if (lane < GT) s_off[lane] = v - c;
-        if (lane == 31) s_off[GT] = v;
-      }
-      __syncthreads();
-      const unsigned long long total = s_off[GT];
-      const unsigned long long excl = lookback(ts, tile, total, epoch, ctrl, op, &s_slot);
-      const unsigned long long out0 = ubase + excl;
-      if (last < GT) {  // a warp without a group in a short last tile writes nothing
-        group_write<W>(G, O, out0 + s_off[last], cls, coef, ex, trunc, thr);
-        for (unsigned j = warp; j < last; j += kRunWarps) {
-          __syncwarp();
-          group_load<W>(G, g0 + j, rd, R, s_gidx, ord, coef, ex, wcap, maxw);
-          group_butterfly<W>(G, cls, ord, s_gidx, s_cs, s_sn, coef, ex, nullptr);
-          group_write<W>(G, O, out0 + s_off[j], cls, coef, ex, trunc, thr);
-        }
-      }
-      __syncwarp();
-      if (tile == ntiles - 1 && threadIdx.x == 0) {
-        ctrl->cap_needed = out0 + total;
-        if (out0 + total > O.cap) set_err(ctrl, kErrCapacity, op);
+        for (int c = 0; c < (1 << kRunLaneK); ++c)
+          if (c < (1 << LG.k)) mine += lane_keep<W>(LG, c, trunc, thr);
       }
     }
+    const unsigned big = __ballot_sync(kFull, valid && !small);
+    unsigned off = kTileSlots, used = 0;  // a large group's slots (kTileSlots: none kept)
+    auto large = [&](WarpGroup<W>& B, unsigned l) {  // lane l's group on the warp
+#pragma unroll
+      for (int w = 0; w < W; ++w) {
+        B.v[w] = __shfl_sync(kFull, LG.v[w], l);
+        B.f0[w] = __shfl_sync(kFull, LG.f0[w], l);
+      }
+      B.coordinates(Q, maxw);
+    };
+    for (unsigned bb = big; bb; bb &= bb - 1) {
+      const unsigned l = (unsigned)(__ffs(bb) - 1);
+      WarpGroup<W> B;
+      large(B, l);
+      B.gates(G, rd, s_gidx);
+      const unsigned size = B.slots();
+      const bool fits = B.k <= 9 && used + size <= (unsigned)kTileSlots;
+      if (!fits) {  // it goes through the slots from the first on: what was kept there is run again too
+        off = kTileSlots;
+        used = kTileSlots;
+      }
+      const unsigned at = fits ? used : 0u;
+      const unsigned n = B.survivors(G, slots + at, R, __shfl_sync(kFull, gs, l), __shfl_sync(kFull, gc, l), eps_a,
+                                     trunc, thr, s_created, -1);
+      if (fits) used += size;
+      if (lane == l) {
+        mine = n;
+        off = fits ? at : (unsigned)kTileSlots;
+      }
+    }
+    unsigned incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned v = __shfl_up_sync(kFull, incl, o);
+      if (lane >= (unsigned)o) incl += v;
+    }
+    const unsigned total = __shfl_sync(kFull, incl, 31);
+    const unsigned pre = incl - mine;
+    const unsigned long long base = ubase + warp_lookback(ts, t, total, epoch, ctrl, op);
+    if (valid && small) lane_write<W>(LG, O, base + pre, cls, trunc, thr);
+    for (unsigned bb = __ballot_sync(kFull, valid && !small && mine); bb; bb &= bb - 1) {
+      const unsigned l = (unsigned)(__ffs(bb) - 1);
+      const unsigned long long at = base + __shfl_sync(kFull, pre, l);
+      const unsigned o = __shfl_sync(kFull, off, l);
+      WarpGroup<W> B;
+      large(B, l);
+      const bool again = o >= (unsigned)kTileSlots;
+      B.emit(O, at, cls, G, slots + (again ? 0u : o), again, rd, s_gidx, R, __shfl_sync(kFull, gs, l),
+             __shfl_sync(kFull, gc, l), eps_a, trunc, thr);
+    }
+    if (t == ntiles - 1 && lane == 0) {
+      ctrl->cap_needed = base + total;
+      if (base + total > O.cap) set_err(ctrl, kErrCapacity, op);
+    }
+    __syncwarp();
   }
   __syncthreads();
   for (unsigned j = threadIdx.x; j < L; j += blockDim.x)
-    if (s_created[j]) atomicAdd(&R.created[j], s_created[j]);
-  if (last_block_done(&ctrl->done) && warp == 0) run_commit(ctrl, R, op, (int)L, trunc_op, log, scratch, O.cap);
+    if (s_created[j]) atomicAdd(&R.created[j], (unsigned long long)s_created[j]);
+  if (last_of_blocks(&ctrl->done, blocks) && warp == 0) run_commit(ctrl, R, op, (int)L, trunc_op, log, false, O.cap);
 }
 
-// Scratch mode of a fused run (many groups): k_run_groups left each group's survivors in a
+constexpr unsigned long long kTileManyGroups = 1ull << 15;  // from here on a warp takes several groups of a tile
+
+// The groups of a run in tiles of consecutive groups, a tile per block and ticket, PER groups per warp:
+// keys and coordinates, the butterflies in registers (tile_survivors), one look-back per tile for
+// the output offset, and the survivors written chunk by chunk of 32 slots, in coordinate order.
+// PER is 1 below kTileManyGroups groups, where a tile's latency is what counts (ticket, dependent
+// loads, look-back, about a microsecond each), and 4 (2 above 256 qubits) from there on, where the look-backs and barriers per group
+// do: the warp's keys, starts and members then come in one load each.  A warp whose groups do not fit
+// its slots together runs those that are left out again to write them.
+// From scratch_min groups on the tiles' order is left to k_run_place (scratch mode): waiting for
+// its place, every tile in flight waits for the slowest before it (RX run of 2.6M groups, 1 in
+// 500 of 8 to 10 coordinates: 6.9 ms in order).
+template <int W>
+__global__ void __launch_bounds__(kTileWarps * 32, 3)
+k_run_tiles(Planes O, Planes S, Ctrl* ctrl, const RunDesc* rd, RunScratch R, int trunc, double thr,
+            unsigned long long maxw, unsigned long long* ts, unsigned epoch, int op, int trunc_op, OpLog* log,
+            unsigned long long scratch_min, unsigned mode) {
+  pdl_wait();
+  constexpr int BLOCK = kTileWarps * 32;
+  constexpr unsigned MANY = W <= 4 ? 4 : 2;  // a warp's keys: MANY * 2W <= 32 words, one per lane
+  __shared__ unsigned long long s_slot[kTileWarps][kTileSlots];
+  __shared__ TileGates s_g[kTileWarps];
+  __shared__ unsigned s_created[kRunMaxGates];
+  __shared__ uint16_t s_gidx[64 * W];  // qubit -> its gate's index in the run
+  __shared__ unsigned s_cnt[kTileWarps], s_tile;
+  __shared__ unsigned long long s_base;
+  const RunCounts rc = run_counts(ctrl);
+  if (ld_volatile_int(&ctrl->err) || run_lanes(rc.groups, rc.members, mode)) return;
+  const unsigned long long ngroups = rc.groups, ubase = rc.untouched;  // untouched survivors go first
+  const bool scratch = ngroups >= scratch_min;  // the same in every block
+  const unsigned per = scratch || ngroups >= kTileManyGroups ? MANY : 1u;
+  const unsigned long long ntiles = (ngroups + kTileWarps * per - 1) / (kTileWarps * per);
+  const unsigned blocks = (unsigned)(ntiles < 1 ? 1 : ntiles < gridDim.x ? ntiles : gridDim.x);
+  if (blockIdx.x >= blocks) return;
+  const uint32_t L = rd->L, cls = rd->cls;
+  for (unsigned j = threadIdx.x; j < L; j += BLOCK) {
+    s_created[j] = 0;
+    s_gidx[rd->q[j]] = (uint16_t)j;  // the qubits of a run are distinct
+  }
+  uint64_t Q[W];
+#pragma unroll
+  for (int w = 0; w < W; ++w) Q[w] = rd->Q[w];
+  const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const double eps_a = cls == 0 ? 1.0 : -1.0;
+  TileGates& G = s_g[warp];
+  unsigned long long* slots = s_slot[warp];
+  // The warp's groups of a tile; per lane b: group b's start, members, survivors and slots (kTileSlots:
+  // none kept), beside one word of the warp's keys.
+  struct Held {
+    uint64_t kw;
+    unsigned gs, gc, n, off, ng;
+  } H;
+  auto load = [&](WarpGroup<W>& B, unsigned b) {
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+      B.v[w] = __shfl_sync(kFull, H.kw, b * 2 * W + w);
+      B.f0[w] = __shfl_sync(kFull, H.kw, b * 2 * W + W + w);
+    }
+    B.coordinates(Q, maxw);
+  };
+  // Groups g0, g0 + 1, ... (at most per): run and counted; returns their survivors.
+  auto count = [&](unsigned long long g0) -> unsigned {
+    H.ng = g0 >= ngroups ? 0u : (unsigned)(ngroups - g0 < per ? ngroups - g0 : per);
+    H.kw = lane < H.ng * 2 * W ? R.gkey[g0 * 2 * W + lane] : 0ull;
+    H.gs = lane < H.ng ? R.g_start[g0 + lane] : 0u;
+    H.gc = lane < H.ng ? R.g_cnt[g0 + lane] : 0u;
+    H.n = 0;
+    H.off = kTileSlots;
+    if (H.ng > 1) {  // the members of all the warp's groups lie together: on their way while the keys are read
+      const unsigned m0 = __shfl_sync(kFull, H.gs, 0);
+      const unsigned m1 = __shfl_sync(kFull, H.gs, H.ng - 1) + __shfl_sync(kFull, H.gc, H.ng - 1);
+      if (m0 + lane * 4 < m1) {
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(R.mcoef + m0 + lane * 4));
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(R.mcoord + m0 + lane * 4));
+      }
+    }
+    unsigned used = 0, mine = 0;
+    for (unsigned b = 0; b < H.ng; ++b) {
+      WarpGroup<W> B;
+      load(B, b);
+      B.gates(G, rd, s_gidx);
+      const unsigned size = B.slots();
+      const bool fits = B.k <= 9 && used + size <= (unsigned)kTileSlots;
+      if (!fits) {  // it goes through the slots from the first on: what was kept there is run again too
+        if (lane < b) H.off = kTileSlots;
+        used = kTileSlots;
+      }
+      const unsigned off = fits ? used : 0u;
+      const unsigned n = B.survivors(G, slots + off, R, __shfl_sync(kFull, H.gs, b), __shfl_sync(kFull, H.gc, b), eps_a,
+                                     trunc, thr, s_created, -1);
+      if (fits) used += size;
+      if (lane == b) {
+        H.n = n;
+        H.off = fits ? off : (unsigned)kTileSlots;
+      }
+      mine += n;
+    }
+    return mine;
+  };
+  // Their survivors to D, from index `out` on.
+  auto emit = [&](const Planes& D, unsigned long long out) {
+    for (unsigned b = 0; b < H.ng; ++b) {
+      const unsigned n = __shfl_sync(kFull, H.n, b);
+      if (n == 0) continue;
+      const unsigned off = __shfl_sync(kFull, H.off, b);
+      const bool again = off >= (unsigned)kTileSlots;
+      WarpGroup<W> B;
+      load(B, b);
+      B.emit(D, out, cls, G, slots + (again ? 0u : off), again, rd, s_gidx, R, __shfl_sync(kFull, H.gs, b),
+             __shfl_sync(kFull, H.gc, b), eps_a, trunc, thr);
+      out += n;
+    }
+  };
+  __syncthreads();
+  if (scratch) {
+    // many groups: the warps work on their own, each one's survivors to the scratch planes wherever a
+    // counter puts them; k_run_place moves every group's block to its place
+    for (;;) {
+      unsigned long long t = 0;
+      if (lane == 0) t = atomicAdd(&ctrl->tickets[2], 1ull);
+      const unsigned long long g0 = __shfl_sync(kFull, t, 0) * per;
+      if (g0 >= ngroups) break;
+      const unsigned mine = count(g0);
+      unsigned long long at = 0;
+      if (lane == 0) at = atomicAdd(&ctrl->scr_top, (unsigned long long)mine);
+      at = __shfl_sync(kFull, at, 0);
+      unsigned pre = H.n;  // lane b: survivors of the groups up to b
+#pragma unroll
+      for (int o = 1; o < 4; o <<= 1) {
+        const unsigned u = __shfl_up_sync(kFull, pre, o);
+        if (lane >= (unsigned)o) pre += u;
+      }
+      if (lane < H.ng) {
+        const unsigned long long b = at + pre - H.n;
+        R.g_rep[g0 + lane] = (uint32_t)(b < 0xFFFFFFFFull ? b : 0xFFFFFFFFull);  // (< capacity < 2^32)
+        R.g_fill[g0 + lane] = H.n;
+      }
+      emit(S, at);
+      __syncwarp();
+    }
+  } else {
+    while (ntiles) {
+      const unsigned tile = next_tile(&ctrl->tickets[2], &s_tile);
+      if (tile >= ntiles) break;
+      const unsigned mine = count(((unsigned long long)tile * kTileWarps + warp) * per);
+      if (lane == 0) s_cnt[warp] = mine;
+      __syncthreads();
+      unsigned total = 0, before = 0;
+#pragma unroll
+      for (int w = 0; w < kTileWarps; ++w) {
+        const unsigned n = s_cnt[w];
+        if (w < (int)warp) before += n;
+        total += n;
+      }
+      const unsigned long long base = ubase + lookback(ts, tile, total, epoch, ctrl, op, &s_base);
+      if (tile == ntiles - 1 && threadIdx.x == 0) {
+        ctrl->cap_needed = base + total;
+        if (base + total > O.cap) set_err(ctrl, kErrCapacity, op);
+      }
+      emit(O, base + before);
+    }
+  }
+  __syncthreads();
+  for (unsigned j = threadIdx.x; j < L; j += BLOCK)
+    if (s_created[j]) atomicAdd(&R.created[j], (unsigned long long)s_created[j]);
+  if (last_of_blocks(&ctrl->done, blocks) && warp == 0)
+    run_commit(ctrl, R, op, (int)L, trunc_op, log, scratch, O.cap);
+}
+
+// Scratch mode of a fused run (many groups): k_run_tiles left each group's survivors in a
 // contiguous block of the scratch planes S, at R.g_rep[g] (R.g_fill[g] of them).  Groups are
 // taken in tiles of BLOCK * ITEMS, in group order: one decoupled look-back per tile gives the
 // tile's output offset, a block scan the offsets of its groups, and the block's warps then
@@ -995,7 +1141,7 @@ k_run_groups(Planes O, Planes S, Ctrl* ctrl, const RunDesc* rd, RunScratch R, in
 template <int W, int BLOCK, int ITEMS>
 __global__ void __launch_bounds__(BLOCK)
 k_run_place(Planes S, Planes O, Ctrl* ctrl, RunScratch R, unsigned long long scratch_min, unsigned long long* ts,
-            unsigned epoch, int op, unsigned tile_mode) {
+            unsigned epoch, int op, unsigned mode) {
   pdl_wait();
   constexpr int NW = BLOCK / 32;
   constexpr int TILE = BLOCK * ITEMS;
@@ -1008,7 +1154,7 @@ k_run_place(Planes S, Planes O, Ctrl* ctrl, RunScratch R, unsigned long long scr
   if (threadIdx.x == 0) {
     const unsigned long long ng = ld_volatile(&ctrl->n_pairs);
     s_skip = ld_volatile_int(&ctrl->err) || ng == 0 || ng < scratch_min ||
-             run_lanes(ng, ld_volatile(&ctrl->n_side), tile_mode);
+             run_lanes(ng, ld_volatile(&ctrl->n_side), mode);
   }
   __syncthreads();
   if (s_skip) return;  // the same in every block (look-back mode, or an earlier error)

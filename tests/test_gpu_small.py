@@ -19,7 +19,8 @@ import pytest
 from ppvm_b200 import gates as G
 from ppvm_b200.paulisum import PauliSum
 
-from tests.helpers import oracle_dict, oracle_from, term_dict
+from tests.helpers import oracle_from
+from tests.test_gpu_parity import same, same_set
 
 pytestmark = pytest.mark.gpu
 
@@ -107,13 +108,11 @@ def test_interpreter_matches_the_oracle(exact):
         s.run(ops)
         want = o.run_ops(ops, counts=True)
         assert np.array_equal(s.live_counts(), want), n
-        assert term_dict(*s.export(), n) == oracle_dict(o), n
+        same_set(s, o)
         for op in ops[:12]:  # one call per op
             s.run([op])
             o.run_ops([op])
-        assert term_dict(*s.export(), n) == oracle_dict(o), n
-        if exact:
-            assert all(np.array_equal(a, b) for a, b in zip(s.export(), o.export())), n
+        (same if exact else same_set)(s, o)
 
 
 def test_parity_cases_through_the_pipelines():
