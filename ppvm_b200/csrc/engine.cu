@@ -464,7 +464,7 @@ ppvm_status grow(ppvm_sum* s, unsigned long long new_cap) {
   CUDA_TRY(pool_malloc((void**)&s->table, sizeof(unsigned long long) * s->table_cap, site));
   CUDA_TRY(cudaMemsetAsync(s->table, 0, sizeof(unsigned long long) * s->table_cap, s->stream));
   s->table_epoch = 0;
-  // one tile-state word per look-back tile: the smallest tile is k_run_groups' kRunWarps groups
+  // tile-state words: one per look-back tile, a group or more each
   s->tstate_cap = new_cap + 64;  // one tile-state word per group of a fused run at most
   CUDA_TRY(pool_malloc((void**)&s->tstate, sizeof(unsigned long long) * s->tstate_cap, site));
   CUDA_TRY(cudaMemsetAsync(s->tstate, 0, sizeof(unsigned long long) * s->tstate_cap, s->stream));
@@ -1008,7 +1008,7 @@ struct K {
     PPVM_TRY(stage_put(s, &rd, sizeof(RunDesc), &d_rd_v));
     const RunDesc* d_rd = static_cast<const RunDesc*>(d_rd_v);
     // grp_min, grp_cnt and created are clean here: k_run_scatter and the last block of
-    // k_run_groups reset what a run used, grow() clears them on allocation and run_list()
+    // k_run_tiles or k_run_lanes reset what a run used, grow() clears them on allocation and run_list()
     // after a device error
     const int trunc = trunc_op >= 0 ? 1 : 0;
     {
@@ -1215,6 +1215,15 @@ struct K {
     k_shard_scatter<W><<<(unsigned)ntiles, kShardBlock, 0, s->stream>>>(P, N, m, nparts, hist, rows);
     k_shard_append<W><<<1, 32, 0, s->stream>>>(P, s->d_ctrl, nullptr, 0ull, 0ull);  // the sum is now empty
     s->launch_count += 4;
+  }
+  static void shard_rows(ppvm_sum* s, uint64_t* rows) {
+    const Planes P = s->planes_view();
+    k_shard_rows<W><<<grid_for(s->n_host, 256, 8), 256, 0, s->stream>>>(P, s->n_host, rows);
+    k_shard_append<W><<<1, 32, 0, s->stream>>>(P, s->d_ctrl, nullptr, 0ull, 0ull);  // the sum is now empty
+    s->launch_count += 2;
+  }
+  static void copy_terms(const Planes& A, const Planes& B, unsigned long long n, cudaStream_t st) {
+    if (n) k_copy_terms<W><<<grid_for(n, 256, 8), 256, 0, st>>>(A, B, n);
   }
   static void shard_append(ppvm_sum* s, const uint64_t* rows, unsigned long long k) {
     k_shard_append<W><<<(unsigned)grid_for(k, 256, 8), 256, 0, s->stream>>>(s->planes_view(), s->d_ctrl, rows, k,
@@ -1958,9 +1967,8 @@ ppvm_status ppvm_sum_clone(const ppvm_sum* src, ppvm_sum** out) {
                             src->flags, src->device));
   ppvm_sum* s = const_cast<ppvm_sum*>(src);
   CUDA_TRY(cudaStreamSynchronize(s->stream));
-  for (int w = 0; w < 2 * src->W + 1; ++w)
-    CUDA_TRY(cudaMemcpyAsync(d->planes + (size_t)w * d->cap, src->planes + (size_t)w * src->cap,
-                             sizeof(uint64_t) * src->n_host, cudaMemcpyDeviceToDevice, d->stream));
+  DISPATCH_W(d->W, copy_terms(src->planes_view(), d->planes_view(), src->n_host, d->stream));
+  CUDA_TRY(cudaGetLastError());
   d->n_host = src->n_host;
   d->n_ub = src->n_host;
   d->maxlw = src->maxlw;
@@ -2039,6 +2047,18 @@ ppvm_status ppvm_sum_shard_export(ppvm_sum* s, const uint64_t* mask_x, const uin
   for (int w = 0; w < s->W; ++w) {
     m.gx[w] = mask_x[w];
     m.gz[w] = mask_z[w];
+  }
+  if (n_parts == 1) {
+    DISPATCH_W(s->W, shard_rows(s, static_cast<uint64_t*>(d_rows)));
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
+    if (e != cudaSuccess) {
+      s->poisoned = true;
+      return fail(PPVM_ECUDA, std::string("shard export: ") + cudaGetErrorString(e));
+    }
+    counts[0] = N;
+    s->n_host = s->n_ub = 0;
+    return PPVM_OK;
   }
   const unsigned long long ntiles = (N + kShardBlock - 1) / kShardBlock;
   unsigned long long* hist = nullptr;

@@ -9,7 +9,7 @@
 // [0, 2^|M|).  The reference processes the run gate by gate over the whole map
 // (PauliSum::map_insert per gate, crates/ppvm-pauli-sum/src/sum/data.rs:204-226); here each
 // group is loaded once, the gates of the run are applied in the same order with the same
-// arithmetic as a butterfly over coordinates c in shared memory (existence tracked
+// arithmetic as a butterfly over coordinates c in registers (existence tracked
 // separately from the coefficient, as a map entry exists even with coefficient 0), and the
 // truncation that ends the run is applied before anything is written back.  The term set
 // and every coefficient are identical to the reference's; only the output order differs
@@ -18,15 +18,16 @@
 // Kernels, in order: k_run_classify (group keys into a hash table, members counted; terms
 // outside every group compacted to the output with the truncation), k_run_order
 // (deterministic group numbering by first member, member offsets), k_run_scatter (member
-// lists), k_run_groups (butterfly + truncation + ordered write; its last block publishes the
-// counts and the op log).
+// lists), then k_run_tiles or, for many single-member groups, k_run_lanes (butterfly + truncation +
+// ordered write; the last block publishes the counts and the op log), and k_run_place when the
+// tiles left their order to it.
 #pragma once
 
 #include "kernels.cuh"
 
 namespace ppvm {
 
-constexpr int kRunMaxK = 10;       // groups up to 2^10 coordinates in shared memory
+constexpr int kRunMaxK = 10;       // groups of up to 10 coordinates (2^10 slots) are fused
 constexpr int kRunMaxGates = 256;  // gates per fused run
 constexpr int kRunWarps = 4;       // warps of a k_run_lanes block
 constexpr unsigned long long kRunTileMinGroups = 8192;  // fewer groups: never one per lane
@@ -321,9 +322,9 @@ k_run_order(Ctrl* ctrl, RunScratch R, unsigned long long* ts_a, unsigned long lo
 }
 
 // Lays out each group's members contiguously, as (coordinate index, coefficient) records,
-// and the group's key (from its representative), so k_run_groups reads one span per group
+// and the group's key (from its representative), so that the group kernels read one span per group
 // instead of gathering members by index.  A member's coordinate index has bit t set when f
-// has a 1 at the t-th lowest qubit of M = v & Q (the order k_run_groups uses).  Also hands
+// has a 1 at the t-th lowest qubit of M = v & Q (the order the group kernels use).  Also hands
 // the group table back clean: grp_min and grp_cnt were last read by k_run_order, so every
 // member resets its slot (same values from every member), and the next run needs no
 // clearing pass.  After a device error the host clears both arrays instead.
@@ -969,12 +970,15 @@ constexpr unsigned long long kTileManyGroups = 1ull << 15;  // from here on a wa
 // keys and coordinates, the butterflies in registers (tile_survivors), one look-back per tile for
 // the output offset, and the survivors written chunk by chunk of 32 slots, in coordinate order.
 // PER is 1 below kTileManyGroups groups, where a tile's latency is what counts (ticket, dependent
-// loads, look-back, about a microsecond each), and 4 (2 above 256 qubits) from there on, where the look-backs and barriers per group
-// do: the warp's keys, starts and members then come in one load each.  A warp whose groups do not fit
-// its slots together runs those that are left out again to write them.
+// loads, look-back, about a microsecond each), and 4 (2 above 256 qubits) from there on, where the
+// look-backs and barriers per group do: the warp's keys, starts and members then come in one load
+// each.  A warp whose groups do not fit its slots together runs those that are left out again to
+// write them.  On the 12 x 12 headline (5,400 groups of 120 slots, 640,000 terms out) a run takes 54 us;
+// one warp per group in shared memory, placed group by group, took 72.
 // From scratch_min groups on the tiles' order is left to k_run_place (scratch mode): waiting for
 // its place, every tile in flight waits for the slowest before it (RX run of 2.6M groups, 1 in
-// 500 of 8 to 10 coordinates: 6.9 ms in order).
+// 500 of 8 to 10 coordinates: 6.9 ms in order, 4.3 + 1.6 ms placed; 4.4 + 1.5 with a warp per group
+// and two atomics each).
 template <int W>
 __global__ void __launch_bounds__(kTileWarps * 32, 3)
 k_run_tiles(Planes O, Planes S, Ctrl* ctrl, const RunDesc* rd, RunScratch R, int trunc, double thr,
