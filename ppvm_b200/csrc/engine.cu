@@ -1909,6 +1909,7 @@ namespace ppvm {
 cudaError_t cache_malloc(void** out, size_t bytes) { return pool_malloc(out, bytes); }
 void cache_free(void* p) { pool_free(p); }
 void release_batch_staging();  // batch.cu: frees the pinned staging buffer of the uploads
+void release_mlp_staging();    // learned.cu: frees the kept pinned buffer of the sample orders
 }  // namespace ppvm
 
 extern "C" {
@@ -2644,6 +2645,7 @@ ppvm_status ppvm_release_cached_memory(void) {
   }
   for (ppvm_sum* h : handles) destroy_now(h);  // their buffers go back to the pool first
   ppvm::release_batch_staging();
+  ppvm::release_mlp_staging();
   std::lock_guard<std::mutex> lk(g_pool_mu);
   for (int d = 0; d < 64; ++d) {
     if (g_pool_free[d].empty()) continue;

@@ -13,6 +13,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -40,7 +41,7 @@ struct ppvm_mlp {
   float* d_tgt = nullptr;
   uint32_t* d_order = nullptr;  // sample orders and learning rates of two epochs, and their pinned twin
   uint32_t* h_order = nullptr;
-  size_t order_cap = 0;
+  size_t order_cap = 0, pinned_words = 0;
   cudaEvent_t half_free[2] = {nullptr, nullptr};  // each half's last upload
   float* d_out = nullptr;
   size_t data_cap = 0;
@@ -618,18 +619,49 @@ ppvm_status ensure_data(ppvm_mlp* m, size_t n) {
   return PPVM_OK;
 }
 
+// One pinned buffer of a destroyed network is kept for the next one (page-locking and unlocking take
+// milliseconds); ppvm_release_cached_memory gives it back.
+constexpr size_t kKeepPinnedWords = (size_t)4 << 20;
+std::mutex g_pinned_mu;
+uint32_t* g_pinned = nullptr;
+size_t g_pinned_words = 0;
+
+uint32_t* take_pinned(size_t words, size_t* got) {
+  std::lock_guard<std::mutex> lk(g_pinned_mu);
+  if (!g_pinned || g_pinned_words < words) return nullptr;
+  uint32_t* p = g_pinned;
+  *got = g_pinned_words;
+  g_pinned = nullptr;
+  return p;
+}
+
+void give_pinned(uint32_t* p, size_t words) {  // no copy from it is in flight
+  if (!p) return;
+  std::lock_guard<std::mutex> lk(g_pinned_mu);
+  if (!g_pinned && words <= kKeepPinnedWords) {
+    g_pinned = p;
+    g_pinned_words = words;
+  } else {
+    cudaFreeHost(p);
+  }
+}
+
 // Room for `words` 4-byte words of orders and learning rates (the stream is idle).
 ppvm_status ensure_order(ppvm_mlp* m, size_t words) {
   for (cudaEvent_t& e : m->half_free)
     if (!e) MCUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   if (words <= m->order_cap) return PPVM_OK;
   cudaFree(m->d_order);
-  cudaFreeHost(m->h_order);
+  give_pinned(m->h_order, m->pinned_words);
   m->d_order = nullptr;
   m->h_order = nullptr;
   m->order_cap = 0;
   MCUDA(cudaMalloc(&m->d_order, sizeof(uint32_t) * words));
-  MCUDA(cudaMallocHost(&m->h_order, sizeof(uint32_t) * words));
+  m->h_order = take_pinned(words, &m->pinned_words);
+  if (!m->h_order) {
+    MCUDA(cudaMallocHost(&m->h_order, sizeof(uint32_t) * words));
+    m->pinned_words = words;
+  }
   m->order_cap = words;
   return PPVM_OK;
 }
@@ -662,6 +694,14 @@ uint64_t splitmix(uint64_t& s) {
 
 }  // namespace
 
+namespace ppvm {
+void release_mlp_staging() {
+  std::lock_guard<std::mutex> lk(g_pinned_mu);
+  if (g_pinned) cudaFreeHost(g_pinned);
+  g_pinned = nullptr;
+}
+}  // namespace ppvm
+
 extern "C" {
 
 ppvm_status ppvm_mlp_destroy(ppvm_mlp* m) {
@@ -678,7 +718,7 @@ ppvm_status ppvm_mlp_destroy(ppvm_mlp* m) {
   cudaFree(m->d_feats);
   cudaFree(m->d_tgt);
   cudaFree(m->d_order);
-  cudaFreeHost(m->h_order);
+  give_pinned(m->h_order, m->pinned_words);
   for (cudaEvent_t e : m->half_free)
     if (e) cudaEventDestroy(e);
   cudaFree(m->d_out);
