@@ -96,10 +96,10 @@ struct ProfLaunch {
 };
 
 enum Family {
-  F_SCAN = 0, F_PAIR, F_APPLY, F_COMMIT, F_CLIFF, F_TRUNC, F_READ,
+  F_PAIR = 0, F_APPLY, F_COMMIT, F_CLIFF, F_TRUNC, F_READ,
   F_RUN_CLASSIFY, F_RUN_ORDER, F_RUN_SCATTER, F_RUN_GROUPS, F_RUN_PLACE, F_TABLEAU, F_LOSS, F_SMALL, F_COUNT
 };
-const char* kFamilyNames[F_COUNT] = {"rot_scan", "rot_pair", "rot_apply", "rot_commit",
+const char* kFamilyNames[F_COUNT] = {"rot_pair", "rot_apply", "rot_commit",
                                      "clifford", "truncate", "readout",
                                      "run_classify", "run_order", "run_scatter", "run_groups", "run_place",
                                      "tableau", "loss", "small"};
@@ -610,7 +610,6 @@ uint64_t launch_bytes(const ppvm_sum* s, const ProfLaunch& L, const std::vector<
   const uint64_t B = 16ull * s->W + 8;
   const OpLog& g = s->h_log[L.op];
   switch (L.family) {
-    case F_SCAN: return g.n_in * 16ull + g.n_s * (B + B + 8);  // damping: test words + gather + record/idx/partner
     case F_PAIR: {  // test words of every term, the anticommuting terms' keys, one table slot each
       const int tw = (L.op < (int)test_words.size()) ? test_words[L.op] : 1;
       return g.n_in * 8ull * tw + g.n_s * (B - 8 + 8);
@@ -896,35 +895,19 @@ struct K {
   // AmplitudeDamping::amplitude_damping (noise.rs:132-163) on qubit q: see noise.cuh.
   static void damping(ppvm_sum* s, uint32_t q, double gamma, int op) {
     const Planes P = s->planes_view();
-    Gen g;
-    std::memset(&g, 0, sizeof(g));
-    g.gz[q >> 6] = 1ull << (q & 63);
-    const unsigned qmask = 1u << (q >> 6);
-    const double om = 1.0 - gamma;    // T::Coeff::from(1.0) - gamma
+    const uint64_t bit = 1ull << (q & 63);
+    const double om = 1.0 - gamma;     // T::Coeff::from(1.0) - gamma
     const double sxy = std::sqrt(om);  // (1 - gamma).sqrt()
     const unsigned long long nub = std::max<unsigned long long>(s->n_ub, 1);
     {
-      ProfScope ps(s, F_SCAN, op, 1);
-      launch(k_damp_scan<W, kScanBlock, ITEMS>, grid_for(nub, TILE, 8), kScanBlock, 0, s->stream,
-          P, s->d_ctrl, g, qmask, s->s_idx, s->s_rec, s->R.gslot, s->tstate,
-          s->next_tile_epoch(), op, s->d_log);  // gslot: free outside fused runs, the parents' partners here
-    }
-    const unsigned tep = s->next_table_epoch();
-    {
       ProfScope ps(s, F_PAIR, op, 1);
-      launch(k_damp_index<W>, grid_for(nub, kPairBlock, 8), kPairBlock, 0, s->stream,
-          s->d_ctrl, g, s->s_rec, s->table, s->table_cap, tep, op);
-      launch(k_damp_probe<W>, grid_for(nub, kPairBlock, 8), kPairBlock, 0, s->stream,
-          P, s->d_ctrl, g, q >> 6, s->s_rec, s->R.gslot, s->table, s->table_cap, tep, sxy, op);
+      launch(k_damp_pair<W>, grid_for(nub, kPairBlock, 8), kPairBlock, 0, s->stream,
+          P, s->d_ctrl, q >> 6, bit, s->link, s->table, s->table_cap, s->next_table_epoch(), op);
     }
     {
       ProfScope ps(s, F_APPLY, op, 1);
       launch(k_damp_apply<W, kScanBlock, ITEMS>, grid_for(nub, TILE, 8), kScanBlock, 0, s->stream,
-          P, s->d_ctrl, g, om, gamma, s->s_idx, s->s_rec, s->R.gslot, s->tstate, s->next_tile_epoch(), op);
-    }
-    {
-      ProfScope ps(s, F_COMMIT, op, 1);
-      launch(k_commit_damp, 1, 1, 0, s->stream, s->d_ctrl, op, s->d_log);
+          P, s->d_ctrl, q >> 6, bit, om, gamma, sxy, s->link, s->tstate, s->next_tile_epoch(), op, s->d_log);
     }
     s->n_ub = std::min<unsigned long long>(s->cap, 2 * s->n_ub);
   }
