@@ -894,20 +894,29 @@ struct K {
 
   // AmplitudeDamping::amplitude_damping (noise.rs:132-163) on qubit q: see noise.cuh.
   static void damping(ppvm_sum* s, uint32_t q, double gamma, int op) {
+    Branch b;
+    std::memset(&b, 0, sizeof(b));
+    b.bit = 1ull << (q & 63);
+    b.qw = b.pw = q >> 6;
+    b.parent = 1.0 - gamma;           // T::Coeff::from(1.0) - gamma
+    b.child = gamma;
+    b.ident = 1.0;
+    b.other = std::sqrt(b.parent);    // (1 - gamma).sqrt()
+    branch(s, b, op);
+  }
+
+  static void branch(ppvm_sum* s, const Branch& b, int op) {
     const Planes P = s->planes_view();
-    const uint64_t bit = 1ull << (q & 63);
-    const double om = 1.0 - gamma;     // T::Coeff::from(1.0) - gamma
-    const double sxy = std::sqrt(om);  // (1 - gamma).sqrt()
     const unsigned long long nub = std::max<unsigned long long>(s->n_ub, 1);
     {
-      ProfScope ps(s, F_PAIR, op, 1);
-      launch(k_damp_pair<W>, grid_for(nub, kPairBlock, 8), kPairBlock, 0, s->stream,
-          P, s->d_ctrl, q >> 6, bit, s->link, s->table, s->table_cap, s->next_table_epoch(), op);
+      ProfScope ps(s, b.loss ? F_LOSS : F_PAIR, op, 1);
+      launch(k_branch_pair<W>, grid_for(nub, kPairBlock, 8), kPairBlock, 0, s->stream,
+          P, s->d_ctrl, b, s->link, s->table, s->table_cap, s->next_table_epoch(), op);
     }
     {
-      ProfScope ps(s, F_APPLY, op, 1);
-      launch(k_damp_apply<W, kScanBlock, ITEMS>, grid_for(nub, TILE, 8), kScanBlock, 0, s->stream,
-          P, s->d_ctrl, q >> 6, bit, om, gamma, sxy, s->link, s->tstate, s->next_tile_epoch(), op, s->d_log);
+      ProfScope ps(s, b.loss ? F_LOSS : F_APPLY, op, 1);
+      launch(k_branch_apply<W, kScanBlock, ITEMS>, grid_for(nub, TILE, 8), kScanBlock, 0, s->stream,
+          P, s->d_ctrl, b, s->link, s->tstate, s->next_tile_epoch(), op, s->d_log);
     }
     s->n_ub = std::min<unsigned long long>(s->cap, 2 * s->n_ub);
   }
@@ -915,21 +924,30 @@ struct K {
   // LossChannel / ResetLossChannel / CorrelatedLossChannel (noise.rs:165-275) on a lossy sum:
   // see loss.cuh.  Writes the whole output into the alternate planes, then swaps.
   static void loss(ppvm_sum* s, const ppvm_op& o, int op) {
+    if (o.code == PPVM_OP_LOSS_CHANNEL) {  // one child per parent: in place, as damping (noise.cuh)
+      Branch b;
+      std::memset(&b, 0, sizeof(b));
+      b.bit = 1ull << (o.q0 & 63);
+      b.qw = o.q0 >> 6;
+      b.pw = (uint32_t)s->wr + b.qw;
+      b.loss = 1;
+      b.parent = 1.0;
+      b.child = o.theta;
+      b.ident = b.other = 1.0 - o.theta;  // T::Coeff::from(1.0) - p
+      branch(s, b, op);
+      return;
+    }
     const Planes P = s->planes_view(), O = s->alt_view();
     const unsigned long long nub = std::max<unsigned long long>(s->n_ub, 1);
     unsigned long long tsize = next_pow2(std::max<unsigned long long>(2 * nub, 1024));
     if (tsize > s->table_cap) tsize = s->table_cap;
     LossOp lo;
     std::memset(&lo, 0, sizeof(lo));
-    lo.mode = o.code == PPVM_OP_LOSS_CHANNEL ? kLossChannel
-              : o.code == PPVM_OP_RESET_LOSS_CHANNEL ? kResetLoss : kCorrelatedLoss;
+    lo.mode = o.code == PPVM_OP_RESET_LOSS_CHANNEL ? kResetLoss : kCorrelatedLoss;
     lo.qa = o.q0;
     lo.qb = lo.mode == kCorrelatedLoss ? o.q1 : o.q0;
     lo.lw = (uint32_t)s->wr;
-    if (lo.mode == kLossChannel) {
-      lo.p0 = o.theta;
-      lo.keep1 = 1.0 - o.theta;  // T::Coeff::from(1.0) - p
-    } else if (lo.mode == kCorrelatedLoss) {
+    if (lo.mode == kCorrelatedLoss) {
       lo.p0 = o.p[0];
       lo.p1 = o.p[1];
       lo.p2 = o.p[2];
@@ -947,9 +965,7 @@ struct K {
         launch(emit_k, grid_for(nub, 256, 8), 256, 0, s->stream, P, O, s->d_ctrl, lo, s->table, tsize - 1, tep,
                s->tstate, s->tstate2, e1, e2, op, s->d_log);
       };
-      if (lo.mode == kLossChannel)
-        count_emit(k_loss_count<W, kLossChannel>, k_loss_emit<W, 256, kLossChannel>);
-      else if (lo.mode == kResetLoss)
+      if (lo.mode == kResetLoss)
         count_emit(k_loss_count<W, kResetLoss>, k_loss_emit<W, 256, kResetLoss>);
       else
         count_emit(k_loss_count<W, kCorrelatedLoss>, k_loss_emit<W, 256, kCorrelatedLoss>);

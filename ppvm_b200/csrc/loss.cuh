@@ -17,8 +17,10 @@
 // into a fresh map, and consume (data.rs:180-189) then merges the smaller of (children, data)
 // into the larger, whose order the result keeps.
 //
-// A child key can have up to three parents (reset: the I and Z terms; correlated (I,I): the
-// (L,L), (I,L) and (L,I) terms), all of which differ from it only on the channel's qubits.
+// The loss channel gives every child one parent, so it runs in place with amplitude damping's
+// kernels (noise.cuh).  In the other two a child key can have up to three parents (reset: the
+// I and Z terms; correlated (I,I): the (L,L), (I,L) and (L,I) terms), all of which differ from
+// it only on the channel's qubits.
 // So every output is computed by pulling: each output key enumerates its possible parents,
 // finds them in an index of the sum, orders them by (parent index, child slot) — the order in
 // which the reference generates children — and folds their contributions as the reference
@@ -37,14 +39,14 @@
 
 namespace ppvm {
 
-enum LossMode : int { kLossChannel = 0, kResetLoss = 1, kCorrelatedLoss = 2 };
+enum LossMode : int { kResetLoss = 1, kCorrelatedLoss = 2 };
 
 struct LossOp {
   int mode;
-  uint32_t qa, qb;  // qubits (qb = qa for the one-qubit channels)
+  uint32_t qa, qb;  // qubits (qb = qa for the reset)
   uint32_t lw;      // first loss word of the X plane (= Wr)
   double p0, p1, p2;
-  double keep1;     // loss: 1 - p;  correlated: 1 - p2 (one lost qubit)
+  double keep1;     // correlated: 1 - p2 (one lost qubit)
   double keep0;     // correlated: 1 - 2 p1 - p0 (no lost qubit)
 };
 
@@ -86,11 +88,6 @@ __device__ __forceinline__ void loss_set(uint64_t (&x)[W], uint64_t (&z)[W], uns
 // how many (0..3).
 __device__ __forceinline__ int loss_parents(const LossOp& op, int ca, int cb, int (&pa)[3], int (&pb)[3],
                                             int (&slot)[3], double (&f)[3]) {
-  if (op.mode == kLossChannel) {
-    if (ca != 0) return 0;
-    pa[0] = 4, pb[0] = cb, slot[0] = 0, f[0] = op.p0;
-    return 1;
-  }
   if (op.mode == kResetLoss) {
     if (ca != 4) return 0;
     pa[0] = 0, pb[0] = cb, slot[0] = 0, f[0] = 1.0;  // the child keeps v: v * 1.0 is v exactly
@@ -125,11 +122,6 @@ __device__ __forceinline__ int loss_parents(const LossOp& op, int ca, int cb, in
 // The codes on (qa, qb) of child `slot` of a term with codes (ca, cb); false if it has none.
 __device__ __forceinline__ bool loss_child(const LossOp& op, int ca, int cb, int slot, int& na, int& nb) {
   na = ca, nb = cb;
-  if (op.mode == kLossChannel) {
-    if (slot != 0 || ca != 4) return false;
-    na = 0;
-    return true;
-  }
   if (op.mode == kResetLoss) {
     if (slot != 0 || !(ca == 0 || ca == 2)) return false;
     na = 4;
@@ -155,7 +147,6 @@ __device__ __forceinline__ bool loss_child(const LossOp& op, int ca, int cb, int
 
 // The coefficient of an existing term after the channel's own scaling.
 __device__ __forceinline__ double loss_own(const LossOp& op, int ca, int cb, double v) {
-  if (op.mode == kLossChannel) return ca == 4 ? v : __dmul_rn(v, op.keep1);
   if (op.mode == kResetLoss) return ca == 4 ? __dmul_rn(v, 0.0) : v;
   if (ca == 4 && cb == 4) return v;
   if (ca == 4 || cb == 4) return __dmul_rn(v, op.keep1);
@@ -202,7 +193,7 @@ __device__ __forceinline__ void loss_find_parents(const LossOp& op, const Planes
 }
 
 // The key's coefficient after the channel.  own: its scaled coefficient if it is a term of
-// the sum (has_own).  map_insert (loss, reset): own, then each child added in order;
+// the sum (has_own).  map_insert (reset): own, then each child added in order;
 // map_insert_multiple (correlated): the children summed in order, then added to own.
 __device__ __forceinline__ double loss_fold(const LossOp& op, bool has_own, double own, const LossFound& F) {
   if (op.mode != kCorrelatedLoss) {
@@ -285,18 +276,9 @@ k_loss_count(Planes P, Ctrl* ctrl, LossOp op_in, const unsigned long long* table
        i += (unsigned long long)gridDim.x * blockDim.x) {
     uint64_t x[W], z[W];
     load_key<W>(P, i, x, z);
-    if constexpr (M == kLossChannel) {
-      // a lost qubit's term is the only parent of its child (the qubit as I): the child is new
-      // when that key is absent
-      if (loss_code<W>(x, z, op.lw, op.qa) == 4) {
-        loss_set<W>(x, z, op.lw, op.qa, 0);
-        nn += index_find<W>(P, x, z, table, mask, tepoch) < 0;
-      }
-    } else {
-      bool first[3], isnew[3];
-      na += loss_children<W>(op, P, i, x, z, table, mask, tepoch, first, isnew);
-      nn += (unsigned)isnew[0] + (unsigned)isnew[1] + (unsigned)isnew[2];
-    }
+    bool first[3], isnew[3];
+    na += loss_children<W>(op, P, i, x, z, table, mask, tepoch, first, isnew);
+    nn += (unsigned)isnew[0] + (unsigned)isnew[1] + (unsigned)isnew[2];
   }
   if (nn) atomicAdd(&s_new, nn);
   if (na) atomicAdd(&s_aux, na);
@@ -356,54 +338,6 @@ k_loss_emit(Planes P, Planes O, Ctrl* ctrl, LossOp op_in, const unsigned long lo
   // consume keeps the order of the larger map: the child keys' when they outnumber the terms
   const bool aux_first = op.mode == kCorrelatedLoss && n_aux > N;
   const unsigned long long ntiles = (N + BLOCK - 1) / BLOCK;
-  if constexpr (M == kLossChannel) {
-    // per term one index lookup: a term with L on qa keeps v and, when the key with I there is
-    // absent, makes it as a new key with v * p (appended in parent order); a term with I on
-    // qa takes v * (1 - p) plus p times the coefficient of the key with L there, if present;
-    // X, Y, Z take v * (1 - p)
-    for (;;) {
-      const unsigned tile = next_tile(&ctrl->tickets[0], &s_tile);
-      if (tile >= ntiles) break;
-      const unsigned long long i = (unsigned long long)tile * BLOCK + threadIdx.x;
-      uint64_t x[W], z[W];
-      bool isnew = false;
-      double v = 0.0, own = 0.0;
-      if (i < N) {
-        load_key<W>(P, i, x, z);
-        v = P.c[i];
-        const int ca = loss_code<W>(x, z, op.lw, op.qa);
-        if (ca == 4 || ca == 0) {
-          uint64_t kx[W], kz[W];
-#pragma unroll
-          for (int w = 0; w < W; ++w) kx[w] = x[w], kz[w] = z[w];
-          loss_set<W>(kx, kz, op.lw, op.qa, ca == 4 ? 0 : 4);
-          const long long j = index_find<W>(P, kx, kz, table, mask, tepoch);
-          if (ca == 4) {
-            own = v;
-            isnew = j < 0;
-          } else {
-            own = __dmul_rn(v, op.keep1);
-            if (j >= 0) own = __dadd_rn(own, __dmul_rn(P.c[j], op.p0));
-          }
-        } else {
-          own = __dmul_rn(v, op.keep1);
-        }
-      }
-      unsigned t1;
-      const unsigned e1 = block_excl<BLOCK>(isnew ? 1u : 0u, s_w, t1);
-      const unsigned long long x1 = lookback(ts, tile, t1, epoch, ctrl, opi, &s_slot);
-      if (i < N) {
-        store_key<W>(O, i, x, z);
-        O.c[i] = own;
-        if (isnew) {
-          const unsigned long long r = N + x1 + e1;
-          loss_set<W>(x, z, op.lw, op.qa, 0);
-          store_key<W>(O, r, x, z);
-          O.c[r] = __dmul_rn(v, op.p0);
-        }
-      }
-    }
-  } else
   for (;;) {
     const unsigned tile = next_tile(&ctrl->tickets[0], &s_tile);
     if (tile >= ntiles) break;

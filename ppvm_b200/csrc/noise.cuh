@@ -1,4 +1,5 @@
-// noise.cuh — amplitude damping (crates/ppvm-pauli-sum/src/sum/noise.rs:132-163).
+// noise.cuh — the channels with one child per parent: amplitude damping and the loss channel
+// (crates/ppvm-pauli-sum/src/sum/noise.rs:132-163, 165-181).
 //
 // The Heisenberg adjoint of amplitude damping on qubit q maps
 //   I -> I,   X -> sqrt(1-g) X,   Y -> sqrt(1-g) Y,   Z -> (1-g) Z + g I,
@@ -6,30 +7,50 @@
 // the same word with I on q and coefficient v * g, is merged with `+=` into an existing term
 // or appended after all terms, in parent order.  Unlike a rotation's child, this child can
 // only land on a term with I on q, which is not a parent itself, so every key still receives
-// at most two contributions and the result is bit-identical to the reference's.
+// at most two contributions and the result is bit-identical to the reference's.  The loss
+// channel of a lossy sum has the same shape, with L in the place of Z:
+//   L -> L + p I,   I, X, Y, Z -> (1-p) themselves.
 //
-//   k_damp_pair   every term with I or Z on q meets its counterpart (the other of the two) in the
-//                 epoch-tagged table, and the second to arrive hands each the other's
-//                 coefficient, as k_rot_pair does for a rotation
-//   k_damp_apply  parents scaled by (1-g), I terms add their parent's child, X and Y scaled by
-//                 sqrt(1-g); the children without a term appended, in parent order; its last
-//                 block publishes the live count
+//   k_branch_pair   every term with I or the parent letter on q meets its counterpart (the other of
+//                   the two) in the epoch-tagged table, and the second to arrive hands each the
+//                   other's coefficient, as k_rot_pair does for a rotation
+//   k_branch_apply  every term scaled by its letter's factor; I terms add their parent's child; the
+//                   children without a term appended, in parent order; its last block
+//                   publishes the live count
 //
 // (A scan into records, an index of the children, a probe of every I term, an apply pass and a
-// commit took five launches: 45 us on a sum of 75,000 terms, against 20 for the two.)  The
-// capacity check runs in k_damp_apply before any coefficient changes, so a replay after growth
-// starts from unmodified terms.
+// commit took five launches for damping, index, count and emit into the other planes three for the
+// loss channel.  These are launches between dependent small passes: five layers of a noisy 7x7
+// lattice take 11.8 ms instead of 12.1, four lossy layers on 40 qubits 6.1 instead of 7.4.)
+// The capacity check runs in k_branch_apply before any coefficient changes, so a replay after
+// growth starts from unmodified terms.
 #pragma once
 
 #include "kernels.cuh"
 
 namespace ppvm {
 
-// qw, bit: the plane word and bit of the damped qubit.
+// A channel on one qubit: word qw and bit of the qubit, word pw of the plane that tells the
+// parent letter from I (damping: the Z plane's qw; loss: the X plane's loss word), and the factors.
+struct Branch {
+  uint64_t bit;
+  uint32_t qw, pw;
+  uint32_t loss;  // 1: loss channel (parents L), 0: amplitude damping (parents Z)
+  // factors: the parent's own, its child's, an I term's, any other term's
+  double parent, child, ident, other;
+};
+
+// Whether term i is touched (I or the parent letter on the qubit) and whether it is a parent.
+__device__ __forceinline__ bool branch_touched(const Planes& P, const Branch& b, unsigned long long i, bool& parent) {
+  const uint64_t x = P.x[(unsigned long long)b.qw * P.cap + i], z = P.z[(unsigned long long)b.qw * P.cap + i];
+  parent = ((b.loss ? P.x[(unsigned long long)b.pw * P.cap + i] : z) & b.bit) != 0;
+  return !((b.loss ? x | z : x) & b.bit);
+}
+
 template <int W>
 __global__ void __launch_bounds__(256)
-k_damp_pair(Planes P, Ctrl* ctrl, unsigned qw, uint64_t bit, unsigned long long* link, unsigned long long* table,
-            unsigned long long table_cap, unsigned tepoch, int op) {
+k_branch_pair(Planes P, Ctrl* ctrl, Branch b, unsigned long long* link, unsigned long long* table,
+              unsigned long long table_cap, unsigned tepoch, int op) {
   pdl_wait();
   __shared__ unsigned s_cnt[2];
   if (ld_volatile_int(&ctrl->err)) return;
@@ -43,18 +64,18 @@ k_damp_pair(Planes P, Ctrl* ctrl, unsigned qw, uint64_t bit, unsigned long long*
   const unsigned long long mask = tsize - 1;
   unsigned parents = 0, pairs = 0;
   for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += stride) {
-    if (P.x[(unsigned long long)qw * P.cap + i] & bit) continue;  // X or Y
-    uint64_t x[W], z[W], kz[W];
+    bool parent;
+    if (!branch_touched(P, b, i, parent)) continue;
+    uint64_t x[W], z[W], kx[W], kz[W];
     load_key<W>(P, i, x, z);
-    bool parent = false;
 #pragma unroll
-    for (int w = 0; w < W; ++w) {
-      const uint64_t m = w == (int)qw ? bit : 0ull;
-      parent |= (z[w] & m) != 0;
-      kz[w] = z[w] & ~m;  // they meet at the key with I
+    for (int w = 0; w < W; ++w) {  // they meet at the key with I
+      const uint64_t m = w == (int)b.pw ? b.bit : 0ull;
+      kx[w] = x[w] & ~(b.loss ? m : 0ull);
+      kz[w] = z[w] & ~(b.loss ? 0ull : m);
     }
     parents += parent;
-    const uint64_t h = table_hash<W>(x, kz);
+    const uint64_t h = table_hash<W>(kx, kz);
     const unsigned tag = (unsigned)(h >> 48) & 0xFFFFu;
     const unsigned long long mine = make_slot(tepoch, tag, (unsigned)i);
     unsigned long long slot = h & mask, probes = 0, cur = ld_volatile(&table[slot]);
@@ -71,7 +92,10 @@ k_damp_pair(Planes P, Ctrl* ctrl, unsigned qw, uint64_t bit, unsigned long long*
         load_key<W>(P, j, jx, jz);
         bool eq = true;
 #pragma unroll
-        for (int w = 0; w < W; ++w) eq &= (jx[w] == x[w]) & (jz[w] == (z[w] ^ (w == (int)qw ? bit : 0ull)));
+        for (int w = 0; w < W; ++w) {
+          const uint64_t m = w == (int)b.pw ? b.bit : 0ull;
+          eq &= (jx[w] == (x[w] ^ (b.loss ? m : 0ull))) & (jz[w] == (z[w] ^ (b.loss ? 0ull : m)));
+        }
         if (eq) {
           link[i] = link_bits(P.c[j]);
           link[j] = link_bits(P.c[i]);
@@ -98,11 +122,10 @@ k_damp_pair(Planes P, Ctrl* ctrl, unsigned qw, uint64_t bit, unsigned long long*
     atomicAdd(threadIdx.x == 0 ? &ctrl->rot_s : &ctrl->rot_pairs, (unsigned long long)s_cnt[threadIdx.x]);
 }
 
-// om = 1 - g, gm = g, sxy = sqrt(1 - g).
 template <int W, int BLOCK, int ITEMS>
 __global__ void __launch_bounds__(BLOCK)
-k_damp_apply(Planes P, Ctrl* ctrl, unsigned qw, uint64_t bit, double om, double gm, double sxy,
-             unsigned long long* link, unsigned long long* ts, unsigned epoch, int op, OpLog* log) {
+k_branch_apply(Planes P, Ctrl* ctrl, Branch b, unsigned long long* link, unsigned long long* ts, unsigned epoch,
+               int op, OpLog* log) {
   pdl_wait();
   __shared__ unsigned s_tile;
   __shared__ unsigned long long s_slot;
@@ -131,13 +154,12 @@ k_damp_apply(Planes P, Ctrl* ctrl, unsigned qw, uint64_t bit, double om, double 
     unsigned ballots[ITEMS];
     double kc[ITEMS];
     unsigned long long kl[ITEMS];
-    bool xy[ITEMS], zz[ITEMS];
+    bool touched[ITEMS], parent[ITEMS];
 #pragma unroll
     for (int k = 0; k < ITEMS; ++k) {
       const unsigned long long i = base + (unsigned long long)k * BLOCK + threadIdx.x;
       if (i < N) {
-        xy[k] = (P.x[(unsigned long long)qw * P.cap + i] & bit) != 0;
-        zz[k] = (P.z[(unsigned long long)qw * P.cap + i] & bit) != 0;
+        touched[k] = branch_touched(P, b, i, parent[k]);
         kl[k] = link[i];
         kc[k] = P.c[i];
       }
@@ -148,14 +170,11 @@ k_damp_apply(Planes P, Ctrl* ctrl, unsigned qw, uint64_t bit, double om, double 
       bool child = false;
       if (i < N) {
         const bool linked = kl[k] != kNoLink;
-        if (xy[k]) {
-          P.c[i] = __dmul_rn(kc[k], sxy);
-        } else if (zz[k]) {
-          P.c[i] = __dmul_rn(kc[k], om);
-          child = !linked;
-        } else if (linked) {
-          P.c[i] = __dadd_rn(kc[k], __dmul_rn(__longlong_as_double((long long)kl[k]), gm));
-        }
+        // a factor of 1 leaves every value as it is
+        double nc = __dmul_rn(kc[k], !touched[k] ? b.other : parent[k] ? b.parent : b.ident);
+        if (touched[k] && parent[k]) child = !linked;
+        else if (linked) nc = __dadd_rn(nc, __dmul_rn(__longlong_as_double((long long)kl[k]), b.child));
+        P.c[i] = nc;
         if (linked) link[i] = kNoLink;
       }
       ballots[k] = __ballot_sync(kFull, child);
@@ -173,9 +192,9 @@ k_damp_apply(Planes P, Ctrl* ctrl, unsigned qw, uint64_t bit, double om, double 
           load_key<W>(P, i, x, z);
 #pragma unroll
           for (int w = 0; w < W; ++w)
-            if (w == (int)qw) z[w] &= ~bit;
+            if (w == (int)b.pw) (b.loss ? x : z)[w] &= ~b.bit;
           store_key<W>(P, r, x, z);
-          P.c[r] = __dmul_rn(kc[k], gm);
+          P.c[r] = __dmul_rn(kc[k], b.child);
         }
       }
     }
