@@ -320,8 +320,8 @@ def batched_shard_seed(rank: int) -> int:
 # dram__bytes_write.sum of every launch of the kernel in the step).  Filled from a capture of
 # the current kernels; a workload or kernel without an entry reports null.
 CAPTURED_TRAFFIC: dict = {
-    "kicked_ising_2d": {"run_groups": 66548 + 402, "tableau": 237986 + 0},          # 21 and 19 launches
-    "clifford_t": {"run_groups": 7685530 + 5397443, "tableau": 8022518 + 3209472},  # 25 and 25 launches
+    "kicked_ising_2d": {"tableau": 237986 + 0},          # 19 launches
+    "clifford_t": {"tableau": 8022518 + 3209472},        # 25 launches
 }
 TRAFFIC_SOURCE = ("ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum --clock-control none over one step "
                   "of this workload (every launch of the kernel), mean per launch")
