@@ -53,6 +53,7 @@ struct Ctrl {
   unsigned long long scr_top;  // fused run in scratch mode: group outputs placed in the scratch so far
   unsigned long long rot_s;      // rotation: anticommuting terms found by k_rot_pair (0 between rotations)
   unsigned long long rot_pairs;  // rotation: partner pairs among them (0 between rotations)
+  unsigned long long rot_n;      // live terms that the pair kernel of a rotation or one-child channel saw
   unsigned long long small_pc;   // ops of the list that k_small has applied
   unsigned spin_limit;         // polls a look-back waits before it gives up; 0 = kSpinLimit
   unsigned reserved;

@@ -120,6 +120,7 @@ k_rot_pair(Planes P, Ctrl* ctrl, Gen g, unsigned xmask, unsigned zmask, unsigned
   if (ld_volatile_int(&ctrl->err)) return;
   const unsigned long long N = ld_volatile(&ctrl->n);
   const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
+  if (blockIdx.x == 0 && threadIdx.x == 0) ctrl->rot_n = N;  // for the apply kernel
   if ((unsigned long long)blockIdx.x * blockDim.x >= N) return;
   if (threadIdx.x < 2) s_cnt[threadIdx.x] = 0;
   __syncthreads();
@@ -216,7 +217,11 @@ k_rot_pair(Planes P, Ctrl* ctrl, Gen g, unsigned xmask, unsigned zmask, unsigned
 // k_rot_apply: new coefficients in place, children appended in parent order (one decoupled
 // look-back per tile of terms).  xmask/zmask: the test's words, gm: the words of the generator (of
 // both planes; the sign needs them).  The last of the blocks that have tiles publishes the
-// live count.  A streaming pass: every access but the appended children is at the term itself.
+// live count.  Which blocks have tiles follows from the count the pair kernel saw (rot_n), not from
+// the live one: a block that starts after the commit (the grid can be larger than what is resident
+// at once) would take the new count's tiles for its own.  A late block may also read rot_s after its
+// reset: then there are no tiles, and block 0 alone, which is never late, takes part.
+// A streaming pass: every access but the appended children is at the term itself.
 template <int W, int BLOCK, int ITEMS>
 __global__ void __launch_bounds__(BLOCK)
 k_rot_apply(Planes P, Ctrl* ctrl, Gen g, unsigned xmask, unsigned zmask, unsigned gm, double sn, double cs,
@@ -226,7 +231,7 @@ k_rot_apply(Planes P, Ctrl* ctrl, Gen g, unsigned xmask, unsigned zmask, unsigne
   __shared__ unsigned long long s_slot;
   __shared__ unsigned s_base[ITEMS * (BLOCK / 32) + 1];
   if (ld_volatile_int(&ctrl->err)) return;
-  const unsigned long long N = ld_volatile(&ctrl->n);
+  const unsigned long long N = ld_volatile(&ctrl->rot_n);
   const unsigned long long ns = ld_volatile(&ctrl->rot_s);
   const unsigned long long nchild = ns - 2 * ld_volatile(&ctrl->rot_pairs);
   if (N + nchild > P.cap) {  // nothing has been written: the host grows the storage and replays this op

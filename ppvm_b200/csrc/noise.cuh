@@ -56,6 +56,7 @@ k_branch_pair(Planes P, Ctrl* ctrl, Branch b, unsigned long long* link, unsigned
   if (ld_volatile_int(&ctrl->err)) return;
   const unsigned long long N = ld_volatile(&ctrl->n);
   const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
+  if (blockIdx.x == 0 && threadIdx.x == 0) ctrl->rot_n = N;  // for the apply kernel
   if ((unsigned long long)blockIdx.x * blockDim.x >= N) return;
   if (threadIdx.x < 2) s_cnt[threadIdx.x] = 0;
   __syncthreads();
@@ -131,7 +132,8 @@ k_branch_apply(Planes P, Ctrl* ctrl, Branch b, unsigned long long* link, unsigne
   __shared__ unsigned long long s_slot;
   __shared__ unsigned s_base[ITEMS * (BLOCK / 32) + 1];
   if (ld_volatile_int(&ctrl->err)) return;
-  const unsigned long long N = ld_volatile(&ctrl->n);
+  // as in k_rot_apply: the blocks that take part follow from a count that the commit below leaves alone
+  const unsigned long long N = ld_volatile(&ctrl->rot_n);
   const unsigned long long ns = ld_volatile(&ctrl->rot_s);
   const unsigned long long nchild = ns - ld_volatile(&ctrl->rot_pairs);
   if (N + nchild > P.cap) {  // nothing has been written: the host grows the storage and replays this op
