@@ -128,10 +128,14 @@ __device__ __forceinline__ bool last_block_done(unsigned long long* counter) {
 }
 
 // last_block_done for a launch of which only the first `blocks` blocks take part (the others
-// returned at once): the last of those to call it.
+// returned at once): the last of those to call it.  A block on its own needs no counter, but the
+// barrier all the same: what its other warps wrote is read by the caller.
 __device__ __forceinline__ bool last_of_blocks(unsigned long long* counter, unsigned blocks) {
   __shared__ bool s_last;
-  if (blocks == 1) return true;
+  if (blocks == 1) {
+    __syncthreads();
+    return true;
+  }
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) {
