@@ -257,7 +257,8 @@ __device__ __forceinline__ void small_run_sort(const Region<W>& R, unsigned N0, 
         unsigned first = 0;
         for (unsigned long long probes = 0; probes <= mask; ++probes) {  // found: the group has an original member
           const unsigned long long cur = R.table[slot];
-          if (slot_epoch(cur) == (epoch & 0xFFFFu) && slot_tag(cur) == tag) {
+          if (slot_epoch(cur) != (epoch & 0xFFFFu)) break;
+          if (slot_tag(cur) == tag) {
             uint64_t jv[W], jf[W];
             group(slot_idx(cur), jv, jf);
             bool eq = true;
@@ -445,7 +446,7 @@ k_small(Planes P, Ctrl* ctrl, const SmallOp* __restrict__ ops, const SmallInline
     const DevOp d = op.d;
     if (op.run) {  // a fused run starts: its terms as they are, in case it outgrows the region
       run_rx = (d.ax & 1) != 0;
-      if (!small_run_begin<W>(R, N, ops ? ops + pc : s_ops, op.run, run_rx, s_q, Q)) break;  // too wide: the pipeline cuts it
+      if (!small_run_begin<W>(R, N, ops ? ops + pc : s_ops + pc, op.run, run_rx, s_q, Q)) break;  // too wide: the pipeline cuts it
       run_at = pc;
       run_end = pc + op.run;
       run_n = N;
