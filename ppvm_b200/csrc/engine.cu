@@ -908,15 +908,26 @@ struct K {
   static void branch(ppvm_sum* s, const Branch& b, int op) {
     const Planes P = s->planes_view();
     const unsigned long long nub = std::max<unsigned long long>(s->n_ub, 1);
-    {
-      ProfScope ps(s, b.loss ? F_LOSS : F_PAIR, op, 1);
+    auto pair = [&] {
       launch(k_branch_pair<W>, grid_for(nub, kPairBlock, 8), kPairBlock, 0, s->stream,
           P, s->d_ctrl, b, s->link, s->table, s->table_cap, s->next_table_epoch(), op);
-    }
-    {
-      ProfScope ps(s, b.loss ? F_LOSS : F_APPLY, op, 1);
+    };
+    auto apply = [&] {
       launch(k_branch_apply<W, kScanBlock, ITEMS>, grid_for(nub, TILE, 8), kScanBlock, 0, s->stream,
           P, s->d_ctrl, b, s->link, s->tstate, s->next_tile_epoch(), op, s->d_log);
+    };
+    if (b.loss) {  // the loss family's bytes are the op's: both kernels in one record
+      ProfScope ps(s, F_LOSS, op, 1);
+      ++s->launch_count;
+      pair();
+      apply();
+    } else {
+      {
+        ProfScope ps(s, F_PAIR, op, 1);
+        pair();
+      }
+      ProfScope ps(s, F_APPLY, op, 1);
+      apply();
     }
     s->n_ub = std::min<unsigned long long>(s->cap, 2 * s->n_ub);
   }
@@ -1052,33 +1063,39 @@ struct K {
     const Planes S = allow ? s->view_of(s->scr) : O;
     const unsigned long long scratch_min = allow ? smin : ~0ull;
     const unsigned mode = run_group_mode();
-    if (mode != 3) {
-      ProfScope ps(s, F_RUN_GROUPS, op0, L);
-      // no more blocks than fit on the GPU at once: blocks take tiles by ticket, so more would
-      // only queue on the ticket counter
-      static int resident = 0;  // blocks per SM (the same on every B200)
-      if (!resident) {
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_run_tiles<W>, kTileWarps * 32, 0) !=
-                cudaSuccess || resident < 1)
-          resident = 1;
-      }
-      launch(k_run_tiles<W>, grid_for(nub, kTileWarps, std::min(resident, 8)), kTileWarps * 32, 0, s->stream,
-          O, S, s->d_ctrl, d_rd, s->R, trunc, s->thr, s->maxw, s->tstate, s->next_tile_epoch(), op0,
-          trunc_op, s->d_log, scratch_min, mode);  // its last block publishes the counts and the op log
-    }
+    const bool tiles = mode != 3;
     // ngroups <= live terms <= nub: below the threshold the device takes tiles, and the lane kernel
     // is not needed
-    if (mode == 3 || (mode == 0 && nub >= kRunTileMinGroups)) {
+    const bool lanes = mode == 3 || (mode == 0 && nub >= kRunTileMinGroups);
+    {
+      // the run's groups go through one of the two kernels, the other returns at once: one record
+      // with the run's bytes and the time of both
       ProfScope ps(s, F_RUN_GROUPS, op0, L);
-      static int resident = 0;
-      if (!resident) {
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_run_lanes<W>, kRunWarps * 32, 0) !=
-                cudaSuccess || resident < 1)
-          resident = 1;
+      if (tiles && lanes) ++s->launch_count;
+      if (tiles) {
+        // no more blocks than fit on the GPU at once: blocks take tiles by ticket, so more would
+        // only queue on the ticket counter
+        static int resident = 0;  // blocks per SM (the same on every B200)
+        if (!resident) {
+          if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_run_tiles<W>, kTileWarps * 32, 0) !=
+                  cudaSuccess || resident < 1)
+            resident = 1;
+        }
+        launch(k_run_tiles<W>, grid_for(nub, kTileWarps, std::min(resident, 8)), kTileWarps * 32, 0, s->stream,
+            O, S, s->d_ctrl, d_rd, s->R, trunc, s->thr, s->maxw, s->tstate, s->next_tile_epoch(), op0,
+            trunc_op, s->d_log, scratch_min, mode);  // its last block publishes the counts and the op log
       }
-      launch(k_run_lanes<W>, grid_for(nub, 32 * kRunWarps, std::min(resident, 8)), kRunWarps * 32, 0, s->stream,
-          O, s->d_ctrl, d_rd, s->R, trunc, s->thr, s->maxw, s->tstate, s->next_tile_epoch(), op0,
-          trunc_op, s->d_log, mode);
+      if (lanes) {
+        static int resident = 0;
+        if (!resident) {
+          if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_run_lanes<W>, kRunWarps * 32, 0) !=
+                  cudaSuccess || resident < 1)
+            resident = 1;
+        }
+        launch(k_run_lanes<W>, grid_for(nub, 32 * kRunWarps, std::min(resident, 8)), kRunWarps * 32, 0, s->stream,
+            O, s->d_ctrl, d_rd, s->R, trunc, s->thr, s->maxw, s->tstate, s->next_tile_epoch(), op0,
+            trunc_op, s->d_log, mode);
+      }
     }
     if (allow && mode != 3) {
       ProfScope ps(s, F_RUN_PLACE, op0, L);
