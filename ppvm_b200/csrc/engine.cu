@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <map>
 #include <mutex>
 #include <set>
@@ -84,7 +85,7 @@ uint64_t h_hash_key(const uint64_t* x, const uint64_t* z, int W) {
   return h;
 }
 
-int g_sm_count = 0;
+std::atomic<int> g_sm_count{0};
 
 struct ProfLaunch {
   int family;
@@ -376,7 +377,11 @@ ppvm_status ensure_device(int dev) {
     return fail(PPVM_ENODEV, std::string("no CUDA device: ") + cudaGetErrorString(e));
   if (dev < 0 || dev >= count) return fail(PPVM_EINVAL, "device ordinal out of range");
   CUDA_TRY(cudaSetDevice(dev));
-  if (g_sm_count == 0) CUDA_TRY(cudaDeviceGetAttribute(&g_sm_count, cudaDevAttrMultiProcessorCount, dev));
+  if (g_sm_count == 0) {
+    int n = 0;
+    CUDA_TRY(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
+    g_sm_count = n;
+  }
   return PPVM_OK;
 }
 
@@ -564,7 +569,7 @@ void launch(void (*kern)(KArgs...), unsigned grid, unsigned block, size_t smem, 
 
 unsigned grid_for(unsigned long long work, unsigned long long per_block, int max_per_sm) {
   unsigned long long g = (work + per_block - 1) / per_block;
-  const unsigned long long cap = (unsigned long long)g_sm_count * max_per_sm;
+  const unsigned long long cap = (unsigned long long)g_sm_count.load(std::memory_order_relaxed) * max_per_sm;
   if (g > cap) g = cap;
   if (g == 0) g = 1;
   return (unsigned)g;
@@ -861,6 +866,13 @@ Lattice lattice_of(int L) {
   return lat;
 }
 
+// Resident blocks per SM of a kernel without dynamic shared memory (the same on every B200).
+template <typename F>
+int blocks_per_sm(F* kern, int block) {
+  int n = 0;
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, block, 0) == cudaSuccess && n > 0 ? n : 1;
+}
+
 // ---- kernel enqueue (templated on W) ------------------------------------------------------------
 template <int W>
 struct K {
@@ -1075,23 +1087,13 @@ struct K {
       if (tiles) {
         // no more blocks than fit on the GPU at once: blocks take tiles by ticket, so more would
         // only queue on the ticket counter
-        static int resident = 0;  // blocks per SM (the same on every B200)
-        if (!resident) {
-          if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_run_tiles<W>, kTileWarps * 32, 0) !=
-                  cudaSuccess || resident < 1)
-            resident = 1;
-        }
+        static const int resident = blocks_per_sm(k_run_tiles<W>, kTileWarps * 32);
         launch(k_run_tiles<W>, grid_for(nub, kTileWarps, std::min(resident, 8)), kTileWarps * 32, 0, s->stream,
             O, S, s->d_ctrl, d_rd, s->R, trunc, s->thr, s->maxw, s->tstate, s->next_tile_epoch(), op0,
             trunc_op, s->d_log, scratch_min, mode);  // its last block publishes the counts and the op log
       }
       if (lanes) {
-        static int resident = 0;
-        if (!resident) {
-          if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_run_lanes<W>, kRunWarps * 32, 0) !=
-                  cudaSuccess || resident < 1)
-            resident = 1;
-        }
+        static const int resident = blocks_per_sm(k_run_lanes<W>, kRunWarps * 32);
         launch(k_run_lanes<W>, grid_for(nub, 32 * kRunWarps, std::min(resident, 8)), kRunWarps * 32, 0, s->stream,
             O, s->d_ctrl, d_rd, s->R, trunc, s->thr, s->maxw, s->tstate, s->next_tile_epoch(), op0,
             trunc_op, s->d_log, mode);
@@ -1128,11 +1130,12 @@ struct K {
     }
     const size_t smem = t.rows.size() * sizeof(uint64_t) + t.ph.size() + (chunk_min >= 0 ? kTabChunkSmem : 0);
     if (smem > kTabMaxSmem) return fail(PPVM_EINVAL, "internal: tableau exceeds shared memory");
-    static unsigned long long attr_set = 0;  // one bit per device
-    if (!((attr_set >> s->device) & 1ull)) {
+    static std::atomic<unsigned long long> attr_set{0};  // one bit per device; sums of other threads come here too
+    const unsigned long long bit = 1ull << (s->device & 63);
+    if (!(attr_set.load(std::memory_order_acquire) & bit)) {
       CUDA_TRY(cudaFuncSetAttribute(k_tableau<W, kTabBlock, ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)kTabMaxSmem));
-      attr_set |= 1ull << s->device;
+      attr_set.fetch_or(bit, std::memory_order_release);
     }
     // blocks per SM: with the tables, as many as 227 KB of shared memory hold (3)
     const int bps = chunk_min >= 0 ? (int)std::max<size_t>(1, std::min<size_t>(4, (227 * 1024) / (smem + 2048)))
@@ -1151,11 +1154,12 @@ struct K {
 
   // ops[0..nops) (small ops, list indices from op0) on a sum of at most kSmallStart terms.
   static ppvm_status small(ppvm_sum* s, const SmallOp* d_ops, const SmallInline& few, int nops, int op0) {
-    static unsigned long long attr_set = 0;  // one bit per device
-    if (!((attr_set >> s->device) & 1ull)) {
+    static std::atomic<unsigned long long> attr_set{0};  // one bit per device
+    const unsigned long long bit = 1ull << (s->device & 63);
+    if (!(attr_set.load(std::memory_order_acquire) & bit)) {
       CUDA_TRY(cudaFuncSetAttribute(k_small<W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)SmallFor<W>::smem));
-      attr_set |= 1ull << s->device;
+      attr_set.fetch_or(bit, std::memory_order_release);
     }
     ProfScope ps(s, F_SMALL, op0, nops);
     launch(k_small<W>, 1, kSmallBlock, SmallFor<W>::smem, s->stream, s->planes_view(), s->d_ctrl, d_ops, few,
@@ -1947,7 +1951,7 @@ ppvm_status ppvm_sum_destroy(ppvm_sum* s) {
       s->event_pool.push_back(L.b);
     }
     s->prof_pending.clear();
-      cudaFree(s->d_pres_keys);
+    cudaFree(s->d_pres_keys);
     cudaFree(s->d_pres_table);
     s->d_pres_keys = nullptr;
     s->d_pres_table = nullptr;

@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -669,10 +670,11 @@ ppvm_status ensure_order(ppvm_mlp* m, size_t words) {
 // Forward + backward of one minibatch into the slabs; *nslabs = the number of slabs written.
 ppvm_status launch_train(ppvm_mlp* m, const uint32_t* d_order, unsigned long long start, unsigned long long count, float inv_n,
                          int* nslabs) {
-  static unsigned long long attr = 0;
-  if (!((attr >> m->device) & 1ull)) {
+  static std::atomic<unsigned long long> attr{0};  // one bit per device
+  const unsigned long long bit = 1ull << (m->device & 63);
+  if (!(attr.load(std::memory_order_acquire) & bit)) {
     MCUDA(cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)train_smem()));
-    attr |= 1ull << m->device;
+    attr.fetch_or(bit, std::memory_order_release);
   }
   const unsigned long long tiles = (count + 15) / 16;
   const unsigned grid = (unsigned)std::max<unsigned long long>(
