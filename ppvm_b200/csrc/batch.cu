@@ -755,11 +755,15 @@ ppvm_status ensure_graphs(ppvm_batch* b) {
 }
 
 // After a launch sequence: grows the regions of instances that ran out of capacity.
-// Returns the first layer to relaunch through *first (UINT32_MAX when nothing failed).
-ppvm_status grow_failed(ppvm_batch* b, uint32_t* first) {
+// Returns the first layer to relaunch through *first (UINT32_MAX when nothing failed); *inside says
+// whether regions grew inside the launches since the pool was last laid out.
+ppvm_status grow_failed(ppvm_batch* b, uint32_t* first, bool* inside) {
   *first = 0xFFFFFFFFu;
   bool grow = false;
-  for (size_t i = 0; i < b->ninst; ++i) b->cap[i] = b->h_inst[i].cap;  // some grew inside the launches
+  for (size_t i = 0; i < b->ninst; ++i) {
+    *inside |= b->cap[i] != b->h_inst[i].cap;
+    b->cap[i] = b->h_inst[i].cap;
+  }
   for (size_t i = 0; i < b->ninst; ++i) {
     BInst& I = b->h_inst[i];
     if (!I.err) continue;
@@ -773,7 +777,10 @@ ppvm_status grow_failed(ppvm_batch* b, uint32_t* first) {
     while (L < I.n_layers && b->lends[i][L] <= I.pc - I.op_begin) ++L;
     *first = std::min(*first, L);
   }
-  if (grow) BTRY(layout(b, true));
+  if (grow) {
+    BTRY(layout(b, true));
+    *inside = false;
+  }
   return PPVM_OK;
 }
 
@@ -783,6 +790,7 @@ ppvm_status run_all(ppvm_batch* b, bool use_graphs, bool persistent) {
   if (b->layout_dirty || !b->pool) BTRY(layout(b, false));
   BTRY(load_initial(b));
   uint32_t first = 0;
+  bool inside = false;
   for (int attempt = 0; attempt < 64; ++attempt) {
     if (persistent) {
       BCUDA(launch_any(b, -1));
@@ -796,15 +804,10 @@ ppvm_status run_all(ppvm_batch* b, bool use_graphs, bool persistent) {
     BCUDA(cudaMemcpyAsync(b->h_inst, b->d_inst, sizeof(BInst) * b->ninst, cudaMemcpyDeviceToHost, b->stream));
     BCUDA(cudaStreamSynchronize(b->stream));
     b->xfer_d2h += sizeof(BInst) * b->ninst;
-    BTRY(grow_failed(b, &first));
+    BTRY(grow_failed(b, &first, &inside));
     if (first == 0xFFFFFFFFu) {
       b->ran = true;
-      bool grown = false;  // inside the launches, into the pool's spare words
-      for (size_t i = 0; i < b->ninst; ++i) {
-        grown |= b->cap[i] != b->h_inst[i].cap;
-        b->cap[i] = b->h_inst[i].cap;
-      }
-      if (grown) {  // lay the next run out anew if every instance could be resident at these sizes
+      if (inside) {  // lay the next run out anew if every instance could be resident at these sizes
         const unsigned long long now = b->resident_bytes;
         BTRY(choose_resident(b));
         b->layout_dirty |= b->resident_bytes > now;
