@@ -47,7 +47,7 @@ namespace ppvm {
 void set_last_error(const std::string& msg);
 // The per-device buffer cache of the sums (engine.cu): buffers handed back once their
 // stream is idle are reused by later batches and sums without cudaMalloc/cudaFree.
-cudaError_t cache_malloc(void** out, size_t bytes);
+cudaError_t cache_malloc(void** out, size_t bytes, bool batch_growth = false);
 void cache_free(void* p);
 }
 
@@ -648,9 +648,10 @@ bool grow_on_device() {
   return v;
 }
 
-// Lays the pool out for the current capacities.  With keep, live terms move over.
-ppvm_status layout(ppvm_batch* b, bool keep) {
-  std::vector<BInst> old(b->h_inst, b->h_inst + b->ninst);
+// Lays the pool out for the current capacities.  With keep, live terms move over.  If that fails, the
+// instance table describes the old pool again, and the next run lays out anew: it must not run on the
+// old pool with the new offsets.
+ppvm_status layout_at(ppvm_batch* b, bool keep, const std::vector<BInst>& old) {
   unsigned long long words = 0;
   for (size_t i = 0; i < b->ninst; ++i) {
     BInst& I = b->h_inst[i];
@@ -670,12 +671,12 @@ ppvm_status layout(ppvm_batch* b, bool keep) {
   BTRY(choose_resident(b));
   BCUDA(cudaStreamSynchronize(b->stream));
   void* np = nullptr;
-  if (spare && ppvm::cache_malloc(&np, bytes + spare) != cudaSuccess) {
+  if (spare && ppvm::cache_malloc(&np, bytes + spare, keep) != cudaSuccess) {
     cudaGetLastError();
     np = nullptr;
     spare = 0;
   }
-  if (!np) BCUDA(ppvm::cache_malloc(&np, bytes));
+  if (!np) BCUDA(ppvm::cache_malloc(&np, bytes, keep));
   // zeroed: pair-table slots of an earlier user must not carry a live epoch (an instance that
   // takes spare words clears them itself)
   cudaError_t e = cudaMemsetAsync(np, 0, bytes, b->stream);
@@ -707,6 +708,14 @@ ppvm_status layout(ppvm_batch* b, bool keep) {
   b->layout_dirty = false;
   drop_graphs(b);
   return PPVM_OK;
+}
+
+ppvm_status layout(ppvm_batch* b, bool keep) {
+  const std::vector<BInst> old(b->h_inst, b->h_inst + b->ninst);
+  b->layout_dirty = true;
+  const ppvm_status st = layout_at(b, keep, old);
+  if (st != PPVM_OK) std::copy(old.begin(), old.end(), b->h_inst);
+  return st;
 }
 
 // Resets every instance to its initial terms (resident in the input block, scattered into
@@ -767,10 +776,12 @@ ppvm_status grow_failed(ppvm_batch* b, uint32_t* first, bool* inside) {
   for (size_t i = 0; i < b->ninst; ++i) {
     BInst& I = b->h_inst[i];
     if (!I.err) continue;
+    b->layout_dirty = true;  // the failed op has left links in the region: the pool is laid out anew in any case
     if (I.err != kErrCapacity)
       return bfail(PPVM_ECUDA, "batch instance " + std::to_string(i) + ": device error " + std::to_string(I.err));
-    b->cap[i] = grown_cap(b->cap[i], I.need);
-    if (b->cap[i] >= 0xFFFFFFF0ull) return bfail(PPVM_ECAPACITY, "batch instance capacity limit (2^32) exceeded");
+    const unsigned long long cap = grown_cap(b->cap[i], I.need);
+    if (cap >= 0xFFFFFFF0ull) return bfail(PPVM_ECAPACITY, "batch instance capacity limit (2^32) exceeded");
+    b->cap[i] = cap;
     I.err = 0;
     grow = true;
     uint32_t L = 0;  // the layer holding the failing op

@@ -237,10 +237,11 @@ void pool_release_device(int dev) {  // caller holds g_pool_mu; dev is current
 }
 
 // Where a pool allocation is made, for the allocation-failure test hook below.
-enum AllocSite : unsigned { kAllocCreate = 0, kAllocGrowth = 1, kAllocRunScratch = 2 };
+enum AllocSite : unsigned { kAllocCreate = 0, kAllocGrowth = 1, kAllocRunScratch = 2, kAllocBatchPool = 3 };
 
 // Test hook: PPVM_TEST_FAIL_ALLOC names allocation sites ("growth": storage growth of a live
-// sum; "run-scratch": the fused runs' scratch planes; comma-separated) whose pool
+// sum; "run-scratch": the fused runs' scratch planes; "batch-pool": a batch's larger pool when
+// instances outgrow theirs; comma-separated) whose pool
 // allocations fail as if the device had no memory left, without calling cudaMalloc.  Read
 // once per process; the failure-handling tests set it in a child process.
 bool alloc_fails(AllocSite site) {
@@ -251,6 +252,7 @@ bool alloc_fails(AllocSite site) {
       const std::string v(e);
       if (v.find("growth") != std::string::npos) m |= 1u << kAllocGrowth;
       if (v.find("run-scratch") != std::string::npos) m |= 1u << kAllocRunScratch;
+      if (v.find("batch-pool") != std::string::npos) m |= 1u << kAllocBatchPool;
     }
     return m;
   }();
@@ -1926,7 +1928,9 @@ ppvm_sum* take_cached(int device, int W) {
 namespace ppvm {
 // The buffer cache for the other translation units (batch.cu): same rules as for the sums,
 // a buffer goes back only when the stream that used it is idle.
-cudaError_t cache_malloc(void** out, size_t bytes) { return pool_malloc(out, bytes); }
+cudaError_t cache_malloc(void** out, size_t bytes, bool batch_growth) {
+  return pool_malloc(out, bytes, batch_growth ? kAllocBatchPool : kAllocCreate);
+}
 void cache_free(void* p) { pool_free(p); }
 void release_batch_staging();  // batch.cu: frees the pinned staging buffer of the uploads
 void release_mlp_staging();    // learned.cu: frees the kept pinned buffer of the sample orders
