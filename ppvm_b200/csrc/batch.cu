@@ -442,6 +442,7 @@ struct ppvm_batch {
   uint64_t* d_init = nullptr;
   uint64_t* pool = nullptr;
   BSpare* d_spare = nullptr;
+  size_t spare_bytes = 0;  // of the pool, counted among the device's
   unsigned long long resident_bytes = 0;  // dynamic shared memory per CTA for resident instances
   double* d_out = nullptr;
   bool inputs_dirty = true;
@@ -637,7 +638,22 @@ ppvm_status choose_resident(ppvm_batch* b) {
   return PPVM_OK;
 }
 
-constexpr size_t kSpareMax = (size_t)1 << 30;
+// Spare words of one batch, and of all live batches of a device together: beyond that a batch grows through
+// the host.  Spare words are room that sums and other batches do not get.
+constexpr size_t kSpareMin = (size_t)16 << 20, kSpareMax = (size_t)1 << 30, kSpareTotal = (size_t)4 << 30;
+std::atomic<size_t> g_spare_live[64];
+
+// Up to `want` bytes of the device's spare room, or none when less than kSpareMin is left.
+size_t take_spare(int device, size_t want) {
+  std::atomic<size_t>& live = g_spare_live[device & 63];
+  size_t now = live.load();
+  for (;;) {
+    const size_t got = std::min(want, kSpareTotal - now) & ~(size_t)255;
+    if (got < std::min(want, kSpareMin)) return 0;
+    if (live.compare_exchange_weak(now, now + got)) return got;
+  }
+}
+void give_spare(int device, size_t bytes) { g_spare_live[device & 63] -= bytes; }
 
 // PPVM_BATCH_GROW=host: no spare words, every growth through the host (for the tests).
 bool grow_on_device() {
@@ -666,16 +682,20 @@ ppvm_status layout_at(ppvm_batch* b, bool keep, const std::vector<BInst>& old) {
   // Spare words after the regions, for instances to grow into inside a launch: 31 times the
   // regions, between 16 MB and 1 GB.  A device that cannot spare them runs without (growth
   // through the host).
-  size_t spare = bytes >= kSpareMax / 31 ? kSpareMax : std::max<size_t>(31 * bytes, (size_t)16 << 20);
-  if (!grow_on_device()) spare = 0;
   BTRY(choose_resident(b));
   BCUDA(cudaStreamSynchronize(b->stream));
+  give_spare(b->device, b->spare_bytes);  // the old pool's: it goes when this layout succeeds, and is not grown into again
+  b->spare_bytes = 0;
+  size_t spare = bytes >= kSpareMax / 31 ? kSpareMax : std::max<size_t>(31 * bytes, kSpareMin);
+  spare = grow_on_device() ? take_spare(b->device, spare) : 0;
   void* np = nullptr;
   if (spare && ppvm::cache_malloc(&np, bytes + spare, keep) != cudaSuccess) {
     cudaGetLastError();
     np = nullptr;
+    give_spare(b->device, spare);
     spare = 0;
   }
+  b->spare_bytes = spare;
   if (!np) BCUDA(ppvm::cache_malloc(&np, bytes, keep));
   // zeroed: pair-table slots of an earlier user must not carry a live epoch (an instance that
   // takes spare words clears them itself)
@@ -960,6 +980,7 @@ ppvm_status ppvm_batch_destroy(ppvm_batch* b) {
   cudaSetDevice(b->device);
   if (b->stream) cudaStreamSynchronize(b->stream);
   drop_graphs(b);
+  give_spare(b->device, b->spare_bytes);
   ppvm::cache_free(b->d_inst);
   cudaFreeHost(b->h_inst);
   ppvm::cache_free(b->d_input);
