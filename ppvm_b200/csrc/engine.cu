@@ -153,6 +153,7 @@ struct ppvm_sum {
   unsigned long long* link = nullptr;  // per term: its rotation partner's coefficient (kNoLink between rotations)
   unsigned long long* table = nullptr;
   unsigned long long table_cap = 0;
+  unsigned run_turn = 0;           // alternates the fused runs' counts of large groups (Ctrl::run_large)
   unsigned long long run_slots_used = 0;  // group-table slots the fused runs since the last clean state hashed into
   unsigned long long* tstate = nullptr;
   unsigned long long tstate_cap = 0;
@@ -315,8 +316,8 @@ unsigned long long run_scratch_min_groups() {
   return v;
 }
 
-// The group mode of the fused runs: 0 chosen per run (many single-member groups: one group per lane;
-// otherwise tiles of groups), 1 tiles, 3 one group per lane.  PPVM_RUN_GROUP_MODE=tiled|lanes forces
+// The group mode of the fused runs: 0 chosen per run (run_lanes: many groups, few of them large, go one
+// per lane; otherwise tiles of groups), 1 tiles, 3 one group per lane.  PPVM_RUN_GROUP_MODE=tiled|lanes forces
 // one ("warp", once a mode of its own, is tiles); the tests run the fused-run cases in each.
 unsigned run_group_mode() {
   static const unsigned v = [] {
@@ -1035,12 +1036,13 @@ struct K {
     // k_run_tiles or k_run_lanes reset what a run used, grow() clears them on allocation and run_list()
     // after a device error
     const int trunc = trunc_op >= 0 ? 1 : 0;
+    const unsigned turn = s->run_turn ^= 1u;  // which count of large groups this run uses
     {
       ProfScope ps(s, F_RUN_CLASSIFY, op0, L);
       const unsigned tep = s->next_table_epoch();
       launch(k_run_classify<W, kScanBlock, ITEMS>, grid_for(nub, TILE, 8), kScanBlock, 0, s->stream, P, O,
              s->d_ctrl, d_rd, s->R, s->table, tsize - 1, tep, trunc, s->thr, s->maxw, s->tstate,
-             s->next_tile_epoch(), op0);
+             s->next_tile_epoch(), op0, turn);
     }
     {
       ProfScope ps(s, F_RUN_ORDER, op0, L);
@@ -1050,7 +1052,7 @@ struct K {
     }
     {
       ProfScope ps(s, F_RUN_SCATTER, op0, L);
-      launch(k_run_scatter<W>, grid_for(nub, 256, 8), 256, 0, s->stream, P, s->d_ctrl, d_rd, s->R);
+      launch(k_run_scatter<W>, grid_for(nub, 256, 8), 256, 0, s->stream, P, s->d_ctrl, d_rd, s->R, turn);
     }
     // Many groups: scratch mode (group outputs placed by k_run_place, one look-back per tile
     // of groups instead of one per group).  ngroups <= live terms <= nub, so below the
@@ -1092,19 +1094,19 @@ struct K {
         static const int resident = blocks_per_sm(k_run_tiles<W>, kTileWarps * 32);
         launch(k_run_tiles<W>, grid_for(nub, kTileWarps, std::min(resident, 8)), kTileWarps * 32, 0, s->stream,
             O, S, s->d_ctrl, d_rd, s->R, trunc, s->thr, s->maxw, s->tstate, s->next_tile_epoch(), op0,
-            trunc_op, s->d_log, scratch_min, mode);  // its last block publishes the counts and the op log
+            trunc_op, s->d_log, scratch_min, mode, turn);  // its last block publishes the counts and the op log
       }
       if (lanes) {
         static const int resident = blocks_per_sm(k_run_lanes<W>, kRunWarps * 32);
         launch(k_run_lanes<W>, grid_for(nub, 32 * kRunWarps, std::min(resident, 8)), kRunWarps * 32, 0, s->stream,
             O, s->d_ctrl, d_rd, s->R, trunc, s->thr, s->maxw, s->tstate, s->next_tile_epoch(), op0,
-            trunc_op, s->d_log, mode);
+            trunc_op, s->d_log, mode, turn);
       }
     }
     if (allow && mode != 3) {
       ProfScope ps(s, F_RUN_PLACE, op0, L);
       launch(k_run_place<W, 256, 2>, grid_for(nub, 512, 4), 256, 0, s->stream,
-          S, O, s->d_ctrl, s->R, scratch_min, s->tstate, s->next_tile_epoch(), op0, mode);
+          S, O, s->d_ctrl, s->R, scratch_min, s->tstate, s->next_tile_epoch(), op0, mode, turn);
     }
     std::swap(s->planes, s->alt);
     s->swaps.push_back(op0);
@@ -1321,6 +1323,7 @@ ppvm_status clear_err(ppvm_sum* s) {
   c.done = 0;  // blocks that returned early on the error never counted
   c.scr_top = 0;
   c.rot_s = c.rot_pairs = 0;
+  c.run_large[0] = c.run_large[1] = 0;
   for (int t = 0; t < 4; ++t) c.tickets[t] = 0;
   CUDA_TRY(cudaMemcpyAsync(s->d_ctrl, &c, sizeof(Ctrl), cudaMemcpyHostToDevice, s->stream));
   CUDA_TRY(cudaStreamSynchronize(s->stream));

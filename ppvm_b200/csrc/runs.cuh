@@ -18,8 +18,8 @@
 // Kernels, in order: k_run_classify (group keys into a hash table, members counted; terms
 // outside every group compacted to the output with the truncation), k_run_order
 // (deterministic group numbering by first member, member offsets), k_run_scatter (member
-// lists), then k_run_tiles or, for many single-member groups, k_run_lanes (butterfly + truncation +
-// ordered write; the last block publishes the counts and the op log), and k_run_place when the
+// lists), then k_run_tiles or, for many small groups, k_run_lanes (butterfly + truncation + ordered
+// write; the last block publishes the counts and the op log), and k_run_place when the
 // tiles left their order to it.
 #pragma once
 
@@ -29,6 +29,7 @@ namespace ppvm {
 
 constexpr int kRunMaxK = 10;       // groups of up to 10 coordinates (2^10 slots) are fused
 constexpr int kRunMaxGates = 256;  // gates per fused run
+constexpr int kRunLaneK = 3;       // groups of up to 3 coordinates (8 slots) run on one lane
 constexpr int kRunWarps = 4;       // warps of a k_run_lanes block
 constexpr unsigned long long kRunTileMinGroups = 8192;  // fewer groups: never one per lane
 constexpr unsigned long long kRunLogScratchBit = 1ull << 63;  // in the op log of a run's first gate
@@ -77,13 +78,15 @@ template <int W, int BLOCK, int ITEMS>
 __global__ void __launch_bounds__(BLOCK)
 k_run_classify(Planes P, Planes O, Ctrl* ctrl, const RunDesc* rd, RunScratch R, unsigned long long* table,
                unsigned long long tmask, unsigned tepoch, int trunc, double thr, unsigned long long maxw,
-               unsigned long long* ts, unsigned epoch, int op) {
+               unsigned long long* ts, unsigned epoch, int op, unsigned turn) {
   pdl_wait();
   __shared__ unsigned s_tile;
   __shared__ unsigned long long s_slot;
   __shared__ unsigned s_base[ITEMS * (BLOCK / 32) + 1];
   __shared__ int s_err;
+  __shared__ unsigned s_large;
   __shared__ uint16_t s_gidx[64 * W];  // qubit -> its gate's index in the run
+  if (threadIdx.x == 0) s_large = 0;
   if (threadIdx.x == 0) s_err = ld_volatile_int(&ctrl->err);
   for (unsigned j = threadIdx.x; j < rd->L; j += BLOCK) s_gidx[rd->q[j]] = (uint16_t)j;
   __syncthreads();
@@ -99,6 +102,7 @@ k_run_classify(Planes P, Planes O, Ctrl* ctrl, const RunDesc* rd, RunScratch R, 
   const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   constexpr int NW = BLOCK / 32;
   const bool wcap = maxw != ~0ull;
+  unsigned large = 0;  // groups opened by this thread that are too large for a lane
   for (;;) {
     const unsigned tile = next_tile(&ctrl->tickets[1], &s_tile);
     if (tile >= ntiles) break;
@@ -165,6 +169,7 @@ k_run_classify(Planes P, Planes O, Ctrl* ctrl, const RunDesc* rd, RunScratch R, 
             if (slot_epoch(cur) != (tepoch & 0xFFFFu)) {
               const unsigned long long prev = atomicCAS(&table[slot], cur, mine);
               if (prev != cur) continue;
+              large += k > (unsigned)kRunLaneK;
               break;  // new group
             }
             if (slot_tag(cur) == tag) {
@@ -207,6 +212,10 @@ k_run_classify(Planes P, Planes O, Ctrl* ctrl, const RunDesc* rd, RunScratch R, 
       }
     if (tile == ntiles - 1 && threadIdx.x == 0) ctrl->n_s = excl + agg;
   }
+  large = __reduce_add_sync(kFull, large);
+  if (lane == 0 && large) atomicAdd(&s_large, large);
+  __syncthreads();
+  if (threadIdx.x == 0 && s_large) atomicAdd(&ctrl->run_large[turn], (unsigned long long)s_large);
 }
 
 // Numbers the groups by their smallest member (index order) and lays out member lists.
@@ -329,9 +338,10 @@ k_run_order(Ctrl* ctrl, RunScratch R, unsigned long long* ts_a, unsigned long lo
 // member resets its slot (same values from every member), and the next run needs no
 // clearing pass.  After a device error the host clears both arrays instead.
 template <int W>
-__global__ void __launch_bounds__(256) k_run_scatter(Planes P, Ctrl* ctrl, const RunDesc* rd, RunScratch R) {
+__global__ void __launch_bounds__(256) k_run_scatter(Planes P, Ctrl* ctrl, const RunDesc* rd, RunScratch R, unsigned turn) {
   pdl_wait();
   if (ld_volatile_int(&ctrl->err)) return;
+  if (blockIdx.x == 0 && threadIdx.x == 0) ctrl->run_large[turn ^ 1u] = 0;  // for the next run
   const unsigned long long N = ld_volatile(&ctrl->n);
   const uint32_t cls = rd->cls;
   uint64_t Q[W];
@@ -665,7 +675,6 @@ struct WarpGroup {
 };
 
 // ---- lane mode: one group per lane ------------------------------------------------------
-constexpr int kRunLaneK = 3;  // groups of up to 3 coordinates (8 slots) run on one lane
 
 // A small group on one lane: its slots in registers (slot c at coef[c], existence bit c of
 // ex), its key and coordinate qubits, the gates of its coordinates in run order.
@@ -828,19 +837,26 @@ __device__ __forceinline__ void lane_write(const LaneGroup<W>& G, Planes D, unsi
   }
 }
 
-// Whether a run's groups go one per lane: forced (mode 3), or chosen for many groups of mostly one
-// member.
-__device__ __forceinline__ bool run_lanes(unsigned long long ngroups, unsigned long long members, unsigned mode) {
-  return mode == 3 || (mode == 0 && ngroups >= kRunTileMinGroups && 2 * members < 3 * ngroups);
+// Whether a run's groups go one per lane: forced (mode 3), or chosen for many groups of which at most
+// one in 8 is too large for a lane (the warp runs those one after the other).  RX runs of 10 gates on
+// groups of one coordinate, a share p of them of K, group kernel and placement in us, tiles / lanes:
+//   300,000 groups on 144 qubits, p = 1 % of K = 5: 598 / 101, of K = 10: 1834 / 687;
+//   p = 20 % of K = 6: 872 / 415;  all of K = 5: 947 / 947 (602 / 813 on 40 qubits);
+//   40,000 groups on 144 qubits, p = 5 % of K = 4: 94 / 44, of K = 10: 693 / 551;
+//   p = 20 % of K = 7: 139 / 181;  all of K = 4: 108 / 195.
+// Counting members instead (lanes up to 1.5 per group) sent runs of a few gates, whose groups are all
+// small but full, to the tiles.
+__device__ __forceinline__ bool run_lanes(unsigned long long ngroups, unsigned long long large, unsigned mode) {
+  return mode == 3 || (mode == 0 && ngroups >= kRunTileMinGroups && 8 * large <= ngroups);
 }
 
 // Whether this launch's groups go one per lane (k_run_lanes) or in tiles (k_run_tiles); both
 // kernels of a run read the same counts and decide alike, and the other returns at once.
 struct RunCounts {
-  unsigned long long groups, members, untouched;
+  unsigned long long groups, large, untouched;
 };
-__device__ __forceinline__ RunCounts run_counts(const Ctrl* ctrl) {
-  return {ld_volatile(&ctrl->n_pairs), ld_volatile(&ctrl->n_side), ld_volatile(&ctrl->n_s)};
+__device__ __forceinline__ RunCounts run_counts(const Ctrl* ctrl, unsigned turn) {
+  return {ld_volatile(&ctrl->n_pairs), ld_volatile(&ctrl->run_large[turn]), ld_volatile(&ctrl->n_s)};
 }
 
 // One group per lane, for runs of many small groups (run_lanes).  A warp takes 32 consecutive groups
@@ -851,15 +867,15 @@ __device__ __forceinline__ RunCounts run_counts(const Ctrl* ctrl) {
 template <int W>
 __global__ void __launch_bounds__(kRunWarps * 32, 5)
 k_run_lanes(Planes O, Ctrl* ctrl, const RunDesc* rd, RunScratch R, int trunc, double thr, unsigned long long maxw,
-            unsigned long long* ts, unsigned epoch, int op, int trunc_op, OpLog* log, unsigned mode) {
+            unsigned long long* ts, unsigned epoch, int op, int trunc_op, OpLog* log, unsigned mode, unsigned turn) {
   pdl_wait();
   __shared__ unsigned long long s_slot[kRunWarps][kTileSlots];
   __shared__ TileGates s_g[kRunWarps];
   __shared__ unsigned s_created[kRunMaxGates];
   __shared__ double s_cs[kRunMaxGates], s_sn[kRunMaxGates];
   __shared__ uint16_t s_gidx[64 * W];  // qubit -> its gate's index in the run
-  const RunCounts rc = run_counts(ctrl);
-  if (ld_volatile_int(&ctrl->err) || !run_lanes(rc.groups, rc.members, mode)) return;
+  const RunCounts rc = run_counts(ctrl, turn);
+  if (ld_volatile_int(&ctrl->err) || !run_lanes(rc.groups, rc.large, mode)) return;
   const unsigned long long ngroups = rc.groups, ubase = rc.untouched;  // untouched survivors go first
   const unsigned long long ntiles = (ngroups + 31) / 32;
   const unsigned long long want = (ntiles + kRunWarps - 1) / kRunWarps;
@@ -983,7 +999,7 @@ template <int W>
 __global__ void __launch_bounds__(kTileWarps * 32, 3)
 k_run_tiles(Planes O, Planes S, Ctrl* ctrl, const RunDesc* rd, RunScratch R, int trunc, double thr,
             unsigned long long maxw, unsigned long long* ts, unsigned epoch, int op, int trunc_op, OpLog* log,
-            unsigned long long scratch_min, unsigned mode) {
+            unsigned long long scratch_min, unsigned mode, unsigned turn) {
   pdl_wait();
   constexpr int BLOCK = kTileWarps * 32;
   constexpr unsigned MANY = W <= 4 ? 4 : 2;  // a warp's keys: MANY * 2W <= 32 words, one per lane
@@ -993,8 +1009,8 @@ k_run_tiles(Planes O, Planes S, Ctrl* ctrl, const RunDesc* rd, RunScratch R, int
   __shared__ uint16_t s_gidx[64 * W];  // qubit -> its gate's index in the run
   __shared__ unsigned s_cnt[kTileWarps], s_tile;
   __shared__ unsigned long long s_base;
-  const RunCounts rc = run_counts(ctrl);
-  if (ld_volatile_int(&ctrl->err) || run_lanes(rc.groups, rc.members, mode)) return;
+  const RunCounts rc = run_counts(ctrl, turn);
+  if (ld_volatile_int(&ctrl->err) || run_lanes(rc.groups, rc.large, mode)) return;
   const unsigned long long ngroups = rc.groups, ubase = rc.untouched;  // untouched survivors go first
   const bool scratch = ngroups >= scratch_min;  // the same in every block
   const unsigned per = scratch || ngroups >= kTileManyGroups ? MANY : 1u;
@@ -1145,7 +1161,7 @@ k_run_tiles(Planes O, Planes S, Ctrl* ctrl, const RunDesc* rd, RunScratch R, int
 template <int W, int BLOCK, int ITEMS>
 __global__ void __launch_bounds__(BLOCK)
 k_run_place(Planes S, Planes O, Ctrl* ctrl, RunScratch R, unsigned long long scratch_min, unsigned long long* ts,
-            unsigned epoch, int op, unsigned mode) {
+            unsigned epoch, int op, unsigned mode, unsigned turn) {
   pdl_wait();
   constexpr int NW = BLOCK / 32;
   constexpr int TILE = BLOCK * ITEMS;
@@ -1158,7 +1174,7 @@ k_run_place(Planes S, Planes O, Ctrl* ctrl, RunScratch R, unsigned long long scr
   if (threadIdx.x == 0) {
     const unsigned long long ng = ld_volatile(&ctrl->n_pairs);
     s_skip = ld_volatile_int(&ctrl->err) || ng == 0 || ng < scratch_min ||
-             run_lanes(ng, ld_volatile(&ctrl->n_side), mode);
+             run_lanes(ng, ld_volatile(&ctrl->run_large[turn]), mode);
   }
   __syncthreads();
   if (s_skip) return;  // the same in every block (look-back mode, or an earlier error)
