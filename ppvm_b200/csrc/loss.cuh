@@ -313,8 +313,11 @@ __device__ __forceinline__ unsigned block_excl(unsigned v, unsigned* s_w, unsign
   return base + inc - v;
 }
 
+// The reset channel above 192 qubits (W = 8) at two blocks an SM: the compiler otherwise takes 215
+// registers for it, one block, and the channel 1345 us instead of 1050 on 1.8 million terms.  (0: no
+// bound.  On 40 qubits any bound costs: reset 440 -> 563 us, correlated loss 600 -> 859.)
 template <int W, int BLOCK, int M>
-__global__ void __launch_bounds__(BLOCK)
+__global__ void __launch_bounds__(BLOCK, W == 8 && M == kResetLoss ? 2 : 0)
 k_loss_emit(Planes P, Planes O, Ctrl* ctrl, LossOp op_in, const unsigned long long* table, unsigned long long mask,
             unsigned tepoch, unsigned long long* ts, unsigned long long* ts2, unsigned epoch, unsigned epoch2,
             int opi, OpLog* log) {
