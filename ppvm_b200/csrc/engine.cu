@@ -1530,8 +1530,8 @@ ppvm_status run_small(ppvm_sum* s, const ppvm_op* ops, size_t n_ops, size_t* sta
         r.c = std::sqrt(r.b);
       } else if (is_local(s, op)) {
         size_t j = i;
-        while (j < n_ops && j - i <= (size_t)kSmallLocal && ops[j].flags == 0 && is_local(s, ops[j])) ++j;
-        if (j - i > (size_t)kSmallLocal) break;
+        while (j < n_ops && j - i <= (size_t)small_local(s->W) && ops[j].flags == 0 && is_local(s, ops[j])) ++j;
+        if (j - i > (size_t)small_local(s->W)) break;
         for (; i < j; ++i) {
           r.kind = S_LOCAL;
           r.d = to_devop(ops[i]);
@@ -1563,8 +1563,7 @@ ppvm_status run_small(ppvm_sum* s, const ppvm_op* ops, size_t n_ops, size_t* sta
       rec.push_back(r);
       ++i;
     }
-    // a short head of a long list is not worth the launch and the synchronisation
-    if (rec.empty() || (rec.size() < 64 && *start + rec.size() < n_ops)) return PPVM_OK;
+    if (rec.empty() || (rec.size() < kSmallHead && *start + rec.size() < n_ops)) return PPVM_OK;
     const void* d_ops = nullptr;
     SmallInline few;
     if (rec.size() <= (size_t)kSmallInline) {

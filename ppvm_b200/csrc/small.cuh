@@ -23,8 +23,20 @@ namespace ppvm {
 constexpr int kSmallBlock = 512;
 constexpr int kSmallItems = 4;
 constexpr int kSmallOps = 2048;                  // ops per launch
-constexpr unsigned long long kSmallStart = 512;  // sums of more terms take the pipelines at once
-constexpr int kSmallLocal = 64;                  // longer stretches of local ops: the composed pass
+// Sums of more terms take the pipelines at once.  200 rotations on a closed sum, interpreter / pipelines:
+// 450 terms 525 / 1704 us on 20 qubits, 880 / 2408 on 400.  Above 512 it would still be the faster on a sum
+// that stays as it is (900 terms, 20 qubits: 1178 / 2708), but not where the region holds 1024
+// terms (900 terms, 400 qubits: 3018 / 2814, as it is left and entered in vain), and a sum that grows
+// leaves it after a few ops.
+constexpr unsigned long long kSmallStart = 512;
+// A head of fewer ops before one that the interpreter does not take (a long stretch of local ops, a
+// two-qubit Pauli error) is left to the pipelines.  Interpreting it would pay from about 4 ops on (16
+// rotations before 100 Cliffords, 20 qubits, 20 terms: 88 / 147 us); the line is a safe one.
+constexpr size_t kSmallHead = 64;
+// Longer stretches of local ops go to the composed Clifford pass, whose cost hardly depends on their
+// length.  Six stretches of k ops between rotations, 300 terms, interpreter / pipelines: 150 qubits, k = 48
+// 208 / 248 us, k = 64 248 / 264; 400 qubits, k = 48 297 / 294, k = 64 408 / 301.
+constexpr int small_local(int W) { return W <= 4 ? 64 : 48; }
 
 // Terms the region holds: as many as fit into shared memory with the pair table and the sort keys.
 template <int W>
