@@ -837,26 +837,34 @@ __device__ __forceinline__ void lane_write(const LaneGroup<W>& G, Planes D, unsi
   }
 }
 
-// Whether a run's groups go one per lane: forced (mode 3), or chosen for many groups of which at most
-// one in 8 is too large for a lane (the warp runs those one after the other).  RX runs of 10 gates on
-// groups of one coordinate, a share p of them of K, group kernel and placement in us, tiles / lanes:
-//   300,000 groups on 144 qubits, p = 1 % of K = 5: 598 / 101, of K = 10: 1834 / 687;
-//   p = 20 % of K = 6: 872 / 415;  all of K = 5: 947 / 947 (602 / 813 on 40 qubits);
-//   40,000 groups on 144 qubits, p = 5 % of K = 4: 94 / 44, of K = 10: 693 / 551;
-//   p = 20 % of K = 7: 139 / 181;  all of K = 4: 108 / 195.
-// Counting members instead (lanes up to 1.5 per group) sent runs of a few gates, whose groups are all
-// small but full, to the tiles.
-__device__ __forceinline__ bool run_lanes(unsigned long long ngroups, unsigned long long large, unsigned mode) {
-  return mode == 3 || (mode == 0 && ngroups >= kRunTileMinGroups && 8 * large <= ngroups);
-}
-
-// Whether this launch's groups go one per lane (k_run_lanes) or in tiles (k_run_tiles); both
-// kernels of a run read the same counts and decide alike, and the other returns at once.
+// Whether a run's groups go one per lane: forced (mode 3), or chosen from kRunTileMinGroups groups on, by
+// how many of them are too large for a lane.  The warp runs those one after the other, and the order
+// puts alike groups side by side, so that one warp may get 32 of them: 0.16 ms of tail at 4 to 6
+// coordinates, 0.5 at 8, 2.3 at 10, while the other lanes' groups cost nearly nothing.  RX runs of 10
+// gates on groups of one coordinate and a share of K, group kernel and placement in us, tiles / lanes:
+//   none large: always lanes (3 gates, 3.0M terms in full groups on 200 qubits: 1920 / 260);
+//   300,000 groups, scattered: 1 % of K = 5 598 / 101 (144 qubits), of K = 10 1834 / 687, 20 % of K = 6
+//   531 / 339 (40 qubits), all of K = 5 602 / 813; side by side, the worst: 0.2 % of K = 10 2365 / 2385;
+//   40,000 groups, scattered: 5 % of K = 4 94 / 44, 20 % of K = 7 139 / 181; side by side: 5 % of K = 4
+//   92 / 187, of K = 8 149 / 646.
+// So lanes are taken when no group is large; from kRunLaneMany groups on, where tiles leave their order to
+// k_run_place, up to one in 16 may be (at one in 6 a kicked-Ising layer of 4M terms takes 12.6 ms in tiles
+// and 14.8 in lanes); and in runs of mostly single members (Clifford+T: 26 layers 3.35 ms, 6.0 in
+// tiles).
+constexpr unsigned long long kRunLaneMany = 1ull << 18;
 struct RunCounts {
-  unsigned long long groups, large, untouched;
+  unsigned long long groups, members, large, untouched;
 };
 __device__ __forceinline__ RunCounts run_counts(const Ctrl* ctrl, unsigned turn) {
-  return {ld_volatile(&ctrl->n_pairs), ld_volatile(&ctrl->run_large[turn]), ld_volatile(&ctrl->n_s)};
+  return {ld_volatile(&ctrl->n_pairs), ld_volatile(&ctrl->n_side), ld_volatile(&ctrl->run_large[turn]),
+          ld_volatile(&ctrl->n_s)};
+}
+// The group kernels and k_run_place read the same counts and decide alike; those not needed return.
+__device__ __forceinline__ bool run_lanes(const RunCounts& c, unsigned mode) {
+  if (mode != 0) return mode == 3;
+  if (c.groups < kRunTileMinGroups) return false;
+  return c.large == 0 || 2 * c.members < 3 * c.groups ||
+         (c.groups >= kRunLaneMany && 16 * c.large <= c.groups);
 }
 
 // One group per lane, for runs of many small groups (run_lanes).  A warp takes 32 consecutive groups
@@ -875,7 +883,7 @@ k_run_lanes(Planes O, Ctrl* ctrl, const RunDesc* rd, RunScratch R, int trunc, do
   __shared__ double s_cs[kRunMaxGates], s_sn[kRunMaxGates];
   __shared__ uint16_t s_gidx[64 * W];  // qubit -> its gate's index in the run
   const RunCounts rc = run_counts(ctrl, turn);
-  if (ld_volatile_int(&ctrl->err) || !run_lanes(rc.groups, rc.large, mode)) return;
+  if (ld_volatile_int(&ctrl->err) || !run_lanes(rc, mode)) return;
   const unsigned long long ngroups = rc.groups, ubase = rc.untouched;  // untouched survivors go first
   const unsigned long long ntiles = (ngroups + 31) / 32;
   const unsigned long long want = (ntiles + kRunWarps - 1) / kRunWarps;
@@ -1010,7 +1018,7 @@ k_run_tiles(Planes O, Planes S, Ctrl* ctrl, const RunDesc* rd, RunScratch R, int
   __shared__ unsigned s_cnt[kTileWarps], s_tile;
   __shared__ unsigned long long s_base;
   const RunCounts rc = run_counts(ctrl, turn);
-  if (ld_volatile_int(&ctrl->err) || run_lanes(rc.groups, rc.large, mode)) return;
+  if (ld_volatile_int(&ctrl->err) || run_lanes(rc, mode)) return;
   const unsigned long long ngroups = rc.groups, ubase = rc.untouched;  // untouched survivors go first
   const bool scratch = ngroups >= scratch_min;  // the same in every block
   const unsigned per = scratch || ngroups >= kTileManyGroups ? MANY : 1u;
@@ -1172,9 +1180,8 @@ k_run_place(Planes S, Planes O, Ctrl* ctrl, RunScratch R, unsigned long long scr
   __shared__ unsigned long long s_dst[TILE];
   __shared__ int s_skip;
   if (threadIdx.x == 0) {
-    const unsigned long long ng = ld_volatile(&ctrl->n_pairs);
-    s_skip = ld_volatile_int(&ctrl->err) || ng == 0 || ng < scratch_min ||
-             run_lanes(ng, ld_volatile(&ctrl->run_large[turn]), mode);
+    const RunCounts rc = run_counts(ctrl, turn);
+    s_skip = ld_volatile_int(&ctrl->err) || rc.groups == 0 || rc.groups < scratch_min || run_lanes(rc, mode);
   }
   __syncthreads();
   if (s_skip) return;  // the same in every block (look-back mode, or an earlier error)
