@@ -54,9 +54,9 @@ struct Ctrl {
   unsigned long long rot_s;      // rotation: anticommuting terms found by k_rot_pair (0 between rotations)
   unsigned long long rot_pairs;  // rotation: partner pairs among them (0 between rotations)
   unsigned long long rot_n;      // live terms that the pair kernel of a rotation or one-child channel saw
-  // fused runs, by turns: groups of more than kRunLaneK coordinates that k_run_classify found (the other
-  // turn's word is cleared by k_run_scatter)
-  unsigned long long run_large[2];
+  // fused runs, by turns: groups of more than kRunLaneK coordinates that k_run_classify found, and the slots
+  // of all groups (the other turn's words are cleared by k_run_scatter)
+  unsigned long long run_large[2], run_slots[2];
   unsigned long long small_pc;   // ops of the list that k_small has applied
   unsigned spin_limit;         // polls a look-back waits before it gives up; 0 = kSpinLimit
   unsigned reserved;

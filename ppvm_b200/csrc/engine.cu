@@ -869,11 +869,25 @@ Lattice lattice_of(int L) {
   return lat;
 }
 
-// Resident blocks per SM of a kernel without dynamic shared memory (the same on every B200).
+// Resident blocks per SM of a kernel (the same on every B200).
 template <typename F>
-int blocks_per_sm(F* kern, int block) {
+int blocks_per_sm(F* kern, int block, size_t smem = 0) {
   int n = 0;
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, block, 0) == cudaSuccess && n > 0 ? n : 1;
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, block, smem) == cudaSuccess && n > 0 ? n : 1;
+}
+
+// The kernel's dynamic shared memory limit, set on its first use on the sum's device (sums of other threads
+// come here too).
+template <typename F>
+ppvm_status max_smem_once(const ppvm_sum* s, F* kern, size_t smem) {
+  static std::mutex mu;
+  static std::set<std::pair<const void*, int>> done;
+  std::lock_guard<std::mutex> lk(mu);
+  if (!done.count({(const void*)kern, s->device})) {
+    CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    done.insert({(const void*)kern, s->device});
+  }
+  return PPVM_OK;
 }
 
 // ---- kernel enqueue (templated on W) ------------------------------------------------------------
@@ -1091,8 +1105,9 @@ struct K {
       if (tiles) {
         // no more blocks than fit on the GPU at once: blocks take tiles by ticket, so more would
         // only queue on the ticket counter
-        static const int resident = blocks_per_sm(k_run_tiles<W>, kTileWarps * 32);
-        launch(k_run_tiles<W>, grid_for(nub, kTileWarps, std::min(resident, 8)), kTileWarps * 32, 0, s->stream,
+        PPVM_TRY(max_smem_once(s, k_run_tiles<W>, kTileSmem));
+        static const int resident = blocks_per_sm(k_run_tiles<W>, kTileWarps * 32, kTileSmem);
+        launch(k_run_tiles<W>, grid_for(nub, kTileWarps, std::min(resident, 8)), kTileWarps * 32, kTileSmem, s->stream,
             O, S, s->d_ctrl, d_rd, s->R, trunc, s->thr, s->maxw, s->tstate, s->next_tile_epoch(), op0,
             trunc_op, s->d_log, scratch_min, mode, turn);  // its last block publishes the counts and the op log
       }
@@ -1323,7 +1338,7 @@ ppvm_status clear_err(ppvm_sum* s) {
   c.done = 0;  // blocks that returned early on the error never counted
   c.scr_top = 0;
   c.rot_s = c.rot_pairs = 0;
-  c.run_large[0] = c.run_large[1] = 0;
+  c.run_large[0] = c.run_large[1] = c.run_slots[0] = c.run_slots[1] = 0;
   for (int t = 0; t < 4; ++t) c.tickets[t] = 0;
   CUDA_TRY(cudaMemcpyAsync(s->d_ctrl, &c, sizeof(Ctrl), cudaMemcpyHostToDevice, s->stream));
   CUDA_TRY(cudaStreamSynchronize(s->stream));

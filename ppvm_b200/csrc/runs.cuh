@@ -84,9 +84,9 @@ k_run_classify(Planes P, Planes O, Ctrl* ctrl, const RunDesc* rd, RunScratch R, 
   __shared__ unsigned long long s_slot;
   __shared__ unsigned s_base[ITEMS * (BLOCK / 32) + 1];
   __shared__ int s_err;
-  __shared__ unsigned s_large;
+  __shared__ unsigned long long s_large, s_slots;
   __shared__ uint16_t s_gidx[64 * W];  // qubit -> its gate's index in the run
-  if (threadIdx.x == 0) s_large = 0;
+  if (threadIdx.x == 0) s_large = s_slots = 0;
   if (threadIdx.x == 0) s_err = ld_volatile_int(&ctrl->err);
   for (unsigned j = threadIdx.x; j < rd->L; j += BLOCK) s_gidx[rd->q[j]] = (uint16_t)j;
   __syncthreads();
@@ -102,7 +102,9 @@ k_run_classify(Planes P, Planes O, Ctrl* ctrl, const RunDesc* rd, RunScratch R, 
   const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   constexpr int NW = BLOCK / 32;
   const bool wcap = maxw != ~0ull;
-  unsigned large = 0;  // groups opened by this thread that are too large for a lane
+  // groups opened by this thread that are too large for a lane, and the slots of all it opened
+  unsigned large = 0;
+  unsigned long long slots = 0;
   for (;;) {
     const unsigned tile = next_tile(&ctrl->tickets[1], &s_tile);
     if (tile >= ntiles) break;
@@ -170,6 +172,7 @@ k_run_classify(Planes P, Planes O, Ctrl* ctrl, const RunDesc* rd, RunScratch R, 
               const unsigned long long prev = atomicCAS(&table[slot], cur, mine);
               if (prev != cur) continue;
               large += k > (unsigned)kRunLaneK;
+              slots += 1u << k;
               break;  // new group
             }
             if (slot_tag(cur) == tag) {
@@ -212,10 +215,18 @@ k_run_classify(Planes P, Planes O, Ctrl* ctrl, const RunDesc* rd, RunScratch R, 
       }
     if (tile == ntiles - 1 && threadIdx.x == 0) ctrl->n_s = excl + agg;
   }
+#pragma unroll
+  for (int o = 16; o; o >>= 1) slots += __shfl_down_sync(kFull, slots, o);
   large = __reduce_add_sync(kFull, large);
-  if (lane == 0 && large) atomicAdd(&s_large, large);
+  if (lane == 0 && slots) {
+    atomicAdd(&s_slots, slots);
+    if (large) atomicAdd(&s_large, (unsigned long long)large);
+  }
   __syncthreads();
-  if (threadIdx.x == 0 && s_large) atomicAdd(&ctrl->run_large[turn], (unsigned long long)s_large);
+  if (threadIdx.x == 0 && s_slots) {
+    atomicAdd(&ctrl->run_slots[turn], s_slots);
+    if (s_large) atomicAdd(&ctrl->run_large[turn], s_large);
+  }
 }
 
 // Numbers the groups by their smallest member (index order) and lays out member lists.
@@ -341,7 +352,7 @@ template <int W>
 __global__ void __launch_bounds__(256) k_run_scatter(Planes P, Ctrl* ctrl, const RunDesc* rd, RunScratch R, unsigned turn) {
   pdl_wait();
   if (ld_volatile_int(&ctrl->err)) return;
-  if (blockIdx.x == 0 && threadIdx.x == 0) ctrl->run_large[turn ^ 1u] = 0;  // for the next run
+  if (blockIdx.x == 0 && threadIdx.x == 0) ctrl->run_large[turn ^ 1u] = ctrl->run_slots[turn ^ 1u] = 0;  // for the next run
   const unsigned long long N = ld_volatile(&ctrl->n);
   const uint32_t cls = rd->cls;
   uint64_t Q[W];
@@ -451,7 +462,8 @@ __device__ __forceinline__ void run_commit(Ctrl* ctrl, RunScratch R, int op0, in
 
 // ---- a group on a warp ------------------------------------------------------------------------
 constexpr int kTileWarps = 8;             // warps of a k_run_tiles block
-constexpr int kTileSlots = 512;           // slots of shared memory per warp (a group of 2^10 goes through them twice)
+constexpr int kTileSlots = 1 << kRunMaxK;  // slots of shared memory per warp: the largest group's
+constexpr size_t kTileSmem = sizeof(unsigned long long) * kTileWarps * kTileSlots;
 constexpr unsigned long long kNoSlot = ~0ull;  // a slot without a term (see link_bits for that NaN)
 
 // The gates of a group's coordinates in run order.
@@ -467,36 +479,28 @@ struct TileGates {
 // coordinate bits pairs lanes (shuffles), on a higher one registers; either way a slot's new value
 // is the reference's map_insert on the pair (crates/ppvm-pauli-sum/src/sum/rot1.rs:73,124: eps of a member
 // with bit b is +1 for b = 0 under RX, for b = 1 under RZ), with existence tracked apart from the value.
-// part < 0: the survivors of the run's TRUNCATE are counted, and written back to the shared slots
-// (the others empty) when they fit; part 0, 1: those of that half of 1024 slots are written.  Children
+// The survivors of the run's TRUNCATE are counted and written back to the shared slots (the others empty).  Children
 // made per gate are added to created (null: not).  In shared memory, a pair per lane and step, the
 // same butterflies took 4 times the instructions and a round of shared-memory latency per pair.
 template <int NR>
 __device__ __noinline__ unsigned tile_survivors(const TileGates& g, unsigned long long* slots,
                                                 const uint32_t* __restrict__ mcoord, const double* __restrict__ mcoef,
                                                 unsigned cnt, double eps_a, bool trunc, bool wok, double thr,
-                                                unsigned* created, int part) {
+                                                unsigned* created) {
   const unsigned lane = threadIdx.x & 31;
-  constexpr int NH = NR < 16 ? NR : 16;  // registers loaded at a time (512 slots)
   double c[NR];
   unsigned ex = 0;
+  __syncwarp();
 #pragma unroll
-  for (int h = 0; h < NR / NH; ++h) {
-    __syncwarp();
+  for (int r = 0; r < NR; ++r) slots[32 * r + lane] = kNoSlot;
+  __syncwarp();
+  for (unsigned m = lane; m < cnt; m += 32) slots[mcoord[m]] = link_bits(mcoef[m]);
+  __syncwarp();
 #pragma unroll
-    for (int r = 0; r < NH; ++r) slots[32 * r + lane] = kNoSlot;
-    __syncwarp();
-    for (unsigned m = lane; m < cnt; m += 32) {
-      const unsigned s = mcoord[m];
-      if (NR == NH || (int)(s >> 9) == h) slots[s & (32 * NH - 1)] = link_bits(mcoef[m]);
-    }
-    __syncwarp();
-#pragma unroll
-    for (int r = 0; r < NH; ++r) {
-      const unsigned long long u = slots[32 * r + lane];
-      c[h * NH + r] = __longlong_as_double((long long)u);
-      ex |= (unsigned)(u != kNoSlot) << (h * NH + r);
-    }
+  for (int r = 0; r < NR; ++r) {
+    const unsigned long long u = slots[32 * r + lane];
+    c[r] = __longlong_as_double((long long)u);
+    ex |= (unsigned)(u != kNoSlot) << r;
   }
   for (unsigned i = 0; i < g.k; ++i) {
     const unsigned t = g.bit[i];
@@ -550,15 +554,8 @@ __device__ __noinline__ unsigned tile_survivors(const TileGates& g, unsigned lon
   }
   const unsigned n = __reduce_add_sync(kFull, __popc(keep));
   __syncwarp();
-  if (NR == NH || part >= 0) {
 #pragma unroll
-    for (int h = 0; h < NR / NH; ++h)
-      if (NR == NH || h == part) {
-#pragma unroll
-        for (int r = 0; r < NH; ++r)
-          slots[32 * r + lane] = (keep >> (h * NH + r)) & 1u ? link_bits(c[h * NH + r]) : kNoSlot;
-      }
-  }
+  for (int r = 0; r < NR; ++r) slots[32 * r + lane] = (keep >> r) & 1u ? link_bits(c[r]) : kNoSlot;
   __syncwarp();
   return n;
 }
@@ -605,28 +602,26 @@ struct WarpGroup {
     __syncwarp();
   }
 
-  // Slots of the warp's shared memory that the group's survivors take (at most kTileSlots at a time).
-  __device__ __forceinline__ unsigned slots() const {
-    return k <= 5 ? 32u : k > 9 ? (unsigned)kTileSlots : 1u << k;
-  }
+  // Slots of the warp's shared memory that the group's survivors take.
+  __device__ __forceinline__ unsigned slots() const { return k <= 5 ? 32u : 1u << k; }
 
   __device__ __forceinline__ unsigned survivors(const TileGates& G, unsigned long long* sl, const RunScratch& R,
                                                 unsigned start, unsigned cnt, double eps_a, bool trunc, double thr,
-                                                unsigned* created, int part) const {
+                                                unsigned* created) const {
     const uint32_t* mc = R.mcoord + start;
     const double* mv = R.mcoef + start;
-    if (k <= 5) return tile_survivors<1>(G, sl, mc, mv, cnt, eps_a, trunc, wok, thr, created, part);
+    if (k <= 5) return tile_survivors<1>(G, sl, mc, mv, cnt, eps_a, trunc, wok, thr, created);
     switch (k) {
-      case 6: return tile_survivors<2>(G, sl, mc, mv, cnt, eps_a, trunc, wok, thr, created, part);
-      case 7: return tile_survivors<4>(G, sl, mc, mv, cnt, eps_a, trunc, wok, thr, created, part);
-      case 8: return tile_survivors<8>(G, sl, mc, mv, cnt, eps_a, trunc, wok, thr, created, part);
-      case 9: return tile_survivors<16>(G, sl, mc, mv, cnt, eps_a, trunc, wok, thr, created, part);
-      default: return tile_survivors<32>(G, sl, mc, mv, cnt, eps_a, trunc, wok, thr, created, part);
+      case 6: return tile_survivors<2>(G, sl, mc, mv, cnt, eps_a, trunc, wok, thr, created);
+      case 7: return tile_survivors<4>(G, sl, mc, mv, cnt, eps_a, trunc, wok, thr, created);
+      case 8: return tile_survivors<8>(G, sl, mc, mv, cnt, eps_a, trunc, wok, thr, created);
+      case 9: return tile_survivors<16>(G, sl, mc, mv, cnt, eps_a, trunc, wok, thr, created);
+      default: return tile_survivors<32>(G, sl, mc, mv, cnt, eps_a, trunc, wok, thr, created);
     }
   }
 
   // Writes the survivors to O from index `out` on, in coordinate order: from sl where tile_survivors
-  // left them, or (again) after running the group once more through sl; 1024 slots always so.
+  // left them, or (again) after running the group once more through sl.
   __device__ __forceinline__ void emit(const Planes& O, unsigned long long out, uint32_t cls, TileGates& G,
                                        unsigned long long* sl, bool again, const RunDesc* rd, const uint16_t* s_gidx,
                                        const RunScratch& R, unsigned start, unsigned cnt, double eps_a, bool trunc,
@@ -634,7 +629,7 @@ struct WarpGroup {
     const unsigned lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
     if (again) {
       gates(G, rd, s_gidx);
-      if (k <= 9) survivors(G, sl, R, start, cnt, eps_a, trunc, thr, nullptr, -1);
+      survivors(G, sl, R, start, cnt, eps_a, trunc, thr, nullptr);
     }
     uint64_t fl[W];  // f with this lane's low coordinate bits; a chunk of 32 slots adds its high ones
 #pragma unroll
@@ -646,31 +641,28 @@ struct WarpGroup {
         if (t < k && (int)(qt >> 6) == w && ((lane >> t) & 1u)) fl[w] |= 1ull << (qt & 63);
       }
     }
-    const unsigned nparts = k > 9 ? 2u : 1u, nchunk = k > 9 ? 16u : k > 5 ? 1u << (k - 5) : 1u;
-    for (unsigned part = 0; part < nparts; ++part) {
-      if (nparts > 1) survivors(G, sl, R, start, cnt, eps_a, trunc, thr, nullptr, (int)part);  // half at a time
-      for (unsigned ch = 0; ch < nchunk; ++ch) {
-        const unsigned long long u = sl[32 * ch + lane];
-        const unsigned bal = __ballot_sync(kFull, u != kNoSlot);
-        uint64_t f[W];
+    const unsigned nchunk = k > 5 ? 1u << (k - 5) : 1u;
+    for (unsigned ch = 0; ch < nchunk; ++ch) {
+      const unsigned long long u = sl[32 * ch + lane];
+      const unsigned bal = __ballot_sync(kFull, u != kNoSlot);
+      uint64_t f[W];
 #pragma unroll
-        for (int w = 0; w < W; ++w) f[w] = fl[w];
-        for (unsigned hb = part * 16 + ch; hb; hb &= hb - 1) {
-          const unsigned qt = __shfl_sync(kFull, q, 4u + (unsigned)__ffs((int)hb));
+      for (int w = 0; w < W; ++w) f[w] = fl[w];
+      for (unsigned hb = ch; hb; hb &= hb - 1) {
+        const unsigned qt = __shfl_sync(kFull, q, 4u + (unsigned)__ffs((int)hb));
 #pragma unroll
-          for (int w = 0; w < W; ++w)
-            if ((int)(qt >> 6) == w) f[w] |= 1ull << (qt & 63);
-        }
-        const unsigned long long r = out + __popc(bal & lt);
-        if (u != kNoSlot && r < O.cap) {
-          if (cls == 0) store_key<W>(O, r, f, v);
-          else store_key<W>(O, r, v, f);
-          O.c[r] = __longlong_as_double((long long)u);
-        }
-        out += __popc(bal);
+        for (int w = 0; w < W; ++w)
+          if ((int)(qt >> 6) == w) f[w] |= 1ull << (qt & 63);
       }
-      __syncwarp();
+      const unsigned long long r = out + __popc(bal & lt);
+      if (u != kNoSlot && r < O.cap) {
+        if (cls == 0) store_key<W>(O, r, f, v);
+        else store_key<W>(O, r, v, f);
+        O.c[r] = __longlong_as_double((long long)u);
+      }
+      out += __popc(bal);
     }
+    __syncwarp();
   }
 };
 
@@ -847,24 +839,33 @@ __device__ __forceinline__ void lane_write(const LaneGroup<W>& G, Planes D, unsi
 //   531 / 339 (40 qubits), all of K = 5 602 / 813; side by side, the worst: 0.2 % of K = 10 2365 / 2385;
 //   40,000 groups, scattered: 5 % of K = 4 94 / 44, 20 % of K = 7 139 / 181; side by side: 5 % of K = 4
 //   92 / 187, of K = 8 149 / 646.
-// So lanes are taken when no group is large; from kRunLaneMany groups on, where tiles leave their order to
-// k_run_place, up to one in 16 may be (at one in 6 a kicked-Ising layer of 4M terms takes 12.6 ms in tiles
-// and 14.8 in lanes); and in runs of mostly single members (Clifford+T: 26 layers 3.35 ms, 6.0 in
-// tiles).
+// So lanes are taken when no group is large; in runs of mostly single members up to one in 8 may be (all
+// large: 1.3M groups of 90 slots 23.7 ms, 12.4 in tiles); from kRunLaneMany groups on, where tiles leave their
+// order to k_run_place, one in 16 whatever the members (at one in 6 a kicked-Ising layer of 4M terms takes 12.6
+// ms in tiles and 14.8 in lanes).
 constexpr unsigned long long kRunLaneMany = 1ull << 18;
 struct RunCounts {
-  unsigned long long groups, members, large, untouched;
+  unsigned long long groups, members, large, slots, untouched;
 };
 __device__ __forceinline__ RunCounts run_counts(const Ctrl* ctrl, unsigned turn) {
   return {ld_volatile(&ctrl->n_pairs), ld_volatile(&ctrl->n_side), ld_volatile(&ctrl->run_large[turn]),
-          ld_volatile(&ctrl->n_s)};
+          ld_volatile(&ctrl->run_slots[turn]), ld_volatile(&ctrl->n_s)};
 }
 // The group kernels and k_run_place read the same counts and decide alike; those not needed return.
 __device__ __forceinline__ bool run_lanes(const RunCounts& c, unsigned mode) {
   if (mode != 0) return mode == 3;
   if (c.groups < kRunTileMinGroups) return false;
-  return c.large == 0 || 2 * c.members < 3 * c.groups ||
+  return c.large == 0 || (2 * c.members < 3 * c.groups && 8 * c.large <= c.groups) ||
          (c.groups >= kRunLaneMany && 16 * c.large <= c.groups);
+}
+
+// Whether tiles leave their order to k_run_place (scratch mode): from scratch_min groups on, unless the
+// groups are large.  Placing moves every term once more: 1.3M groups of 90 slots (1.1e8 terms) 13.1 + 5.9 ms,
+// 12.4 in order; 2.6M groups of a kicked-Ising layer 4.3 + 1.6, 6.9 in order.  A threshold set below the
+// default asks for scratch mode whatever the groups.
+constexpr unsigned long long kScratchSlots = 32;
+__device__ __forceinline__ bool run_scratch(const RunCounts& c, unsigned long long scratch_min) {
+  return c.groups >= scratch_min && (scratch_min < kRunLaneMany || c.slots <= kScratchSlots * c.groups);
 }
 
 // One group per lane, for runs of many small groups (run_lanes).  A warp takes 32 consecutive groups
@@ -942,14 +943,14 @@ k_run_lanes(Planes O, Ctrl* ctrl, const RunDesc* rd, RunScratch R, int trunc, do
       large(B, l);
       B.gates(G, rd, s_gidx);
       const unsigned size = B.slots();
-      const bool fits = B.k <= 9 && used + size <= (unsigned)kTileSlots;
+      const bool fits = used + size <= (unsigned)kTileSlots;
       if (!fits) {  // it goes through the slots from the first on: what was kept there is run again too
         off = kTileSlots;
         used = kTileSlots;
       }
       const unsigned at = fits ? used : 0u;
       const unsigned n = B.survivors(G, slots + at, R, __shfl_sync(kFull, gs, l), __shfl_sync(kFull, gc, l), eps_a,
-                                     trunc, thr, s_created, -1);
+                                     trunc, thr, s_created);
       if (fits) used += size;
       if (lane == l) {
         mine = n;
@@ -994,24 +995,25 @@ constexpr unsigned long long kTileManyGroups = 1ull << 15;  // from here on a wa
 // keys and coordinates, the butterflies in registers (tile_survivors), one look-back per tile for
 // the output offset, and the survivors written chunk by chunk of 32 slots, in coordinate order.
 // PER is 1 below kTileManyGroups groups, where a tile's latency is what counts (ticket, dependent
-// loads, look-back, about a microsecond each), and 4 (2 above 256 qubits) from there on, where the
-// look-backs and barriers per group do: the warp's keys, starts and members then come in one load
-// each.  A warp whose groups do not fit its slots together runs those that are left out again to
-// write them.  On the 12 x 12 headline (5,400 groups of 120 slots, 640,000 terms out) a run takes 54 us;
+// loads, look-back, about a microsecond each), and up to 4 (2 above 256 qubits) from there on, where the
+// look-backs and barriers per group do, as far as the groups fit a warp's slots on average (60,000
+// groups of 256 slots: 325 us with 4, 416 with 1): the warp's keys, starts and members then come in one
+// load each.  A warp whose groups do not fit its slots together runs those that are left out again to
+// write them.  On the 12 x 12 headline (5,400 groups of 120 slots, 640,000 terms out) a run takes 50 us;
 // one warp per group in shared memory, placed group by group, took 72.
-// From scratch_min groups on the tiles' order is left to k_run_place (scratch mode): waiting for
-// its place, every tile in flight waits for the slowest before it (RX run of 2.6M groups, 1 in
-// 500 of 8 to 10 coordinates: 6.9 ms in order, 4.3 + 1.6 ms placed; 4.4 + 1.5 with a warp per group
-// and two atomics each).
+// 1024 slots a warp and two blocks an SM: with 512 slots a group of 10 coordinates went through them
+// twice and was run three times (5,400 of them 357 us instead of 121; 1.1e8 terms of an unbudgeted 10 x 10
+// circuit 28.9 ms instead of 12.4); three blocks leave 80 registers, whose spills and less L1 make the
+// headline 2.75 ms instead of 2.68 and a kicked-Ising layer of 4M terms 12.9 instead of 12.0.
 template <int W>
-__global__ void __launch_bounds__(kTileWarps * 32, 3)
+__global__ void __launch_bounds__(kTileWarps * 32, 2)
 k_run_tiles(Planes O, Planes S, Ctrl* ctrl, const RunDesc* rd, RunScratch R, int trunc, double thr,
             unsigned long long maxw, unsigned long long* ts, unsigned epoch, int op, int trunc_op, OpLog* log,
             unsigned long long scratch_min, unsigned mode, unsigned turn) {
   pdl_wait();
   constexpr int BLOCK = kTileWarps * 32;
   constexpr unsigned MANY = W <= 4 ? 4 : 2;  // a warp's keys: MANY * 2W <= 32 words, one per lane
-  __shared__ unsigned long long s_slot[kTileWarps][kTileSlots];
+  extern __shared__ unsigned long long s_tiles[];  // kTileWarps * kTileSlots
   __shared__ TileGates s_g[kTileWarps];
   __shared__ unsigned s_created[kRunMaxGates];
   __shared__ uint16_t s_gidx[64 * W];  // qubit -> its gate's index in the run
@@ -1020,8 +1022,9 @@ k_run_tiles(Planes O, Planes S, Ctrl* ctrl, const RunDesc* rd, RunScratch R, int
   const RunCounts rc = run_counts(ctrl, turn);
   if (ld_volatile_int(&ctrl->err) || run_lanes(rc, mode)) return;
   const unsigned long long ngroups = rc.groups, ubase = rc.untouched;  // untouched survivors go first
-  const bool scratch = ngroups >= scratch_min;  // the same in every block
-  const unsigned per = scratch || ngroups >= kTileManyGroups ? MANY : 1u;
+  const bool scratch = run_scratch(rc, scratch_min);  // the same in every block
+  unsigned per = scratch || ngroups >= kTileManyGroups ? MANY : 1u;
+  while (per > 1 && per * rc.slots > (unsigned long long)kTileSlots * ngroups) per >>= 1;  // so many fit on average
   const unsigned long long ntiles = (ngroups + kTileWarps * per - 1) / (kTileWarps * per);
   const unsigned blocks = (unsigned)(ntiles < 1 ? 1 : ntiles < gridDim.x ? ntiles : gridDim.x);
   if (blockIdx.x >= blocks) return;
@@ -1036,7 +1039,7 @@ k_run_tiles(Planes O, Planes S, Ctrl* ctrl, const RunDesc* rd, RunScratch R, int
   const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const double eps_a = cls == 0 ? 1.0 : -1.0;
   TileGates& G = s_g[warp];
-  unsigned long long* slots = s_slot[warp];
+  unsigned long long* slots = s_tiles + warp * kTileSlots;
   // The warp's groups of a tile; per lane b: group b's start, members, survivors and slots (kTileSlots:
   // none kept), beside one word of the warp's keys.
   struct Held {
@@ -1073,14 +1076,14 @@ k_run_tiles(Planes O, Planes S, Ctrl* ctrl, const RunDesc* rd, RunScratch R, int
       load(B, b);
       B.gates(G, rd, s_gidx);
       const unsigned size = B.slots();
-      const bool fits = B.k <= 9 && used + size <= (unsigned)kTileSlots;
+      const bool fits = used + size <= (unsigned)kTileSlots;
       if (!fits) {  // it goes through the slots from the first on: what was kept there is run again too
         if (lane < b) H.off = kTileSlots;
         used = kTileSlots;
       }
       const unsigned off = fits ? used : 0u;
       const unsigned n = B.survivors(G, slots + off, R, __shfl_sync(kFull, H.gs, b), __shfl_sync(kFull, H.gc, b), eps_a,
-                                     trunc, thr, s_created, -1);
+                                     trunc, thr, s_created);
       if (fits) used += size;
       if (lane == b) {
         H.n = n;
@@ -1181,7 +1184,7 @@ k_run_place(Planes S, Planes O, Ctrl* ctrl, RunScratch R, unsigned long long scr
   __shared__ int s_skip;
   if (threadIdx.x == 0) {
     const RunCounts rc = run_counts(ctrl, turn);
-    s_skip = ld_volatile_int(&ctrl->err) || rc.groups == 0 || rc.groups < scratch_min || run_lanes(rc, mode);
+    s_skip = ld_volatile_int(&ctrl->err) || rc.groups == 0 || !run_scratch(rc, scratch_min) || run_lanes(rc, mode);
   }
   __syncthreads();
   if (s_skip) return;  // the same in every block (look-back mode, or an earlier error)
